@@ -1,0 +1,61 @@
+"""Digit products on the tensor cores (hsr_digits.cuh) where they can go wrong:
+sizes at the edges of their tiles (128 rows, 64 columns, 16 and 192 inner),
+graded and non-finite inputs.  Each is compared with the same formula in
+extended precision; tolerances follow from the FP64 operations that remain
+around the exact digit sums."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+EPS = np.finfo(np.float64).eps
+
+
+def _cols(torch, A, pad):
+    """Columns of A as rows of a device tensor with a padded leading dimension."""
+    out = torch.full((A.shape[1], A.shape[0] + pad), 5.0, dtype=torch.float64, device="cuda")
+    out[:, :A.shape[0]] = torch.from_numpy(np.ascontiguousarray(A.T))
+    return out
+
+
+@pytest.mark.parametrize("n,ncols,pad,graded", [
+    (127, 3, 0, False), (128, 64, 1, False), (129, 65, 0, False), (191, 1, 3, False), (193, 63, 0, False),
+    (255, 130, 1, False), (385, 70, 0, True), (640, 33, 2, True)])
+def test_residuals_against_extended(gpu_lib, n, ncols, pad, graded):
+    """Every operation after the exact products rounds once in FP64: the sum
+    of n squares and the two norms, at most n eps / 2 each, and a few more."""
+    import torch
+    import hsrq3in_gb300 as hsr
+    rng = np.random.default_rng(n)
+    H = rng.standard_normal((n, n))
+    X = rng.standard_normal((n, ncols))
+    if graded:                                   # columns of H over 60 decades, x the other way
+        d = 10.0 ** rng.uniform(-30, 30, n)
+        H, X = H * d, X / d[:, None]
+    wr = rng.uniform(-2, 2, ncols)
+    got = hsr.residuals_device(_cols(torch, H, pad), torch.from_numpy(wr).cuda(), _cols(torch, X, pad)).cpu().numpy()
+    L = np.longdouble
+    Hh, Xl = np.triu(H, -1).astype(L), X.astype(L)
+    R = np.array([(Hh * Xl[:, c]).sum(1) for c in range(ncols)]).T - Xl * wr.astype(L)
+    ref = np.sqrt((R * R).sum(0)) / (np.sqrt((Hh * Hh).sum()) * np.sqrt((Xl * Xl).sum(0)))
+    np.testing.assert_allclose(got, ref.astype(np.float64), rtol=(2 * n + 32) * EPS)
+
+
+def test_residuals_non_finite(gpu_lib):
+    """A column of x with an Inf or a NaN gives NaN, a zero one Inf, the others
+    their value; garbage below the subdiagonal of H does not enter."""
+    import torch
+    import hsrq3in_gb300 as hsr
+    n = 300
+    rng = np.random.default_rng(1)
+    H, X, wr = rng.standard_normal((n, n)), rng.standard_normal((n, 5)), rng.uniform(-1, 1, 5)
+    X[7, 1], X[299, 2], X[:, 3] = np.inf, np.nan, 0.0
+    H[np.tril_indices(n, -2)] = np.nan
+    got = hsr.residuals_device(_cols(torch, H, 0), torch.from_numpy(wr).cuda(), _cols(torch, X, 1)).cpu().numpy()
+    Hh = np.triu(H, -1)
+    for c in (0, 4):
+        ref = np.linalg.norm(Hh @ X[:, c] - wr[c] * X[:, c]) / (np.linalg.norm(Hh) * np.linalg.norm(X[:, c]))
+        np.testing.assert_allclose(got[c], ref, rtol=1e-12)
+    assert np.isnan(got[1]) and np.isnan(got[2]) and np.isposinf(got[3])
+    H[5, 200] = np.inf
+    assert np.isnan(hsr.residuals_device(_cols(torch, H, 0), torch.from_numpy(wr).cuda(),
+                                         _cols(torch, X, 0)).cpu().numpy()[[0, 1, 2, 4]]).all()
