@@ -21,7 +21,9 @@
 //     the same truncations came to 2^-51 a chunk, more than an FP64 chain's;
 //   * every 192 columns the accumulators are added to two 64-bit integers per
 //     entry, exactly, so the order of the columns does not matter and results
-//     are the same for every tiling.
+//     are the same for every tiling.  A sum over at most 128 columns goes into
+//     one integer in units of 2^-55 (DgOne), half an ulp of an entry of size
+//     1/4 where every product's bound is 1.
 //
 // What is lost is the rounding of t (2^-63 of the row's largest entry) and
 // the products with p + q >= 8 (2^-60 of the largest product), below the
@@ -56,7 +58,6 @@ constexpr int kDgGroups = 7;                       // accumulators: d = 0 .. 5 a
 constexpr int kDgChunk = 12;                       // stages (of 16 columns) between drains
 constexpr int kDgStages = 4;
 constexpr int kDgABytes = kDgBM * kDgBK * kDgDigits * 2, kDgBBytes = kDgBN * kDgBK * kDgDigits * 2;
-constexpr int kDgThreads = 320;                    // copy warp, MMA warp, eight drain warps
 constexpr int kDgSmem = kDgStages * (kDgABytes + kDgBBytes) + 1024;
 constexpr int kDgZero = -(1 << 20);                // exponent of an all-zero row
 constexpr int kDgBad = 1 << 20;                    // exponent field of a row with an Inf or NaN
@@ -194,6 +195,42 @@ __global__ void __launch_bounds__(256) k_dg_split(Ld ld, int RB, int Rpad, long 
     dg_store8(u, out + dg_place(r, c8, RB, steps), RB * kDgBK * 2);
 }
 
+// Exponents and digits in one pass for K <= 128: a thread keeps its eight
+// entries between the two.  RC: a CTA takes 32 rows, else 8; its 16 thread
+// groups one group of eight columns each.
+template <class Ld, bool RC>
+__global__ void __launch_bounds__(RC ? 512 : 128) k_dg_small(Ld ld, int RB, int R, int Rpad, int K, const int *dk,
+                                                             int sign, int *ex, unsigned char *out) {
+    constexpr int ROWS = RC ? 32 : 8;
+    __shared__ int red[ROWS][17];
+    const int t = threadIdx.x, rr = RC ? t & 31 : t & 7, c8 = RC ? t >> 5 : t >> 3;
+    const int r = blockIdx.x * ROWS + rr;
+    const int steps = (K + kDgBK - 1) / kDgBK;
+    double x[8];
+    int m = kDgZero;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const int k = c8 * 8 + e;
+        x[e] = r < R && k < K ? ld(r, k) : 0.0;
+        const int ee = dg_exp(x[e]);
+        m = max(m, dk && ee != kDgZero ? ee + sign * dk[k] : ee);
+    }
+    red[rr][c8] = m;
+    __syncthreads();
+    m = kDgZero;
+#pragma unroll
+    for (int q = 0; q < 16; ++q) m = max(m, red[rr][q]);
+    if (c8 == 0 && r < R) ex[r] = m;
+    if (c8 >= 2 * steps || r >= Rpad) return;
+    unsigned long long u[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const int k = c8 * 8 + e;
+        u[e] = dg_digits(x[e], dk && k < K ? m - 9 - sign * dk[k] : m - 9);
+    }
+    dg_store8(u, out + dg_place(r, c8, RB, steps), RB * kDgBK * 2);
+}
+
 // ------------------------------------------------------- tcgen05 wrappers
 __device__ __forceinline__ uint64_t dg_desc(uint32_t addr) {
     // K-major, no swizzle: core matrices 128 B apart along K (leading offset),
@@ -214,13 +251,21 @@ __device__ __forceinline__ void dg_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
 }
-__device__ __forceinline__ void dg_ld32(uint32_t addr, float (&v)[32]) {
+__device__ __forceinline__ void dg_ld(uint32_t addr, float (&v)[32]) {
     uint32_t r[32];
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
                  : "r"(addr));
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void dg_ld(uint32_t addr, float (&v)[16]) {
+    uint32_t r[16];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(addr));
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 __device__ __forceinline__ void dg_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void dg_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -234,9 +279,12 @@ __device__ __forceinline__ void dg_bulk(void *dst, const void *src, uint32_t byt
         ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
         : "memory");
 }
-// One tile: its row and column block, a split index and its stages [s0, s1).
+// One tile: its row and column block, a part index, the places of its first
+// stage in A and B (counted in stages) and the number of stages.
 struct DgTile {
-    int bx, by, bz, s0, s1;
+    int bx, by, bz;
+    long long a, b;
+    int stages;
 };
 // Bounded wait without a device error word: false after the poll limit.
 __device__ __forceinline__ bool dg_wait(uint64_t *bar, uint32_t parity) {
@@ -280,6 +328,55 @@ __device__ __forceinline__ double dg_value(long long hi, long long lo, int e) {
     return from_bits(sign | (((unsigned long long)(f - 1) << 52) + m));
 }
 
+// The same for one word, T 2^(e - 55), |T| <= 2^62.
+__device__ __forceinline__ double dg_value(long long T, int e) {
+    if (T == 0) return 0.0;
+    const unsigned long long sign = (unsigned long long)T & 0x8000000000000000ULL;
+    const unsigned long long a = (unsigned long long)(T < 0 ? -T : T);
+    const int z = __clzll((long long)a);
+    const unsigned long long m = ((a << z) + (1ULL << 10)) >> 11;    // a <= 2^62: no carry out of 64 bits
+    const int f = 1023 + 63 - z - 55 + e;
+    if (f <= 0 || f >= 0x7fe) return dg_ldexp_rare(from_bits(sign | (0x3ffULL << 52)) * (double)m, f - 1075);
+    return from_bits(sign | (((unsigned long long)(f - 1) << 52) + m));
+}
+
+// A thread's sums: kCols columns of one row, as hi 2^-28 + lo 2^-64 ...
+template <int N>
+struct DgTwo {
+    static constexpr int kCols = N;
+    long long hi[N], lo[N];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int c = 0; c < N; ++c) hi[c] = lo[c] = 0;
+    }
+    __device__ __forceinline__ void add(int g, int c, float v) {  // one wide multiply-add each
+        const float unit = g == 0 ? 0x1p12f : g == 1 ? 0x1p20f : g == 2 ? 0x1p28f : g == 3 ? 0x1p36f
+                         : g == 4 ? 0x1p44f : g == 5 ? 0x1p52f : 0x1p64f;
+        const int i = __float2int_rn(v * unit);
+        if (g < 3) hi[c] += (long long)i * (1 << (16 - 8 * g));
+        else lo[c] += (long long)i * (1 << (g == 6 ? 0 : 28 - 8 * (g - 3)));
+    }
+    __device__ __forceinline__ double value(int c, int e) const { return dg_value(hi[c], lo[c], e - 64); }
+};
+// ... or, for at most 128 columns, as T 2^-55.
+template <int N>
+struct DgOne {
+    static constexpr int kCols = N;
+    long long T[N];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int c = 0; c < N; ++c) T[c] = 0;
+    }
+    __device__ __forceinline__ void add(int g, int c, float v) {
+        const float unit = g == 0 ? 0x1p12f : g == 1 ? 0x1p20f : g == 2 ? 0x1p28f : g == 3 ? 0x1p36f
+                         : g == 4 ? 0x1p44f : g == 5 ? 0x1p52f : 0x1p55f;
+        const int i = __float2int_rn(v * unit);
+        if (g < 2) T[c] += (long long)((unsigned long long)(unsigned)(i << (11 - 8 * g)) << 32);   // the high word only
+        else T[c] += (long long)i * (1 << (g == 6 ? 0 : 27 - 8 * (g - 2)));
+    }
+    __device__ __forceinline__ double value(int c, int e) const { return dg_value(T[c], e); }
+};
+
 // One elected lane of a converged warp.
 __device__ __forceinline__ bool dg_elect() {
     uint32_t p;
@@ -317,9 +414,9 @@ __device__ __forceinline__ bool dg_group(uint32_t tmem, uint64_t da, uint64_t db
     return ok;
 }
 
-// Tiles of 128 x 64 of A B.  A: digits of row blocks of 128, B: of 64,
-// `steps` stages each.  epi.tile(t, ...) gives tile t's blocks and stages;
-// epi.finish takes a thread's row and 32 columns of it in 64-bit integers.
+// Tiles of 128 x 64 of A B.  A: digits of row blocks of 128, B: of 64.
+// epi.tile(t) gives tile t's blocks and stages; epi.finish takes a thread's
+// row and Epi::Sum::kCols columns of it as integers.
 //
 // Persistent: CTA c works through tiles c, c + gridDim.x, ...; the copy and
 // MMA warps run on into the next tile while the drain warps finish the last
@@ -331,11 +428,10 @@ __device__ __forceinline__ bool dg_group(uint32_t tmem, uint64_t da, uint64_t db
 // per product measured, 48 by its bytes.  A wait that runs out (a copy that
 // never lands) ends the CTA's work, and epi.poison marks the results.  H x at
 // n = 5000 with 5000 columns: one tile per CTA with one drain barrier 5.3 ms,
-// this form 3.8 ms; the fma chain on the FP64 pipe 114 ms.
+// this form 3.7 ms; the fma chain on the FP64 pipe 114 ms.
 template <class Epi>
-__global__ void __launch_bounds__(kDgThreads, 1)
-k_dg_gemm(const unsigned char *__restrict__ A, const unsigned char *__restrict__ B, long long steps, int tiles,
-          Epi epi) {
+__global__ void __launch_bounds__(64 + 32 * Epi::kWarps, 1)
+k_dg_gemm(const unsigned char *__restrict__ A, const unsigned char *__restrict__ B, int tiles, Epi epi) {
     extern __shared__ __align__(1024) unsigned char dg_sm[];
     __shared__ __align__(8) uint64_t full[kDgStages], empty[kDgStages], acc_full[kDgGroups], acc_empty[kDgGroups];
     __shared__ uint32_t tmem_base;
@@ -348,7 +444,7 @@ k_dg_gemm(const unsigned char *__restrict__ A, const unsigned char *__restrict__
         }
         for (int g = 0; g < kDgGroups; ++g) {
             mbar_init(&acc_full[g], 1);
-            mbar_init(&acc_empty[g], 8);
+            mbar_init(&acc_empty[g], Epi::kWarps);
         }
         mbar_fence_init();
         failed = 0;
@@ -372,9 +468,8 @@ k_dg_gemm(const unsigned char *__restrict__ A, const unsigned char *__restrict__
             bool ok = true;
             for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
                 const DgTile q = epi.tile(tile);
-                const unsigned char *ga = A + ((size_t)q.bx * (size_t)steps + (size_t)q.s0) * kDgABytes;
-                const unsigned char *gb = B + ((size_t)q.by * (size_t)steps + (size_t)q.s0) * kDgBBytes;
-                for (int t = 0; t < q.s1 - q.s0; ++t, ++it) {
+                const unsigned char *ga = A + (size_t)q.a * kDgABytes, *gb = B + (size_t)q.b * kDgBBytes;
+                for (int t = 0; t < q.stages; ++t, ++it) {
                     const unsigned st = it % kDgStages;
                     if (it >= kDgStages && !dg_wait(&empty[st], (it / kDgStages - 1) & 1)) {
                         ok = false;
@@ -396,7 +491,7 @@ k_dg_gemm(const unsigned char *__restrict__ A, const unsigned char *__restrict__
         bool ok = true;
         for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
             const DgTile q = epi.tile(tile);
-            const int nst = q.s1 - q.s0;
+            const int nst = q.stages;
             for (int t = 0; t < nst && ok; ++t, ++it) {
                 const int in_chunk = t % kDgChunk;
                 const unsigned st = it % kDgStages;
@@ -436,44 +531,36 @@ k_dg_gemm(const unsigned char *__restrict__ A, const unsigned char *__restrict__
         if (it > 0) ok = ok && dg_wait(&empty[(it - 1) % kDgStages], ((it - 1) / kDgStages) & 1);
         if (!ok) failed = 1;
     } else {
-        // Warp w reads TMEM lanes 32 (w mod 4) ..; the warps of a pair take 32
-        // columns each.
-        const int quad = wid & 3, half = (wid - 2) >> 2;
+        // Warp w reads TMEM lanes 32 (w mod 4) .. and kCols of the 64 columns.
+        constexpr int kCols = kDgBN * 4 / Epi::kWarps;
+        const int quad = wid & 3, part = (wid - 2) >> 2;
         const int row = quad * 32 + lane;
-        const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * 32);
+        const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(part * kCols);
         unsigned chunk = 0;
         bool ok = true;
         for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
             const DgTile q = epi.tile(tile);
-            long long hi[32], lo[32];
-#pragma unroll
-            for (int c = 0; c < 32; ++c) hi[c] = lo[c] = 0;
-            const int nchunk = (q.s1 - q.s0 + kDgChunk - 1) / kDgChunk;
+            typename Epi::Sum sum;
+            sum.zero();
+            const int nchunk = (q.stages + kDgChunk - 1) / kDgChunk;
             for (int ch = 0; ch < nchunk && ok; ++ch, ++chunk) {
 #pragma unroll
                 for (int g = 0; g < kDgGroups; ++g) {
                     ok = __all_sync(0xffffffffu, dg_wait(&acc_full[g], chunk & 1));
                     if (!ok) break;
                     dg_fence_after();
-                    float v[32];
-                    dg_ld32(base + (uint32_t)(g * kDgBN), v);
+                    float v[kCols];
+                    dg_ld(base + (uint32_t)(g * kDgBN), v);
                     dg_wait_ld();
                     dg_fence_before();
                     __syncwarp();
                     if (lane == 0) dg_arrive(&acc_empty[g]);
+                    // Groups 0 .. 5 are exact integers in units of 2^(-12 - 8 g).
 #pragma unroll
-                    for (int c = 0; c < 32; ++c) {
-                        // hi 2^-28 + lo 2^-64 of the entry: groups 0 .. 5 are
-                        // exact integers in units of 2^(-12 - 8 g).
-                        const float unit = g == 0 ? 0x1p12f : g == 1 ? 0x1p20f : g == 2 ? 0x1p28f : g == 3 ? 0x1p36f
-                                         : g == 4 ? 0x1p44f : g == 5 ? 0x1p52f : 0x1p64f;
-                        const long long i = (long long)__float2int_rn(v[c] * unit);
-                        if (g < 3) hi[c] += i << (16 - 8 * g);
-                        else lo[c] += i << (g == 6 ? 0 : 28 - 8 * (g - 3));
-                    }
+                    for (int c = 0; c < kCols; ++c) sum.add(g, c, v[c]);
                 }
             }
-            if (ok) epi.finish(q, q.bx * kDgBM + row, q.by * kDgBN + half * 32, hi, lo);
+            if (ok) epi.finish(q, q.bx * kDgBM + row, q.by * kDgBN + part * kCols, sum);
         }
         if (!ok) failed = 1;
     }
@@ -484,6 +571,97 @@ k_dg_gemm(const unsigned char *__restrict__ A, const unsigned char *__restrict__
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
     if (failed) epi.poison();
 }
+
+// ------------------------------------------------------------- epilogues
+__device__ __forceinline__ bool dg_bad(int ex) { return ex >= kDgBad / 2; }
+__device__ __forceinline__ double dg_nan() { return __longlong_as_double(0x7ff8000000000000LL); }
+
+// Stages [0, steps) of every tile cut into nz parts of `per` stages; part z
+// of C(i, j) goes to out[z * cz + i * si + j * sj].
+template <class S, int W>
+struct DgStore {
+    using Sum = S;
+    static constexpr int kWarps = W;
+    int mblocks, nblocks, steps, per, M, N;
+    const int *ea, *eb;
+    double *out;
+    long long si, sj, cz;
+    __device__ __forceinline__ DgTile tile(int t) const {
+        const int mn = mblocks * nblocks, bz = t / mn, r = t - bz * mn, by = r / mblocks;
+        const int bx = r - by * mblocks, s0 = bz * per;
+        return DgTile{bx, by, bz, (long long)bx * steps + s0, (long long)by * steps + s0, min(steps - s0, per)};
+    }
+    __device__ __forceinline__ void finish(const DgTile &q, int i, int j0, const Sum &sum) const {
+        const int lane = threadIdx.x & 31;
+        const int ecl = max(eb[min(j0 + lane, N - 1)], kDgZero), er = max(ea[min(i, M - 1)], kDgZero);
+        double *o = out + (size_t)q.bz * cz + (size_t)i * si + (size_t)j0 * sj;
+#pragma unroll
+        for (int c = 0; c < S::kCols; ++c) {
+            const int ec = __shfl_sync(0xffffffffu, ecl, c);
+            const double v = sum.value(c, er + ec - 2044);
+            if (i < M && j0 + c < N) o[(size_t)c * sj] = dg_bad(er) || dg_bad(ec) ? dg_nan() : v;
+        }
+    }
+    __device__ void poison() const {
+        for (long long e = threadIdx.x; e < (long long)M * N; e += blockDim.x)
+            out[(e % M) * si + (e / M) * sj] = dg_nan();
+    }
+};
+using DgStoreLong = DgStore<DgTwo<16>, 16>;
+using DgStoreShort = DgStore<DgOne<16>, 16>;
+// C(i, j) -= sum over at most 128 columns; cex (optional): the columns'
+// exponents are raised to the new entries'.  One FP64 instruction per entry (a
+// warp's takes 64 clocks), the rest on the integer pipe.  Sixteen drain warps
+// with one word per sum: with eight and two words (168 registers, two warps
+// per scheduler) this end took 13,000 clocks of a tile whose products take
+// 14,000, and the two did not overlap.
+struct DgUpdate {
+    using Sum = DgOne<16>;
+    static constexpr int kWarps = 16;
+    int mblocks, steps, M, N;
+    const int *ea, *eb;
+    double *C;
+    long long ldc;
+    int *cex;
+    __device__ __forceinline__ DgTile tile(int t) const {
+        const int by = t / mblocks;
+        const int bx = t - by * mblocks;
+        return DgTile{bx, by, 0, (long long)bx * steps, (long long)by * steps, steps};
+    }
+    __device__ __forceinline__ void finish(const DgTile &, int i, int j0, const Sum &sum) const {
+        // Lane c holds column j0 + c's exponents, loaded once.
+        const int lane = threadIdx.x & 31, jl = min(j0 + lane, N - 1);
+        const int ecl = max(eb[jl], kDgZero), er = max(ea[min(i, M - 1)], kDgZero);
+        const bool in = i < M, any_bad = __any_sync(0xffffffffu, dg_bad(er) || dg_bad(ecl));
+        const int cl = cex ? cex[jl] : 0;
+        unsigned big = 0;                                        // largest high word of the lane's column
+        double *Ci = C + min(i, M - 1) + (size_t)j0 * ldc;
+        const int cols = min(Sum::kCols, N - j0);
+        double x[Sum::kCols];
+#pragma unroll
+        for (int c = 0; c < Sum::kCols; ++c) x[c] = c < cols ? Ci[(size_t)c * ldc] : 0.0;
+#pragma unroll
+        for (int c = 0; c < Sum::kCols; ++c) {
+            const int ec = __shfl_sync(0xffffffffu, ecl, c);
+            x[c] = x[c] - sum.value(c, er + ec - 2044);
+            if (any_bad && (dg_bad(er) || dg_bad(ec))) x[c] = dg_nan();
+            if (in && c < cols) Ci[(size_t)c * ldc] = x[c];
+        }
+        if (!cex) return;
+#pragma unroll
+        for (int c = 0; c < Sum::kCols; ++c) {
+            const unsigned m = __reduce_max_sync(0xffffffffu, in ? (unsigned)(ubits(x[c]) >> 32) & 0x7fffffffu : 0u);
+            if (lane == c) big = m;
+        }
+        if (lane < cols) {
+            const int m = big >= 0x7ff00000u ? kDgBad : max((int)(big >> 20), 1);
+            if (m > cl) atomicMax(&cex[jl], m);
+        }
+    }
+    __device__ void poison() const {
+        for (long long e = threadIdx.x; e < (long long)M * N; e += blockDim.x) C[(e % M) + (e / M) * ldc] = dg_nan();
+    }
+};
 
 // Host side: one growing device buffer per thread.  A call on another stream
 // than the last one first waits for that one's work.
@@ -537,12 +715,12 @@ struct DgScratch {
     bool capturing = false;
 };
 template <class Epi>
-inline cudaError_t dg_gemm(int tiles, int sms, const unsigned char *A, const unsigned char *B, long long steps,
-                           const Epi &epi, cudaStream_t st) {
+inline cudaError_t dg_gemm(int tiles, int sms, const unsigned char *A, const unsigned char *B, const Epi &epi,
+                           cudaStream_t st) {
     const cudaError_t e =
         cudaFuncSetAttribute(k_dg_gemm<Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDgSmem);
     if (e != cudaSuccess) return e;
-    k_dg_gemm<Epi><<<std::min(tiles, sms), kDgThreads, kDgSmem, st>>>(A, B, steps, tiles, epi);
+    k_dg_gemm<Epi><<<std::min(tiles, sms), 64 + 32 * Epi::kWarps, kDgSmem, st>>>(A, B, tiles, epi);
     return cudaGetLastError();
 }
 

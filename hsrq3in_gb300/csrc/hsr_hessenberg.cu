@@ -32,6 +32,7 @@
 // order: no block waits for another, and results are reproducible run to run.
 #include "../../include/hsrq3in_gb300.h"
 #include "hsr_device.cuh"
+#include "hsr_digits.cuh"
 
 #include <algorithm>
 #include <cfloat>
@@ -442,6 +443,300 @@ __global__ void k_hq_tfactor(int ib, const double *tau, const double *G, double 
     }
 }
 
+// ------------------------------------------------ back-transform by digits
+// The same back-transform with the products on the bf16 tensor cores
+// (hsr_digits.cuh), in blocks of kHqNb = 128 reflectors, one row block of
+// digits.  Blocks are taken in groups whose digits of V fit kHqVBytes: for a
+// group, the digits, the Gram matrices V^T V and the factors T of all its
+// blocks at once (they do not depend on X), then per block W = V^T X, T W and
+// X -= V (T W).
+constexpr int kHqNb = 128;
+// Smallest order: a reflector of the DFMA form costs about 5.5 us (three thin
+// products and a serial factor per 64), this form 215 us and 0.5 us each
+// (n = 20: 155 us as DFMA; 64: 337 against 225; 300: 1,780 against 390;
+// 5000 with 2500 columns: 175.4 ms against 8.5).  The DFMA form also stays for
+// a scratch buffer that cannot be had.
+constexpr int kHqDigitsN = 40;
+// Most scratch for digits of X's columns and of V (three layouts) at a time.
+constexpr size_t kHqXBytes = (size_t)1 << 30, kHqVBytes = (size_t)4 << 30;
+constexpr int kHqMaxSplit = 16;
+
+// The blocks of a group, last first: block g of the group begins at reflector
+// k0(g) and has rows k0 + 1 .. n - 1.  Its row blocks of 128 count from the
+// bottom, so that block g has g more of them than block 0 and places are
+// sums: `rb0` row blocks in block 0.
+struct HqGroup {
+    const double *A;
+    long long lda;
+    int n, klast, rb0;                                           // klast: k0 of block 0
+    __host__ __device__ __forceinline__ int k0(int g) const { return klast - g * kHqNb; }
+    __host__ __device__ __forceinline__ int rblocks(int g) const { return rb0 + g; }
+    __host__ __device__ __forceinline__ long long before(int g) const {      // row blocks of blocks 0 .. g-1
+        return (long long)g * rb0 + (long long)g * (g - 1) / 2;
+    }
+    // V(i, q) of block g.
+    __device__ __forceinline__ double at(int g, int i, int q) const {
+        const int j = k0(g) + q;
+        if (j >= n - 2 || i >= n || i < j + 1) return 0.0;
+        return i == j + 1 ? 1.0 : A[i + (size_t)j * lda];
+    }
+};
+// Exponents of V's columns (row g * 128 + q: column q of block g).
+struct HqVCols {
+    HqGroup h;
+    __device__ __forceinline__ double operator()(int r, int k) const {
+        const int g = r / kHqNb;
+        return h.at(g, h.k0(g) + 1 + k, r % kHqNb);
+    }
+};
+// Digits of V's columns as row blocks of RB (128: the A side, 64: the B
+// side): block (x, y) = eight columns and 256 rows of block z of the group.
+template <int RB>
+__global__ void __launch_bounds__(256) k_hq_vcols(HqGroup h, const int *ex, unsigned char *out) {
+    const int t = threadIdx.x, g = blockIdx.z, r = blockIdx.x * 8 + (t & 7), c8 = blockIdx.y * 32 + (t >> 3);
+    const int steps = h.rblocks(g) * (kHqNb / kDgBK);
+    if (c8 >= 2 * steps) return;
+    const int base = max(ex[g * kHqNb + r], kDgZero) - 9, i0 = h.k0(g) + 1 + c8 * 8;
+    unsigned long long u[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) u[e] = dg_digits(h.at(g, i0 + e, r), base);
+    dg_store8(u, out + (size_t)h.before(g) * kHqNb * kHqNb * kDgDigits * 2 + dg_place(r, c8, RB, steps), RB * kDgBK * 2);
+}
+// Exponents and digits of V's rows: 32 rows of one block of the group.
+__global__ void __launch_bounds__(512) k_hq_vrows(HqGroup h, int *ex, unsigned char *out) {
+    __shared__ int red[32][17];
+    const int t = threadIdx.x, g = blockIdx.y, rr = t & 31, c8 = t >> 5, r = blockIdx.x * 32 + rr;
+    if (r - rr >= h.rblocks(g) * kHqNb) return;                  // uniform over the block
+    double x[8];
+    int m = kDgZero;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        x[e] = h.at(g, h.k0(g) + 1 + r, c8 * 8 + e);
+        m = max(m, dg_exp(x[e]));
+    }
+    red[rr][c8] = m;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 16; ++q) m = max(m, red[rr][q]);
+    const size_t row = (size_t)h.before(g) * kHqNb + r;
+    if (c8 == 0) ex[row] = m;
+    unsigned long long u[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) u[e] = dg_digits(x[e], m - 9);
+    dg_store8(u, out + (size_t)h.before(g) * kHqNb * kHqNb * kDgDigits * 2 + dg_place(r, c8, kDgBM, kHqNb / kDgBK),
+              kDgBM * kDgBK * 2);
+}
+// Gram matrices of a group: part z of block g to S[(g * nz + z)].
+struct HqGram {
+    using Sum = DgTwo<16>;
+    static constexpr int kWarps = 16;
+    HqGroup h;
+    int nz;
+    const int *ex;
+    double *S;
+    __device__ __forceinline__ DgTile tile(int t) const {
+        const int g = t / (2 * nz), r = t - g * 2 * nz, z = r >> 1, by = r & 1;
+        const int steps = h.rblocks(g) * (kHqNb / kDgBK), per = (steps + nz - 1) / nz, s0 = min(z * per, steps);
+        const long long at = h.before(g) * (kHqNb / kDgBK);
+        return DgTile{g, by, z, at + s0, 2 * at + (long long)by * steps + s0, min(steps - s0, per)};
+    }
+    __device__ __forceinline__ void finish(const DgTile &q, int i, int j0, const Sum &sum) const {
+        const int p = i - q.bx * kDgBM, lane = threadIdx.x & 31;
+        const int ecl = max(ex[q.bx * kHqNb + j0 + (lane & 15)], kDgZero), er = max(ex[q.bx * kHqNb + p], kDgZero);
+        double *o = S + ((size_t)q.bx * nz + q.bz) * kHqNb * kHqNb + p + (size_t)j0 * kHqNb;
+#pragma unroll
+        for (int c = 0; c < Sum::kCols; ++c) {
+            const int ec = __shfl_sync(0xffffffffu, ecl, c);
+            const double v = sum.value(c, er + ec - 2044);
+            o[(size_t)c * kHqNb] = dg_bad(er) || dg_bad(ec) ? dg_nan() : v;
+        }
+    }
+    __device__ void poison() const {
+        for (int e = threadIdx.x; e < nz * kHqNb * kHqNb; e += blockDim.x) S[e] = dg_nan();
+    }
+};
+// Rows of the operand are columns of a column-major matrix.
+struct HqCols {
+    const double *X;
+    long long ld;
+    int cols, rows;
+    __device__ __forceinline__ double operator()(int r, int k) const {
+        return r < cols && k < rows ? X[k + (size_t)r * ld] : 0.0;
+    }
+    __device__ __forceinline__ int first(int) const { return 0; }
+};
+// W(:, j) as the sum of nz partial products, in order.
+struct HqSum {
+    const double *Wp;
+    int nz;
+    long long cz;
+    __device__ __forceinline__ double operator()(int r, int k) const {
+        double s = 0.0;
+        for (int z = 0; z < nz; ++z) s += Wp[(size_t)z * cz + k + (size_t)r * kHqNb];
+        return s;
+    }
+};
+// Factors T of all blocks, stacked (row r of the operand: row r % 128 of block r / 128).
+struct HqT {
+    const double *T;
+    __device__ __forceinline__ double operator()(int r, int k) const {
+        return T[(size_t)(r / kHqNb) * kHqNb * kHqNb + (r % kHqNb) + (size_t)k * kHqNb];
+    }
+};
+
+// dlarft of a block of 128 in three parts, from S = V^T V (summed from its
+// partial products): the factors T11 and T22 of its halves, T(0:i, i) =
+// -tau_i T(0:i, 0:i) S(0:i, i), T(i, i) = tau_i, by one CTA each, four threads
+// per row; then T12 = -T11 S12 T22, eight columns per CTA.  Bound by the FP64
+// pipe of the SMs that take part (a warp's FMA 64 clocks): one CTA for the
+// whole block 254 us, this form 79 + 50 us, for any number of blocks.
+constexpr int kHqHalf = kHqNb / 2;
+__device__ __forceinline__ int hq_packed(int p, int i) { return p + i * (i + 1) / 2; }
+__device__ __forceinline__ double hq_gram(const double *S, int nz, int p, int i) {
+    double s = 0.0;
+#pragma unroll 4
+    for (int z = 0; z < nz; ++z) s += S[(size_t)z * kHqNb * kHqNb + p + (size_t)i * kHqNb];
+    return s;
+}
+__global__ void __launch_bounds__(4 * kHqHalf) k_hq_thalf(HqGroup h, const double *tau, const double *Sp, int nz, double *T) {
+    __shared__ double ts[kHqHalf * (kHqHalf + 1) / 2], ss[kHqHalf * (kHqHalf + 1) / 2], part[4][kHqHalf];
+    const int p = threadIdx.x % kHqHalf, w = threadIdx.x / kHqHalf, o = blockIdx.y * kHqHalf;
+    const int k0 = h.k0(blockIdx.x) + o, ib = max(0, min(kHqHalf, h.n - 2 - k0));
+    const double *S = Sp + (size_t)blockIdx.x * nz * kHqNb * kHqNb + o + (size_t)o * kHqNb;
+    double *To = T + (size_t)blockIdx.x * kHqNb * kHqNb + o + (size_t)o * kHqNb;
+    for (int i = w; i < kHqHalf; i += 4) {
+        if (p < i) ss[hq_packed(p, i)] = hq_gram(S, nz, p, i);
+        if (p > i || i >= ib) To[p + (size_t)i * kHqNb] = 0.0;
+    }
+    for (int i = 0; i < ib; ++i) {
+        __syncthreads();                                         // S, T(:, i - 1)
+        double a = 0.0;
+        for (int q = p + w; q < i; q += 4) a = fma(ts[hq_packed(p, q)], ss[hq_packed(q, i)], a);
+        part[w][p] = a;
+        __syncthreads();
+        if (w == 0 && p <= i) {
+            const double t = tau[k0 + i];
+            const double v = p < i ? -t * ((part[0][p] + part[1][p]) + (part[2][p] + part[3][p])) : t;
+            ts[hq_packed(p, i)] = v;
+            To[p + (size_t)i * kHqNb] = v;
+        }
+    }
+}
+__global__ void __launch_bounds__(8 * kHqHalf) k_hq_tcross(HqGroup, const double *Sp, int nz, double *T) {
+    __shared__ double s12[kHqHalf][kHqHalf + 1], t22[kHqHalf][8], u[kHqHalf][8];
+    const int p = threadIdx.x % kHqHalf, c = threadIdx.x / kHqHalf, col = blockIdx.y * 8 + c;
+    const double *S = Sp + (size_t)blockIdx.x * nz * kHqNb * kHqNb + (size_t)kHqHalf * kHqNb;   // S(0.., 64..)
+    double *To = T + (size_t)blockIdx.x * kHqNb * kHqNb;
+    for (int r = c; r < kHqHalf; r += 8) s12[r][p] = hq_gram(S, nz, p, r);       // S12(p, r)
+    t22[p][c] = To[kHqHalf + p + (size_t)(kHqHalf + col) * kHqNb];
+    __syncthreads();
+    double a0 = 0.0, a1 = 0.0;
+    for (int r = 0; r <= col; r += 2) {                          // T22 is zero below its diagonal
+        a0 = fma(s12[r][p], t22[r][c], a0);
+        a1 = fma(s12[r + 1][p], t22[r + 1][c], a1);
+    }
+    u[p][c] = a0 + a1;
+    __syncthreads();
+    a0 = a1 = 0.0;
+    for (int q = p & ~31; q < kHqHalf; q += 2) {                 // T11 likewise
+        a0 = fma(To[p + (size_t)q * kHqNb], u[q][c], a0);
+        a1 = fma(To[p + (size_t)(q + 1) * kHqNb], u[q + 1][c], a1);
+    }
+    To[p + (size_t)(kHqHalf + col) * kHqNb] = -(a0 + a1);
+    To[kHqHalf + p + (size_t)col * kHqNb] = 0.0;                 // T21
+}
+
+// False when the scratch cannot be had: nothing has been enqueued then.
+bool hq_digits(int n, const double *dA, int lda, const double *dtau, int ncols, double *dX, int ldx, int dev, int sms,
+               cudaStream_t st, int *rc) {
+    static thread_local DgScratch dg;
+    constexpr int ksteps = kHqNb / kDgBK;
+    constexpr size_t vblock = (size_t)kHqNb * kHqNb * kDgDigits * 2, small = (size_t)kHqNb * kDgDigits * 2;
+    const int nblk = (n - 3) / kHqNb + 1;                        // blocks of reflectors
+    const int rbmax = (n - 1 + kHqNb - 1) / kHqNb;               // row blocks of the first one
+    const size_t per_row = (size_t)rbmax * kHqNb * kDgDigits * 2;
+    const size_t fit = std::max<size_t>(1, kHqXBytes / (per_row * kDgBN)) * kDgBN;
+    const int cch = (int)std::min<size_t>(fit, (size_t)((ncols + kDgBN - 1) / kDgBN) * kDgBN);
+    const int gmax = (int)std::max<size_t>(1, std::min<size_t>(nblk, kHqVBytes / (3 * vblock * rbmax)));
+    const size_t vrb = (size_t)gmax * rbmax;                     // row blocks of a group, at most
+    size_t off = 0;
+    const auto take = [&](size_t bytes) {
+        const size_t o = off;
+        off += (bytes + 255) / 256 * 256;
+        return o;
+    };
+    const size_t oXN = take((size_t)cch * per_row), oVM = take(vrb * vblock), oVN = take(vrb * vblock),
+                 oVA = take(vrb * vblock), oTM = take((size_t)gmax * kHqNb * small), oWN = take((size_t)cch * small),
+                 oS = take((size_t)gmax * kHqMaxSplit * kHqNb * kHqNb * 8), oT = take((size_t)gmax * kHqNb * kHqNb * 8),
+                 oWp = take((size_t)kHqMaxSplit * kHqNb * cch * 8), oW2 = take((size_t)kHqNb * cch * 8),
+                 oEx = take(((size_t)ncols + cch + vrb * kHqNb + (size_t)2 * gmax * kHqNb) * sizeof(int));
+    if (!dg.ensure(off, dev, st)) return false;
+    unsigned char *const b = dg.p, *XN = b + oXN, *VM = b + oVM, *VN = b + oVN, *VA = b + oVA, *TM = b + oTM, *WN = b + oWN;
+    double *S = reinterpret_cast<double *>(b + oS), *T = reinterpret_cast<double *>(b + oT),
+           *Wp = reinterpret_cast<double *>(b + oWp), *W2 = reinterpret_cast<double *>(b + oW2);
+    int *exX = reinterpret_cast<int *>(b + oEx), *exW = exX + ncols, *exVA = exW + cch, *exV = exVA + vrb * kHqNb,
+        *exT = exV + gmax * kHqNb;
+    *rc = HSR_ERR_CUDA;
+    // Parts of a sum over `steps` stages for `tiles` tiles: as many as give
+    // the fewest stages on the busiest SM, five stages' time counted for the
+    // end of each part.
+    const auto parts = [&](int tiles, long long steps, int &per) {
+        long long best = LLONG_MAX;
+        int nz = 1;
+        for (int z = 1; z <= kHqMaxSplit && (z == 1 || (long long)z * kDgChunk / 2 <= steps); ++z) {
+            const long long pz = (steps + z - 1) / z, cost = (((long long)tiles * z + sms - 1) / sms) * (pz + 5);
+            if (cost < best) {
+                best = cost;
+                nz = z;
+            }
+        }
+        per = (int)((steps + nz - 1) / nz);
+        return (int)((steps + per - 1) / per);
+    };
+    k_dg_exp_k<<<ncols, 256, 0, st>>>(HqCols{dX, ldx, ncols, n}, n, nullptr, 0, exX);
+    for (int last = nblk - 1; last >= 0; last -= gmax) {
+        const int ng = std::min(gmax, last + 1);
+        const HqGroup h{dA, lda, n, last * kHqNb, (n - 1 - last * kHqNb + kHqNb - 1) / kHqNb};
+        const int rmax = h.rblocks(ng - 1), gz = std::min(kHqMaxSplit, std::max(1, 2 * sms / (2 * ng)));
+        k_dg_exp_k<<<ng * kHqNb, 256, 0, st>>>(HqVCols{h}, n - h.k0(ng - 1) - 1, nullptr, 0, exV);
+        const dim3 gv(kHqNb / 8, (unsigned)((2 * rmax * ksteps + 31) / 32), ng);
+        k_hq_vcols<kDgBM><<<gv, 256, 0, st>>>(h, exV, VM);
+        k_hq_vcols<kDgBN><<<gv, 256, 0, st>>>(h, exV, VN);
+        k_hq_vrows<<<dim3(rmax * (kHqNb / 32), ng), 512, 0, st>>>(h, exVA, VA);
+        if (dg_gemm(2 * gz * ng, sms, VM, VN, HqGram{h, gz, exV, S}, st) != cudaSuccess) return true;
+        k_hq_thalf<<<dim3(ng, 2), 4 * kHqHalf, 0, st>>>(h, dtau, S, gz, T);
+        k_hq_tcross<<<dim3(ng, kHqHalf / 8), 8 * kHqHalf, 0, st>>>(h, S, gz, T);
+        k_dg_small<HqT, true><<<ng * (kHqNb / 32), 512, 0, st>>>(HqT{T}, kDgBM, ng * kHqNb, ng * kHqNb, kHqNb, nullptr, 0,
+                                                                exT, TM);
+        for (int c0 = 0; c0 < ncols; c0 += cch) {
+            const int cols = std::min(cch, ncols - c0), cb = (cols + kDgBN - 1) / kDgBN;
+            for (int g = 0; g < ng; ++g) {
+                const int k0 = h.k0(g), kr = n - k0 - 1, rb = h.rblocks(g), steps = rb * ksteps;
+                const long long at = h.before(g);
+                double *X = dX + (size_t)c0 * ldx + k0 + 1;
+                k_dg_split<HqCols, false><<<dim3(cb * (kDgBN / 8), (unsigned)((2 * steps + 31) / 32)), 256, 0, st>>>(
+                    HqCols{X, ldx, cols, kr}, kDgBN, cb * kDgBN, steps, exX + c0, nullptr, 0, cols, kr, XN);
+                int per = 0;
+                const int nz = parts(cb, steps, per);
+                const DgStoreLong e1{1, cb, steps, per, kHqNb, cols, exV + g * kHqNb, exX + c0, Wp, 1, kHqNb,
+                                     (long long)kHqNb * cols};
+                if (dg_gemm(cb * nz, sms, VM + (size_t)at * vblock, XN, e1, st) != cudaSuccess) return true;
+                k_dg_small<HqSum, false><<<cb * (kDgBN / 8), 128, 0, st>>>(HqSum{Wp, nz, (long long)kHqNb * cols}, kDgBN,
+                                                                         cols, cb * kDgBN, kHqNb, nullptr, 0, exW, WN);
+                const DgStoreShort e2{1, cb, ksteps, ksteps, kHqNb, cols, exT + g * kHqNb, exW, W2, 1, kHqNb, 0};
+                if (dg_gemm(cb, sms, TM + (size_t)g * kHqNb * small, WN, e2, st) != cudaSuccess) return true;
+                k_dg_small<HqSum, false><<<cb * (kDgBN / 8), 128, 0, st>>>(HqSum{W2, 1, 0}, kDgBN, cols, cb * kDgBN, kHqNb,
+                                                                         nullptr, 0, exW, WN);
+                const DgUpdate e3{rb, ksteps, kr, cols, exVA + at * kHqNb, exW, X, ldx, exX + c0};
+                if (dg_gemm(rb * cb, sms, VA + (size_t)at * vblock, WN, e3, st) != cudaSuccess) return true;
+            }
+        }
+    }
+    dg.done(st);
+    *rc = cudaGetLastError() == cudaSuccess ? HSR_OK : HSR_ERR_CUDA;
+    return true;
+}
+
 struct HhScratch {
     int device = -1;
     double *p = nullptr;
@@ -560,8 +855,11 @@ extern "C" int hsr_hessenberg_apply_q_device(int n, const double *dA, int lda, c
     if (ncols == 0 || n <= 2) return HSR_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     static thread_local HhScratch sc;
-    int dev = 0;
+    int dev = 0, sms = 0, rc = HSR_OK;
     if (cudaGetDevice(&dev) != cudaSuccess) return HSR_ERR_CUDA;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (n >= kHqDigitsN && hq_digits(n, dA, lda, dtau, ncols, dX, ldx, dev, sms, st, &rc))
+        return rc;
     const size_t nb = kHbNb;
     const size_t need = (size_t)n * nb + 2 * nb * nb + (size_t)kHbMaxSplit * nb * nb +
                         (size_t)(kHbMaxSplit + 2) * nb * ncols;
@@ -569,8 +867,6 @@ extern "C" int hsr_hessenberg_apply_q_device(int n, const double *dA, int lda, c
     double *V = sc.p, *G = V + (size_t)n * nb, *T = G + nb * nb, *Gp = T + nb * nb;
     double *Wp = Gp + (size_t)kHbMaxSplit * nb * nb, *W = Wp + (size_t)kHbMaxSplit * nb * ncols,
            *W2 = W + nb * (size_t)ncols;
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     auto split_for = [&](int tiles, int kr) {
         int sp = (2 * sms + tiles - 1) / tiles;
         return std::max(1, std::min(sp, std::min(kHbMaxSplit, (kr + kHbTk - 1) / kHbTk)));

@@ -21,7 +21,7 @@
 // The digit product takes over at order 128 (kValDigitsN), for any number of
 // columns: below, its seven more launches cost more than the product (n = 64:
 // 69 us against 60; n = 128: 76 against 93; n = 1000 with 1000 columns: 173
-// against 2,127; n = 5000 with 5000 columns: 4.35 ms against 114.5).  The DFMA
+// against 2,127; n = 5000 with 5000 columns: 4.22 ms against 114.7).  The DFMA
 // form also stays for a scratch buffer that cannot be had.  Error of the
 // residuals against a double-double evaluation, n = 3000: 1.4e-13 relative,
 // DFMA 1.1e-12.
@@ -238,12 +238,14 @@ __global__ void k_val_cols(int cols, const double *wr, const unsigned long long 
     if (c >= cols) return;
     const double sh = inv_pow2_of(*hmax), xs = inv_pow2_of(xmax[c]);
     const int esh = (int)((ubits(sh) >> 52) & 0x7ff) - 1023, exs = (int)((ubits(xs) >> 52) & 0x7ff) - 1023;
-    col[c] = ValCol{-(wr[c] * sh), exs, max(xex[c], kDgZero) + exs + esh - 2044 - 64};
+    col[c] = ValCol{-(wr[c] * sh), exs, max(xex[c], kDgZero) + exs + esh - 2044};
 }
 // r = H x - lambda x of a tile (scaled by the exact powers of two of H and x),
 // its sum of squares per column.  Tiles in row-block order: the longest (the
 // first rows) first, and CTAs that run together share H's digits.
 struct ValEpi {
+    using Sum = DgTwo<16>;
+    static constexpr int kWarps = 16;
     int row0, rows, cols, steps, cblocks;
     const double *X;
     long long ldx;
@@ -252,18 +254,19 @@ struct ValEpi {
     double *rsum;
     __device__ __forceinline__ DgTile tile(int t) const {
         const int bx = t / cblocks;
-        return DgTile{bx, t - bx * cblocks, 0, max(row0 + bx * kDgBM - 1, 0) / kDgBK, steps};
+        const int by = t - bx * cblocks, s0 = max(row0 + bx * kDgBM - 1, 0) / kDgBK;
+        return DgTile{bx, by, 0, (long long)bx * steps + s0, (long long)by * steps + s0, steps - s0};
     }
-    __device__ __forceinline__ void finish(const DgTile &, int row, int col0, const long long (&hi)[32],
-                                           const long long (&lo)[32]) const {
+    __device__ __forceinline__ void finish(const DgTile &, int row, int col0, const Sum &sum) const {
         const bool in = row < rows;
         const int lane = threadIdx.x & 31;
         const int er = in ? max(hex[row], kDgZero) : 0;
-        double r2[32];
+        constexpr int NC = Sum::kCols;
+        double r2[NC];
         // Eight columns at a time, their x loaded ahead of the arithmetic (one
-        // load at a time pays its latency 32 times over).
+        // load at a time pays its latency for every column).
 #pragma unroll
-        for (int c0 = 0; c0 < 32; c0 += 8) {
+        for (int c0 = 0; c0 < NC; c0 += 8) {
             double x[8];
 #pragma unroll
             for (int c = 0; c < 8; ++c)
@@ -271,22 +274,25 @@ struct ValEpi {
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
                 const ValCol k = col[min(col0 + c0 + c, cols - 1)];
-                const double r = fma(k.nlam, dg_ldexp(x[c], k.ex), dg_value(hi[c0 + c], lo[c0 + c], er + k.ep));
+                const double r = fma(k.nlam, dg_ldexp(x[c], k.ex), sum.value(c0 + c, er + k.ep));
                 r2[c0 + c] = in ? r * r : 0.0;
             }
         }
-        // Sum over the warp's rows; lane l ends with column l.
+        // Sum over the warp's rows: lanes l and l + 16 end with halves of
+        // column l mod 16, added last.
+        static_assert(NC == 16, "the exchange below");
 #pragma unroll
-        for (int o = 16; o; o >>= 1) {
+        for (int o = NC / 2; o; o >>= 1) {
             const bool up = (lane & o) != 0;
 #pragma unroll
-            for (int c = 0; c < 16; ++c) {
+            for (int c = 0; c < NC / 2; ++c) {
                 if (c >= o) break;
                 const double keep = up ? r2[c + o] : r2[c], send = up ? r2[c] : r2[c + o];
                 r2[c] = keep + __shfl_xor_sync(0xffffffffu, send, o);
             }
         }
-        if (col0 + lane < cols) atomicAdd(&rsum[col0 + lane], r2[0]);
+        r2[0] += __shfl_xor_sync(0xffffffffu, r2[0], 16);
+        if (lane < NC && col0 + lane < cols) atomicAdd(&rsum[col0 + lane], r2[0]);
     }
     __device__ void poison() const {
         for (int c = threadIdx.x; c < cols; c += blockDim.x) rsum[c] = __longlong_as_double(0x7ff8000000000000LL);
@@ -370,7 +376,7 @@ extern "C" int hsr_residuals_device(int n, const double *dH, int lddH, int ncols
                     lx, kDgBN, cb * kDgBN, steps, xex, hcol, 1, cols, n, xdig);
                 k_val_cols<<<(cols + 127) / 128, 128, 0, st>>>(cols, dwr + c0, hmax, xmax + c0, xex, vcol);
                 const ValEpi epi{r0, rows, cols, (int)steps, cb, Xc, lddX, hex, vcol, rsum + c0};
-                if (dg_gemm(rb * cb, sms, hdig, xdig, steps, epi, st) != cudaSuccess) return HSR_ERR_CUDA;
+                if (dg_gemm(rb * cb, sms, hdig, xdig, epi, st) != cudaSuccess) return HSR_ERR_CUDA;
             }
         }
         dg.done(st);

@@ -59,3 +59,57 @@ def test_residuals_non_finite(gpu_lib):
     H[5, 200] = np.inf
     assert np.isnan(hsr.residuals_device(_cols(torch, H, 0), torch.from_numpy(wr).cuda(),
                                          _cols(torch, X, 0)).cpu().numpy()[[0, 1, 2, 4]]).all()
+
+
+def _reflectors(rng, n):
+    """(A, tau): random Householder vectors as hsr_hessenberg_device leaves them."""
+    A = rng.standard_normal((n, n))
+    tau = np.zeros(n)
+    for k in range(n - 2):
+        x = A[k + 1:, k]
+        beta = -np.copysign(np.linalg.norm(x), x[0])
+        tau[k] = (beta - x[0]) / beta
+        A[k + 2:, k] /= x[0] - beta
+    return A, tau
+
+
+@pytest.mark.parametrize("n,ncols,pad", [(40, 1, 0), (127, 63, 1), (128, 64, 0), (129, 65, 3), (130, 3, 0),
+                                         (131, 130, 0), (258, 16, 1), (259, 5, 0), (515, 70, 0)])
+def test_back_transform_against_extended(gpu_lib, n, ncols, pad):
+    """Reflector by reflector in extended precision; n Householder reflectors
+    in FP64 are within n eps of it, column by column."""
+    import torch
+    import hsrq3in_gb300 as hsr
+    rng = np.random.default_rng(n)
+    A, tau = _reflectors(rng, n)
+    X = rng.standard_normal((n, ncols)) * 10.0 ** rng.uniform(-200, 200, ncols)
+    dX = _cols(torch, X, pad)
+    hsr.hessenberg_apply_q_device(_cols(torch, A, pad), torch.from_numpy(tau).cuda(), dX)
+    R = X.astype(np.longdouble)
+    for k in range(n - 3, -1, -1):
+        v = A[k + 1:, k].astype(np.longdouble)
+        v[0] = 1.0
+        R[k + 1:] -= np.outer(v, tau[k] * (v[:, None] * R[k + 1:]).sum(0))
+    got = dX.cpu().numpy()
+    err = np.sqrt((((got[:, :n].T - R) / np.abs(R).max(0)) ** 2).sum(0)) / np.sqrt(((R / np.abs(R).max(0)) ** 2).sum(0))
+    assert err.max() <= n * EPS, err.max()
+    assert np.all(got[:, n:] == 5.0)
+
+
+def test_back_transform_non_finite(gpu_lib):
+    """An Inf or NaN in a column of X spoils that column's rows from 1 on, as
+    the reflectors do one by one, and no other column."""
+    import torch
+    import hsrq3in_gb300 as hsr
+    n = 200
+    rng = np.random.default_rng(3)
+    A, tau = _reflectors(rng, n)
+    X = rng.standard_normal((n, 4))
+    ref = _cols(torch, X, 0)
+    hsr.hessenberg_apply_q_device(_cols(torch, A, 0), torch.from_numpy(tau).cuda(), ref)
+    X[60, 1], X[150, 2] = np.nan, np.inf
+    dX = _cols(torch, X, 0)
+    hsr.hessenberg_apply_q_device(_cols(torch, A, 0), torch.from_numpy(tau).cuda(), dX)
+    got, ref = dX.cpu().numpy(), ref.cpu().numpy()
+    assert np.array_equal(got[[0, 3]], ref[[0, 3]])
+    assert not np.isfinite(got[1:3, 1:]).any() and np.array_equal(got[1:3, 0], X[0, 1:3])
