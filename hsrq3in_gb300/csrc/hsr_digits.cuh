@@ -133,6 +133,11 @@ __device__ __forceinline__ size_t dg_place(int r, int c8, int RB, long long step
     return blk * (size_t)(RB * kDgBK * kDgDigits * 2) + (size_t)((rr >> 3) * 256 + kc * 128 + (rr & 7) * 16);
 }
 
+__device__ __forceinline__ int dg_dk(const int *dk, int k) {     // no scaling by a zero or non-finite column
+    const int d = dk[k];
+    return d <= -kDgBad / 2 || d >= kDgBad / 2 ? 0 : d;
+}
+
 // ---------------------------------------------------------- preparation
 // Exponents and digits of an operand of R rows and K columns, read through a
 // loader ld(r, k) (0 outside the operand).  dk (optional): exponents taken
@@ -213,7 +218,7 @@ __global__ void __launch_bounds__(RC ? 512 : 128) k_dg_small(Ld ld, int RB, int 
         const int k = c8 * 8 + e;
         x[e] = r < R && k < K ? ld(r, k) : 0.0;
         const int ee = dg_exp(x[e]);
-        m = max(m, dk && ee != kDgZero ? ee + sign * dk[k] : ee);
+        m = max(m, dk && k < K && ee != kDgZero ? ee + sign * dg_dk(dk, k) : ee);
     }
     red[rr][c8] = m;
     __syncthreads();
@@ -226,7 +231,7 @@ __global__ void __launch_bounds__(RC ? 512 : 128) k_dg_small(Ld ld, int RB, int 
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
         const int k = c8 * 8 + e;
-        u[e] = dg_digits(x[e], dk && k < K ? m - 9 - sign * dk[k] : m - 9);
+        u[e] = dg_digits(x[e], dk && k < K ? m - 9 - sign * dg_dk(dk, k) : m - 9);
     }
     dg_store8(u, out + dg_place(r, c8, RB, steps), RB * kDgBK * 2);
 }
@@ -610,7 +615,7 @@ struct DgStore {
 using DgStoreLong = DgStore<DgTwo<16>, 16>;
 using DgStoreShort = DgStore<DgOne<16>, 16>;
 // C(i, j) -= sum over at most 128 columns; cex (optional): the columns'
-// exponents are raised to the new entries'.  One FP64 instruction per entry (a
+// exponents are raised to the new entries' in rows cex_row ...  One FP64 instruction per entry (a
 // warp's takes 64 clocks), the rest on the integer pipe.  Sixteen drain warps
 // with one word per sum: with eight and two words (168 registers, two warps
 // per scheduler) this end took 13,000 clocks of a tile whose products take
@@ -622,7 +627,7 @@ struct DgUpdate {
     const int *ea, *eb;
     double *C;
     long long ldc;
-    int *cex;
+    int *cex, cex_row;
     __device__ __forceinline__ DgTile tile(int t) const {
         const int by = t / mblocks;
         const int bx = t - by * mblocks;
@@ -650,7 +655,8 @@ struct DgUpdate {
         if (!cex) return;
 #pragma unroll
         for (int c = 0; c < Sum::kCols; ++c) {
-            const unsigned m = __reduce_max_sync(0xffffffffu, in ? (unsigned)(ubits(x[c]) >> 32) & 0x7fffffffu : 0u);
+            const unsigned m = __reduce_max_sync(
+                0xffffffffu, in && i >= cex_row ? (unsigned)(ubits(x[c]) >> 32) & 0x7fffffffu : 0u);
             if (lane == c) big = m;
         }
         if (lane < cols) {
@@ -714,6 +720,22 @@ struct DgScratch {
     }
     bool capturing = false;
 };
+// Parts of a sum over `steps` stages for `tiles` tiles (per: stages of a
+// part): as many as give the fewest stages on the busiest SM, five stages'
+// time counted for the end of each part.
+inline int dg_parts(int tiles, int sms, int most, int steps, int &per) {
+    long long best = LLONG_MAX;
+    int nz = 1;
+    for (int z = 1; z <= most && (z == 1 || z * kDgChunk / 2 <= steps); ++z) {
+        const long long pz = (steps + z - 1) / z, cost = (((long long)tiles * z + sms - 1) / sms) * (pz + 5);
+        if (cost < best) {
+            best = cost;
+            nz = z;
+        }
+    }
+    per = (steps + nz - 1) / nz;
+    return (steps + per - 1) / per;
+}
 template <class Epi>
 inline cudaError_t dg_gemm(int tiles, int sms, const unsigned char *A, const unsigned char *B, const Epi &epi,
                            cudaStream_t st) {

@@ -26,7 +26,8 @@
 //                runs dlarfg (with its safe-minimum rescaling)
 //   k_hb_gemv    A(:, j+1 : n-1) v in column chunks, and partial V^T v
 // After the panel the trailing columns c1 = k0 + nb ... get both sides of
-// the block reflector with FP64 GEMMs (k_hb_gemm, DFMA, 64x64 tiles):
+// the block reflector: in one rank-128 product by digits on the tensor cores
+// (hb_trailing), or with FP64 GEMMs (k_hb_gemm, DFMA, 64x64 tiles):
 //   A(:, c1:) -= Y V(c1:, :)^T;  W = T^T V^T A(k0+1:, c1:);  A(k0+1:, c1:) -= V W
 // The "last block" reductions use a completion counter and a fixed summation
 // order: no block waits for another, and results are reproducible run to run.
@@ -677,22 +678,6 @@ bool hq_digits(int n, const double *dA, int lda, const double *dtau, int ncols, 
     int *exX = reinterpret_cast<int *>(b + oEx), *exW = exX + ncols, *exVA = exW + cch, *exV = exVA + vrb * kHqNb,
         *exT = exV + gmax * kHqNb;
     *rc = HSR_ERR_CUDA;
-    // Parts of a sum over `steps` stages for `tiles` tiles: as many as give
-    // the fewest stages on the busiest SM, five stages' time counted for the
-    // end of each part.
-    const auto parts = [&](int tiles, long long steps, int &per) {
-        long long best = LLONG_MAX;
-        int nz = 1;
-        for (int z = 1; z <= kHqMaxSplit && (z == 1 || (long long)z * kDgChunk / 2 <= steps); ++z) {
-            const long long pz = (steps + z - 1) / z, cost = (((long long)tiles * z + sms - 1) / sms) * (pz + 5);
-            if (cost < best) {
-                best = cost;
-                nz = z;
-            }
-        }
-        per = (int)((steps + nz - 1) / nz);
-        return (int)((steps + per - 1) / per);
-    };
     k_dg_exp_k<<<ncols, 256, 0, st>>>(HqCols{dX, ldx, ncols, n}, n, nullptr, 0, exX);
     for (int last = nblk - 1; last >= 0; last -= gmax) {
         const int ng = std::min(gmax, last + 1);
@@ -717,7 +702,7 @@ bool hq_digits(int n, const double *dA, int lda, const double *dtau, int ncols, 
                 k_dg_split<HqCols, false><<<dim3(cb * (kDgBN / 8), (unsigned)((2 * steps + 31) / 32)), 256, 0, st>>>(
                     HqCols{X, ldx, cols, kr}, kDgBN, cb * kDgBN, steps, exX + c0, nullptr, 0, cols, kr, XN);
                 int per = 0;
-                const int nz = parts(cb, steps, per);
+                const int nz = dg_parts(cb, sms, kHqMaxSplit, steps, per);
                 const DgStoreLong e1{1, cb, steps, per, kHqNb, cols, exV + g * kHqNb, exX + c0, Wp, 1, kHqNb,
                                      (long long)kHqNb * cols};
                 if (dg_gemm(cb * nz, sms, VM + (size_t)at * vblock, XN, e1, st) != cudaSuccess) return true;
@@ -727,7 +712,7 @@ bool hq_digits(int n, const double *dA, int lda, const double *dtau, int ncols, 
                 if (dg_gemm(cb, sms, TM + (size_t)g * kHqNb * small, WN, e2, st) != cudaSuccess) return true;
                 k_dg_small<HqSum, false><<<cb * (kDgBN / 8), 128, 0, st>>>(HqSum{W2, 1, 0}, kDgBN, cols, cb * kDgBN, kHqNb,
                                                                          nullptr, 0, exW, WN);
-                const DgUpdate e3{rb, ksteps, kr, cols, exVA + at * kHqNb, exW, X, ldx, exX + c0};
+                const DgUpdate e3{rb, ksteps, kr, cols, exVA + at * kHqNb, exW, X, ldx, exX + c0, 0};
                 if (dg_gemm(rb * cb, sms, VA + (size_t)at * vblock, WN, e3, st) != cudaSuccess) return true;
             }
         }
@@ -735,6 +720,193 @@ bool hq_digits(int n, const double *dA, int lda, const double *dtau, int ncols, 
     dg.done(st);
     *rc = cudaGetLastError() == cudaSuccess ? HSR_OK : HSR_ERR_CUDA;
     return true;
+}
+
+// ------------------------------------------------ trailing update by digits
+// Both sides of a panel's block reflector in one rank-128 product: with Y =
+// A V T and W0 = V^T A(k0+1:, c1:) over the panel-start A,
+//   (I - V T^T V^T) (A - Y V^T) = A - Y V^T - V Z,
+//   Z = T^T W0 - T^T (V^T Y) V(c1:, :)^T,
+// so the trailing columns are read once for W0 and read and written once for
+// A -= [Y V] [V(c1:, :)^T; Z], where the two sides one after the other pass
+// over them five times.  V^T Y comes with W0 (Y's columns follow A's).
+constexpr size_t kHbDigitBytes = (size_t)2 << 30;   // most scratch for digits of A's columns at a time
+constexpr int kHbParts = 16;
+// Smallest order: the DFMA form's thin products take about 65 us each on the
+// few SMs they fill (n = 10, no trailing product worth the name: 331 us
+// against 354; 40: 1,729 against 1,664; 700: 41.4 ms against 39.4; 6000: 1,130
+// against 691, the rest of it the panels).  The DFMA form also stays for a
+// scratch buffer that cannot be had.
+constexpr int kHbDigitsN = 32;
+
+// Columns c0 + r of A, then Y's; rows k0 + 1 + k.
+struct HbTrail {
+    const double *A, *Y;
+    long long lda;
+    int n, k0, c0;
+    __device__ __forceinline__ double operator()(int r, int k) const {
+        const int i = k0 + 1 + k, c = c0 + r;
+        if (i >= n || c >= n + kHbNb) return 0.0;
+        return c < n ? A[i + (size_t)c * lda] : Y[i + (size_t)(c - n) * n];
+    }
+    __device__ __forceinline__ int first(int) const { return 0; }
+};
+// Columns of [Y V] (rows k0 + 1 + k), for their exponents, and V's alone.
+struct HbPanelCols {
+    const double *Y, *V;
+    int n, k0;
+    __device__ __forceinline__ double operator()(int r, int k) const {
+        const int i = k0 + 1 + k;
+        if (i >= n) return 0.0;
+        return r < kHbNb ? Y[i + (size_t)r * n] : V[i + (size_t)(r - kHbNb) * n];
+    }
+    __device__ __forceinline__ int first(int) const { return 0; }
+};
+struct HbVCols {
+    const double *V;
+    int n, k0;
+    __device__ __forceinline__ double operator()(int r, int k) const {
+        const int i = k0 + 1 + k;
+        return i < n ? V[i + (size_t)r * n] : 0.0;
+    }
+    __device__ __forceinline__ int first(int) const { return 0; }
+};
+// [T^T, -T^T (V^T Y)], 64 x 128.
+struct HbM1 {
+    const double *M;
+    __device__ __forceinline__ double operator()(int r, int k) const { return M[r + k * kHbNb]; }
+};
+// Column j of [W0; V(c1:, :)^T].
+struct HbB1 {
+    const double *Wp, *V;
+    int nz, n, c1;
+    long long cz;
+    __device__ __forceinline__ double operator()(int r, int k) const {
+        if (k >= kHbNb) return V[c1 + r + (size_t)(k - kHbNb) * n];
+        double s = 0.0;
+        for (int z = 0; z < nz; ++z) s += Wp[(size_t)z * cz + k + (size_t)r * kHbNb];
+        return s;
+    }
+};
+// Row i of [Y V], column j of [V(c1:, :)^T; Z].
+struct HbA2 {
+    const double *Y, *V;
+    int n;
+    __device__ __forceinline__ double operator()(int r, int k) const {
+        return k < kHbNb ? Y[r + (size_t)k * n] : V[r + (size_t)(k - kHbNb) * n];
+    }
+};
+struct HbB2 {
+    const double *V, *Z;
+    int n, c1;
+    __device__ __forceinline__ double operator()(int r, int k) const {
+        return k < kHbNb ? V[c1 + r + (size_t)k * n] : Z[k - kHbNb + (size_t)r * kHbNb];
+    }
+};
+
+// M1 = [T^T, -T^T VY] (VY: the last 64 columns of W0), eight columns per CTA,
+// and their exponents.
+__global__ void __launch_bounds__(8 * kHbNb) k_hb_m1(const double *T, const double *VYp, int nz, long long cz, double *M,
+                                                     int *dk) {
+    __shared__ double vy[8][kHbNb];
+    __shared__ int red[8][2];
+    const int q = threadIdx.x % kHbNb, c = threadIdx.x / kHbNb, k = blockIdx.x * 8 + c;
+    double v;
+    if (k < kHbNb) {
+        v = T[k + q * kHbNb];
+    } else {
+        double s = 0.0;
+#pragma unroll 4
+        for (int z = 0; z < nz; ++z) s += VYp[(size_t)z * cz + q + (size_t)(k - kHbNb) * kHbNb];
+        vy[c][q] = s;
+    }
+    __syncthreads();
+    if (k >= kHbNb) {
+        double a0 = 0.0, a1 = 0.0;
+        for (int p = 0; p < kHbNb; p += 2) {
+            a0 = fma(T[p + q * kHbNb], vy[c][p], a0);
+            a1 = fma(T[p + 1 + q * kHbNb], vy[c][p + 1], a1);
+        }
+        v = -(a0 + a1);
+    }
+    M[q + k * kHbNb] = v;
+    const int m = __reduce_max_sync(0xffffffffu, dg_exp(v));
+    if ((q & 31) == 0) red[c][q >> 5] = m;
+    __syncthreads();
+    if (q == 0) dk[k] = max(red[c][0], red[c][1]);
+}
+
+// The scratch of one reduction, laid out once.
+struct HbDigits {
+    unsigned char *AD, *VN, *M1, *B1, *A2, *B2;
+    double *Wp, *M, *Z;
+    int *cex, *exM1, *exB, *exA2, *dk1;                          // cex: n columns of A, then [Y V]
+    int cch;
+};
+size_t hb_digits_layout(int n, unsigned char *base, HbDigits &D) {
+    const size_t rows16 = (size_t)((n + kDgBK - 1) / kDgBK) * kDgBK * kDgDigits * 2;   // bytes of one column's digits
+    const size_t all = (size_t)(n + kHbNb + kDgBM - 1) / kDgBM * kDgBM;
+    const size_t fit = std::max<size_t>(1, kHbDigitBytes / (rows16 * kDgBM)) * kDgBM;
+    D.cch = (int)std::min(all, fit);
+    const size_t small = (size_t)2 * kHbNb * kDgDigits * 2;      // bytes of one 128-column row's digits
+    size_t off = 0;
+    const auto take = [&](size_t bytes) {
+        const size_t o = off;
+        off += (bytes + 255) / 256 * 256;
+        return base + o;
+    };
+    D.AD = take((size_t)D.cch * rows16);
+    D.VN = take((size_t)kDgBN * rows16);
+    D.M1 = take((size_t)kDgBM * small);
+    D.B1 = take(all * small);
+    D.A2 = take(all * small);
+    D.B2 = take(all * small);
+    D.Wp = reinterpret_cast<double *>(take((size_t)kHbParts * kHbNb * all * 8));
+    D.M = reinterpret_cast<double *>(take((size_t)2 * kHbNb * kHbNb * 8));
+    D.Z = reinterpret_cast<double *>(take((size_t)kHbNb * all * 8));
+    D.cex = reinterpret_cast<int *>(take((size_t)(n + 2 * kHbNb) * sizeof(int)));
+    D.exM1 = reinterpret_cast<int *>(take((size_t)kDgBM * sizeof(int)));
+    D.exB = reinterpret_cast<int *>(take(all * sizeof(int)));
+    D.exA2 = reinterpret_cast<int *>(take(all * sizeof(int)));
+    D.dk1 = reinterpret_cast<int *>(take((size_t)2 * kHbNb * sizeof(int)));
+    return off;
+}
+// The trailing columns c1 .. n-1 of panel k0.
+cudaError_t hb_trailing(const HbState &S, const HbDigits &D, int k0, int c1, int sms, cudaStream_t st) {
+    const int n = S.n, m = n - c1, kr = n - k0 - 1, total = m + kHbNb;
+    const int steps = (kr + kDgBK - 1) / kDgBK;
+    constexpr int ksteps = 2 * kHbNb / kDgBK;
+    const int *exY = D.cex + n, *exV = exY + kHbNb;
+    k_dg_exp_k<<<2 * kHbNb, 256, 0, st>>>(HbPanelCols{S.Y, S.V, n, k0}, kr, nullptr, 0, D.cex + n);
+    k_dg_split<HbVCols, false><<<dim3(kDgBN / 8, (unsigned)((2 * steps + 31) / 32)), 256, 0, st>>>(
+        HbVCols{S.V, n, k0}, kDgBN, kDgBN, steps, exV, nullptr, 0, kHbNb, kr, D.VN);
+    int per = 0;
+    const int tiles = (std::min(total, D.cch) + kDgBM - 1) / kDgBM;
+    const int nz = dg_parts(tiles, sms, kHbParts, steps, per);
+    const long long cz = (long long)kHbNb * total;
+    for (int c = 0; c < total; c += D.cch) {
+        const int cols = std::min(D.cch, total - c), mb = (cols + kDgBM - 1) / kDgBM;
+        k_dg_split<HbTrail, false><<<dim3(mb * (kDgBM / 8), (unsigned)((2 * steps + 31) / 32)), 256, 0, st>>>(
+            HbTrail{S.A, S.Y, S.lda, n, k0, c1 + c}, kDgBM, mb * kDgBM, steps, D.cex + c1 + c, nullptr, 0, cols, kr, D.AD);
+        const DgStoreLong e{mb, 1, steps, per, cols, kHbNb, D.cex + c1 + c, exV, D.Wp + (size_t)kHbNb * c, kHbNb, 1, cz};
+        const cudaError_t err = dg_gemm(mb * nz, sms, D.AD, D.VN, e, st);
+        if (err != cudaSuccess) return err;
+    }
+    k_hb_m1<<<2 * kHbNb / 8, 8 * kHbNb, 0, st>>>(S.T, D.Wp + (size_t)kHbNb * m, nz, cz, D.M, D.dk1);
+    k_dg_small<HbM1, true><<<kDgBM / 32, 512, 0, st>>>(HbM1{D.M}, kDgBM, kHbNb, kDgBM, 2 * kHbNb, D.dk1, -1, D.exM1, D.M1);
+    const int nb = (m + kDgBN - 1) / kDgBN, rb = (n + kDgBM - 1) / kDgBM;
+    k_dg_small<HbB1, false><<<nb * (kDgBN / 8), 128, 0, st>>>(HbB1{D.Wp, S.V, nz, n, c1, cz}, kDgBN, m, nb * kDgBN,
+                                                              2 * kHbNb, D.dk1, 1, D.exB, D.B1);
+    const DgStoreShort ez{1, nb, ksteps, ksteps, kHbNb, m, D.exM1, D.exB, D.Z, 1, kHbNb, 0};
+    cudaError_t err = dg_gemm(nb, sms, D.M1, D.B1, ez, st);
+    if (err != cudaSuccess) return err;
+    k_dg_small<HbA2, true><<<rb * (kDgBM / 32), 512, 0, st>>>(HbA2{S.Y, S.V, n}, kDgBM, n, rb * kDgBM, 2 * kHbNb, D.cex + n,
+                                                              -1, D.exA2, D.A2);
+    k_dg_small<HbB2, false><<<nb * (kDgBN / 8), 128, 0, st>>>(HbB2{S.V, D.Z, n, c1}, kDgBN, m, nb * kDgBN, 2 * kHbNb,
+                                                              D.cex + n, 1, D.exB, D.B2);
+    const DgUpdate eu{rb, ksteps, n, m, D.exA2, D.exB, S.A + (size_t)c1 * S.lda, S.lda, D.cex + c1, k0 + 1};
+    err = dg_gemm(rb * nb, sms, D.A2, D.B2, eu, st);
+    return err != cudaSuccess ? err : cudaGetLastError();
 }
 
 struct HhScratch {
@@ -806,10 +978,21 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
     if (cudaMemsetAsync(S.cnt, 0, 4 * sizeof(double), st) != cudaSuccess) return HSR_ERR_CUDA;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    static thread_local DgScratch dg;
+    HbDigits D{};
+    const bool digits = n >= kHbDigitsN && dg.ensure(hb_digits_layout(n, nullptr, D), dev, st);
+    if (digits) {
+        hb_digits_layout(n, dg.p, D);
+        // Exponents of A's columns over the rows that reflectors touch.
+        k_dg_exp_k<<<n, 256, 0, st>>>(HqCols{dA + 1, lda, n, n - 1}, n - 1, nullptr, 0, D.cex);
+    }
     for (int k0 = 0; k0 < n - 2; k0 += kHbNb) {
         const int ib = std::min(kHbNb, n - 2 - k0);
         if (cudaMemsetAsync(S.V, 0, (size_t)n * nb * sizeof(double), st) != cudaSuccess ||
             cudaMemsetAsync(S.T, 0, nb * nb * sizeof(double), st) != cudaSuccess)
+            return HSR_ERR_CUDA;
+        if (ib < kHbNb &&                                        // columns a short panel leaves unwritten
+            cudaMemsetAsync(S.Y + (size_t)ib * n, 0, (size_t)(kHbNb - ib) * n * sizeof(double), st) != cudaSuccess)
             return HSR_ERR_CUDA;
         int nchp = 0;
         for (int i = 0; i < ib; ++i) {
@@ -823,6 +1006,10 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
         k_hb_step<<<nblk, kHbRows, 0, st>>>(S, k0, ib - 1, -1, nchp);
         const int c1 = k0 + ib, m = n - c1;
         if (m <= 0) continue;
+        if (digits) {
+            if (hb_trailing(S, D, k0, c1, sms, st) != cudaSuccess) return HSR_ERR_CUDA;
+            continue;
+        }
         // Right: A(:, c1:) -= Y V(c1:, :)^T
         if (hb_gemm(n, m, ib, -1.0, S.Y, 1, n, S.V + c1, n, 1, 1.0, dA + (size_t)c1 * lda, lda, 1, 0, st) !=
             cudaSuccess)
@@ -846,6 +1033,7 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
                     0, st) != cudaSuccess)
             return HSR_ERR_CUDA;
     }
+    if (digits) dg.done(st);
     return cudaGetLastError() == cudaSuccess ? HSR_OK : HSR_ERR_CUDA;
 }
 

@@ -113,3 +113,43 @@ def test_back_transform_non_finite(gpu_lib):
     got, ref = dX.cpu().numpy(), ref.cpu().numpy()
     assert np.array_equal(got[[0, 3]], ref[[0, 3]])
     assert not np.isfinite(got[1:3, 1:]).any() and np.array_equal(got[1:3, 0], X[0, 1:3])
+
+
+@pytest.mark.parametrize("n,pad,scale", [(32, 0, 1.0), (66, 1, 1e150), (67, 0, 1.0), (130, 0, 1e-150), (193, 3, 1.0),
+                                         (258, 0, 1.0), (322, 1, 1e8)])
+def test_reduction_backward_error(gpu_lib, n, pad, scale):
+    """A = Q H Q^T to within n eps |A|, the backward error of 2n Householder
+    transformations, with Q formed in extended precision from the reflectors."""
+    import torch
+    import hsrq3in_gb300 as hsr
+    A = np.random.default_rng(n).standard_normal((n, n))
+    dA = _cols(torch, A * scale, pad)
+    tau = hsr.hessenberg_device(dA).cpu().numpy()
+    got = dA.cpu().numpy()
+    assert np.all(got[:, n:] == 5.0)
+    F = got[:, :n].T
+    Q = np.eye(n, dtype=np.longdouble)
+    for k in range(n - 3, -1, -1):
+        v = F[k + 1:, k].astype(np.longdouble)
+        v[0] = 1.0
+        Q[k + 1:] -= np.outer(v, tau[k] * (v[:, None] * Q[k + 1:]).sum(0))
+    H = np.triu(F, -1).astype(np.longdouble) / scale
+    R = np.array([(A * Q[:, c]).sum(1) - (Q[:, :c + 2] * H[:c + 2, c]).sum(1) for c in range(n)])   # A Q - Q H
+    err = float(np.sqrt((R * R).sum()))
+    assert err <= n * EPS * np.linalg.norm(A), (err, np.linalg.norm(A))
+
+
+def test_reduction_nan_in_first_row(gpu_lib):
+    """Row 0 takes no part in any reflector: a NaN there stays in that row and
+    the rest is what it is without it."""
+    import torch
+    import hsrq3in_gb300 as hsr
+    n = 150
+    A = np.random.default_rng(5).standard_normal((n, n))
+    clean = _cols(torch, A, 0)
+    tau = hsr.hessenberg_device(clean)
+    A[0, 100] = np.nan
+    got = _cols(torch, A, 0)
+    tau2 = hsr.hessenberg_device(got)
+    assert torch.equal(tau, tau2) and torch.equal(got[:, 1:], clean[:, 1:])
+    assert torch.isnan(got[1:, 0]).all()
