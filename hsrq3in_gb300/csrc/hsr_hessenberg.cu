@@ -319,6 +319,446 @@ __global__ void __launch_bounds__(kHbRows) k_hb_gemv(HbState S, int k0, int i, i
     block_vdot(S, r0, i, cs, S.part2 + (size_t)blockIdx.x * kHbNb);
 }
 
+// --------------------------------------------------- panel in one launch
+// The same column steps as the three kernels above, for all columns of a
+// panel in one cooperative launch.  The first CTAs own R rows each for the
+// vector work and keep their rows of Y and V, and a copy of T, in shared
+// memory; a sum over all rows is left in global memory as one partial per
+// CTA, and after a grid barrier every CTA that needs it adds all of them up
+// in the same order.  Three barriers a column: after the partial V^T c (CTAs
+// with rows only), after the partial norms, and after A v.  All CTAs share
+// A v, a row tile of rpc rows and a share of the columns each.  T's new
+// column is formed while a barrier is awaited, the next column and the first
+// entries of A for A v are loaded ahead of one.
+//
+// Bound for small orders by the L2 round trips of the barriers and sums and
+// by FP64 issue (a warp's instruction takes 64 clocks of its sub-partition):
+// 35,000 clocks a column at n = 700, of which A v 4,000; for large ones by the
+// FP64 pipe in A v (an FMA per 8 bytes of A: 2 a clock and SM, 0.7 of the
+// memory rate; 76,000 of 119,000 clocks at n = 6000).  Against the three
+// launches a column on n / 256 CTAs: n = 700 39.4 ms before, 13.4 now;
+// n = 6000 691 and 370; n = 10 354 us and 225.
+constexpr int kHbThreads = 512;
+constexpr int kHbPiece = 1024;         // columns of v staged at a time (two per thread)
+constexpr int kHbAhead = 8;            // entries of A per thread loaded before v is known
+constexpr int kHbPanelSmem = 220 * 1024;
+constexpr unsigned kHbSpin = 1u << 23; // polls of a barrier before it gives up and says so
+constexpr unsigned kHbDead = 1u << 30; // ... by this bit of both counters
+
+struct HbPanel {
+    HbState S;
+    int k0, ib, R, own;                // CTAs 0 .. own-1 have rows, R each
+    int rpc, tiles, shares;            // A v: row tiles of rpc rows, CTAs (column shares) per tile
+    unsigned *bar;                     // arrivals since the reduction began: of all CTAs, of those with rows
+};
+__host__ __device__ constexpr int hb_pitch(int R) { return R | 1; }     // odd: columns fall on different banks
+__host__ __device__ constexpr size_t hb_panel_smem(int R) {
+    return sizeof(double) * ((size_t)2 * kHbNb * hb_pitch(R) + kHbNb * (kHbNb + 1) + 2 * (size_t)R + 4 * kHbNb +
+                             2 * kHbThreads + kHbPiece + 16);
+}
+// Sum of x over the lanes of an aligned group of g (a power of two), in every lane.
+__device__ __forceinline__ double group_sum(double x, int g) {
+    for (int o = g >> 1; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+
+__global__ void __launch_bounds__(kHbThreads, 1) k_hb_panel(HbPanel P) {
+    extern __shared__ double hsm[];
+    __shared__ int dead;
+    const HbState &S = P.S;
+    const int tid = threadIdx.x, n = S.n, k0 = P.k0, R = P.R, Rp = hb_pitch(R), G = gridDim.x, b = blockIdx.x;
+    double *const Ys = hsm, *const Vs = Ys + kHbNb * Rp, *const Ts = Vs + kHbNb * Rp;      // T(p, q) at p + 65 q
+    double *const cs = Ts + kHbNb * (kHbNb + 1), *const aj = cs + R, *const vv = aj + R, *const wv = vv + kHbNb;
+    double *const w2 = wv + kHbNb, *const vrow = w2 + kHbNb, *const red = vrow + kHbNb, *const gred = red + kHbThreads;
+    double *const vst = gred + kHbThreads, *const sc = vst + kHbPiece;
+    const int rt = b / P.shares, share = b - rt * P.shares;      // place in A v
+    const bool has = b < P.own;
+    const int r0 = min(b * R, n), nr = has ? min(R, n - r0) : 0; // own rows
+    const int rlo = min(max(k0 + 1 - r0, 0), nr);                // first own row that the reflectors touch
+    // A warp's FP64 instruction takes 64 clocks of its sub-partition whether
+    // one lane or all are at work, so the dots below use the fewest warps that
+    // fill four of them, and warps without work stay out.
+    int tpr = 1;                                                 // threads per row
+    while (tpr < 32 && R * tpr * 2 <= 128) tpr *= 2;
+    const int rgrp = kHbThreads / tpr, rs = tid & (tpr - 1), rofs = tid / tpr, wofs = (tid & ~31) / tpr;
+
+    unsigned target[2] = {0, 0};
+    if (tid == 0) {
+        // Arrivals of this launch cannot complete a round before this CTA's own.
+        target[0] = (*reinterpret_cast<volatile unsigned *>(P.bar) & ~kHbDead) / G * G;
+        target[1] = (*reinterpret_cast<volatile unsigned *>(P.bar + 1) & ~kHbDead) / P.own * P.own;
+        dead = 0;
+    }
+    auto arrive = [&](int which) {                               // 0: all CTAs, 1: those with rows
+        __syncthreads();
+        if (tid == 0) {
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(P.bar + which) : "memory");
+            target[which] += which ? P.own : G;
+        }
+    };
+    auto wait = [&](int which) {                                 // false once a barrier gave up
+        if (tid == 0) {
+            unsigned it = 0, v;
+            do {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(P.bar + which) : "memory");
+            } while (!(v & kHbDead) && (int)(v - target[which]) < 0 && ++it < kHbSpin);
+            if (it >= kHbSpin) {
+                atomicOr(P.bar, kHbDead);
+                atomicOr(P.bar + 1, kHbDead);
+            }
+            if (it >= kHbSpin || (v & kHbDead)) dead = 1;
+        }
+        __syncthreads();
+        return dead == 0;
+    };
+    // out[q] = f * sum over the CTAs of part[c][q], q < cnt, in a fixed order:
+    // four or (many CTAs) eight threads per q, up to 13 loads of each in
+    // flight at a time.
+    auto reduce_parts = [&](const double *part, int cnt, double *out, double f) {
+        const int lq = cnt <= 32 ? 5 : 6, q = tid & ((1 << lq) - 1), s = tid >> lq, ns = P.own > 52 ? 8 : 4;
+        if (s < ns) {
+            double a = 0.0;
+            if (q < cnt) {
+                for (int c = s; c < P.own; c += 13 * ns) {
+                    double x[13];
+#pragma unroll
+                    for (int e = 0; e < 13; ++e) x[e] = c + e * ns < P.own ? __ldcg(part + (size_t)(c + e * ns) * kHbNb + q) : 0.0;
+#pragma unroll
+                    for (int e = 0; e < 13; ++e)
+                        if (c + e * ns < P.own) a += x[e];       // uniform over the warp
+                }
+            }
+            red[tid] = a;
+        }
+        __syncthreads();
+        if (tid < cnt) {
+            double u = (red[tid] + red[tid + (1 << lq)]) + (red[tid + (2 << lq)] + red[tid + (3 << lq)]);
+            if (ns == 8) u += (red[tid + (4 << lq)] + red[tid + (5 << lq)]) + (red[tid + (6 << lq)] + red[tid + (7 << lq)]);
+            out[tid] = f * u;
+        }
+        __syncthreads();
+    };
+    // Threads per column for `cnt` column dots: as with the rows.
+    auto per_col = [&](int cnt) { return cnt <= 16 ? 8 : cnt <= 32 ? 4 : 2; };
+    // part[b][q] = sum over own rows of V(r, q) x(r), q < cnt.
+    auto col_dots = [&](const double *x, int cnt, double *part) {
+        const int tq = per_col(cnt), q = tid / tq, s = tid & (tq - 1);
+        if ((tid & ~31) / tq >= cnt) return;
+        double a = 0.0;
+        if (q < cnt)
+            for (int r = rlo + s; r < nr; r += tq) a = fma(Vs[q * Rp + r], x[r], a);
+        a = group_sum(a, tq);
+        if (s == 0 && q < cnt) __stcg(part + (size_t)b * kHbNb + q, a);
+    };
+    // Norm accumulators of c(j+2 :): this CTA's rows to partn, later all CTAs'.
+    auto norms_out = [&](int j, double *out) {
+        Nrm3 acc;
+        acc.init();
+        for (int r = tid; r < nr; r += kHbThreads)
+            if (r0 + r >= j + 2) acc.add(cs[r]);
+        const int warps = min(kHbThreads / 32, (nr + 31) / 32), w = tid >> 5;
+        const bool ends = __syncthreads_or(acc.asml != 0.0 || acc.abig != 0.0);
+        if (w < warps) {
+            const double m = group_sum(acc.amed, 32);
+            if ((tid & 31) == 0) red[w] = m;
+            if (ends) {
+                const double lo = group_sum(acc.asml, 32), hi = group_sum(acc.abig, 32);
+                if ((tid & 31) == 0) {
+                    red[32 + w] = lo;
+                    red[64 + w] = hi;
+                }
+            }
+        }
+        __syncthreads();
+        if (tid < 3) {                                           // asml, amed, abig
+            double u = 0.0;
+            const int at = tid == 0 ? 32 : tid == 1 ? 0 : 64;
+            if (tid == 1 || ends)
+                for (int z = 0; z < warps; ++z) u += red[at + z];
+            __stcg(out + (size_t)b * 3 + tid, u);
+        }
+    };
+    // xnorm (or, as good a test for 0, its square) to sc[0], alpha to sc[1],
+    // beta to sc[2], 1 / (alpha - beta) to sc[4].  With all of c(j+1 :) in the middle range beta is one
+    // square root of the sum of squares.
+    auto norms_in = [&](int j, const double *in) {
+        if (tid < 32) {
+            double x[3][5];
+            Nrm3 tot;
+            tot.init();
+            const double alpha = __ldcg(S.c + j + 1);
+            for (int c = tid; c < P.own; c += 160) {
+#pragma unroll
+                for (int e = 0; e < 5; ++e)
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) x[k][e] = c + 32 * e < P.own ? __ldcg(in + (size_t)(c + 32 * e) * 3 + k) : 0.0;
+#pragma unroll
+                for (int e = 0; e < 5; ++e)
+                    if ((c & ~31) + 32 * e < P.own) tot.amed += x[1][e];
+#pragma unroll
+                for (int e = 0; e < 5; ++e) {
+                    if (mag(x[0][e]) != 0) tot.asml = add_rare(tot.asml, x[0][e]);
+                    if (mag(x[2][e]) != 0) tot.abig = add_rare(tot.abig, x[2][e]);
+                }
+            }
+            const bool ends = __any_sync(0xffffffffu, mag(tot.asml) != 0 || mag(tot.abig) != 0);
+            tot.amed = group_sum(tot.amed, 32);
+            if (ends) {
+                tot.asml = group_sum(tot.asml, 32);
+                tot.abig = group_sum(tot.abig, 32);
+            }
+            if (tid == 0) {
+                const unsigned long long ma = mag(alpha);
+                double xn = tot.amed, beta = alpha;
+                if (!ends && (ma == 0 || (ma > pow2_bits(-500) && ma < pow2_bits(486))) && mag(xn) > pow2_bits(-900)) {
+                    beta = sqrt(fma(alpha, alpha, xn));
+                    beta = ubits(alpha) >> 63 ? beta : neg(beta);
+                } else {
+                    xn = tot.finish();
+                    if (xn != 0.0) beta = -copysign(lapy2(alpha, xn), alpha);
+                }
+                sc[0] = xn;
+                sc[1] = alpha;
+                sc[2] = beta;
+                sc[4] = xn != 0.0 ? 1.0 / (alpha - beta) : 1.0;
+            }
+        }
+        __syncthreads();
+    };
+    // T(0 : ip, ip) = -tau T vv, T(ip, ip) = tau, in shared memory (vv holds -V^T v).
+    auto t_column = [&](int ip, double t) {
+        const int tq = per_col(ip + 1), p = tid / tq, s = tid & (tq - 1);
+        if ((tid & ~31) / tq > ip) return;
+        double a = 0.0;
+        for (int q = p + s; q < ip; q += tq) a = fma(Ts[p + q * (kHbNb + 1)], vv[q], a);
+        a = group_sum(a, tq);
+        if (s == 0 && p <= ip) Ts[p + ip * (kHbNb + 1)] = p < ip ? t * a : t;
+    };
+    // sum_q M(r, q) w[q] over q < cnt for row r, in the row's lanes; `more` is
+    // each lane's own part of something to add.
+    auto row_dot = [&](const double *M, const double *w, int cnt, int r, double more) {
+        double a = more;
+        if (r < nr)
+            for (int q = rs; q < cnt; q += tpr) a = fma(M[q * Rp + r], w[q], a);
+        return group_sum(a, tpr);
+    };
+
+    for (int e = tid; e < kHbNb * (kHbNb + 1); e += kHbThreads) Ts[e] = 0.0;
+    for (int r = tid; r < nr; r += kHbThreads) aj[r] = S.A[r0 + r + (size_t)k0 * S.lda];
+    double t = 0.0;
+    bool ok = true;
+    __syncthreads();
+    for (int i = 0; i <= P.ib; ++i) {
+        const int j = k0 + i, ip = i - 1;
+        if (i == P.ib && !has) break;
+        if (has) {
+            if (i > 0) {
+                // Y(:, ip) = tau (A v - Y (V^T v)).
+                if (tid < i) vrow[tid] = tid == ip ? 1.0 : __ldcg(S.V + j + (size_t)tid * n);
+                double g0[4];                                    // the first row's parts, beside the sums' loads
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    g0[e] = rofs < nr && rs + e * tpr < P.shares ? __ldcg(S.gpart + (size_t)(rs + e * tpr) * n + r0 + rofs) : 0.0;
+                reduce_parts(S.part2, ip, vv, -1.0);                 // -V^T v
+                for (int base = 0; base + wofs < nr; base += rgrp) {
+                    const int r = base + rofs;
+                    double av = 0.0;
+                    if (r < nr) {
+                        for (int c = rs; c < P.shares; c += tpr) av += __ldcg(S.gpart + (size_t)c * n + r0 + r);
+                    }
+                    const double y = t * row_dot(Ys, vv, ip, r, av);
+                    if (r < nr && rs == 0) {
+                        Ys[ip * Rp + r] = y;
+                        S.Y[r0 + r + (size_t)ip * n] = y;
+                    }
+                }
+                if (i == P.ib) break;
+                __syncthreads();
+            }
+            // c = a_j - Y V(j, :)^T.
+            for (int base = 0; base + wofs < nr; base += rgrp) {
+                const int r = base + rofs;
+                const double a = row_dot(Ys, vrow, i, r, 0.0);
+                if (r < nr && rs == 0) cs[r] = aj[r] - a;
+            }
+            __syncthreads();
+            if (i > 0) {
+                // c -= V T^T V^T c.
+                col_dots(cs, i, S.part);
+                arrive(1);
+                t_column(ip, t);
+                ok = wait(1);
+                if (!ok) break;
+                reduce_parts(S.part, i, wv, 1.0);
+                {                                                    // T^T of it
+                    const int tq = per_col(i), p = tid / tq, s = tid & (tq - 1);
+                    if ((tid & ~31) / tq < i) {
+                        double a = 0.0;
+                        if (p < i)
+                            for (int q = s; q <= p; q += tq) a = fma(Ts[q + p * (kHbNb + 1)], wv[q], a);
+                        a = group_sum(a, tq);
+                        if (s == 0 && p < i) w2[p] = a;
+                    }
+                }
+                __syncthreads();
+                for (int base = rlo; base + wofs < nr; base += rgrp) {
+                    const int r = base + rofs;
+                    const double a = row_dot(Vs, w2, i, r, 0.0);
+                    if (r < nr && rs == 0) cs[r] -= a;
+                }
+                __syncthreads();
+            }
+            for (int r = tid; r < nr; r += kHbThreads) {
+                const int g = r0 + r;
+                if (g <= j) S.A[g + (size_t)j * S.lda] = cs[r];      // final entries of H
+                else __stcg(S.c + g, cs[r]);
+            }
+            norms_out(j, S.partn);
+        }
+        arrive(0);
+        if (has && i + 1 < P.ib)                                 // the next column, unchanged since the panel began
+            for (int r = tid; r < nr; r += kHbThreads) aj[r] = S.A[r0 + r + (size_t)(j + 1) * S.lda];
+        // This CTA's share of A v: columns [ca, ce) after j + 1 for its row tile.
+        // The first of A are loaded ahead of the barrier, the first of c ahead
+        // of the norm.
+        const int w = n - j - 1, len = (w + P.shares - 1) / P.shares, ca = min(w, share * len), ce = min(w, ca + len);
+        const int rl = tid & (P.rpc - 1), sub = tid / P.rpc, nsub = kHbThreads / P.rpc, r = rt * P.rpc + rl;
+        const bool work = rt < P.tiles && r < n;
+        const int pl0 = min(ce - ca, kHbPiece), sl0 = (pl0 + nsub - 1) / nsub, qa = min(sub * sl0, pl0), qb = min(qa + sl0, pl0);
+        double y0[kHbAhead], cpre[2];
+#pragma unroll
+        for (int e = 0; e < kHbAhead; ++e)
+            y0[e] = work && qa + e < qb ? S.A[r + (size_t)(j + 1 + ca + qa + e) * S.lda] : 0.0;
+        ok = wait(0);
+        if (!ok) break;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int c = tid + e * kHbThreads;
+            cpre[e] = rt < P.tiles && c < pl0 ? __ldcg(S.c + j + 1 + ca + c) : 0.0;
+        }
+        // dlarfg, the same in every CTA.
+        norms_in(j, S.partn);
+        double xnorm = sc[0], alpha = sc[1], beta = sc[2];
+        const double safmin = 0x1p-969, rsafmn = 0x1p+969;       // dlamch('S') / dlamch('E')
+        int knt = 0;
+        if (xnorm != 0.0 && fabs(beta) < safmin) {
+            do {
+                ++knt;
+                for (int r = tid; r < nr; r += kHbThreads)
+                    if (r0 + r >= j + 2) cs[r] = cs[r] * rsafmn;
+                beta = beta * rsafmn;
+                alpha = alpha * rsafmn;
+            } while (fabs(beta) < safmin && knt < 20);
+            for (int r = tid; r < nr; r += kHbThreads)
+                if (r0 + r >= j + 2) __stcg(S.c + r0 + r, cs[r]);
+            double *const again = S.partn + (size_t)3 * P.own;       // the first sums may still be read
+            if (has) norms_out(j, again);
+            arrive(0);
+            ok = wait(0);
+            if (!ok) break;
+            norms_in(j, again);                                  // (alpha as stored is the unscaled one)
+            xnorm = sc[0];
+            beta = -copysign(lapy2(alpha, xnorm), alpha);
+            __syncthreads();
+            if (tid == 0) sc[4] = 1.0 / (alpha - beta);
+            __syncthreads();
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int c = tid + e * kHbThreads;
+                if (rt < P.tiles && c < pl0) cpre[e] = __ldcg(S.c + j + 1 + ca + c);
+            }
+        }
+        const double rsc = sc[4];
+        if (tid == 32) sc[3] = xnorm != 0.0 ? (beta - alpha) / beta : 0.0;       // tau, for after the product
+        if (b == 0 && tid == 0) {
+            for (int q = 0; q < knt; ++q) beta = beta * safmin;
+            S.A[(j + 1) + (size_t)j * S.lda] = beta;
+        }
+        for (int r = tid; r < nr; r += kHbThreads) {
+            const int g = r0 + r;
+            const double v = g == j + 1 ? 1.0 : (g >= j + 2 ? cs[r] * rsc : 0.0);
+            Vs[i * Rp + r] = v;
+            if (g >= j + 1) S.V[g + (size_t)i * n] = v;
+            if (g >= j + 2) S.A[g + (size_t)j * S.lda] = v;
+        }
+        // A v
+        if (rt < P.tiles) {
+            double x = 0.0;                                      // one chain: four warps share a sub-partition
+            for (int p0 = ca; p0 < ce; p0 += kHbPiece) {
+                const int pl = min(ce - p0, kHbPiece), c0 = j + 1 + p0;
+                if (p0 > ca) __syncthreads();
+                for (int c = tid, e = 0; c < pl; c += kHbThreads, ++e) {
+                    const int g = c0 + c;
+                    vst[c] = g == j + 1 ? 1.0 : (p0 == ca ? cpre[e & 1] : __ldcg(S.c + g)) * rsc;
+                }
+                __syncthreads();
+                const int sl = (pl + nsub - 1) / nsub, q0 = min(sub * sl, pl), q1 = min(q0 + sl, pl);
+                if (r < n) {
+                    int q = q0;
+                    if (p0 == ca) {
+#pragma unroll
+                        for (int e = 0; e < kHbAhead; ++e)
+                            if (q + e < q1) x = fma(y0[e], vst[q + e], x);
+                        q = min(q + kHbAhead, q1);
+                    }
+                    const double *a = S.A + r + (size_t)(c0 + q) * S.lda;
+                    for (; q + 15 < q1; q += 16, a += 16 * S.lda) {
+                        double y[16];
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) y[e] = a[(size_t)e * S.lda];
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) x = fma(y[e], vst[q + e], x);
+                    }
+                    if (q < q1) {                                // the rest, its loads in flight together too
+                        double y[15];
+#pragma unroll
+                        for (int e = 0; e < 15; ++e) y[e] = q + e < q1 ? a[(size_t)e * S.lda] : 0.0;
+#pragma unroll
+                        for (int e = 0; e < 15; ++e)
+                            if (q + e < q1) x = fma(y[e], vst[q + e], x);
+                    }
+                }
+            }
+            if (nsub > 1) {
+                gred[tid] = x;
+                __syncthreads();
+                int left = nsub;                                 // by fours, then what is left
+                if (left > 4) {
+                    left /= 4;
+                    if (sub < left) {
+                        x = (x + gred[(sub + left) * P.rpc + rl]) + (gred[(sub + 2 * left) * P.rpc + rl] + gred[(sub + 3 * left) * P.rpc + rl]);
+                        gred[tid] = x;
+                    }
+                    __syncthreads();
+                }
+                if (sub == 0)
+                    for (int z = 1; z < left; ++z) x += gred[z * P.rpc + rl];
+            }
+            if (sub == 0 && r < n) __stcg(S.gpart + (size_t)share * n + r, x);
+        }
+        __syncthreads();
+        t = sc[3];
+        if (b == 0 && tid == 0) S.tau[j] = t;
+        if (has && i > 0) col_dots(Vs + i * Rp, i, S.part2);     // V^T v
+        arrive(0);
+        ok = wait(0);
+        if (!ok) break;
+    }
+    if (!ok) {                                                   // a barrier gave up: results say so
+        if (b == 0) {
+            for (int q = tid; q < n; q += kHbThreads) S.tau[q] = dg_nan();
+            for (int q = tid; q < kHbNb * kHbNb; q += kHbThreads) S.T[q] = dg_nan();
+        }
+        return;
+    }
+    if (b == 0) {
+        __syncthreads();
+        t_column(P.ib - 1, t);
+        __syncthreads();
+        for (int e = tid; e < kHbNb * kHbNb; e += kHbThreads) S.T[e] = Ts[(e % kHbNb) + (e / kHbNb) * (kHbNb + 1)];
+    }
+}
+
 // C(i, j) = beta C(i, j) + alpha sum_k A(i, k) B(k, j) over k in this block's
 // split-K range, with A(i, k) = A[i*sai + k*sak], B(k, j) = B[k*sbk + j*sbj]
 // (one of each pair of strides is 1: loads coalesce along it) and
@@ -946,12 +1386,32 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
     const int nblk = (n + kHbRows - 1) / kHbRows;
     const int maxch = (n + kHbChunk - 1) / kHbChunk;
     const size_t nb = kHbNb;
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // The one-launch panel: CTAs, rows per CTA, rows per tile of A v.
+    // Rows: every CTA with rows adds one part to the sums that each of them
+    // forms, 48 clocks of the FP64 pipe a column, and its own rows cost 80.
+    const int ctas = std::max(1, std::min(sms, (n + 3) / 4));
+    const int R = std::max((n + ctas - 1) / ctas, (int)(n / (1.3 * std::sqrt((double)n)))), own = (n + R - 1) / R;
+    // The lowest row tile that keeps nearly as many CTAs busy as the best one:
+    // fewer column shares, whose parts each row adds up.
+    const auto busy = [&](int h) {
+        const int rt = (n + h - 1) / h;
+        return rt <= ctas ? (long long)(ctas / rt) * n / h : 0LL;
+    };
+    int rpc = 32;
+    long long best = 0;
+    for (int h = 32; h <= kHbThreads; h *= 2) best = std::max(best, busy(h));
+    while (rpc < kHbThreads && 10 * busy(rpc) < 9 * best) rpc *= 2;
+    const int rtiles = (n + rpc - 1) / rpc, shares = std::max(1, ctas / rtiles);
+    const bool one = rtiles <= ctas && hb_panel_smem(R) <= kHbPanelSmem &&
+                     cudaFuncSetAttribute(k_hb_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, kHbPanelSmem) == cudaSuccess;
     const size_t need = 2 * (size_t)n * nb           // Y, V
                         + nb * nb                     // T
                         + (size_t)n                   // c
-                        + 2 * (size_t)nblk * nb       // part, part2
-                        + 3 * (size_t)nblk            // partn
-                        + (size_t)maxch * n           // gpart
+                        + 2 * (size_t)std::max(nblk, ctas) * nb   // part, part2
+                        + 6 * (size_t)std::max(nblk, ctas)        // partn
+                        + std::max((size_t)maxch, (size_t)shares) * n   // gpart
                         + nb + 8                      // sc
                         + (size_t)(kHbMaxSplit + 2) * nb * n   // W partials, W, W2
                         + 4;                          // counters
@@ -965,10 +1425,10 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
     S.V = p; p += (size_t)n * nb;
     S.T = p; p += nb * nb;
     S.c = p; p += n;
-    S.part = p; p += (size_t)nblk * nb;
-    S.part2 = p; p += (size_t)nblk * nb;
-    S.partn = p; p += 3 * (size_t)nblk;
-    S.gpart = p; p += (size_t)maxch * n;
+    S.part = p; p += (size_t)std::max(nblk, ctas) * nb;
+    S.part2 = p; p += (size_t)std::max(nblk, ctas) * nb;
+    S.partn = p; p += 6 * (size_t)std::max(nblk, ctas);
+    S.gpart = p; p += std::max((size_t)maxch, (size_t)shares) * n;
     S.sc = p; p += nb + 8;
     double *Wp = p; p += (size_t)kHbMaxSplit * nb * n;
     double *W = p; p += nb * (size_t)n;
@@ -976,8 +1436,6 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
     S.cnt = reinterpret_cast<unsigned int *>(p);
     S.tau = dtau;
     if (cudaMemsetAsync(S.cnt, 0, 4 * sizeof(double), st) != cudaSuccess) return HSR_ERR_CUDA;
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     static thread_local DgScratch dg;
     HbDigits D{};
     const bool digits = n >= kHbDigitsN && dg.ensure(hb_digits_layout(n, nullptr, D), dev, st);
@@ -994,16 +1452,24 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
         if (ib < kHbNb &&                                        // columns a short panel leaves unwritten
             cudaMemsetAsync(S.Y + (size_t)ib * n, 0, (size_t)(kHbNb - ib) * n * sizeof(double), st) != cudaSuccess)
             return HSR_ERR_CUDA;
-        int nchp = 0;
-        for (int i = 0; i < ib; ++i) {
-            const int j = k0 + i;
-            const int nch = (n - j - 1 + kHbChunk - 1) / kHbChunk;
-            k_hb_step<<<nblk, kHbRows, 0, st>>>(S, k0, i - 1, i, nchp);
-            k_hb_larfg<<<nblk, kHbRows, 0, st>>>(S, k0, i, j);
-            k_hb_gemv<<<dim3(nblk, nch), kHbRows, 0, st>>>(S, k0, i, j);
-            nchp = nch;
+        if (one) {
+            HbPanel pp{S, k0, ib, R, own, rpc, rtiles, shares, S.cnt + 2};
+            void *args[] = {&pp};
+            if (cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_hb_panel), dim3(ctas), dim3(kHbThreads), args,
+                                            hb_panel_smem(R), st) != cudaSuccess)
+                return HSR_ERR_CUDA;
+        } else {
+            int nchp = 0;
+            for (int i = 0; i < ib; ++i) {
+                const int j = k0 + i;
+                const int nch = (n - j - 1 + kHbChunk - 1) / kHbChunk;
+                k_hb_step<<<nblk, kHbRows, 0, st>>>(S, k0, i - 1, i, nchp);
+                k_hb_larfg<<<nblk, kHbRows, 0, st>>>(S, k0, i, j);
+                k_hb_gemv<<<dim3(nblk, nch), kHbRows, 0, st>>>(S, k0, i, j);
+                nchp = nch;
+            }
+            k_hb_step<<<nblk, kHbRows, 0, st>>>(S, k0, ib - 1, -1, nchp);
         }
-        k_hb_step<<<nblk, kHbRows, 0, st>>>(S, k0, ib - 1, -1, nchp);
         const int c1 = k0 + ib, m = n - c1;
         if (m <= 0) continue;
         if (digits) {
