@@ -6,7 +6,9 @@
 // kernels reproduce the CPU oracle's "fma" arithmetic bit for bit.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
+#include <cstring>
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -187,6 +189,95 @@ __device__ __forceinline__ bool ddiv2_rn(double a1, double a2, double b, double 
     return true;
 }
 
+// a / b, correctly rounded.
+__device__ __forceinline__ double ddiv_rn(double a, double b) {
+    const unsigned long long ua = ubits(a), ub = ubits(b);
+    const int ea = (int)((ua >> 52) & 0x7ff), eb = (int)((ub >> 52) & 0x7ff);
+    const unsigned long long fb = ub & kSigMask;
+    if (!ip_div_ok(ea, eb, fb)) return div_fp64(a, b);
+    const unsigned long long mb = fb | kHidden;
+    return from_bits(ip_quot((ua & kSigMask) | kHidden, mb, ip_recip(mb), ea - eb + 1023, (ua ^ ub) & 0x8000000000000000ULL));
+}
+
+// -------------------------------------------- square root, integer pipe
+// An FP64 square root issues about ten FP64 instructions (some 700 cycles).
+// ip_sqrt returns the correctly rounded root of a positive normal u (as bits)
+// and, in y, 2^62 over the root of u's significand z in [1, 4).  With the
+// FP32 approximation y0 of 1 / sqrt(z) and e = 1 - z y0^2 in 60-bit fixed
+// point, y = y0 (1 + e/2 + 3 e^2 / 8) (Householder's iteration of order two,
+// error 5/16 e^3 < 2^-62); s = z y, lowered by the error bound, is the root's
+// floor to 54 bits or one less, which the exact remainder modulo 2^64 decides.
+// The 54th bit rounds: m 2^t with t >= 54 has no root of exactly 54 bits, so
+// there are no ties.
+__host__ __device__ __forceinline__ float rsqrt_approx_f32(float x) {
+#ifdef __CUDA_ARCH__
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+#else
+    return 1.0f / sqrtf(x);
+#endif
+}
+__host__ __device__ __forceinline__ float ip_float_of(unsigned b) {
+#ifdef __CUDA_ARCH__
+    return __uint_as_float(b);
+#else
+    float f;
+    memcpy(&f, &b, 4);
+    return f;
+#endif
+}
+__host__ __device__ __forceinline__ unsigned ip_bits_of(float f) {
+#ifdef __CUDA_ARCH__
+    return __float_as_uint(f);
+#else
+    unsigned b;
+    memcpy(&b, &f, 4);
+    return b;
+#endif
+}
+__host__ __device__ __forceinline__ unsigned long long ip_sqrt(unsigned long long u, unsigned long long &y) {
+    const int ex = (int)(u >> 52), odd = (ex & 1) ^ 1;           // z = m 2^(odd - 52)
+    const unsigned long long m = (u & kSigMask) | kHidden, Z = m << (10 + odd);            // z 2^62
+    const float zf = ip_float_of(((unsigned)(127 + odd) << 23) | ((unsigned)(m >> 29) & 0x7fffffu));
+    const float yf = fmaxf(fminf(rsqrt_approx_f32(zf), 0x1.fffffep-1f), 0.5f);
+    const unsigned y0 = ((ip_bits_of(yf) & 0x7fffffu) | 0x800000u) << 7;                    // 2^31 / sqrt(z)
+    const long long e = (1LL << 60) - (long long)umulhi64(Z, (unsigned long long)y0 * y0);
+    const int e20 = (int)(e >> 20);
+    const long long h = (e >> 1) + ((3LL * ((long long)e20 * e20)) >> 23);
+    const unsigned long long ah = h < 0 ? (unsigned long long)(-h) : (unsigned long long)h;
+    const unsigned long long dy = umulhi64((unsigned long long)y0 << 32, ah << 3);
+    y = ((unsigned long long)y0 << 31) + (h < 0 ? 0ULL - dy : dy);
+    unsigned long long s = (umulhi64(Z, y) - 4) >> 7;
+    const unsigned long long r = (m << (54 + odd)) - s * s;
+    s += r > 2 * s ? 1 : 0;
+    const unsigned long long q = (s >> 1) + (s & 1ULL);
+    return ((unsigned long long)(((ex - 1129 - odd) >> 1) + 1075) << 52) + q;
+}
+// Reciprocal for ip_quot of the root d (bits db, not a power of two) from y.
+__host__ __device__ __forceinline__ unsigned long long ip_recip_root(unsigned long long db, unsigned long long y) {
+    return ip_recip_step((db & kSigMask) | kHidden, y << 2);
+}
+// d = sqrt(ss), q1 = a1 / d and q2 = a2 / d, each correctly rounded, for a
+// positive normal ss; a1 and a2 normal or (quotients near the exponent limits
+// and roots that are powers of two likewise) through the FP64 division.
+__device__ __forceinline__ double dsqrt_div2_rn(double ss, double a1, double a2, double &q1, double &q2) {
+    unsigned long long y;
+    const unsigned long long db = ip_sqrt(ubits(ss), y), fb = db & kSigMask;
+    const unsigned long long u1 = ubits(a1), u2 = ubits(a2);
+    const int e1 = (int)((u1 >> 52) & 0x7ff), e2 = (int)((u2 >> 52) & 0x7ff), eb = (int)(db >> 52);
+    const double d = from_bits(db);
+    if (!ip_div_ok(e1, eb, fb) || !ip_div_ok(e2, eb, fb)) {
+        q1 = div_fp64(a1, d);
+        q2 = div_fp64(a2, d);
+        return d;
+    }
+    const unsigned long long mb = fb | kHidden, rec = ip_recip_root(db, y);
+    q1 = from_bits(ip_quot((u1 & kSigMask) | kHidden, mb, rec, e1 - eb + 1023, u1 & 0x8000000000000000ULL));
+    q2 = from_bits(ip_quot((u2 & kSigMask) | kHidden, mb, rec, e2 - eb + 1023, u2 & 0x8000000000000000ULL));
+    return d;
+}
+
 // ------------------------------------------------ scaling-factor algebra
 // robust.c:24-121.  `is` selects base-2 exponents (INTSCALING) at run time.
 __device__ __forceinline__ double sc_one(bool is) { return is ? 0.0 : 1.0; }
@@ -282,7 +373,7 @@ __device__ __forceinline__ int solve_1x1(double smin, double t, double lambda, d
         info = 1;
     }
     const double alpha = protect_real_division(x, csr);
-    x = scale_by(alpha, x) / csr;
+    x = ddiv_rn(scale_by(alpha, x), csr);
     if (is_one(alpha) && is_one(s)) scale = sc_one(is);
     else scale = solve_1x1_scale(alpha, s, is);
     return info;
@@ -322,8 +413,7 @@ __device__ __forceinline__ void givens(double f, double g, double &c, double &s)
     } else if (mf > kRtminBits && mf < kRtmaxBits && mg > kRtminBits && mg < kRtmaxBits) {
         // c = |f| / d and sv = g / copysign(d, f) = +-(g / d), exactly as the
         // FP64 divisions round them, from one reciprocal of d.
-        const double d = sqrt(f * f + g * g);
-        ddiv2_rn(absd(f), g, d, c, sv);
+        dsqrt_div2_rn(f * f + g * g, absd(f), g, c, sv);
         if (ubits(f) >> 63) sv = neg(sv);
     } else {
         const RotCS r = givens_scaled(f, g);
@@ -511,8 +601,9 @@ __device__ __forceinline__ void c_dladiv(double a, double b, double c, double d,
 }
 // Complex 1x1 solve x := (scale x) / (t - l) (solve_1x1_cmplx_system,
 // robust.c:677-773, with a complex t); returns 1 if |t - l| was lifted to smin.
-__device__ __forceinline__ int csolve_1x1(double smin, double tr, double ti, double lr, double li, dcplx &x,
-                                          double &scale, bool is) {
+// The general form, with every protection evaluated.
+static __device__ __noinline__ int csolve_1x1_full(double smin, double tr, double ti, double lr, double li, dcplx &x,
+                                                   double &scale, bool is) {
     int info = 0;
     const double s = fmin(protect_sum(tr, -lr), protect_sum(ti, -li));
     double csr = (s * tr) - (s * lr);
@@ -527,6 +618,42 @@ __device__ __forceinline__ int csolve_1x1(double smin, double tr, double ti, dou
     scale = is ? (double)ilogb((1.0 / s) * alpha) : (1.0 / s) * alpha;
     return info;
 }
+// The same where no protection can fire and no operand is zero: then every
+// scaling factor is 1, the multiplications and divisions by them are skipped,
+// and what is left are c_dladiv's own operations in its order -- two divisions
+// and ten other FP64 instructions of some sixty.  Magnitudes are compared as
+// bit patterns.  Anything else (zeros, exponents far out, non-finite values)
+// takes the general form.
+__device__ __forceinline__ int csolve_1x1(double smin, double tr, double ti, double lr, double li, dcplx &x,
+                                          double &scale, bool is) {
+    const unsigned long long lim = pow2_bits(200);
+    const unsigned long long xa = mag(x.re), xb = mag(x.im);
+    if (mag(tr) < lim && mag(ti) < lim && mag(lr) < lim && mag(li) < lim && xa < lim && xb < lim) {
+        double csr = tr - lr, csi = ti - li;
+        int info = 0;
+        if (ubits(absd(csr) + absd(csi)) < ubits(smin)) {
+            csr = smin;
+            csi = 0.0;
+            info = 1;
+        }
+        const bool swap = mag(csi) >= mag(csr);                  // c_dladiv's choice
+        const double a = swap ? x.im : x.re, b = swap ? x.re : x.im, c = swap ? csi : csr, d = swap ? csr : csi;
+        // d = 0 (r = 0) and a vanishing numerator part take other branches there.
+        if (mag(d) > pow2_bits(-200) && xa > pow2_bits(-400) && xb > pow2_bits(-400)) {
+            const double r = ddiv_rn(d, c), sum = c + d * r;
+            const double ar = neg(a) * r, br = b * r;
+            const double p = a + br, q = b + ar;
+            // |sum| >= |c| >= |d| > 2^-200 and |r| > 2^-401: every protected
+            // quantity is far inside its bound, and neither product is 0.
+            const double t = ddiv_rn(1.0, sum);
+            x.re = p * t;
+            x.im = swap ? neg(q * t) : q * t;
+            scale = sc_one(is);
+            return info;
+        }
+    }
+    return csolve_1x1_full(smin, tr, ti, lr, li, x, scale, is);
+}
 
 // Complex Givens rotation of (f, g), f complex, g real: c real >= 0 and
 // sigma with sigma f + c g = 0.  Exact power-of-two scaling: the phase of f
@@ -538,17 +665,7 @@ __device__ __forceinline__ int exp_clamped(double m) {
     return e > 1000 ? 1000 : (e < -1000 ? -1000 : e);
 }
 __device__ __forceinline__ double pow2d(int e) { return __longlong_as_double((long long)pow2_bits(e)); }
-__device__ __forceinline__ void cgivens(dcplx f, double g, double &c, dcplx &sg) {
-    if (is_zero(g)) {
-        c = 1.0;
-        sg = cmk(0.0, 0.0);
-        return;
-    }
-    if (is_zero(f.re) && is_zero(f.im)) {
-        c = 0.0;
-        sg = cmk(-copysign(1.0, g), 0.0);
-        return;
-    }
+static __device__ __noinline__ void cgivens_full(dcplx f, double g, double &c, dcplx &sg) {
     const int ef = exp_clamped(fmax(absd(f.re), absd(f.im)));
     const int eg = exp_clamped(absd(g));
     const int e = ef > eg ? ef : eg;
@@ -562,6 +679,35 @@ __device__ __forceinline__ void cgivens(dcplx f, double g, double &c, dcplx &sg)
     c = af / d;
     const double t = gs / d;
     sg = cmk(-(t * pr), t * pi);
+}
+// With exponents within +-200 the scalings by powers of two are exponent
+// additions, and the two roots and four quotients run on the integer pipe:
+// the same bits, six FP64 instructions instead of some seventy.
+__device__ __forceinline__ double add_exp(double x, int e) { return from_bits(ubits(x) + ((unsigned long long)(long long)e << 52)); }
+__device__ __forceinline__ void cgivens(dcplx f, double g, double &c, dcplx &sg) {
+    if (is_zero(g)) {
+        c = 1.0;
+        sg = cmk(0.0, 0.0);
+        return;
+    }
+    if (is_zero(f.re) && is_zero(f.im)) {
+        c = 0.0;
+        sg = cmk(-copysign(1.0, g), 0.0);
+        return;
+    }
+    const unsigned long long mr = mag(f.re), mi = mag(f.im), mg = mag(g);
+    const unsigned long long lo = pow2_bits(-200), hi = pow2_bits(200);
+    if (mr > lo && mr < hi && mi > lo && mi < hi && mg > lo && mg < hi) {
+        const int ef = (int)(umax64(mr, mi) >> 52) - 1023, eg = (int)(mg >> 52) - 1023, e = ef > eg ? ef : eg;
+        const double fsr = add_exp(f.re, -ef), fsi = add_exp(f.im, -ef);
+        double pr, pi, t;
+        const double af1 = dsqrt_div2_rn(fma(fsr, fsr, fsi * fsi), fsr, fsi, pr, pi);
+        const double af = add_exp(af1, ef - e), gs = add_exp(g, -e);
+        dsqrt_div2_rn(fma(af, af, gs * gs), af, gs, c, t);
+        sg = cmk(neg(t * pr), t * pi);
+        return;
+    }
+    cgivens_full(f, g, c, sg);
 }
 
 // ------------------------------------------------ mbarrier + TMA (PTX)
