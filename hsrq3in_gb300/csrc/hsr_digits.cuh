@@ -275,9 +275,6 @@ __device__ __forceinline__ void dg_ld(uint32_t addr, float (&v)[16]) {
 __device__ __forceinline__ void dg_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void dg_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void dg_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void dg_arrive(uint64_t *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 __device__ __forceinline__ void dg_bulk(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
     asm volatile(
         "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -559,7 +556,7 @@ k_dg_gemm(const unsigned char *__restrict__ A, const unsigned char *__restrict__
                     dg_wait_ld();
                     dg_fence_before();
                     __syncwarp();
-                    if (lane == 0) dg_arrive(&acc_empty[g]);
+                    if (lane == 0) mbar_arrive(&acc_empty[g]);
                     // Groups 0 .. 5 are exact integers in units of 2^(-12 - 8 g).
 #pragma unroll
                     for (int c = 0; c < kCols; ++c) sum.add(g, c, v[c]);

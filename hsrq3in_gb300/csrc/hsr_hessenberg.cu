@@ -564,7 +564,17 @@ __global__ void __launch_bounds__(kHbThreads, 1) k_hb_panel(HbPanel P) {
                     const int r = base + rofs;
                     double av = 0.0;
                     if (r < nr) {
-                        for (int c = rs; c < P.shares; c += tpr) av += __ldcg(S.gpart + (size_t)c * n + r0 + r);
+                        for (int c = rs; c < P.shares; c += 4 * tpr) {
+                            double x[4];
+#pragma unroll
+                            for (int e = 0; e < 4; ++e)
+                                x[e] = base == 0 && c == rs      ? g0[e]
+                                       : c + e * tpr < P.shares ? __ldcg(S.gpart + (size_t)(c + e * tpr) * n + r0 + r)
+                                                                : 0.0;
+#pragma unroll
+                            for (int e = 0; e < 4; ++e)
+                                if (c - rs + e * tpr < P.shares) av += x[e];     // uniform over the warp
+                        }
                     }
                     const double y = t * row_dot(Ys, vv, ip, r, av);
                     if (r < nr && rs == 0) {
@@ -1200,7 +1210,6 @@ struct HbPanelCols {
         if (i >= n) return 0.0;
         return r < kHbNb ? Y[i + (size_t)r * n] : V[i + (size_t)(r - kHbNb) * n];
     }
-    __device__ __forceinline__ int first(int) const { return 0; }
 };
 struct HbVCols {
     const double *V;

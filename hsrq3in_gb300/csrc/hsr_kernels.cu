@@ -198,11 +198,9 @@ cudaError_t launch_init(const DevProblem &P, int mode, const double *eps3_dev, i
 constexpr int kDiagWarps = 4;     // single-problem path, v/y in global scratch
 constexpr int kDiagWarpsSmem = 8; // single-problem path, v/y in shared memory
 constexpr int kDiagWarpsB = 1;    // batched path
-// Single-problem path, 8 or 16 shifts per CTA: three warps (the chain and
-// two row warps) need 3 x 32 x 120 registers, which fit beside the two
-// 256-thread CTAs of the concurrent GEMM on one SM (a fourth warp would not,
-// and the diagonal CTA would wait for a GEMM CTA to finish).
-constexpr int kDiagWarpsNarrow = 3;
+// Single-problem path, 8 or 16 shifts per CTA: the rotation's chain, the
+// solve's chain and six row warps (diag_body_narrow).
+constexpr int kDiagWarpsNarrow = 8;
 
 constexpr int kDiagBcast = 8;      // per-lane step results broadcast by warp 0
 // Staging buffers for columns of H: the pipelined multi-warp body keeps three
@@ -917,34 +915,50 @@ __device__ __forceinline__ unsigned long long gemm_epilogue_elem(const DevProble
 }
 
 // Narrow form of the pipelined body for solves with few shifts: SC (< 32)
-// shifts per CTA, so that a small shift count still spreads over many SMs.
-// The scalar chain of each step runs on warp 0, lane s (and its duplicates
-// s + SC, s + 2 SC, ..., which compute the same values and store nothing);
-// the row warps 1 .. NW-1 hold RL = 32 / SC rows x SC shifts per
-// instruction, so a step's vector work takes RL times fewer instructions than
-// with a lane per shift.  Every (row, shift) element sees the same operations
-// in the same order as in diag_body_pipe, and the maxima cover the same rows
-// (a maximum does not depend on the order it is taken in), so the result is
-// bit-identical to the wide form.  v/y live in shared memory as [row][SC].
+// shifts per CTA, so that a small shift count still spreads over many SMs, and
+// the step's serial chain split over two warps.  The rotation of a step
+// depends on the running column v alone, so
+//   warp 0 (lane s and its duplicates s + SC, ... of shift s) runs the Givens
+//     chain: rotation j, then rows j-1 and j-2 of v, one group of lanes each;
+//     the two quotients of the rotation, two group's worth of work, likewise;
+//   warp 4 (sub-partition 0 too) runs the solve chain one step behind: the
+//     1x1 solve, the decisions, rows j-1 and j-2 of y;
+//   warps 1-3 and 5-7 update rows 0 .. j-3 of v and y, 32 / SC rows x SC
+//     shifts per instruction.
+// Rotation j-1 runs while the rows of step j are updated.  Three mbarriers
+// carry the step: the rotation is there, the solve's factors are there, the
+// rows are done.  Every (row, shift) element sees the same operations in the
+// same order as in diag_body_pipe, so the result is bit-identical to the wide
+// form.  For the third decision the row warps fold the high words of |y| and
+// |v|; only where those do not already show that it cannot fire does warp 4
+// take the maxima themselves, over the rows in shared memory (a maximum does
+// not depend on the order it is taken in).  v and y live in shared memory as
+// [row][SC].
+//
+// Bound by the two chains' latency (rotation about 900 clocks, solve 700) and
+// by the rows' FP64 issue, 4 instructions of 64 clocks per 32 / SC rows on
+// three sub-partitions.  With one chain warp, two row warps and two block
+// barriers a step: %%DIAG%%
+constexpr int kNarrowRowWarps = 6;
 template <int SC>
-__host__ __device__ constexpr size_t diag_narrow_smem_bytes(int b, int nw) {
-    return (size_t)(3 * (b + 1) + nw * 2 * SC + kDiagBcast * SC + 2 * SC * b) * sizeof(double);
+__host__ __device__ constexpr size_t diag_narrow_smem_bytes(int b) {
+    return (size_t)(4 * (b + 2) + (2 * 4 + 2 * 5) * SC + 8 * SC + 2 * SC * b) * sizeof(double);
 }
 
-template <int SC, int NW>
+template <int SC>
 __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int bx) {
-    static_assert(32 % SC == 0 && SC >= 4 && SC < 32, "shifts per CTA");
-    static_assert(NW >= 2, "a chain warp and at least one row warp");
+    static_assert(SC == 8 || SC == 16, "shifts per CTA");
+    constexpr int NW = kDiagWarpsNarrow, NR = kNarrowRowWarps;
+    static_assert(NW == 8, "two chain warps on sub-partition 0, six row warps");
     constexpr int RL = 32 / SC;                                               // rows per row-warp instruction
-    // Warps w = 0, 4, ... share sub-partition 0, whose FP64 unit the scalar
-    // chain (warp 0) needs to itself: rows go to the other warps only.
-    constexpr int NR = NW - (NW + 3) / 4;                                     // row warps
     extern __shared__ double sm[];
+    __shared__ __align__(8) uint64_t bars[5];                                 // rotation x 2, rows x 2, factors
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int wid = tid >> 5;
     const int sh = lane % SC;                                                 // shift slot
-    const int rs = lane / SC;                                                 // row slot (row warps)
+    const int rs = lane / SC;                                                 // row slot, lane group
+    const bool odd = (rs & 1) != 0;                                           // which of two values the group takes
     const bool store_lane = lane < SC;                                        // chain results are stored once
     const bool row_warp = (wid & 3) != 0;
     const int rw = wid - 1 - wid / 4;                                         // row-warp index, 0 .. NR-1
@@ -955,17 +969,27 @@ __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int
     const bool is = P.is != 0;
     const size_t Spad = (size_t)P.Spad;
 
-    double *hc = sm;                                                          // [3][b+1]
-    unsigned long long *pm = reinterpret_cast<unsigned long long *>(sm + 3 * (b + 1));   // [NW][2][SC]
-    double *bc = sm + 3 * (b + 1) + NW * 2 * SC;                              // [kDiagBcast][SC]
-    double *v = bc + kDiagBcast * SC;                                         // [b][SC]
+    double *hc = sm;                                                          // [4][b+2]
+    double *sa = sm + 4 * (b + 2);                                            // [2][4][SC]: c, s, v(j), v(j-1)
+    double *sb = sa + 2 * 4 * SC;                                             // [2][5][SC]: yc, ys, a1, a2, a3
+    unsigned *pm = reinterpret_cast<unsigned *>(sb + 2 * 5 * SC);             // [NR][2][SC], high words
+    double *v = sb + 2 * 5 * SC + 8 * SC;                                     // [b][SC]
     double *y = v + (size_t)SC * b;                                           // [b][SC]
 #define V(i) v[(size_t)(i) * SC + sh]
 #define Y(i) y[(size_t)(i) * SC + sh]
 #define PM(w, which) pm[(((w) * 2) + (which)) * SC + sh]
-#define BC(q) bc[(q) * SC + sh]
-#define HCOL(col) (hc + (size_t)((col) % 3) * (b + 1))
+#define SA(t, q) sa[((((t) & 1) * 4) + (q)) * SC + sh]
+#define SB(t, q) sb[((((t) & 1) * 5) + (q)) * SC + sh]
+#define HCOL(col) (hc + (size_t)((col) & 3) * (b + 2))
 
+    if (tid == 0) {
+        mbar_init(&bars[0], 1);
+        mbar_init(&bars[1], 1);
+        mbar_init(&bars[2], NR);
+        mbar_init(&bars[3], NR);
+        mbar_init(&bars[4], 1);
+        mbar_fence_init();
+    }
     for (int idx = tid; idx < SC * b; idx += 32 * NW) {
         const int c = idx / b, i = idx - c * b;
         const int kc = k0 + c;
@@ -977,172 +1001,209 @@ __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int
             y[(size_t)i * SC + c] = 0.0;
         }
     }
-
     const double mu = act ? P.wr[k] : 0.0;
     const double smin = fmax(DBL_EPSILON / 2 * absd(mu), P.smlnum);
-    const double Hnorm = P.Hn[J + (size_t)J * P.T];
     double beta = act ? P.beta[(size_t)J * Spad + k] : sc_one(is);
     int pert = 0;
-
     const double *Hd = P.H + l + (size_t)l * P.ldh;                           // H(l, l)
     auto stage_col = [&](int col) {                                           // H(l : l+col+1, l+col), warp 0
-        int rows = col + 2;
-        if (rows > b) rows = b;
-        const double *src = Hd + (size_t)col * P.ldh;
-        double *dst = HCOL(col);
-        for (int i = lane; i < rows; i += 32) cp_async8(dst + i, src + i);
-        cp_async_commit();
-    };
-    if (wid == 0 && b >= 2) stage_col(b - 2);
-    if (wid == 0 && b >= 3) stage_col(b - 3);
-    if (wid == 0) cp_async_wait_all();
-    __syncthreads();                                                          // tiles and columns loaded
-
-    // Maxima over the RL row slots of one shift (lanes sh, sh + SC, ...).
-    auto slot_max = [&](unsigned long long m) {
-#pragma unroll
-        for (int o = SC; o < 32; o <<= 1) m = umax64(m, __shfl_xor_sync(0xffffffffu, m, o));
-        return m;
-    };
-    // Maxima of |y(0:b-3)| and |v(0:b-3)| for the first step, by the row warps.
-    {
-        unsigned long long ym = 0, vm = 0;
-        if (row_warp)
-            for (int i = rw * RL + rs; i < b - 2; i += NR * RL) {
-                ym = umax64(ym, abs_bits(Y(i)));
-                vm = umax64(vm, abs_bits(V(i)));
-            }
-        ym = slot_max(ym);
-        vm = slot_max(vm);
-        if (store_lane) {
-            PM(wid, 0) = ym;
-            PM(wid, 1) = vm;
+        if (col >= 0) {
+            const int rows = min(col + 2, b);
+            const double *src = Hd + (size_t)col * P.ldh;
+            double *dst = HCOL(col);
+            for (int i = lane; i < rows; i += 32) cp_async8(dst + i, src + i);
         }
+        cp_async_commit();                                                    // one group per column, empty ones too
+    };
+    if (wid == 0) {
+        stage_col(b - 2);
+        stage_col(b - 3);
     }
+    __syncthreads();                                                          // tile and barriers ready
 
-    // Chain state of warp 0.
-    double vcar = V(b - 1), ycar = Y(b - 1);
-    double c = 0.0, s = 0.0, yc = 0.0, ys = 0.0, a1 = 1.0, a2 = 1.0, a3 = 1.0, yj = 0.0, yjm1 = 0.0;
-
-    auto chain12 = [&](int jj, double vjm1, double yjm1_in) {
-        const double *hcol = HCOL(jj - 1);
-        const double hsub = hcol[jj];
-        const double hdiag = hcol[jj - 1] - mu;
-        const double vj = vcar;
-        yj = ycar;
-        yjm1 = yjm1_in;
-        givens(vj, hsub, c, s);
-        if (act && store_lane) {
-            P.Cr[(size_t)(l + jj) * Spad + k] = c;
-            P.Sr[(size_t)(l + jj) * Spad + k] = s;
-        }
-        double phi = sc_one(is);
-        pert |= solve_1x1(smin, c * vj, s * hsub, yj, phi, is);
-        beta = sc_combine(beta, phi, is);
-        a1 = sc_value(phi, is);
-        yjm1 = scale_by(a1, yjm1);
-        phi = protect_double_update(absd(vjm1), absd(yj), absd(hdiag), absd(yj), absd(yjm1), is);
-        a2 = sc_value(phi, is);
-        if (!is_one(a2)) {
-            yj = mul_rare(a2, yj);
-            yjm1 = mul_rare(a2, yjm1);
-        }
-        beta = sc_combine(beta, phi, is);
-        yc = yj * c;
-        ys = yj * s;
-        yjm1 = fma(ys, hdiag, fma(-yc, vjm1, yjm1));
-        vcar = fma(c, hdiag, s * vjm1);
+    // Step t's barriers (t = b - 1 - j).  The rotation and the rows alternate
+    // between two, so that neither can complete the phase after the one that
+    // a late warp still has to wait for; the factors of step t + 1 follow the
+    // rows of step t, which every row warp ends after its wait for step t's.
+    // A wait that runs out is recorded; the warp then waits no more.
+    constexpr int kRot = 0, kRows = 2, kFac = 4;
+    bool ok = true;
+    auto await = [&](int which, int t) {
+        ok = ok && mbar_wait(&bars[which == kFac ? kFac : which + (t & 1)], (uint32_t)(which == kFac ? t & 1 : (t >> 1) & 1), P.err);
     };
-    auto chain3 = [&](int jj) {
-        unsigned long long ymb = 0, vmb = 0;
+    auto post = [&](int which, int t) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars[which == kFac ? kFac : which + (t & 1)]);
+    };
+    const unsigned hi497 = (unsigned)(pow2_bits(497) >> 32), hi995 = (unsigned)(pow2_bits(995) >> 32);
+    auto hi_mag = [](double x) { return (unsigned)(ubits(x) >> 32) & 0x7fffffffu; };
+
+    double v0 = 0.0, y0 = 0.0;                                                // rows 0 of v (warp 0) and y (warp 4)
+    if (wid == 0) {
+        double vj = V(b - 1), vw = b >= 2 ? V(b - 2) : 0.0;                   // v(j); v(j-1)
+        for (int j = b - 1, t = 0; j >= 1; --j, ++t) {
+            cp_async_wait_one();                                              // column j-1
+            __syncwarp();
+            const double *hcol = HCOL(j - 1);
+            const double hsub = hcol[j], hdiag = hcol[j - 1] - mu;
+            double c, s;
+            {
+                // As givens(), the squares and the quotients of f and g on
+                // two lane groups.
+                const unsigned long long mf = mag(vj), mg = mag(hsub);
+                bool fast = mf > kRtminBits && mf < kRtmaxBits && mg > kRtminBits && mg < kRtmaxBits;
+                const double fg = odd ? hsub : vj, sq = fg * fg;
+                const double ss = __shfl_sync(0xffffffffu, sq, sh) + __shfl_sync(0xffffffffu, sq, sh + SC);
+                unsigned long long yr;
+                const unsigned long long db = ip_sqrt(fast ? ubits(ss) : kOneBits + 1, yr), fb = db & kSigMask;
+                const int eb = (int)(db >> 52);
+                const unsigned long long num = odd ? ubits(hsub) : mf;
+                const int en = (int)((num >> 52) & 0x7ff);
+                fast = fast && ip_div_ok(en, eb, fb);
+                if (__all_sync(0xffffffffu, fast)) {
+                    const double q = from_bits(ip_quot((num & kSigMask) | kHidden, fb | kHidden, ip_recip_root(db, yr),
+                                                       en - eb + 1023, num & 0x8000000000000000ULL));
+                    c = __shfl_sync(0xffffffffu, q, sh);
+                    s = __shfl_sync(0xffffffffu, q, sh + SC);
+                    if (!(ubits(vj) >> 63)) s = neg(s);
+                } else {
+                    givens(vj, hsub, c, s);
+                }
+            }
+            if (store_lane) {
+                SA(t, 0) = c;
+                SA(t, 1) = s;
+                SA(t, 2) = vj;
+                SA(t, 3) = vw;
+            }
+            post(kRot, t);
+            if (act && store_lane) {
+                P.Cr[(size_t)(l + j) * Spad + k] = c;
+                P.Sr[(size_t)(l + j) * Spad + k] = s;
+            }
+            await(kRows, t);                                                      // rows of step j+1: row j-2 is in V
+            const double h = !odd ? hdiag : (j >= 2 ? hcol[j - 2] : 0.0);
+            const double vo = !odd ? vw : (j >= 2 ? V(j - 2) : 0.0);
+            const double vn = fma(c, h, s * vo);
+            vj = __shfl_sync(0xffffffffu, vn, sh);
+            vw = __shfl_sync(0xffffffffu, vn, sh + SC);
+            stage_col(j - 3);                                                 // over column j+1
+        }
+        v0 = vj;
+    } else if (wid == 4) {
+        const double Hnorm = P.Hn[J + (size_t)J * P.T];
+        double ycar = Y(b - 1), ynext = b >= 2 ? Y(b - 2) : 0.0;              // y(j), y(j-1)
+        for (int j = b - 1, t = 0; j >= 1; --j, ++t) {
+            await(kRot, t);
+            const double *hcol = HCOL(j - 1);
+            const double c = SA(t, 0), s = SA(t, 1), vjm1 = SA(t, 3);
+            const double hdiag = hcol[j - 1] - mu;
+            double yj = ycar, yjm1 = ynext;
+            const double pr = (odd ? s : c) * (odd ? hcol[j] : SA(t, 2));     // c v(j), s H(j, j-1)
+            double phi = sc_one(is);
+            pert |= solve_1x1(smin, __shfl_sync(0xffffffffu, pr, sh), __shfl_sync(0xffffffffu, pr, sh + SC), yj, phi, is);
+            beta = sc_combine(beta, phi, is);
+            const double a1 = sc_value(phi, is);
+            yjm1 = scale_by(a1, yjm1);
+            phi = protect_double_update(absd(vjm1), absd(yj), absd(hdiag), absd(yj), absd(yjm1), is);
+            const double a2 = sc_value(phi, is);
+            if (!is_one(a2)) {
+                yj = mul_rare(a2, yj);
+                yjm1 = mul_rare(a2, yjm1);
+            }
+            beta = sc_combine(beta, phi, is);
+            const double py = yj * (odd ? s : c);
+            double yc = __shfl_sync(0xffffffffu, py, sh), ys = __shfl_sync(0xffffffffu, py, sh + SC);
+            yjm1 = fma(ys, hdiag, fma(-yc, vjm1, yjm1));
+            await(kRows, t);                                                      // rows of step j+1
+            unsigned ymh = 0, vmh = 0;
 #pragma unroll
-        for (int w = 1; w < NW; ++w) {
-            ymb = umax64(ymb, PM(w, 0));
-            vmb = umax64(vmb, PM(w, 1));
-        }
-        double ymax = from_bits(ymb);
-        if (!is_one(a1)) ymax = from_bits(abs_bits(mul_rare(a1, ymax)));
-        if (!is_one(a2)) ymax = from_bits(abs_bits(mul_rare(a2, ymax)));
-        const double phi = protect_double_update(from_bits(vmb), absd(yj), Hnorm, absd(yj), ymax, is);
-        a3 = sc_value(phi, is);
-        if (!is_one(a3)) {
-            yj = mul_rare(a3, yj);
-            yjm1 = mul_rare(a3, yjm1);
-            yc = mul_rare(yj, c);
-            ys = mul_rare(yj, s);
-        }
-        beta = sc_combine(beta, phi, is);
-        if (store_lane) {
-            BC(0) = c;
-            BC(1) = s;
-            BC(2) = yc;
-            BC(3) = ys;
-            BC(4) = a1;
-            BC(5) = a2;
-            BC(6) = a3;
-            Y(jj) = yj;
-        }
-        ycar = yjm1;
-    };
-
-    if (wid == 0 && b >= 2) chain12(b - 1, V(b - 2), Y(b - 2));
-    __syncthreads();                                                          // first maxima in
-    if (wid == 0 && b >= 2) chain3(b - 1);
-    __syncthreads();                                                          // step b-1's scalars visible
-
-    for (int j = b - 1; j >= 1; --j) {
-        double sc_c = c, sc_s = s, sc_yc = yc, sc_ys = ys, s1 = a1, s2 = a2, s3 = a3;
-        if (wid != 0) {
-            sc_c = BC(0);
-            sc_s = BC(1);
-            sc_yc = BC(2);
-            sc_ys = BC(3);
-            s1 = BC(4);
-            s2 = BC(5);
-            s3 = BC(6);
-        }
-        const bool scaled = (!is_one(s1)) || (!is_one(s2)) || (!is_one(s3));
-        const double *hcol = HCOL(j - 1);
-        if (wid == 0) {
-            // Row j-2 first: it enters step j-1's chain.
-            double vn = 0.0, yn = 0.0;
-            if (j >= 2) {
-                const double h = hcol[j - 2];
-                double yi = Y(j - 2);
-                const double vi = V(j - 2);
-                if (scaled) {
-                    yi = scale_by(s1, yi);
-                    yi = scale_by(s2, yi);
-                    yi = scale_by(s3, yi);
+            for (int w = 0; w < NR; ++w) {
+                ymh = max(ymh, PM(w, 0));
+                vmh = max(vmh, PM(w, 1));
+            }
+            double a3 = 1.0;
+            phi = sc_one(is);
+            if (!(ymh < hi995 && vmh < hi497 && hi_mag(yj) < hi497 && hi_mag(Hnorm) < hi497 && is_one(a1) && is_one(a2))) {
+                unsigned long long ymb = 0, vmb = 0;                          // the maxima over rows 0 .. j-2
+                for (int i = 0; i <= j - 2; ++i) {
+                    ymb = umax64(ymb, abs_bits(Y(i)));
+                    vmb = umax64(vmb, abs_bits(V(i)));
                 }
-                yn = fma(sc_ys, h, fma(-sc_yc, vi, yi));
-                vn = fma(sc_c, h, sc_s * vi);
-                __syncwarp();                                                 // every lane read row j-2
-                if (store_lane) {
-                    Y(j - 2) = yn;
-                    V(j - 2) = vn;
+                double ymax = from_bits(ymb);
+                if (!is_one(a1)) ymax = from_bits(abs_bits(mul_rare(a1, ymax)));
+                if (!is_one(a2)) ymax = from_bits(abs_bits(mul_rare(a2, ymax)));
+                phi = protect_double_update(from_bits(vmb), absd(yj), Hnorm, absd(yj), ymax, is);
+                a3 = sc_value(phi, is);
+                if (!is_one(a3)) {
+                    yj = mul_rare(a3, yj);
+                    yjm1 = mul_rare(a3, yjm1);
+                    yc = mul_rare(yj, c);
+                    ys = mul_rare(yj, s);
                 }
             }
-            if (j >= 2) {
-                cp_async_wait_all();                                          // column j-2, staged last step
-                __syncwarp();                                                 // ... by all lanes of warp 0
-                chain12(j - 1, vn, yn);
+            beta = sc_combine(beta, phi, is);
+            const double yi0 = j >= 2 ? Y(j - 2) : 0.0, vi = j >= 2 ? V(j - 2) : 0.0;
+            if (store_lane) {
+                SB(t, 0) = yc;
+                SB(t, 1) = ys;
+                SB(t, 2) = a1;
+                SB(t, 3) = a2;
+                SB(t, 4) = a3;
+                Y(j) = yj;
             }
-            if (j >= 3) stage_col(j - 3);                                     // for step j-2's chain
-        } else if (row_warp) {
-            if (scaled) {
-                for (int i = j + 1 + rw * RL + rs; i < b; i += NR * RL) {
-                    double t = Y(i);
-                    t = scale_by(s1, t);
-                    t = scale_by(s2, t);
-                    t = scale_by(s3, t);
-                    Y(i) = t;
-                }
+            post(kFac, t);
+            // Row j-2 of y, for the next step's chain.
+            double yi = yi0;
+            if (!is_one(a1) || !is_one(a2) || !is_one(a3)) {
+                yi = scale_by(a1, yi);
+                yi = scale_by(a2, yi);
+                yi = scale_by(a3, yi);
             }
-            unsigned long long ymx = 0, vmx = 0;
+            ynext = j >= 2 ? fma(ys, hcol[j - 2], fma(-yc, vi, yi)) : 0.0;
+            ycar = yjm1;
+        }
+        y0 = ycar;
+    } else {
+        // High words of the first step's bounds, then the rows of every step.
+        unsigned ym = 0, vm = 0;
+        for (int i = rw * RL + rs; i < b - 2; i += NR * RL) {
+            ym = max(ym, hi_mag(Y(i)));
+            vm = max(vm, hi_mag(V(i)));
+        }
+        auto fold = [&](unsigned ymx, unsigned vmx) {
+#pragma unroll
+            for (int o = SC; o < 32; o <<= 1) {
+                ymx = max(ymx, __shfl_xor_sync(0xffffffffu, ymx, o));
+                vmx = max(vmx, __shfl_xor_sync(0xffffffffu, vmx, o));
+            }
+            if (store_lane) {
+                PM(rw, 0) = ymx;
+                PM(rw, 1) = vmx;
+            }
+        };
+        fold(ym, vm);
+        post(kRows, 0);
+        for (int j = b - 1, t = 0; j >= 1; --j, ++t) {
+            await(kRot, t);
+            const double sc_c = SA(t, 0), sc_s = SA(t, 1);
+            const double *hcol = HCOL(j - 1);
             const int lim = j - 2;                                            // rows 0 .. j-3
-            int i = rw * RL + rs;
             constexpr int ST = NR * RL;                                       // row stride of one lane
+            int i = rw * RL + rs;
+            await(kFac, t);
+            const double sc_yc = SB(t, 0), sc_ys = SB(t, 1), s1 = SB(t, 2), s2 = SB(t, 3), s3 = SB(t, 4);
+            const bool scaled = !is_one(s1) || !is_one(s2) || !is_one(s3);
+            if (scaled) {
+                for (int q = j + 1 + rw * RL + rs; q < b; q += NR * RL) {
+                    double u = Y(q);
+                    u = scale_by(s1, u);
+                    u = scale_by(s2, u);
+                    u = scale_by(s3, u);
+                    Y(q) = u;
+                }
+            }
+            ym = vm = 0;
             for (; i + 3 * ST < lim; i += 4 * ST) {
                 double hh[4], yy[4], vv[4];
 #pragma unroll
@@ -1166,11 +1227,10 @@ __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int
                 }
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const int r = i + q * ST;
-                    Y(r) = yy[q];
-                    V(r) = vv[q];
-                    ymx = umax64(ymx, abs_bits(yy[q]));
-                    vmx = umax64(vmx, abs_bits(vv[q]));
+                    Y(i + q * ST) = yy[q];
+                    V(i + q * ST) = vv[q];
+                    ym = max(ym, hi_mag(yy[q]));
+                    vm = max(vm, hi_mag(vv[q]));
                 }
             }
             for (; i < lim; i += ST) {
@@ -1185,62 +1245,53 @@ __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int
                 vi = fma(sc_c, h, sc_s * vi);
                 Y(i) = yi;
                 V(i) = vi;
-                ymx = umax64(ymx, abs_bits(yi));
-                vmx = umax64(vmx, abs_bits(vi));
+                ym = max(ym, hi_mag(yi));
+                vm = max(vm, hi_mag(vi));
             }
-            ymx = slot_max(ymx);
-            vmx = slot_max(vmx);
-            if (store_lane) {
-                PM(wid, 0) = ymx;
-                PM(wid, 1) = vmx;
-            }
+            fold(ym, vm);
+            post(kRows, t + 1);
         }
-        __syncthreads();                                                      // rows of step j done, maxima in
-        if (wid == 0 && j >= 2) chain3(j - 1);
-        __syncthreads();                                                      // step j-1's scalars visible
     }
+    __syncthreads();                                                          // the last step's rows written
 
     double c0 = 0.0, s0 = 0.0;
+    if (wid == 0) {
+        if (J > 0) {
+            // Final rotation with H(l, l-1) (reduce.c:53-61, solve-task.c:111-118).
+            const double hleft = P.H[l + (size_t)(l - 1) * P.ldh];
+            if (hleft != 0) {
+                givens(v0, hleft, c0, s0);
+            } else {
+                c0 = 1.0;
+                s0 = 0.0;
+            }
+            if (act && store_lane) {
+                P.Cr[(size_t)l * Spad + k] = c0;
+                P.Sr[(size_t)l * Spad + k] = s0;
+            }
+            v0 = fma(v0, c0, -(hleft * s0));
+        }
+        if (store_lane) {
+            SA(0, 0) = c0;
+            SA(0, 1) = s0;
+            SA(0, 2) = v0;
+        }
+    }
+    __syncthreads();
+    c0 = SA(0, 0);
+    s0 = SA(0, 1);
+    if (wid == 4) {
+        double phi = sc_one(is);
+        pert |= solve_1x1(smin, SA(0, 2), 0.0, y0, phi, is);
+        beta = sc_combine(beta, phi, is);
+        if (store_lane) SB(0, 2) = sc_value(phi, is);
+    }
+    __syncthreads();
     {
-        double y0 = 0.0, a = 1.0;
-        if (wid == 0) {
-            double v0 = b >= 2 ? vcar : V(0);
-            y0 = b >= 2 ? ycar : Y(0);
-            if (J > 0) {
-                // Final rotation with H(l, l-1) (reduce.c:53-61, solve-task.c:111-118).
-                const double hleft = P.H[l + (size_t)(l - 1) * P.ldh];
-                if (hleft != 0) {
-                    givens(v0, hleft, c0, s0);
-                } else {
-                    c0 = 1.0;
-                    s0 = 0.0;
-                }
-                if (act && store_lane) {
-                    P.Cr[(size_t)l * Spad + k] = c0;
-                    P.Sr[(size_t)l * Spad + k] = s0;
-                }
-                v0 = fma(v0, c0, -(hleft * s0));
-            }
-            double phi = sc_one(is);
-            pert |= solve_1x1(smin, v0, 0.0, y0, phi, is);
-            beta = sc_combine(beta, phi, is);
-            a = sc_value(phi, is);
-            if (store_lane) {
-                BC(0) = c0;
-                BC(1) = s0;
-                BC(2) = a;
-            }
-        }
-        __syncthreads();                                       // last step's rows (and the scalars) written
-        if (wid != 0) {
-            c0 = BC(0);
-            s0 = BC(1);
-            a = BC(2);
-        }
+        const double a = SB(0, 2);
         if (!is_one(a))
-            for (int i = 1 + wid * RL + rs; i < b; i += NW * RL)
-                Y(i) = a * Y(i);
-        if (wid == 0 && store_lane) Y(0) = y0;
+            for (int i = 1 + wid * RL + rs; i < b; i += NW * RL) Y(i) = a * Y(i);
+        if (wid == 4 && store_lane) Y(0) = y0;
     }
     __syncthreads();
 
@@ -1250,7 +1301,7 @@ __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int
         const int kc = k0 + cc;
         if (kc < P.S) P.X[l + i + (size_t)kc * P.ldx] = y[(size_t)i * SC + cc];
     }
-    if (act && wid == 0 && store_lane) {
+    if (act && wid == 4 && store_lane) {
         P.beta[(size_t)J * Spad + k] = beta;
         if (pert) P.pert[k] = 1;
     }
@@ -1290,8 +1341,9 @@ __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int
 #undef V
 #undef Y
 #undef PM
+#undef SA
+#undef SB
 #undef HCOL
-#undef BC
 }
 
 // The GEMM of stage J+1 over the rows of tile J, for the CTA's own columns
@@ -1408,24 +1460,24 @@ template <int SC, int NW>
 __global__ void __launch_bounds__(32 * NW) k_diag_nf(DevProblem P, DevProblem Pg, int J) {
     const int b = P.fr[J + 1] - P.fr[J];
     const size_t have = dynamic_smem_bytes();
-    if (diag_narrow_smem_bytes<SC>(b, NW) > have || top_staged_bytes<SC>(b) > have) {
+    if (diag_narrow_smem_bytes<SC>(b) > have || top_staged_bytes<SC>(b) > have) {
         if (threadIdx.x == 0) atomicOr(P.err, kErrShape);
         return;
     }
     extern __shared__ double sm[];
     top_rows_staged<SC, NW>(Pg, J, blockIdx.x * SC, sm);
     __syncthreads();                     // this CTA's rows of tile J are final; shared memory free
-    diag_body_narrow<SC, NW>(P, J, blockIdx.x);
+    diag_body_narrow<SC>(P, J, blockIdx.x);
 }
 
 template <int SC, int NW>
 __global__ void __launch_bounds__(32 * NW) k_diag_n(DevProblem P, int J) {
     const int b = P.fr[J + 1] - P.fr[J];
-    if (diag_narrow_smem_bytes<SC>(b, NW) > dynamic_smem_bytes()) {
+    if (diag_narrow_smem_bytes<SC>(b) > dynamic_smem_bytes()) {
         if (threadIdx.x == 0) atomicOr(P.err, kErrShape);
         return;
     }
-    diag_body_narrow<SC, NW>(P, J, blockIdx.x);
+    diag_body_narrow<SC>(P, J, blockIdx.x);
 }
 
 // NW warps: 8 (two per sub-partition, hiding FP64 latency) when v/y sit in
@@ -1460,7 +1512,7 @@ template <int SC, int NW>
 cudaError_t launch_diag_narrow(const DevProblem &P, int J, int b, cudaStream_t st) {
     static size_t configured = 0;
     static bool carve = false;
-    const size_t smem = diag_narrow_smem_bytes<SC>(b, NW);
+    const size_t smem = diag_narrow_smem_bytes<SC>(b);
     cudaError_t e = prefer_max_shared((const void *)k_diag_n<SC, NW>, &carve);
     if (e == cudaSuccess) e = raise_smem_limit((const void *)k_diag_n<SC, NW>, &configured, smem);
     if (e != cudaSuccess) return e;
@@ -1471,7 +1523,7 @@ cudaError_t launch_diag_narrow(const DevProblem &P, int J, int b, cudaStream_t s
 template <int SC, int NW>
 cudaError_t launch_diag_narrow_fused(const DevProblem &P, const DevProblem &Pg, int J, int b, cudaStream_t st) {
     static size_t configured = 0;
-    const size_t smem = std::max(diag_narrow_smem_bytes<SC>(b, NW), top_staged_bytes<SC>(b));
+    const size_t smem = std::max(diag_narrow_smem_bytes<SC>(b), top_staged_bytes<SC>(b));
     static bool carve = false;
     cudaError_t e = prefer_max_shared((const void *)k_diag_nf<SC, NW>, &carve);
     if (e == cudaSuccess) e = raise_smem_limit((const void *)k_diag_nf<SC, NW>, &configured, smem);
