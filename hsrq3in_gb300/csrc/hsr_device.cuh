@@ -137,28 +137,23 @@ __host__ __device__ __forceinline__ unsigned long long ip_recip(unsigned long lo
 }
 // Bits of the correctly rounded ma / mb (significands with the hidden bit),
 // given y = ip_recip(mb), the biased exponent ea - eb + 1023 and the sign.
-// q estimates floor(ma 2^sh / mb) (54 bits) within two; the remainder
-// r = ma 2^sh - q mb, exact modulo 2^64 because |r| < 2^56, moves q to the
-// floor; its last bit and r != 0 round the 53-bit result to nearest even.
+// q, lowered by the estimate's error, is floor(ma 2^sh / mb) (54 bits) or at
+// most two less; the remainder r = ma 2^sh - q mb, exact modulo 2^64 because
+// r < 2^56, moves q to the floor; its last bit and r != 0 round the 53-bit
+// result to nearest even.
 __host__ __device__ __forceinline__ unsigned long long ip_quot(unsigned long long ma, unsigned long long mb,
                                                                unsigned long long y, int ebias,
                                                                unsigned long long sign) {
     const int sh = ma < mb ? 54 : 53;
     const unsigned long long hi = umulhi64(ma, y);
     const unsigned long long lo = ma * y;
-    unsigned long long q = sh == 53 ? ((hi << 1) | (lo >> 63)) : ((hi << 2) | (lo >> 62));
-    long long r = (long long)((ma << sh) - q * mb);
+    unsigned long long q = (sh == 53 ? ((hi << 1) | (lo >> 63)) : ((hi << 2) | (lo >> 62))) - 1;
+    unsigned long long r = (ma << sh) - q * mb;
 #pragma unroll
     for (int i = 0; i < 2; ++i)
-        if (r < 0) {
-            q -= 1;
-            r += (long long)mb;
-        }
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-        if (r >= (long long)mb) {
+        if (r >= mb) {
             q += 1;
-            r -= (long long)mb;
+            r -= mb;
         }
     const unsigned long long guard = q & 1ULL;
     unsigned long long Q = q >> 1;

@@ -920,39 +920,47 @@ __device__ __forceinline__ unsigned long long gemm_epilogue_elem(const DevProble
 // depends on the running column v alone, so
 //   warp 0 (lane s and its duplicates s + SC, ... of shift s) runs the Givens
 //     chain: rotation j, then rows j-1 and j-2 of v, one group of lanes each;
-//     the two quotients of the rotation, two group's worth of work, likewise;
-//   warp 4 (sub-partition 0 too) runs the solve chain one step behind: the
-//     1x1 solve, the decisions, rows j-1 and j-2 of y;
-//   warps 1-3 and 5-7 update rows 0 .. j-3 of v and y, 32 / SC rows x SC
+//     the two quotients of the rotation, two groups' worth of work, likewise;
+//   warp 4 forms the 1x1 system of step j from the rotation, with the
+//     reciprocal of its coefficient, and stages the columns of H;
+//   warp 1 runs the solve chain: the quotient, the decisions, rows j-1 and j-2
+//     of y;
+//   warps 2, 3, 5, 6, 7 update rows 0 .. j-3 of v and y, 32 / SC rows x SC
 //     shifts per instruction.
-// Rotation j-1 runs while the rows of step j are updated.  Three mbarriers
-// carry the step: the rotation is there, the solve's factors are there, the
-// rows are done.  Every (row, shift) element sees the same operations in the
-// same order as in diag_body_pipe, so the result is bit-identical to the wide
-// form.  For the third decision the row warps fold the high words of |y| and
-// |v|; only where those do not already show that it cannot fire does warp 4
-// take the maxima themselves, over the rows in shared memory (a maximum does
-// not depend on the order it is taken in).  v and y live in shared memory as
-// [row][SC].
+// Rotation j-1 runs while the rows of step j are updated, and so does solve
+// j-1: its third decision needs bounds of the rows of step j, but those of
+// step j+1 bound them too (`fits` below).  mbarriers carry the step.  Every
+// (row, shift) element sees the same operations in the same order as in
+// diag_body_pipe, so the result is bit-identical to the wide form.  For the
+// third decision the row warps fold the high words of |y| and |v|; only where
+// those do not show that it cannot fire does warp 1 wait for the rows and take
+// the maxima themselves, in shared memory (a maximum does not depend on the
+// order it is taken in).  v and y live in shared memory as [row][SC].
 //
-// Bound by the two chains' latency (rotation about 900 clocks, solve 700) and
-// by the rows' FP64 issue, 4 instructions of 64 clocks per 32 / SC rows on
-// three sub-partitions.  With one chain warp, two row warps and two block
-// barriers a step: %%DIAG%%
-constexpr int kNarrowRowWarps = 6;
+// Bound by the chains' latency in low tiles (rotation 1,300 clocks, system
+// 700, solve 550) and by the rows' FP64 issue, 4 instructions of 64 clocks per
+// 32 / SC rows, in high ones: about 2,700 clocks a step at tile 64, 3,300 at
+// 160.  With one chain warp, two row warps and two block barriers a step:
+// 6,600 and 7,900 (n = 1000, all shifts, tile 160: 7.17 ms a solve, now 4.37;
+// n = 3001, 301 shifts, tile 200: 22.9 and 14.6).
+// a3 (yold - yc v + ys h), the scaled update of row j-1 (rare).
+static __device__ __noinline__ double scaled_update(double a3, double yc, double ys, double h, double v, double yold) {
+    return a3 * fma(ys, h, fma(-yc, v, yold));
+}
+constexpr int kNarrowRowWarps = 5;
 template <int SC>
 __host__ __device__ constexpr size_t diag_narrow_smem_bytes(int b) {
-    return (size_t)(4 * (b + 2) + (2 * 4 + 2 * 5) * SC + 8 * SC + 2 * SC * b) * sizeof(double);
+    return (size_t)(4 * (b + 2) + (2 * 4 + 2 * 5 + 2 * 4) * SC + 2 * kNarrowRowWarps * SC + 2 * SC * b) * sizeof(double);
 }
 
 template <int SC>
 __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int bx) {
     static_assert(SC == 8 || SC == 16, "shifts per CTA");
     constexpr int NW = kDiagWarpsNarrow, NR = kNarrowRowWarps;
-    static_assert(NW == 8, "two chain warps on sub-partition 0, six row warps");
+    static_assert(NW == 8, "three chain warps, five row warps");
     constexpr int RL = 32 / SC;                                               // rows per row-warp instruction
     extern __shared__ double sm[];
-    __shared__ __align__(8) uint64_t bars[5];                                 // rotation x 2, rows x 2, factors
+    __shared__ __align__(8) uint64_t bars[8];                                 // two each: rotation, system, factors, rows
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int wid = tid >> 5;
@@ -960,8 +968,7 @@ __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int
     const int rs = lane / SC;                                                 // row slot, lane group
     const bool odd = (rs & 1) != 0;                                           // which of two values the group takes
     const bool store_lane = lane < SC;                                        // chain results are stored once
-    const bool row_warp = (wid & 3) != 0;
-    const int rw = wid - 1 - wid / 4;                                         // row-warp index, 0 .. NR-1
+    const int rw = wid < 4 ? wid - 2 : wid - 3;                               // row-warp index, 0 .. NR-1
     const int k0 = bx * SC;
     const int k = k0 + sh;
     const bool act = k < P.S;
@@ -972,22 +979,20 @@ __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int
     double *hc = sm;                                                          // [4][b+2]
     double *sa = sm + 4 * (b + 2);                                            // [2][4][SC]: c, s, v(j), v(j-1)
     double *sb = sa + 2 * 4 * SC;                                             // [2][5][SC]: yc, ys, a1, a2, a3
-    unsigned *pm = reinterpret_cast<unsigned *>(sb + 2 * 5 * SC);             // [NR][2][SC], high words
-    double *v = sb + 2 * 5 * SC + 8 * SC;                                     // [b][SC]
+    double *sc = sb + 2 * 5 * SC;                                             // [2][4][SC]: coefficient, reciprocal, kind, H(j-1, j-1) - mu
+    unsigned *pm = reinterpret_cast<unsigned *>(sc + 2 * 4 * SC);             // [2][NR][2][SC], high words
+    double *v = sc + 2 * 4 * SC + 2 * NR * SC;                                // [b][SC]
     double *y = v + (size_t)SC * b;                                           // [b][SC]
 #define V(i) v[(size_t)(i) * SC + sh]
 #define Y(i) y[(size_t)(i) * SC + sh]
-#define PM(w, which) pm[(((w) * 2) + (which)) * SC + sh]
+#define PM(t, w, which) pm[((((t) & 1) * NR + (w)) * 2 + (which)) * SC + sh]
+#define SX(t, q) sc[((((t) & 1) * 4) + (q)) * SC + sh]
 #define SA(t, q) sa[((((t) & 1) * 4) + (q)) * SC + sh]
 #define SB(t, q) sb[((((t) & 1) * 5) + (q)) * SC + sh]
 #define HCOL(col) (hc + (size_t)((col) & 3) * (b + 2))
 
     if (tid == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
-        mbar_init(&bars[2], NR);
-        mbar_init(&bars[3], NR);
-        mbar_init(&bars[4], 1);
+        for (int q = 0; q < 8; ++q) mbar_init(&bars[q], q < 6 ? 1 : NR);
         mbar_fence_init();
     }
     for (int idx = tid; idx < SC * b; idx += 32 * NW) {
@@ -1006,7 +1011,7 @@ __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int
     double beta = act ? P.beta[(size_t)J * Spad + k] : sc_one(is);
     int pert = 0;
     const double *Hd = P.H + l + (size_t)l * P.ldh;                           // H(l, l)
-    auto stage_col = [&](int col) {                                           // H(l : l+col+1, l+col), warp 0
+    auto stage_col = [&](int col) {                                           // H(l : l+col+1, l+col), warp 4
         if (col >= 0) {
             const int rows = min(col + 2, b);
             const double *src = Hd + (size_t)col * P.ldh;
@@ -1015,25 +1020,22 @@ __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int
         }
         cp_async_commit();                                                    // one group per column, empty ones too
     };
-    if (wid == 0) {
+    if (wid == 4) {
         stage_col(b - 2);
         stage_col(b - 3);
     }
     __syncthreads();                                                          // tile and barriers ready
 
-    // Step t's barriers (t = b - 1 - j).  The rotation and the rows alternate
-    // between two, so that neither can complete the phase after the one that
-    // a late warp still has to wait for; the factors of step t + 1 follow the
-    // rows of step t, which every row warp ends after its wait for step t's.
-    // A wait that runs out is recorded; the warp then waits no more.
-    constexpr int kRot = 0, kRows = 2, kFac = 4;
+    // Step t's barriers (t = b - 1 - j), two of each kind in turn: the phase
+    // after the one that a late warp still has to wait for cannot complete
+    // before that warp's own next post.  A wait that runs out is recorded; the
+    // warp then waits no more.
+    constexpr int kRot = 0, kSys = 2, kFac = 4, kRows = 6;
     bool ok = true;
-    auto await = [&](int which, int t) {
-        ok = ok && mbar_wait(&bars[which == kFac ? kFac : which + (t & 1)], (uint32_t)(which == kFac ? t & 1 : (t >> 1) & 1), P.err);
-    };
+    auto await = [&](int which, int t) { ok = ok && mbar_wait(&bars[which + (t & 1)], (uint32_t)((t >> 1) & 1), P.err); };
     auto post = [&](int which, int t) {
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bars[which == kFac ? kFac : which + (t & 1)]);
+        if (lane == 0) mbar_arrive(&bars[which + (t & 1)]);
     };
     const unsigned hi497 = (unsigned)(pow2_bits(497) >> 32), hi995 = (unsigned)(pow2_bits(995) >> 32);
     auto hi_mag = [](double x) { return (unsigned)(ubits(x) >> 32) & 0x7fffffffu; };
@@ -1041,11 +1043,11 @@ __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int
     double v0 = 0.0, y0 = 0.0;                                                // rows 0 of v (warp 0) and y (warp 4)
     if (wid == 0) {
         double vj = V(b - 1), vw = b >= 2 ? V(b - 2) : 0.0;                   // v(j); v(j-1)
+        // H(j, j-1), H(j-1, j-1) and H(j-2, j-1), two steps ahead.
+        auto entry = [&](int row, int col) { return col >= 0 && row >= 0 ? Hd[row + (size_t)col * P.ldh] : 0.0; };
+        double hsub = entry(b - 1, b - 2), hdiag = entry(b - 2, b - 2) - mu, htop = entry(b - 3, b - 2);
+        double hs1 = entry(b - 2, b - 3), hd1 = entry(b - 3, b - 3), ht1 = entry(b - 4, b - 3);
         for (int j = b - 1, t = 0; j >= 1; --j, ++t) {
-            cp_async_wait_one();                                              // column j-1
-            __syncwarp();
-            const double *hcol = HCOL(j - 1);
-            const double hsub = hcol[j], hdiag = hcol[j - 1] - mu;
             double c, s;
             {
                 // As givens(), the squares and the quotients of f and g on
@@ -1081,69 +1083,132 @@ __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int
                 P.Cr[(size_t)(l + j) * Spad + k] = c;
                 P.Sr[(size_t)(l + j) * Spad + k] = s;
             }
-            await(kRows, t);                                                      // rows of step j+1: row j-2 is in V
-            const double h = !odd ? hdiag : (j >= 2 ? hcol[j - 2] : 0.0);
+            const double hdu = hdiag, htu = htop;                             // the next step's, off the chain's path
+            hsub = hs1;
+            hdiag = hd1 - mu;
+            htop = ht1;
+            hs1 = entry(j - 2, j - 3);
+            hd1 = entry(j - 3, j - 3);
+            ht1 = entry(j - 4, j - 3);
+            await(kRows, t);                                                  // rows of step j+1: row j-2 is in V
             const double vo = !odd ? vw : (j >= 2 ? V(j - 2) : 0.0);
-            const double vn = fma(c, h, s * vo);
+            const double vn = fma(c, !odd ? hdu : htu, s * vo);
             vj = __shfl_sync(0xffffffffu, vn, sh);
             vw = __shfl_sync(0xffffffffu, vn, sh + SC);
-            stage_col(j - 3);                                                 // over column j+1
         }
         v0 = vj;
     } else if (wid == 4) {
-        const double Hnorm = P.Hn[J + (size_t)J * P.T];
-        double ycar = Y(b - 1), ynext = b >= 2 ? Y(b - 2) : 0.0;              // y(j), y(j-1)
         for (int j = b - 1, t = 0; j >= 1; --j, ++t) {
+            cp_async_wait_one();                                              // column j-1, for the other warps too
             await(kRot, t);
-            const double *hcol = HCOL(j - 1);
-            const double c = SA(t, 0), s = SA(t, 1), vjm1 = SA(t, 3);
-            const double hdiag = hcol[j - 1] - mu;
-            double yj = ycar, yjm1 = ynext;
-            const double pr = (odd ? s : c) * (odd ? hcol[j] : SA(t, 2));     // c v(j), s H(j, j-1)
-            double phi = sc_one(is);
-            pert |= solve_1x1(smin, __shfl_sync(0xffffffffu, pr, sh), __shfl_sync(0xffffffffu, pr, sh + SC), yj, phi, is);
-            beta = sc_combine(beta, phi, is);
-            const double a1 = sc_value(phi, is);
-            yjm1 = scale_by(a1, yjm1);
-            phi = protect_double_update(absd(vjm1), absd(yj), absd(hdiag), absd(yj), absd(yjm1), is);
-            const double a2 = sc_value(phi, is);
-            if (!is_one(a2)) {
-                yj = mul_rare(a2, yj);
-                yjm1 = mul_rare(a2, yjm1);
+            __syncwarp();
+            // solve_1x1's coefficient c v(j) - s H(j, j-1), the operands on
+            // two lane groups, and what the decisions need of it, of v(j-1)
+            // and of H: kind has bit 0 where the coefficient was lifted to
+            // smin, bit 1 where warp 1 has to evaluate the decisions in full.
+            const double hdg = HCOL(j - 1)[j - 1] - mu;
+            const double pr = (odd ? SA(t, 1) : SA(t, 0)) * (odd ? HCOL(j - 1)[j] : SA(t, 2));
+            const double tt = __shfl_sync(0xffffffffu, pr, sh), ll = __shfl_sync(0xffffffffu, pr, sh + SC);
+            double csr = tt - ll;
+            unsigned kind = hi_mag(tt) < hi995 && hi_mag(ll) < hi995 && hi_mag(SA(t, 3)) < hi497 && hi_mag(hdg) < hi497 ? 0 : 2;
+            if (mag(csr) < ubits(smin)) {
+                csr = smin;
+                kind |= 1;
             }
-            beta = sc_combine(beta, phi, is);
-            const double py = yj * (odd ? s : c);
-            double yc = __shfl_sync(0xffffffffu, py, sh), ys = __shfl_sync(0xffffffffu, py, sh + SC);
-            yjm1 = fma(ys, hdiag, fma(-yc, vjm1, yjm1));
-            await(kRows, t);                                                      // rows of step j+1
-            unsigned ymh = 0, vmh = 0;
+            const unsigned long long fb = ubits(csr) & kSigMask;
+            const unsigned ed = hi_mag(csr) >> 20;
+            if (fb == 0 || ed == 0 || ed == 0x7ff) kind |= 2;
+            const unsigned long long rec = ip_recip(fb | kHidden | (fb == 0 ? 1 : 0));
+            if (store_lane) {
+                SX(t, 0) = csr;
+                SX(t, 1) = from_bits(rec);
+                SX(t, 2) = from_bits((unsigned long long)kind);
+                SX(t, 3) = hdg;
+            }
+            post(kSys, t);
+            // Column j+1 gives way: the rows that read it ended before this
+            // rotation, warp 1's use before its factors of step j+1.
+            if (t > 0) await(kFac, t - 1);
+            stage_col(j - 3);
+        }
+    } else if (wid == 1) {
+        const double Hnorm = P.Hn[J + (size_t)J * P.T];
+        const unsigned hi490 = (unsigned)(pow2_bits(490) >> 32), hi990 = (unsigned)(pow2_bits(990) >> 32);
+        // fits: bounds |y| < 2^990, |v| < 2^490 over the rows before a step
+        // without scaling, whose factors are below 2^497, show that after it
+        // |y| < 2^990 + 2 2^(497+490) < 2^995 and |v| < 2^490 + |H| < 2^497 (a
+        // rotation's c and s are at most 1, H's entries at most Hnorm < 2^490).
+        const bool hfits = hi_mag(Hnorm) < hi490;
+        bool fits = false;
+        double ycar = Y(b - 1), ynext = b >= 2 ? Y(b - 2) : 0.0;              // y(j), y(j-1)
+        unsigned ymh = 0, vmh = 0;
+        auto bounds = [&](int t) {
+            ymh = vmh = 0;
 #pragma unroll
             for (int w = 0; w < NR; ++w) {
-                ymh = max(ymh, PM(w, 0));
-                vmh = max(vmh, PM(w, 1));
+                ymh = max(ymh, PM(t, w, 0));
+                vmh = max(vmh, PM(t, w, 1));
             }
-            double a3 = 1.0;
-            phi = sc_one(is);
-            if (!(ymh < hi995 && vmh < hi497 && hi_mag(yj) < hi497 && hi_mag(Hnorm) < hi497 && is_one(a1) && is_one(a2))) {
-                unsigned long long ymb = 0, vmb = 0;                          // the maxima over rows 0 .. j-2
-                for (int i = 0; i <= j - 2; ++i) {
-                    ymb = umax64(ymb, abs_bits(Y(i)));
-                    vmb = umax64(vmb, abs_bits(V(i)));
+        };
+        for (int j = b - 1, t = 0; j >= 1; --j, ++t) {
+            await(kSys, t);
+            const double *hcol = HCOL(j - 1);
+            const double c = SA(t, 0), s = SA(t, 1), vjm1 = SA(t, 3), csr = SX(t, 0), hdiag = SX(t, 3);
+            const unsigned kind = (unsigned)ubits(SX(t, 2));
+            double yj = ycar, yold = ynext, yc, ys, yjm1 = 0.0, a1 = 1.0, a2 = 1.0, a3 = 1.0;
+            // The step where no decision fires: the division's operands normal
+            // and no further apart than its protection allows, every bound of
+            // the other two inside.  All of it in one test for the warp.
+            const unsigned long long un = ubits(yj), ud = ubits(csr);
+            const int en = (int)((un >> 52) & 0x7ff), ed = (int)((ud >> 52) & 0x7ff);
+            const double q = from_bits(ip_quot((un & kSigMask) | kHidden, (ud & kSigMask) | kHidden, ubits(SX(t, 1)),
+                                               en - ed + 1023, (un ^ ud) & 0x8000000000000000ULL));
+            const bool plain = kind < 2 && en != 0 && en != 0x7ff && en - ed >= -1021 && en - ed < 990 && hi_mag(q) < hi497 &&
+                               hi_mag(yold) < hi995 && fits;
+            if (__all_sync(0xffffffffu, plain || !act)) {           // columns past the last count as plain
+                pert |= (int)kind;
+                yj = q;
+                const double py = yj * (odd ? s : c);
+                yc = __shfl_sync(0xffffffffu, py, sh);
+                ys = __shfl_sync(0xffffffffu, py, sh + SC);
+            } else {
+                double phi = sc_one(is);
+                pert |= solve_1x1(smin, mul_rare(c, SA(t, 2)), mul_rare(s, hcol[j]), yj, phi, is);
+                beta = sc_combine(beta, phi, is);
+                a1 = sc_value(phi, is);
+                yold = scale_by(a1, yold);
+                phi = protect_double_update(absd(vjm1), absd(yj), absd(hdiag), absd(yj), absd(yold), is);
+                a2 = sc_value(phi, is);
+                if (!is_one(a2)) {
+                    yj = mul_rare(a2, yj);
+                    yold = mul_rare(a2, yold);
                 }
-                double ymax = from_bits(ymb);
-                if (!is_one(a1)) ymax = from_bits(abs_bits(mul_rare(a1, ymax)));
-                if (!is_one(a2)) ymax = from_bits(abs_bits(mul_rare(a2, ymax)));
-                phi = protect_double_update(from_bits(vmb), absd(yj), Hnorm, absd(yj), ymax, is);
-                a3 = sc_value(phi, is);
+                beta = sc_combine(beta, phi, is);
+                yc = mul_rare(yj, c);
+                ys = mul_rare(yj, s);
+                await(kRows, t);                                              // rows of step j+1
+                bounds(t);
+                if (!(ymh < hi995 && vmh < hi497 && hi_mag(yj) < hi497 && hi_mag(Hnorm) < hi497 && is_one(a1) && is_one(a2))) {
+                    unsigned long long ymb = 0, vmb = 0;                      // the maxima over rows 0 .. j-2
+                    for (int i = 0; i <= j - 2; ++i) {
+                        ymb = umax64(ymb, abs_bits(Y(i)));
+                        vmb = umax64(vmb, abs_bits(V(i)));
+                    }
+                    double ymax = from_bits(ymb);
+                    if (!is_one(a1)) ymax = from_bits(abs_bits(mul_rare(a1, ymax)));
+                    if (!is_one(a2)) ymax = from_bits(abs_bits(mul_rare(a2, ymax)));
+                    phi = protect_double_update(from_bits(vmb), absd(yj), Hnorm, absd(yj), ymax, is);
+                    a3 = sc_value(phi, is);
+                    beta = sc_combine(beta, phi, is);
+                }
                 if (!is_one(a3)) {
+                    yjm1 = scaled_update(a3, yc, ys, hdiag, vjm1, yold);
                     yj = mul_rare(a3, yj);
-                    yjm1 = mul_rare(a3, yjm1);
                     yc = mul_rare(yj, c);
                     ys = mul_rare(yj, s);
                 }
             }
-            beta = sc_combine(beta, phi, is);
-            const double yi0 = j >= 2 ? Y(j - 2) : 0.0, vi = j >= 2 ? V(j - 2) : 0.0;
+            const bool scaled = !is_one(a1) || !is_one(a2) || !is_one(a3);
             if (store_lane) {
                 SB(t, 0) = yc;
                 SB(t, 1) = ys;
@@ -1153,14 +1218,21 @@ __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int
                 Y(j) = yj;
             }
             post(kFac, t);
-            // Row j-2 of y, for the next step's chain.
-            double yi = yi0;
-            if (!is_one(a1) || !is_one(a2) || !is_one(a3)) {
-                yi = scale_by(a1, yi);
-                yi = scale_by(a2, yi);
-                yi = scale_by(a3, yi);
+            if (is_one(a3)) yjm1 = fma(ys, hdiag, fma(-yc, vjm1, yold));
+            // Row j-2 of y, for the next step's chain, and the bounds of the
+            // rows of step j+1.
+            await(kRows, t);
+            bounds(t);
+            fits = hfits && !scaled && ymh < hi990 && vmh < hi490 && hi_mag(yc) < hi497 && hi_mag(ys) < hi497;
+            if (j >= 2) {
+                double yi = Y(j - 2);
+                if (scaled) {
+                    yi = scale_by(a1, yi);
+                    yi = scale_by(a2, yi);
+                    yi = scale_by(a3, yi);
+                }
+                ynext = fma(ys, hcol[j - 2], fma(-yc, V(j - 2), yi));
             }
-            ynext = j >= 2 ? fma(ys, hcol[j - 2], fma(-yc, vi, yi)) : 0.0;
             ycar = yjm1;
         }
         y0 = ycar;
@@ -1171,27 +1243,26 @@ __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int
             ym = max(ym, hi_mag(Y(i)));
             vm = max(vm, hi_mag(V(i)));
         }
-        auto fold = [&](unsigned ymx, unsigned vmx) {
+        auto fold = [&](unsigned ymx, unsigned vmx, int tm) {
 #pragma unroll
             for (int o = SC; o < 32; o <<= 1) {
                 ymx = max(ymx, __shfl_xor_sync(0xffffffffu, ymx, o));
                 vmx = max(vmx, __shfl_xor_sync(0xffffffffu, vmx, o));
             }
             if (store_lane) {
-                PM(rw, 0) = ymx;
-                PM(rw, 1) = vmx;
+                PM(tm, rw, 0) = ymx;
+                PM(tm, rw, 1) = vmx;
             }
         };
-        fold(ym, vm);
+        fold(ym, vm, 0);
         post(kRows, 0);
         for (int j = b - 1, t = 0; j >= 1; --j, ++t) {
-            await(kRot, t);
+            await(kFac, t);                                                   // ... and with it the rotation and the column
             const double sc_c = SA(t, 0), sc_s = SA(t, 1);
             const double *hcol = HCOL(j - 1);
             const int lim = j - 2;                                            // rows 0 .. j-3
             constexpr int ST = NR * RL;                                       // row stride of one lane
             int i = rw * RL + rs;
-            await(kFac, t);
             const double sc_yc = SB(t, 0), sc_ys = SB(t, 1), s1 = SB(t, 2), s2 = SB(t, 3), s3 = SB(t, 4);
             const bool scaled = !is_one(s1) || !is_one(s2) || !is_one(s3);
             if (scaled) {
@@ -1248,7 +1319,7 @@ __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int
                 ym = max(ym, hi_mag(yi));
                 vm = max(vm, hi_mag(vi));
             }
-            fold(ym, vm);
+            fold(ym, vm, t + 1);
             post(kRows, t + 1);
         }
     }
@@ -1280,7 +1351,7 @@ __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int
     __syncthreads();
     c0 = SA(0, 0);
     s0 = SA(0, 1);
-    if (wid == 4) {
+    if (wid == 1) {
         double phi = sc_one(is);
         pert |= solve_1x1(smin, SA(0, 2), 0.0, y0, phi, is);
         beta = sc_combine(beta, phi, is);
@@ -1291,7 +1362,7 @@ __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int
         const double a = SB(0, 2);
         if (!is_one(a))
             for (int i = 1 + wid * RL + rs; i < b; i += NW * RL) Y(i) = a * Y(i);
-        if (wid == 4 && store_lane) Y(0) = y0;
+        if (wid == 1 && store_lane) Y(0) = y0;
     }
     __syncthreads();
 
@@ -1301,7 +1372,7 @@ __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int
         const int kc = k0 + cc;
         if (kc < P.S) P.X[l + i + (size_t)kc * P.ldx] = y[(size_t)i * SC + cc];
     }
-    if (act && wid == 4 && store_lane) {
+    if (act && wid == 1 && store_lane) {
         P.beta[(size_t)J * Spad + k] = beta;
         if (pert) P.pert[k] = 1;
     }
@@ -1342,6 +1413,7 @@ __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int
 #undef Y
 #undef PM
 #undef SA
+#undef SX
 #undef SB
 #undef HCOL
 }
