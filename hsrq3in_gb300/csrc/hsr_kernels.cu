@@ -955,7 +955,7 @@ __host__ __device__ constexpr size_t diag_narrow_smem_bytes(int b) {
 
 template <int SC>
 __device__ __forceinline__ void diag_body_narrow(const DevProblem &P, int J, int bx) {
-    static_assert(SC == 8 || SC == 16, "shifts per CTA");
+    static_assert(SC == 4 || SC == 8 || SC == 16, "shifts per CTA");
     constexpr int NW = kDiagWarpsNarrow, NR = kNarrowRowWarps;
     static_assert(NW == 8, "three chain warps, five row warps");
     constexpr int RL = 32 / SC;                                               // rows per row-warp instruction
@@ -1480,6 +1480,7 @@ __device__ __forceinline__ void top_rows_staged(const DevProblem &Pg, int J, int
     unsigned long long m = 0;
     for (int p0 = 0; p0 < rows; p0 += G * EB) {
         int ri[EB];
+        const int ne = min(EB, (rows - p0 + G - 1) / G);        // slabs of G rows this pass has, the same for every thread
 #pragma unroll
         for (int e = 0; e < EB; ++e) ri[e] = min(p0 + g + e * G, rows - 1);   // rows past the tile: computed, dropped
         double aw[EB], az[EB], hl1[EB];
@@ -1507,9 +1508,11 @@ __device__ __forceinline__ void top_rows_staged(const DevProblem &Pg, int J, int
                 const double *hk = hs + (size_t)kk * rows;
 #pragma unroll
                 for (int e = 0; e < EB; ++e) {
-                    const double a = hk[ri[e]];
-                    aw[e] = fma(a, w, aw[e]);
-                    az[e] = fma(a, z, az[e]);
+                    if (e < ne) {
+                        const double a = hk[ri[e]];
+                        aw[e] = fma(a, w, aw[e]);
+                        az[e] = fma(a, z, az[e]);
+                    }
                 }
             }
             __syncthreads();                                    // buffer ch & 1 free for chunk ch + 2
@@ -1604,13 +1607,35 @@ cudaError_t launch_diag_narrow_fused(const DevProblem &P, const DevProblem &Pg, 
     return cudaGetLastError();
 }
 
+// SMs of the device (0 if unknown).
+int device_sms() {
+    static const int sms = []() {
+        int dev = 0, n = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+            return 0;
+        return n;
+    }();
+    return sms;
+}
+
+// Shifts per CTA of a launch: diag_shifts_per_cta, and where that is 8 and
+// CTAs of 4 still find an SM each, 4: the rows and the fused top GEMM are
+// bound by the FP64 pipes of the SMs that take part (n = 3001, 301 shifts,
+// tile 200: 14.6 ms with 8, 12.4 with 4).
+int narrow_shifts(int S) {
+    const int sc = diag_shifts_per_cta(S);
+    return sc == 8 && (S + 3) / 4 <= device_sms() ? 4 : sc;
+}
+
 // Tile J's diagonal solve preceded by stage J+1's GEMM over tile J's rows,
 // in one launch, when the narrow forms apply; false (nothing launched) when
 // the wide form is used and the caller runs the two launches.
 bool launch_diag_fused(const DevProblem &P, const DevProblem &Pg, int J, int b, cudaStream_t st,
                        cudaError_t *err) {
     if (!fused_top_for(P.S)) return false;
-    switch (diag_shifts_per_cta(P.S)) {
+    switch (narrow_shifts(P.S)) {
+    case 4: *err = launch_diag_narrow_fused<4, kDiagWarpsNarrow>(P, Pg, J, b, st); return true;
     case 8: *err = launch_diag_narrow_fused<8, kDiagWarpsNarrow>(P, Pg, J, b, st); return true;
     case 16: *err = launch_diag_narrow_fused<16, kDiagWarpsNarrow>(P, Pg, J, b, st); return true;
     default: return false;
@@ -1680,13 +1705,7 @@ int diag_shifts_per_cta(int S) {
         const int best = nearest_tuned(g_spc_tuned, S);
         if (best) return best;
     }
-    static const int sms = []() {
-        int dev = 0, n = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-            return 0;
-        return n;
-    }();
+    const int sms = device_sms();
     const int wide = (S + 31) / 32;
     if (sms <= 0) return 32;
     if (4 * wide <= sms) return 8;
@@ -1696,7 +1715,8 @@ int diag_shifts_per_cta(int S) {
 
 cudaError_t launch_diag(const DevProblem &P, int J, int b, double *gscratch, cudaStream_t st) {
     const int grid = (P.S + 31) / 32;
-    switch (diag_shifts_per_cta(P.S)) {
+    switch (narrow_shifts(P.S)) {
+    case 4: return launch_diag_narrow<4, kDiagWarpsNarrow>(P, J, b, st);
     case 8: return launch_diag_narrow<8, kDiagWarpsNarrow>(P, J, b, st);
     case 16: return launch_diag_narrow<16, kDiagWarpsNarrow>(P, J, b, st);
     default: break;
