@@ -27,6 +27,7 @@
 #include "hsr_kernels.h"
 
 #include <cfloat>
+#include <type_traits>
 
 namespace hsr {
 
@@ -479,6 +480,566 @@ __global__ void __launch_bounds__(32 * NW) k_diag_c(DevProblem P, int J, double 
 #undef BC
 }
 
+// Narrow form for few pairs: SC pairs per CTA, the step's serial chain on
+// three warps, as diag_body_narrow (hsr_kernels.cu) does it for real shifts:
+//   warp 0  rotation j, rows j-1 and j-2 of v;
+//   warp 4  the 1x1 system: its coefficient and, for c_dladiv, the ratio r of
+//           its parts and t = 1 / (c + d r); stages the columns of H;
+//   warp 1  the solve, the decisions, rows j-1 and j-2 of y;
+//   warps 2, 3, 5, 6, 7  rows 0 .. j-3 of v and y, 32 / SC rows x SC pairs per
+//           instruction.
+// In the chains even lane groups take the real part of a complex result, odd
+// ones the imaginary part (or two quotients of one divisor), so that both cost
+// one FP64 instruction; the partner's part is one exchange away.  Every element
+// sees the operations of k_diag_c in their order: the same bits.
+//
+// Bound by the rows' FP64 issue (11 instructions of 64 clocks per 32 / SC rows
+// on less than three sub-partitions), so SC is the smallest that still fits
+// one wave of CTAs.  %%CDIAG%%
+constexpr int kNarrowCWarps = 8, kNarrowCRows = 5;
+constexpr size_t kNarrowCSmem = 200 * 1024;
+template <int SC>
+__host__ __device__ constexpr size_t diag_cn_smem_bytes(int b) {
+    return (size_t)(4 * (b + 2) + 2 * (7 + 4 + 7) * SC + 2 * kNarrowCRows * SC + 4 * SC * b) * sizeof(double);
+}
+
+template <int SC>
+__global__ void __launch_bounds__(32 * kNarrowCWarps) k_diag_cn(DevProblem P, int J) {
+    static_assert(SC == 4 || SC == 8 || SC == 16, "pairs per CTA");
+    constexpr int NW = kNarrowCWarps, NR = kNarrowCRows, RL = 32 / SC;
+    extern __shared__ double sm[];
+    __shared__ __align__(8) uint64_t bars[8];                          // two each: rotation, system, factors, rows
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int sh = lane % SC, rs = lane / SC;                          // pair slot; row slot, lane group
+    const bool odd = (rs & 1) != 0, store_lane = lane < SC;
+    const int rw = wid < 4 ? wid - 2 : wid - 3;                        // row-warp index
+    const int np = P.S / 2, p0 = blockIdx.x * SC, pidx = p0 + sh;
+    const bool act = pidx < np;
+    const int k = 2 * pidx;
+    const int l = P.fr[J], b = P.fr[J + 1] - l;
+    const bool is = P.is != 0;
+    const size_t Spad = (size_t)P.Spad;
+    if (diag_cn_smem_bytes<SC>(b) > dynamic_smem_bytes()) {
+        if (tid == 0) atomicOr(P.err, kErrShape);
+        return;
+    }
+
+    double *hc = sm;                                                   // [4][b+2]
+    double *sa = hc + 4 * (b + 2);                                     // [2][7][SC]: c, sigma, v(j), v(j-1)
+    double *sx = sa + 2 * 7 * SC;                                      // [2][4][SC]: r, t, kind, Re(H(j-1,j-1) - mu)
+    double *sb = sx + 2 * 4 * SC;                                      // [2][7][SC]: yc, ys, a1, a2, a3
+    unsigned *pm = reinterpret_cast<unsigned *>(sb + 2 * 7 * SC);      // [2][NR][2][SC], high words
+    double *vr_ = sb + 2 * 7 * SC + 2 * NR * SC;
+    double *vi_ = vr_ + (size_t)SC * b, *yr_ = vi_ + (size_t)SC * b, *yi_ = yr_ + (size_t)SC * b;
+#define VR(i) vr_[(size_t)(i) * SC + sh]
+#define VI(i) vi_[(size_t)(i) * SC + sh]
+#define YR(i) yr_[(size_t)(i) * SC + sh]
+#define YI(i) yi_[(size_t)(i) * SC + sh]
+#define SA(t, q) sa[(((t) & 1) * 7 + (q)) * SC + sh]
+#define SX(t, q) sx[(((t) & 1) * 4 + (q)) * SC + sh]
+#define SB(t, q) sb[(((t) & 1) * 7 + (q)) * SC + sh]
+#define PM(t, w, which) pm[((((t) & 1) * NR + (w)) * 2 + (which)) * SC + sh]
+#define HCOL(col) (hc + (size_t)((col) & 3) * (b + 2))
+
+    if (tid == 0) {
+        for (int q = 0; q < 8; ++q) mbar_init(&bars[q], q < 6 ? 1 : NR);
+        mbar_fence_init();
+    }
+    for (int idx = tid; idx < SC * b; idx += 32 * NW) {
+        const int c = idx / b, i = idx - c * b, pc = p0 + c;
+        const size_t at = (size_t)i * SC + c;
+        if (pc < np) {
+            const double *rr = P.R + l + i + (size_t)(2 * pc) * P.ldr, *xr = P.X + l + i + (size_t)(2 * pc) * P.ldx;
+            vr_[at] = rr[0];
+            vi_[at] = rr[P.ldr];
+            yr_[at] = xr[0];
+            yi_[at] = xr[P.ldx];
+        } else {
+            vr_[at] = 1.0;
+            vi_[at] = yr_[at] = yi_[at] = 0.0;
+        }
+    }
+    const dcplx mu = act ? cmk(P.wr[k], P.wr[k + 1]) : cmk(0.0, 0.0);
+    const double smin = fmax(DBL_EPSILON / 2 * cabs1(mu), P.smlnum);
+    double beta = act ? P.beta[(size_t)J * Spad + k] : sc_one(is);
+    int pert = 0;
+    const double *Hd = P.H + l + (size_t)l * P.ldh;
+    auto stage_col = [&](int col) {                                    // H(l : l+col+1, l+col), warp 4
+        if (col >= 0) {
+            const int rows = min(col + 2, b);
+            const double *src = Hd + (size_t)col * P.ldh;
+            double *dst = HCOL(col);
+            for (int i = lane; i < rows; i += 32) cp_async8(dst + i, src + i);
+        }
+        cp_async_commit();                                             // one group per column, empty ones too
+    };
+    if (wid == 4) {
+        stage_col(b - 2);
+        stage_col(b - 3);
+    }
+    __syncthreads();                                                   // tile and barriers ready
+
+    // The barriers of step t = b - 1 - j, as in diag_body_narrow.
+    constexpr int kRot = 0, kSys = 2, kFac = 4, kRows = 6;
+    bool ok = true;
+    auto await = [&](int which, int t) { ok = ok && mbar_wait(&bars[which + (t & 1)], (uint32_t)((t >> 1) & 1), P.err); };
+    auto post = [&](int which, int t) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars[which + (t & 1)]);
+    };
+    constexpr unsigned kAll = 0xffffffffu;
+    auto even_of = [&](double x) { return __shfl_sync(kAll, x, sh); };             // the even group's value
+    auto odd_of = [&](double x) { return __shfl_sync(kAll, x, sh + SC); };
+    auto hi_mag = [](double x) { return (unsigned)(ubits(x) >> 32) & 0x7fffffffu; };
+    auto hi_pow2 = [](int e) { return (unsigned)(pow2_bits(e) >> 32); };
+
+    dcplx v0 = cmk(0.0, 0.0), y0 = v0;                                 // rows 0 of v (warp 0) and y (warp 1)
+    if (wid == 0) {
+        dcplx vj = cmk(VR(b - 1), VI(b - 1)), vw = b >= 2 ? cmk(VR(b - 2), VI(b - 2)) : vj;   // v(j), v(j-1)
+        auto entry = [&](int row, int col) { return col >= 0 && row >= 0 ? Hd[row + (size_t)col * P.ldh] : 0.0; };
+        double hsub = entry(b - 1, b - 2), hdiag = entry(b - 2, b - 2) - mu.re, htop = entry(b - 3, b - 2);
+        double hs1 = entry(b - 2, b - 3), hd1 = entry(b - 3, b - 3), ht1 = entry(b - 4, b - 3);
+        for (int j = b - 1, t = 0; j >= 1; --j, ++t) {
+            double c;
+            dcplx sg;
+            {
+                // cgivens() with the quotients of one divisor on two lane groups.
+                const unsigned long long mr = mag(vj.re), mi = mag(vj.im), mg = mag(hsub);
+                const unsigned long long lo = pow2_bits(-200), hi = pow2_bits(200);
+                const bool in = mr > lo && mr < hi && mi > lo && mi < hi && mg > lo && mg < hi;
+                const int ef = (int)(umax64(mr, mi) >> 52) - 1023, eg = (int)(mg >> 52) - 1023, e = ef > eg ? ef : eg;
+                const double fsr = add_exp(vj.re, -ef), fsi = add_exp(vj.im, -ef);
+                double q1, q2;
+                bool okq = true;
+                auto quots = [&](double ss, double a1) {               // a1 / sqrt(ss) per group; the root returned
+                    unsigned long long y;
+                    const unsigned long long db = ip_sqrt(in ? ubits(ss) : kOneBits + 1, y), fb = db & kSigMask, u = ubits(a1);
+                    const int ea = (int)((u >> 52) & 0x7ff), eb = (int)(db >> 52);
+                    okq = okq && ip_div_ok(ea, eb, fb);
+                    q1 = from_bits(ip_quot((u & kSigMask) | kHidden, fb | kHidden, ip_recip_root(db, y), ea - eb + 1023,
+                                           u & 0x8000000000000000ULL));
+                    return from_bits(db);
+                };
+                const double af1 = quots(fma(fsr, fsr, fsi * fsi), odd ? fsi : fsr);
+                q2 = q1;                                               // pr, pi
+                const double af = add_exp(af1, ef - e), gs = add_exp(hsub, -e);
+                quots(fma(af, af, gs * gs), odd ? gs : af);            // c, t
+                if (__all_sync(kAll, (in && okq) || !act)) {            // pairs past the last count as in range
+                    c = even_of(q1);
+                    const double tt = odd_of(q1), sp = tt * q2;
+                    sg = cmk(neg(even_of(sp)), odd_of(sp));
+                } else {
+                    cgivens(vj, hsub, c, sg);
+                }
+            }
+            if (store_lane) {
+                SA(t, 0) = c;
+                SA(t, 1) = sg.re;
+                SA(t, 2) = sg.im;
+                SA(t, 3) = vj.re;
+                SA(t, 4) = vj.im;
+                SA(t, 5) = vw.re;
+                SA(t, 6) = vw.im;
+            }
+            post(kRot, t);
+            if (act && store_lane) {
+                P.Cr[(size_t)(l + j) * Spad + k] = c;
+                P.Sr[(size_t)(l + j) * Spad + k] = sg.re;
+                P.Sr[(size_t)(l + j) * Spad + k + 1] = sg.im;
+            }
+            const double hdu = hdiag, htu = htop;                      // the next step's, off the chain's path
+            hsub = hs1;
+            hdiag = hd1 - mu.re;
+            htop = ht1;
+            hs1 = entry(j - 2, j - 3);
+            hd1 = entry(j - 3, j - 3);
+            ht1 = entry(j - 4, j - 3);
+            await(kRows, t);                                           // rows of step j+1: row j-2 is in v
+            const dcplx vo = !odd ? vw : (j >= 2 ? cmk(VR(j - 2), VI(j - 2)) : cmk(0.0, 0.0));
+            const dcplx sv = cmul(sg, vo);
+            const double nr = fma(c, !odd ? hdu : htu, sv.re), ni = !odd ? fma(c, -mu.im, sv.im) : sv.im;
+            vj = cmk(even_of(nr), even_of(ni));
+            vw = cmk(odd_of(nr), odd_of(ni));
+        }
+        v0 = vj;
+    } else if (wid == 4) {
+        for (int j = b - 1, t = 0; j >= 1; --j, ++t) {
+            cp_async_wait_one();                                       // column j-1, for the other warps too
+            await(kRot, t);
+            __syncwarp();
+            const double hsub = HCOL(j - 1)[j], hdg = HCOL(j - 1)[j - 1] - mu.re;
+            const double x0 = (odd ? SA(t, 1) : SA(t, 0)) * (odd ? hsub : SA(t, 3));
+            const double x1 = (odd ? neg(SA(t, 2)) : SA(t, 0)) * (odd ? hsub : SA(t, 4));
+            const double tr = even_of(x0), lr = odd_of(x0), ti = even_of(x1), li = odd_of(x1);
+            const double csr = tr - lr, csi = ti - li;
+            // csolve_1x1's conditions on the coefficient, the second
+            // decision's on v(j-1) and H (a |Re| + |Im| below 2^497).
+            const unsigned lim = hi_pow2(200), l495 = hi_pow2(495);
+            const bool swap = mag(csi) >= mag(csr);
+            const double cc = swap ? csi : csr, dd = swap ? csr : csi;
+            bool plain = hi_mag(tr) < lim && hi_mag(ti) < lim && hi_mag(lr) < lim && hi_mag(li) < lim &&
+                         mag(dd) > pow2_bits(-200) && hi_mag(SA(t, 5)) < l495 && hi_mag(SA(t, 6)) < l495 &&
+                         hi_mag(hdg) < l495 && hi_mag(mu.im) < l495;
+            plain = plain && !(ubits(absd(csr) + absd(csi)) < ubits(smin));
+            double r = 0.0, tq = 0.0;
+            if (plain) {
+                r = ddiv_rn(dd, cc);
+                tq = ddiv_rn(1.0, cc + dd * r);
+            }
+            if (store_lane) {
+                SX(t, 0) = r;
+                SX(t, 1) = tq;
+                SX(t, 2) = from_bits(plain ? (swap ? 1ULL : 0ULL) : 2ULL);
+                SX(t, 3) = hdg;
+            }
+            post(kSys, t);
+            if (t > 0) await(kFac, t - 1);                             // column j+1 gives way
+            stage_col(j - 3);
+        }
+    } else if (wid == 1) {
+        const double Hnorm = P.Hn[J + (size_t)J * P.T];
+        const unsigned l200 = hi_pow2(200), lm400 = hi_pow2(-400), l490 = hi_pow2(490), l495 = hi_pow2(495), l497 = hi_pow2(497),
+                       l990 = hi_pow2(990), l993 = hi_pow2(993);
+        // fits: parts of y below 2^990 and of v below 2^490 before a step
+        // without scaling whose factors' parts are below 2^497 give parts
+        // below 2^991 and 2^492 after it (|c|, |sigma| <= 1, |H| < 2^490).
+        const bool hfits = hi_mag(Hnorm) < l490;
+        bool fits = false;
+        // The lane's part (real in even groups) of y(j) and y(j-1).
+        double ycar = odd ? YI(b - 1) : YR(b - 1), ynext = b >= 2 ? (odd ? YI(b - 2) : YR(b - 2)) : 0.0;
+        unsigned ymh = 0, vmh = 0;
+        auto bounds = [&](int t) {
+            ymh = vmh = 0;
+#pragma unroll
+            for (int w = 0; w < NR; ++w) {
+                ymh = max(ymh, PM(t, w, 0));
+                vmh = max(vmh, PM(t, w, 1));
+            }
+        };
+        auto other = [&](double x) { return __shfl_xor_sync(kAll, x, SC); };
+        for (int j = b - 1, t = 0; j >= 1; --j, ++t) {
+            await(kSys, t);
+            const double *hcol = HCOL(j - 1);
+            const double c = SA(t, 0), r = SX(t, 0), tq = SX(t, 1), hdg = SX(t, 3);
+            const dcplx sg = cmk(SA(t, 1), SA(t, 2)), vjm1 = cmk(SA(t, 5), SA(t, 6)), hd = cmk(hdg, -mu.im);
+            const unsigned kind = (unsigned)ubits(SX(t, 2));
+            double yold = ynext, a1 = 1.0, a2 = 1.0, a3 = 1.0, yjm1 = 0.0;
+            const double yo = other(ycar);
+            // (a + b r) t and (b - a r) t of c_dladiv: x.re and x.im, or with
+            // the parts exchanged x.re and -x.im.
+            const bool swap = kind == 1;
+            const double xre = odd ? yo : ycar, xim = odd ? ycar : yo;
+            const double pa = swap ? xim : xre, pb = swap ? xre : xim;
+            double yj = ((odd ? pb : pa) + (odd ? neg(pa) : pb) * r) * tq;
+            if (odd && swap) yj = neg(yj);
+            bool plain = kind < 2 && hi_mag(ycar) < l200 && hi_mag(ycar) > lm400 && hi_mag(yj) < l495 && hi_mag(yold) < l993 && fits;
+            plain = __all_sync(kAll, plain || !act);
+            double yc, ysc;                                            // the lane's parts of yc and ys
+            if (plain) {
+                const double yjo = other(yj);
+                yc = c * yj;
+                const double m = sg.im * yjo;
+                ysc = fma(sg.re, yj, odd ? neg(m) : m);
+            } else {
+                dcplx x = cmk(xre, xim), yp = cmk(even_of(yold), odd_of(yold));
+                double phi = sc_one(is);
+                pert |= csolve_1x1(smin, mul_rare(c, SA(t, 3)), mul_rare(c, SA(t, 4)), mul_rare(sg.re, hcol[j]),
+                                   mul_rare(-sg.im, hcol[j]), x, phi, is);
+                beta = sc_combine(beta, phi, is);
+                a1 = sc_value(phi, is);
+                if (!is_one(a1)) yp = cscal(a1, yp);
+                phi = protect_double_update(cabs1(vjm1), cabs1(x), cabs1(hd), cabs1(x), cabs1(yp), is);
+                a2 = sc_value(phi, is);
+                if (!is_one(a2)) {
+                    x = cscal(a2, x);
+                    yp = cscal(a2, yp);
+                }
+                beta = sc_combine(beta, phi, is);
+                dcplx zc = cscal(c, x), zs = cmulc(sg, x);
+                await(kRows, t);                                       // rows of step j+1
+                unsigned long long ymb = 0, vmb = 0;                   // the maxima over rows 0 .. j-2
+                bounds(t);
+                if (!(ymh < l993 && vmh < l495 && hi_mag(x.re) < l495 && hi_mag(x.im) < l495 && hi_mag(Hnorm) < l497 &&
+                      is_one(a1) && is_one(a2))) {
+                    for (int i = 0; i <= j - 2; ++i) {
+                        ymb = umax64(ymb, abs_bits(cabs1(cmk(YR(i), YI(i)))));
+                        vmb = umax64(vmb, abs_bits(cabs1(cmk(VR(i), VI(i)))));
+                    }
+                    double ymax = from_bits(ymb);
+                    if (!is_one(a1)) ymax = a1 * ymax;
+                    if (!is_one(a2)) ymax = a2 * ymax;
+                    phi = protect_double_update(from_bits(vmb), cabs1(x), Hnorm, cabs1(x), ymax, is);
+                    a3 = sc_value(phi, is);
+                    beta = sc_combine(beta, phi, is);
+                }
+                if (!is_one(a3)) {
+                    const dcplx z = cscal(a3, cfma(zs, hd, cfnma(zc, vjm1, yp)));
+                    yjm1 = odd ? z.im : z.re;
+                    x = cscal(a3, x);
+                    zc = cscal(c, x);
+                    zs = cmulc(sg, x);
+                }
+                yj = odd ? x.im : x.re;
+                yold = odd ? yp.im : yp.re;
+                yc = odd ? zc.im : zc.re;
+                ysc = odd ? zs.im : zs.re;
+            }
+            const bool scaled = !is_one(a1) || !is_one(a2) || !is_one(a3);
+            if (lane < 2 * SC) {
+                SB(t, odd ? 1 : 0) = yc;
+                SB(t, odd ? 3 : 2) = ysc;
+                if (odd) YI(j) = yj;
+                else YR(j) = yj;
+            }
+            if (store_lane) {
+                SB(t, 4) = a1;
+                SB(t, 5) = a2;
+                SB(t, 6) = a3;
+            }
+            post(kFac, t);
+            // y - yc v: fma(-yc.re, v.re, fma(yc.im, v.im, y.re)) and
+            // fma(-yc.re, v.im, fma(-yc.im, v.re, y.im)).
+            const double yco = other(yc), yso = other(ysc);
+            const double ycr = odd ? yco : yc, yci = odd ? yc : yco, ysr = odd ? yso : ysc, ysi = odd ? ysc : yso;
+            auto minus = [&](dcplx v, double y) {
+                return fma(-ycr, odd ? v.im : v.re, fma(odd ? neg(yci) : yci, odd ? v.re : v.im, y));
+            };
+            if (is_one(a3)) {
+                const double u = minus(vjm1, yold);
+                yjm1 = fma(ysr, odd ? hd.im : hd.re, fma(odd ? ysi : neg(ysi), odd ? hd.re : hd.im, u));
+            }
+            // Row j-2 of y, for the next step's chain, and the bounds of the
+            // rows of step j+1.
+            await(kRows, t);
+            bounds(t);
+            fits = hfits && !scaled && ymh < l990 && vmh < l490 && hi_mag(yc) < l497 && hi_mag(yco) < l497 &&
+                   hi_mag(ysc) < l497 && hi_mag(yso) < l497;
+            if (j >= 2) {
+                double yi = odd ? YI(j - 2) : YR(j - 2);
+                if (scaled) {
+                    if (!is_one(a1)) yi = a1 * yi;
+                    if (!is_one(a2)) yi = a2 * yi;
+                    if (!is_one(a3)) yi = a3 * yi;
+                }
+                ynext = fma(odd ? ysi : ysr, hcol[j - 2], minus(cmk(VR(j - 2), VI(j - 2)), yi));
+            }
+            ycar = yjm1;
+        }
+        y0 = cmk(even_of(ycar), odd_of(ycar));
+    } else {
+        unsigned ym = 0, vm = 0;
+        auto note = [&](dcplx y, dcplx v) {
+            ym = max(ym, max(hi_mag(y.re), hi_mag(y.im)));
+            vm = max(vm, max(hi_mag(v.re), hi_mag(v.im)));
+        };
+        auto fold = [&](int tm) {
+#pragma unroll
+            for (int o = SC; o < 32; o <<= 1) {
+                ym = max(ym, __shfl_xor_sync(kAll, ym, o));
+                vm = max(vm, __shfl_xor_sync(kAll, vm, o));
+            }
+            if (store_lane) {
+                PM(tm, rw, 0) = ym;
+                PM(tm, rw, 1) = vm;
+            }
+            post(kRows, tm);
+        };
+        for (int i = rw * RL + rs; i < b - 2; i += NR * RL) note(cmk(YR(i), YI(i)), cmk(VR(i), VI(i)));
+        fold(0);
+        for (int j = b - 1, t = 0; j >= 1; --j, ++t) {
+            await(kFac, t);                                            // ... and with it the rotation and the column
+            const double c = SA(t, 0), s1 = SB(t, 4), s2 = SB(t, 5), s3 = SB(t, 6);
+            const dcplx sg = cmk(SA(t, 1), SA(t, 2)), yc = cmk(SB(t, 0), SB(t, 1)), ys = cmk(SB(t, 2), SB(t, 3));
+            const double *hcol = HCOL(j - 1);
+            const bool scaled = !is_one(s1) || !is_one(s2) || !is_one(s3);
+            auto rescale = [&](dcplx y) {
+                if (!is_one(s1)) y = cscal(s1, y);
+                if (!is_one(s2)) y = cscal(s2, y);
+                if (!is_one(s3)) y = cscal(s3, y);
+                return y;
+            };
+            if (scaled) {
+                for (int q = j + 1 + rw * RL + rs; q < b; q += NR * RL) {
+                    const dcplx u = rescale(cmk(YR(q), YI(q)));
+                    YR(q) = u.re;
+                    YI(q) = u.im;
+                }
+            }
+            ym = vm = 0;
+            constexpr int ST = NR * RL;
+            const int lim = j - 2;                                     // rows 0 .. j-3
+            int i = rw * RL + rs;
+            auto rows = [&](auto tag) {
+                constexpr int U = decltype(tag)::value;
+                double h[U];
+                dcplx y[U], v[U];
+#pragma unroll
+                for (int q = 0; q < U; ++q) {
+                    h[q] = hcol[i + q * ST];
+                    y[q] = cmk(YR(i + q * ST), YI(i + q * ST));
+                    v[q] = cmk(VR(i + q * ST), VI(i + q * ST));
+                    if (scaled) y[q] = rescale(y[q]);
+                }
+#pragma unroll
+                for (int q = 0; q < U; ++q) {
+                    y[q] = cfmar(ys, h[q], cfnma(yc, v[q], y[q]));
+                    const dcplx sv = cmul(sg, v[q]);
+                    v[q] = cmk(fma(c, h[q], sv.re), sv.im);
+                }
+#pragma unroll
+                for (int q = 0; q < U; ++q) {
+                    YR(i + q * ST) = y[q].re;
+                    YI(i + q * ST) = y[q].im;
+                    VR(i + q * ST) = v[q].re;
+                    VI(i + q * ST) = v[q].im;
+                    note(y[q], v[q]);
+                }
+            };
+            for (; i + ST < lim; i += 2 * ST) rows(std::integral_constant<int, 2>{});
+            for (; i < lim; i += ST) rows(std::integral_constant<int, 1>{});
+            fold(t + 1);
+        }
+    }
+    __syncthreads();                                                   // the last step's rows written
+
+    double c0 = 1.0;
+    dcplx s0 = cmk(0.0, 0.0);
+    if (wid == 0) {
+        if (J > 0) {
+            // Final rotation with H(l, l-1) (reduce.c:53-61).
+            const double hleft = P.H[l + (size_t)(l - 1) * P.ldh];
+            if (hleft != 0) cgivens(v0, hleft, c0, s0);
+            if (act && store_lane) {
+                P.Cr[(size_t)l * Spad + k] = c0;
+                P.Sr[(size_t)l * Spad + k] = s0.re;
+                P.Sr[(size_t)l * Spad + k + 1] = s0.im;
+            }
+            v0 = cmk(fma(v0.re, c0, -(hleft * s0.re)), fma(v0.im, c0, hleft * s0.im));
+        }
+        if (store_lane) {
+            SA(0, 0) = c0;
+            SA(0, 1) = s0.re;
+            SA(0, 2) = s0.im;
+            SA(0, 3) = v0.re;
+            SA(0, 4) = v0.im;
+        }
+    }
+    __syncthreads();
+    c0 = SA(0, 0);
+    s0 = cmk(SA(0, 1), SA(0, 2));
+    if (wid == 1) {
+        double phi = sc_one(is);
+        pert |= csolve_1x1(smin, SA(0, 3), SA(0, 4), 0.0, 0.0, y0, phi, is);
+        beta = sc_combine(beta, phi, is);
+        if (store_lane) SB(0, 4) = sc_value(phi, is);
+    }
+    __syncthreads();
+    {
+        const double a = SB(0, 4);
+        if (!is_one(a))
+            for (int i = 1 + wid * RL + rs; i < b; i += NW * RL) {
+                YR(i) = a * YR(i);
+                YI(i) = a * YI(i);
+            }
+        if (wid == 1 && store_lane) {
+            YR(0) = y0.re;
+            YI(0) = y0.im;
+        }
+    }
+    __syncthreads();
+
+    for (int idx = tid; idx < SC * b; idx += 32 * NW) {
+        const int c = idx / b, i = idx - c * b, pc = p0 + c;
+        if (pc < np) {
+            double *xr = P.X + l + i + (size_t)(2 * pc) * P.ldx;
+            xr[0] = yr_[(size_t)i * SC + c];
+            xr[P.ldx] = yi_[(size_t)i * SC + c];
+        }
+    }
+    if (act && wid == 1 && store_lane) {
+        P.beta[(size_t)J * Spad + k] = beta;
+        if (pert) P.pert[k] = P.pert[k + 1] = 1;
+    }
+    if (J == 0) return;
+
+    // The stage operands, a lane's part each (whole warps: the parts meet by
+    // exchange; groups past the second repeat the first two).
+    const int kk = act ? k : 0;
+    const bool st = act && lane < 2 * SC;
+    if (wid == 0) {
+        // W(q) = c_q prod_{p<q} sigma_p, pi = prod sigma (crossover propagation).
+        double pk = odd ? 0.0 : 1.0;
+        for (int q = 0; q < b; ++q) {
+            const double cq = P.Cr[(size_t)(l + q) * Spad + kk];
+            const dcplx sq = cmk(P.Sr[(size_t)(l + q) * Spad + kk], P.Sr[(size_t)(l + q) * Spad + kk + 1]);
+            if (st) P.W[(size_t)q * Spad + k + (odd ? 1 : 0)] = cq * pk;
+            // cmul(pk, sq)
+            const double po = __shfl_xor_sync(kAll, pk, SC), pr = odd ? po : pk, pi = odd ? pk : po;
+            const double m = pi * (odd ? sq.re : sq.im);
+            pk = fma(pr, odd ? sq.im : sq.re, odd ? m : neg(m));
+        }
+        if (st) P.pi[k + (odd ? 1 : 0)] = pk;
+    }
+    if (wid == 1) {
+        // Ytilde2 (update-task.c:170-198): Zs(q) = Ytilde2(q-1), Zs(0) = 0,
+        // zlast = Ytilde2(b-1); ytilde = -conj(sigma_0) x_0 for Part 1.
+        unsigned long long zmx = 0;
+        const double x0 = odd ? YI(0) : YR(0);
+        double z = c0 * x0;
+        if (st) P.Zs[k + (odd ? 1 : 0)] = 0.0;
+        for (int q = 1; q < b; ++q) {
+            const double cq = P.Cr[(size_t)(l + q) * Spad + kk];
+            const dcplx sq = cmk(P.Sr[(size_t)(l + q) * Spad + kk], P.Sr[(size_t)(l + q) * Spad + kk + 1]);
+            const double t2 = odd ? YI(q) : YR(q), t2o = odd ? YR(q) : YI(q), zo_ = __shfl_xor_sync(kAll, z, SC);
+            // crot_out: c z - conj(s) t2; crot_next: c t2 + s z.
+            const double m = sq.im * t2o;
+            const double q2 = fma(sq.re, t2, odd ? neg(m) : m);
+            const double zo = fma(cq, z, neg(q2));
+            const double mz = sq.im * zo_;
+            const double p2 = fma(sq.re, z, odd ? mz : neg(mz));
+            z = fma(cq, t2, p2);
+            if (st) P.Zs[(size_t)q * Spad + k + (odd ? 1 : 0)] = zo;
+            zmx = umax64(zmx, abs_bits(absd(zo) + absd(__shfl_xor_sync(kAll, zo, SC))));
+        }
+        const double zc = __shfl_xor_sync(kAll, z, SC);
+        zmx = umax64(zmx, abs_bits(absd(z) + absd(zc)));
+        if (st) P.zlast[k + (odd ? 1 : 0)] = z;
+        if (act && store_lane) {
+            P.z2n[k] = from_bits(zmx);
+            const dcplx q0 = cmulc(s0, cmk(YR(0), YI(0)));
+            P.ytil[k] = -q0.re;
+            P.ytil[k + 1] = -q0.im;
+        }
+    }
+#undef VR
+#undef VI
+#undef YR
+#undef YI
+#undef SA
+#undef SX
+#undef SB
+#undef PM
+#undef HCOL
+}
+
+// Pairs per CTA of the narrow form (0: the wide one): the smallest that fits
+// one wave.
+int diag_c_narrow(int np) {
+    const int sms = device_sms();
+    for (int sc = 4; sc <= 16; sc *= 2)
+        if ((np + sc - 1) / sc <= sms) return sc;
+    return 0;
+}
+template <int SC>
+cudaError_t launch_diag_cn(const DevProblem &P, int J, int b, cudaStream_t st) {
+    static size_t configured = 0;
+    const size_t smem = diag_cn_smem_bytes<SC>(b);
+    const cudaError_t e = raise_smem_limit((const void *)k_diag_cn<SC>, &configured, smem);
+    if (e != cudaSuccess) return e;
+    k_diag_cn<SC><<<(P.S / 2 + SC - 1) / SC, 32 * kNarrowCWarps, smem, st>>>(P, J);
+    return cudaGetLastError();
+}
+
 // The dynamic shared-memory limit of each k_diag_c form only ever grows.
 template <int NW>
 cudaError_t diag_c_smem_attr(size_t smem) {
@@ -487,6 +1048,11 @@ cudaError_t diag_c_smem_attr(size_t smem) {
 }
 
 cudaError_t launch_diag_c(const DevProblem &P, int J, int b, double *gscratch, cudaStream_t st) {
+    // (A tile too high for the narrow form's shared memory takes the wide one.)
+    const int sc = diag_c_narrow(P.S / 2);
+    if (sc == 4 && diag_cn_smem_bytes<4>(b) <= kNarrowCSmem) return launch_diag_cn<4>(P, J, b, st);
+    if (sc == 8 && diag_cn_smem_bytes<8>(b) <= kNarrowCSmem) return launch_diag_cn<8>(P, J, b, st);
+    if (sc == 16 && diag_cn_smem_bytes<16>(b) <= kNarrowCSmem) return launch_diag_cn<16>(P, J, b, st);
     bool gvy = false;
     const size_t smem = diag_c_smem_bytes(b, &gvy);
     if (gvy && !gscratch) return cudaErrorInvalidValue;

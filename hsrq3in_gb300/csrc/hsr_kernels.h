@@ -69,6 +69,7 @@ cudaError_t launch_norms(const DevProblem &P, unsigned long long *Hn_bits,
 // 2: caller right-hand sides already in X.
 cudaError_t launch_init(const DevProblem &P, int mode, const double *eps3_dev,
                         int its, cudaStream_t st);
+int device_sms();                    // SMs of the current device (0 if unknown)
 cudaError_t launch_diag(const DevProblem &P, int J, int b, double *gscratch, cudaStream_t st);
 // Few shifts: tile J's diagonal solve preceded, in the same CTAs, by the GEMM
 // of stage J+1 over tile J's rows (Pg: the descriptor with stage J+1's
