@@ -748,8 +748,12 @@ int run_pass_c(Solver &s, int mode, int its, int off, int cnt) {
             HSR_LAUNCH_C(kcPart1, M, launch_part1_c(P, J, M));
             HSR_CK(cudaEventRecord(w.ev_top, M));
             HSR_CK(cudaStreamWaitEvent(D, w.ev_top, 0));
-            HSR_LAUNCH_C(kcGemmTop, D,
-                         launch_gemm_c(P, J, s.fr[J - 1], s.fr[J], s.tmH, s.tmW[J & 1], s.tmZ[J & 1], D));
+            if (gemm_prefers_narrow(s.fr[J] - s.fr[J - 1], cc))
+                HSR_LAUNCH_C(kcGemmTop, D,
+                             launch_gemm_c_narrow(P, J, s.fr[J - 1], s.fr[J], s.tmH, s.tmWn[J & 1], s.tmZn[J & 1], D));
+            else
+                HSR_LAUNCH_C(kcGemmTop, D,
+                             launch_gemm_c(P, J, s.fr[J - 1], s.fr[J], s.tmH, s.tmW[J & 1], s.tmZ[J & 1], D));
             HSR_LAUNCH_C(kcDiag, D, launch_diag_c(Pn, J - 1, s.fr[J] - s.fr[J - 1], gs, D));
             HSR_CK(cudaEventRecord(w.ev_diag, D));
             if (s.fr[J - 1] > 0)
@@ -849,6 +853,12 @@ int solve_device_cplx(int n, const double *dH, long long ldh, int np, double *dw
         !make_map(&s.tmZ[1], w.Zs.as<double>() + (size_t)tlsz * Sp, Sp, (unsigned long long)tlsz, Sp, kGemmBN,
                   kGemmKC))
         return HSR_ERR_CUDA;
+    for (int par = 0; par < 2; ++par)
+        if (!make_map(&s.tmWn[par], w.W.as<double>() + (size_t)par * tlsz * Sp, Sp, (unsigned long long)tlsz, Sp,
+                      kGemmBNNarrow, kGemmKC) ||
+            !make_map(&s.tmZn[par], w.Zs.as<double>() + (size_t)par * tlsz * Sp, Sp, (unsigned long long)tlsz, Sp,
+                      kGemmBNNarrow, kGemmKC))
+            return HSR_ERR_CUDA;
 
     unsigned long long *bits = w.bits.as<unsigned long long>();
     HSR_CK(cudaMemsetAsync(bits, 0, (2 * (size_t)T * T + 2) * 8, st));

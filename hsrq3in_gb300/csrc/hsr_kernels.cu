@@ -1970,6 +1970,7 @@ size_t gemm_narrow_smem_bytes() { return sizeof(GemmSmemT<kGemmBNNarrow>) + 128;
 // epilogue becomes its complex counterpart (crossover coefficient pi, Part-1
 // ytilde, shift mu, zlast, the old crossover column); the bound folded into
 // ynorm is the largest cabs1 of the pair's rows, kept at column 2p.
+template <int BN>
 __device__ __forceinline__ void gemm_epilogue_cplx(const DevProblem &P, int J, int row_lo, int row_hi, int row0,
                                                    int col0, const double *eaw, const double *eaz, int kEpiLd) {
     const int tid = threadIdx.x;
@@ -1984,8 +1985,8 @@ __device__ __forceinline__ void gemm_epilogue_cplx(const DevProblem &P, int J, i
     if (I < 0) I = 0;
     const int key = rowok ? I : -1;
     const double hl1 = rowok ? P.H[row + (size_t)(l - 1) * P.ldh] : 0.0;
-    for (int j = 0; j < kGemmBN / 4; j += 2) {
-        const int cc = cg * (kGemmBN / 4) + j;
+    for (int j = 0; j < BN / 4; j += 2) {
+        const int cc = cg * (BN / 4) + j;
         const int col = col0 + cc;
         if (col >= P.S) break;
         const dcplx pik = cmk(P.pi[col], P.pi[col + 1]);
@@ -2042,7 +2043,7 @@ template <bool kCplx, int BN = kGemmBN>
 __device__ __forceinline__ void gemm_body(const DevProblem &P, int J, int row_lo, int row_hi, int bx, int by,
                                           const CUtensorMap *tmH, const CUtensorMap *tmW,
                                           const CUtensorMap *tmZ) {
-    static_assert(BN == kGemmBN || (BN == kGemmBNNarrow && !kCplx), "tile widths");
+    static_assert(BN == kGemmBN || BN == kGemmBNNarrow, "tile widths");
     // Threads per row of the tile (4 columns each) and rows per thread.
     constexpr int TC = BN / 4, RPT = kGemmBM * TC / 256;
     static_assert(RPT == 4 || RPT == 1, "thread tile");
@@ -2165,7 +2166,7 @@ __device__ __forceinline__ void gemm_body(const DevProblem &P, int J, int row_lo
     }
     __syncthreads();
     if constexpr (kCplx) {
-        gemm_epilogue_cplx(P, J, row_lo, row_hi, row0, col0, eaw, eaz, kEpiLd);
+        gemm_epilogue_cplx<BN>(P, J, row_lo, row_hi, row0, col0, eaw, eaz, kEpiLd);
         return;
     }
 
@@ -2261,6 +2262,29 @@ cudaError_t launch_gemm(const DevProblem &P, int J, int row_lo, int row_hi, cons
     const int span = row_hi - (row_lo & ~7);
     dim3 g((span + kGemmBM - 1) / kGemmBM, (P.S + kGemmBN - 1) / kGemmBN);
     k_gemm<<<g, 256, smem, st>>>(P, J, row_lo, row_hi, tmH, tmW, tmZ);
+    return cudaGetLastError();
+}
+
+__global__ void __launch_bounds__(256, 2)
+k_gemm_cn(DevProblem P, int J, int row_lo, int row_hi, const __grid_constant__ CUtensorMap tmH,
+          const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmZ) {
+    gemm_body<true, kGemmBNNarrow>(P, J, row_lo, row_hi, blockIdx.x, blockIdx.y, &tmH, &tmW, &tmZ);
+}
+
+// launch_gemm_narrow with the complex epilogue, for the rows of the next tile
+// that gate its diagonal solve: at n = 2000 with 500 pairs (160 rows, 1000
+// columns) 169 us a tile on 189 CTAs, against 340 us on 48 CTAs with the
+// 64-column tiles; the solve 18.28 -> 17.73 ms.
+cudaError_t launch_gemm_c_narrow(const DevProblem &P, int J, int row_lo, int row_hi, const CUtensorMap &tmH,
+                                 const CUtensorMap &tmW, const CUtensorMap &tmZ, cudaStream_t st) {
+    static size_t configured = 0;
+    const size_t smem = gemm_narrow_smem_bytes();
+    const cudaError_t e = raise_smem_limit((const void *)k_gemm_cn, &configured, smem);
+    if (e != cudaSuccess) return e;
+    if (row_hi <= row_lo) return cudaSuccess;
+    const int span = row_hi - (row_lo & ~7);
+    dim3 g((span + kGemmBM - 1) / kGemmBM, (P.S + kGemmBNNarrow - 1) / kGemmBNNarrow);
+    k_gemm_cn<<<g, 256, smem, st>>>(P, J, row_lo, row_hi, tmH, tmW, tmZ);
     return cudaGetLastError();
 }
 

@@ -178,6 +178,8 @@ cudaError_t launch_init_c(const DevProblem &P, int mode, const double *eps3_dev,
 size_t diag_c_smem_bytes(int b, bool *global_vy);
 cudaError_t launch_diag_c(const DevProblem &P, int J, int b, double *gscratch, cudaStream_t st);
 cudaError_t launch_part1_c(const DevProblem &P, int J, cudaStream_t st);
+cudaError_t launch_gemm_c_narrow(const DevProblem &P, int J, int row_lo, int row_hi, const CUtensorMap &tmH,
+                                 const CUtensorMap &tmW, const CUtensorMap &tmZ, cudaStream_t st);
 cudaError_t launch_gemm_c(const DevProblem &P, int J, int row_lo, int row_hi, const CUtensorMap &tmH,
                           const CUtensorMap &tmW, const CUtensorMap &tmZ, cudaStream_t st);
 // colnorm/status per column (both columns of a pair), scale_out per pair.
