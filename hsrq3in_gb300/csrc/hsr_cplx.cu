@@ -9,11 +9,14 @@
 //               solve-task.c:19-225), the complex 1x1 solves going through the
 //               robust complex division of robust.c:486-773; then the stage
 //               operands W and Zs
+//   k_diag_cn   the same for few pairs: 4, 8 or 16 per CTA, the two chains and
+//               the 1x1 systems on warps of their own
 //   k_part1_c   the exact no-rescale test per (tile, pair), the full complex
 //               Part 1 of update-task.c:68-226 where a decision can fire
-//   k_gemm_c    the real GEMM over H (hsr_kernels.cu) with a complex epilogue:
-//               the imaginary parts are just more columns of W and Zs
-//   k_finalize_c  reconciliation, complex back-transform, 2-norm, convergence
+//   k_gemm_c, k_gemm_cn  the real GEMM over H (hsr_kernels.cu) with a complex
+//               epilogue: the imaginary parts are just more columns of W and Zs
+//   k_finalize<true>  (hsr_kernels.cu) reconciliation, complex back-transform,
+//               2-norm, convergence
 // Layout: pair p holds its real part in column 2p and its imaginary part in
 // column 2p+1 of X, R, W, Zs, Zslow and of the per-column scalars pi, ytil,
 // zlast and the shifts; the cosine of a rotation is Cr[.][2p], the complex
@@ -495,7 +498,8 @@ __global__ void __launch_bounds__(32 * NW) k_diag_c(DevProblem P, int J, double 
 //
 // Bound by the rows' FP64 issue (11 instructions of 64 clocks per 32 / SC rows
 // on less than three sub-partitions), so SC is the smallest that still fits
-// one wave of CTAs.  %%CDIAG%%
+// one wave of CTAs.  n = 2000, 500 pairs, tiles of 160: k_diag_c 3,026 us
+// a tile, k_diag_cn<4> 513 us; the whole solve 49.3 -> 18.3 ms.
 constexpr int kNarrowCWarps = 8, kNarrowCRows = 5;
 constexpr size_t kNarrowCSmem = 200 * 1024;
 template <int SC>
@@ -1267,100 +1271,6 @@ __global__ void __launch_bounds__(256) k_part1_c(DevProblem P, int J) {
 cudaError_t launch_part1_c(const DevProblem &P, int J, cudaStream_t st) {
     const int np = P.S / 2;
     k_part1_c<<<(np + kPart1Shifts - 1) / kPart1Shifts, 256, 0, st>>>(P, J);
-    return cudaGetLastError();
-}
-
-// -------------------------------------------------------------- finalize
-// Lane per pair: smin = min_I beta (robust.c:58-82), complex back-transform
-// with the tile upscalings (shifted_Hessenberg_solve.c:153-215), the
-// three-accumulator 2-norm over real and imaginary parts, convergence
-// ||y|| > 0.1/sqrt(n) (:33-40).  Rows pass through shared memory 32 at a
-// time so that both columns of every pair are read and written coalesced.
-__global__ void __launch_bounds__(32) k_finalize_c(DevProblem P, double *colnorm, int *status,
-                                                   double *scale_out) {
-    __shared__ double bre[32][33], bim[32][33];
-    const int lane = threadIdx.x;
-    const int np = P.S / 2;
-    const int p0 = blockIdx.x * 32;
-    const int pidx = p0 + lane;
-    const bool act = pidx < np;
-    const int k = 2 * pidx;
-    const bool is = P.is != 0;
-    const size_t Spad = (size_t)P.Spad;
-    const int n = P.n;
-
-    double smin = act ? P.beta[k] : sc_one(is);
-    for (int I = 1; I < P.T; ++I)
-        if (act) smin = sc_min(smin, P.beta[(size_t)I * Spad + k], is);
-
-    Nrm3 acc;
-    acc.init();
-    dcplx tau1 = cmk(0.0, 0.0);
-    int I = 0;
-    double alpha = act ? sc_upscale(smin, P.beta[k], is) : 1.0;
-    for (int r0 = 0; r0 < n; r0 += 32) {
-        const int rows = min(32, n - r0);
-        __syncwarp();
-        for (int c = 0; c < 32; ++c) {
-            const int pc = p0 + c;
-            if (pc < np && lane < rows) {
-                bre[lane][c] = P.X[r0 + lane + (size_t)(2 * pc) * P.ldx];
-                bim[lane][c] = P.X[r0 + lane + (size_t)(2 * pc + 1) * P.ldx];
-            }
-        }
-        __syncwarp();
-        for (int t = 0; t < rows; ++t) {
-            const int i = r0 + t;
-            if (i == P.fr[I + 1]) {
-                ++I;
-                alpha = act ? sc_upscale(smin, P.beta[(size_t)I * Spad + k], is) : 1.0;
-            }
-            if (i == 0) {
-                tau1 = cscal(alpha, cmk(bre[0][lane], bim[0][lane]));
-                continue;
-            }
-            const dcplx tau2 = cscal(alpha, cmk(bre[t][lane], bim[t][lane]));
-            const double c = act ? P.Cr[(size_t)i * Spad + k] : 0.0;
-            const dcplx s = act ? cmk(P.Sr[(size_t)i * Spad + k], P.Sr[(size_t)i * Spad + k + 1]) : cmk(0.0, 0.0);
-            const dcplx out = crot_out(c, s, tau1, tau2);
-            tau1 = crot_next(c, s, tau1, tau2);
-            acc.add(out.re);
-            acc.add(out.im);
-            if (t == 0) {
-                if (act) {
-                    P.X[(i - 1) + (size_t)k * P.ldx] = out.re;
-                    P.X[(i - 1) + (size_t)(k + 1) * P.ldx] = out.im;
-                }
-            } else {
-                bre[t - 1][lane] = out.re;
-                bim[t - 1][lane] = out.im;
-            }
-        }
-        __syncwarp();
-        for (int c = 0; c < 32; ++c) {
-            const int pc = p0 + c;
-            if (pc < np && lane < rows - 1) {
-                P.X[r0 + lane + (size_t)(2 * pc) * P.ldx] = bre[lane][c];
-                P.X[r0 + lane + (size_t)(2 * pc + 1) * P.ldx] = bim[lane][c];
-            }
-        }
-    }
-    if (act) {
-        P.X[(n - 1) + (size_t)k * P.ldx] = tau1.re;
-        P.X[(n - 1) + (size_t)(k + 1) * P.ldx] = tau1.im;
-        acc.add(tau1.re);
-        acc.add(tau1.im);
-        const double ynrm = acc.finish();
-        const int ok = (ynrm > 0.1 / sqrt((double)n)) ? 1 : 0;
-        colnorm[k] = colnorm[k + 1] = ynrm;
-        status[k] = status[k + 1] = ok;
-        if (scale_out) scale_out[pidx] = smin;
-    }
-}
-
-cudaError_t launch_finalize_c(const DevProblem &P, double *colnorm, int *status, double *scale_out,
-                              cudaStream_t st) {
-    k_finalize_c<<<(P.S / 2 + 31) / 32, 32, 0, st>>>(P, colnorm, status, scale_out);
     return cudaGetLastError();
 }
 

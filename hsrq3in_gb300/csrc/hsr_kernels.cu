@@ -2396,25 +2396,42 @@ __device__ __forceinline__ void finalize_body(const DevProblem &P, int bx, doubl
     finalize_body_buf(P, bx, colnorm, status, scale_out, fb);
 }
 
-// The plain path's form of finalize_body_buf, on two warps for the same 32
-// shifts.  Warp 0 runs only the per-row recurrence (the back-transform
-// rotation of each row, reading X, the cosines and the sines from shared
-// memory) and leaves each row's result in an output buffer.  Warp 1 brings
-// the next 32-row block in with cp.async, and for the block warp 0 finished
-// one step earlier adds the results to the three-accumulator norm in row
-// order and writes them back to X.  The two warps meet at one barrier per
-// block, with double-buffered inputs and outputs.  Every value sees the
-// operations of finalize_body_buf in the same order, so the result is the
-// same bit for bit; the recurrence's warp no longer carries the loads, the
-// norm and the stores between one row's rotation and the next.
+// The plain path's form of finalize_body_buf, on five warps for the same 32
+// columns.  Warp 0 runs the recurrence alone (the next row's carried value;
+// two FP64 instructions a row, three with a complex sine) and leaves the
+// values it carried; warp 1 makes the results of the block before from them;
+// warp 2 adds the results of the block before that to the three-accumulator
+// norm in row order; warp 4 writes those back to X, and warps 3 and 4 keep two
+// blocks of inputs on their way with cp.async.  They meet at one barrier per
+// block.  Every value sees
+// the operations of finalize_body_buf in the same order, so the result is the
+// same bit for bit.
+//
+// A pass with few shifts has few of these CTAs, so its time is the length of
+// one row's step.  With the results on the recurrence's warp and the norm,
+// loads and stores on a second one, n = 1000 with 1000 shifts took 259 us;
+// this way 189 us.
+//
+// kCplx: a lane is one part of a pair (its real part on the even lane, its
+// imaginary part on the odd one, which is how the columns lie), so that a row
+// costs the recurrence three FP64 instructions and one exchange with the
+// neighbour, and the norm takes a pair's two parts in turn.  n = 2000 with 500
+// pairs: 3,399 us with a lane per pair and one warp doing everything, 709 us
+// this way.
+//
+// 16 rows a block: the inputs are held four deep, and 32 rows would leave
+// one CTA per SM, two waves at 10^4 columns.
+constexpr int kFinRows = 16;
 struct FinalizeWs {
-    double x[2][32][33];                 // X rows of the block, [row][shift]
-    double c[2][32][33];                 // cosines, [row][shift]
-    double s[2][32][33];                 // sines, [row][shift]
-    double o[2][32][33];                 // results: o[t] is row r0 - 1 + t
-    double tail[32];                     // the last row's result, for warp 1
+    double x[4][kFinRows][33];           // X rows of the block, [row][column]
+    alignas(16) double c[4][kFinRows][32];   // cosines, [row][column]
+    alignas(16) double s[4][kFinRows][32];   // sines, [row][column]
+    double t[2][kFinRows][33];           // the value carried into the row
+    double o[2][kFinRows][33];           // results: o[t] is row r0 - 1 + t
+    double tail[32];                     // the last row's result, for warp 2
 };
 
+template <bool kCplx>
 __device__ __forceinline__ void finalize_body_ws(const DevProblem &P, int bx, double *colnorm, int *status,
                                                  double *scale_out, FinalizeWs &fw) {
     const int lane = threadIdx.x & 31;
@@ -2425,84 +2442,174 @@ __device__ __forceinline__ void finalize_body_ws(const DevProblem &P, int bx, do
     const bool is = P.is != 0;
     const size_t Spad = (size_t)P.Spad;
     const int n = P.n;
-    const int nb = (n + 31) / 32;
+    const int nb = (n + kFinRows - 1) / kFinRows;
+    // The columns whose cosine, sine parts and scaling factors this lane uses.
+    const int le = kCplx ? lane & ~1 : lane, lo = kCplx ? lane | 1 : lane;
+    const double *beta = P.beta + k0 + le;
 
-    auto stage = [&](int blk) {                                // warp 1
-        const int r0 = blk * 32, rows = min(32, n - r0), q = blk & 1;
-        for (int c = 0; c < 32; ++c) {
-            const int kc = k0 + c;
-            if (kc < P.S && lane < rows) cp_async8(&fw.x[q][lane][c], P.X + r0 + lane + (size_t)kc * P.ldx);
-        }
-        for (int t = 0; t < rows; ++t) {
-            const size_t at = (size_t)(r0 + t) * Spad + k;
-            if (act) {
-                cp_async8(&fw.c[q][t][lane], P.Cr + at);
-                cp_async8(&fw.s[q][t][lane], P.Sr + at);
-            } else {
-                fw.c[q][t][lane] = 0.0;
-                fw.s[q][t][lane] = 0.0;
-            }
+    // x, with its sign changed where `odd` is: by its bits, not in an FP64 instruction.
+    auto flip = [](double x, int odd) {
+        return from_bits((unsigned long long)__double_as_longlong(x) ^ ((unsigned long long)(odd & 1) << 63));
+    };
+
+    // Warp 3 stages the rotations, warp 4 the rows of X.  An empty block still
+    // commits a group: the waits count groups.
+    auto stage_rot = [&](int blk) {
+        const int r0 = blk * kFinRows, rows = min(kFinRows, n - r0), q = blk & 3;
+        const int c = 2 * (lane & 15);                         // Spad is a multiple of 64: columns past S exist
+        for (int t = lane >> 4; t < rows; t += 2) {
+            const size_t at = (size_t)(r0 + t) * Spad + k0 + c;
+            cp_async16(&fw.c[q][t][c], P.Cr + at);
+            cp_async16(&fw.s[q][t][c], P.Sr + at);
         }
         cp_async_commit();
-        cp_async_wait_all();
+    };
+    auto stage_x = [&](int blk) {
+        const int r0 = blk * kFinRows, rows = min(kFinRows, n - r0), q = blk & 3;
+        const int row = lane & (kFinRows - 1);
+        if (row < rows) {
+            const double *xs = P.X + r0 + row + (size_t)(k0 + lane / kFinRows) * P.ldx;
+            const int cols = min(32, P.S - k0);
+            for (int c = lane / kFinRows; c < cols; c += 32 / kFinRows, xs += (size_t)(32 / kFinRows) * P.ldx)
+                cp_async8(&fw.x[q][row][c], xs);
+        }
+        cp_async_commit();
     };
 
     // Warp 0: the recurrence.
     double tau1 = 0.0, alpha = 1.0, smin = 0.0;
     int I = 0, nbound = 0;
     if (wid == 0) {
-        smin = act ? P.beta[k] : sc_one(is);
+        smin = act ? beta[0] : sc_one(is);
         for (int J = 1; J < P.T; ++J)
-            if (act) smin = sc_min(smin, P.beta[(size_t)J * Spad + k], is);
-        alpha = act ? sc_upscale(smin, P.beta[k], is) : 1.0;
+            if (act) smin = sc_min(smin, beta[(size_t)J * Spad], is);
+        alpha = act ? sc_upscale(smin, beta[0], is) : 1.0;
         nbound = P.fr[1];
     }
-    // Warp 1: the norm.
+    // Warp 2: the norm.
     Nrm3 acc;
     acc.init();
+    auto norm_add = [&](const double *row) {
+        if (kCplx) {                                           // lane p: pair p of the block's 16
+            acc.add(row[2 * (lane & 15)]);
+            acc.add(row[2 * (lane & 15) + 1]);
+        } else {
+            acc.add(row[lane]);
+        }
+    };
 
-    if (wid == 1) stage(0);
+    if (wid == 3) {
+        stage_rot(0);
+        stage_rot(1);
+        cp_async_wait_one();
+    }
+    if (wid == 4) {
+        stage_x(0);
+        stage_x(1);
+        cp_async_wait_one();
+    }
     __syncthreads();                                           // block 0 in
-    for (int blk = 0; blk <= nb; ++blk) {
+    for (int blk = 0; blk < nb + 2; ++blk) {
         if (wid == 0 && blk < nb) {
-            const int r0 = blk * 32, rows = min(32, n - r0), q = blk & 1;
+            const int r0 = blk * kFinRows, rows = min(kFinRows, n - r0), q = blk & 3;
             double (*xb)[33] = fw.x[q];
-            double (*cb)[33] = fw.c[q];
-            double (*sb)[33] = fw.s[q];
-            double (*ob)[33] = fw.o[q];
-            for (int t = 0; t < rows; ++t) {
-                const int i = r0 + t;
-                if (i == nbound) {                             // tile boundary: the next tile's upscaling
+            double (*cb)[32] = fw.c[q];
+            double (*sb)[32] = fw.s[q];
+            double (*tb)[33] = fw.t[blk & 1];
+            int t = 0;
+            while (t < rows) {
+                if (r0 + t == nbound) {                        // tile boundary: the next tile's upscaling
                     ++I;
                     nbound = P.fr[I + 1];
-                    alpha = act ? sc_upscale_rare(smin, P.beta[(size_t)I * Spad + k], is) : 1.0;
+                    alpha = act ? sc_upscale_rare(smin, beta[(size_t)I * Spad], is) : 1.0;
                 }
-                if (i == 0) {
-                    tau1 = scale_by(alpha, xb[0][lane]);
-                    continue;
+                const int te = min(rows, nbound - r0);
+                if (!is_one(alpha))
+                    for (int u = t; u < te; ++u) xb[u][lane] = mul_rare(alpha, xb[u][lane]);
+                if (kCplx) __syncwarp();                       // the pair took the same way
+                if (r0 + t == 0) {
+                    tau1 = xb[0][lane];
+                    ++t;
                 }
-                const double tau2 = scale_by(alpha, xb[t][lane]);
-                const double c = cb[t][lane];
-                const double s = sb[t][lane];
-                ob[t][lane] = fma(c, tau1, -(s * tau2));       // row i - 1
-                tau1 = fma(c, tau2, s * tau1);
+                // One row, or four with their inputs read before the first is
+                // carried on (a store between them would hold the next reads back).
+                auto rows_of = [&](auto count) {
+                    constexpr int N = decltype(count)::value;
+                    double x2[N], c[N], sr[N], si[N];
+#pragma unroll
+                    for (int u = 0; u < N; ++u) {
+                        x2[u] = xb[t + u][lane];
+                        c[u] = cb[t + u][le];
+                        sr[u] = sb[t + u][le];
+                        if (kCplx) {
+                            si[u] = flip(sb[t + u][lo], ~lane);
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < N; ++u) {
+                        tb[t + u][lane] = tau1;
+                        if (kCplx) {                           // c t2 + s t1
+                            const double ot = __shfl_xor_sync(0xffffffffu, tau1, 1);
+                            tau1 = fma(c[u], x2[u], fma(sr[u], tau1, si[u] * ot));
+                        } else {
+                            tau1 = fma(c[u], x2[u], sr[u] * tau1);
+                        }
+                    }
+                    t += N;
+                };
+                while (t + 4 <= te) rows_of(std::integral_constant<int, 4>{});
+                while (t < te) rows_of(std::integral_constant<int, 1>{});
             }
         }
-        if (wid == 1) {
-            if (blk >= 1) {
-                // Results of block blk-1: rows r0-1 .. r0+rows-2 (row -1 does not exist).
-                const int p = blk - 1, r0 = p * 32, rows = min(32, n - r0), q = p & 1;
-                double (*ob)[33] = fw.o[q];
-                for (int t = (r0 == 0 ? 1 : 0); t < rows; ++t) acc.add(ob[t][lane]);
-                __syncwarp();
-                const int lo = r0 == 0 ? 1 : 0;
-                for (int c = 0; c < 32; ++c) {
-                    const int kc = k0 + c;
-                    if (kc < P.S && lane >= lo && lane < rows)
-                        P.X[(r0 - 1 + lane) + (size_t)kc * P.ldx] = ob[lane][c];
+        if (wid == 1 && blk >= 1 && blk <= nb) {
+            const int b = blk - 1, r0 = b * kFinRows, rows = min(kFinRows, n - r0), q = b & 3;
+            double (*xb)[33] = fw.x[q];
+            double (*cb)[32] = fw.c[q];
+            double (*sb)[32] = fw.s[q];
+            double (*tb)[33] = fw.t[b & 1];
+            double (*ob)[33] = fw.o[b & 1];
+            int t = b == 0 ? 1 : 0;
+            auto rows_of = [&](auto count) {                   // rows r0 + t - 1 ..., as above
+                constexpr int N = decltype(count)::value;
+                double out[N];
+#pragma unroll
+                for (int u = 0; u < N; ++u) {
+                    const double c = cb[t + u][le], sr = sb[t + u][le];
+                    double q2 = sr * xb[t + u][lane];
+                    if (kCplx) {                               // c t1 - conj(s) t2
+                        q2 = fma(sr, xb[t + u][lane], flip(sb[t + u][lo], lane) * xb[t + u][lane ^ 1]);
+                    }
+                    out[u] = fma(c, tb[t + u][lane], -q2);
                 }
+#pragma unroll
+                for (int u = 0; u < N; ++u) ob[t + u][lane] = out[u];
+                t += N;
+            };
+            while (t + 4 <= rows) rows_of(std::integral_constant<int, 4>{});
+            while (t < rows) rows_of(std::integral_constant<int, 1>{});
+        }
+        if (wid >= 2) {
+            // Results of block blk-2: rows r0-1 .. r0+rows-2 (row -1 does not exist).
+            const int b = blk - 2, r0 = b * kFinRows, rows = min(kFinRows, n - r0);
+            double (*ob)[33] = fw.o[b & 1];
+            const int first = b == 0 ? 1 : 0;
+            if (wid == 2 && b >= 0) {
+                for (int t = first; t < rows; ++t) norm_add(ob[t]);
             }
-            if (blk + 1 < nb) stage(blk + 1);
+            if (wid == 3) {
+                stage_rot(blk + 2);
+                cp_async_wait_one();                           // block blk + 1 in
+            }
+            if (wid == 4) {
+                stage_x(blk + 2);
+                const int row = lane & (kFinRows - 1);
+                for (int c = b >= 0 ? lane / kFinRows : 32; c < 32; c += 32 / kFinRows) {
+                    const int kc = k0 + c;
+                    if (kc < P.S && row >= first && row < rows)
+                        P.X[(r0 - 1 + row) + (size_t)kc * P.ldx] = ob[row][c];
+                }
+                cp_async_wait_one();                           // block blk + 1 in
+            }
         }
         __syncthreads();
     }
@@ -2510,32 +2617,54 @@ __device__ __forceinline__ void finalize_body_ws(const DevProblem &P, int bx, do
         fw.tail[lane] = tau1;
         if (act) {
             P.X[(n - 1) + (size_t)k * P.ldx] = tau1;
-            if (scale_out) scale_out[k] = smin;
+            if (scale_out && le == lane) scale_out[kCplx ? k / 2 : k] = smin;
         }
     }
     __syncthreads();
-    if (wid == 1 && act) {
-        acc.add(fw.tail[lane]);
+    if (wid == 2) {
+        norm_add(fw.tail);
         const double ynrm = acc.finish();
-        colnorm[k] = ynrm;
-        status[k] = (ynrm > 0.1 / sqrt((double)n)) ? 1 : 0;
+        const int ok = (ynrm > 0.1 / sqrt((double)n)) ? 1 : 0;
+        if (kCplx) {
+            const int kp = k0 + 2 * lane;
+            if (lane < 16 && kp < P.S) {
+                colnorm[kp] = colnorm[kp + 1] = ynrm;
+                status[kp] = status[kp + 1] = ok;
+            }
+        } else if (act) {
+            colnorm[k] = ynrm;
+            status[k] = ok;
+        }
     }
 }
 
-__global__ void __launch_bounds__(64) k_finalize(DevProblem P, double *colnorm, int *status,
+template <bool kCplx>
+__global__ void __launch_bounds__(160) k_finalize(DevProblem P, double *colnorm, int *status,
                                                  double *scale_out) {
     extern __shared__ double fsm[];
-    finalize_body_ws(P, blockIdx.x, colnorm, status, scale_out, *reinterpret_cast<FinalizeWs *>(fsm));
+    finalize_body_ws<kCplx>(P, blockIdx.x, colnorm, status, scale_out, *reinterpret_cast<FinalizeWs *>(fsm));
+}
+
+template <bool kCplx>
+static cudaError_t launch_finalize_form(const DevProblem &P, double *colnorm, int *status, double *scale_out,
+                                        cudaStream_t st) {
+    static size_t configured = 0;
+    const size_t smem = sizeof(FinalizeWs);
+    const cudaError_t e = raise_smem_limit((const void *)k_finalize<kCplx>, &configured, smem);
+    if (e != cudaSuccess) return e;
+    k_finalize<kCplx><<<(P.S + 31) / 32, 160, smem, st>>>(P, colnorm, status, scale_out);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_finalize(const DevProblem &P, double *colnorm, int *status, double *scale_out,
                             cudaStream_t st) {
-    static size_t configured = 0;
-    const size_t smem = sizeof(FinalizeWs);
-    const cudaError_t e = raise_smem_limit((const void *)k_finalize, &configured, smem);
-    if (e != cudaSuccess) return e;
-    k_finalize<<<(P.S + 31) / 32, 64, smem, st>>>(P, colnorm, status, scale_out);
-    return cudaGetLastError();
+    return launch_finalize_form<false>(P, colnorm, status, scale_out, st);
+}
+
+// Complex pairs: column norms and flags per column, one scaling factor per pair.
+cudaError_t launch_finalize_c(const DevProblem &P, double *colnorm, int *status, double *scale_out,
+                              cudaStream_t st) {
+    return launch_finalize_form<true>(P, colnorm, status, scale_out, st);
 }
 
 __global__ void k_normalize(DevProblem P, const double *colnorm, const int *status) {
