@@ -39,6 +39,7 @@
 #include <cfloat>
 #include <cmath>
 #include <cuda_runtime.h>
+#include <type_traits>
 
 namespace hsr {
 namespace {
@@ -334,10 +335,9 @@ __global__ void __launch_bounds__(kHbRows) k_hb_gemv(HbState S, int k0, int i, i
 // Bound for small orders by the L2 round trips of the barriers and sums and
 // by FP64 issue (a warp's instruction takes 64 clocks of its sub-partition):
 // 35,000 clocks a column at n = 700, of which A v 4,000; for large ones by the
-// FP64 pipe in A v (an FMA per 8 bytes of A: 2 a clock and SM, 0.7 of the
-// memory rate; 76,000 of 119,000 clocks at n = 6000).  Against the three
-// launches a column on n / 256 CTAs: n = 700 39.4 ms before, 13.4 now;
-// n = 6000 691 and 370; n = 10 354 us and 225.
+// memory in A v (fixed point, below; with FMAs by the FP64 pipe).  Against the
+// three launches a column on n / 256 CTAs: n = 700 39.4 ms before, 13.4 now;
+// n = 6000 691 and 316; n = 10 354 us and 225.
 constexpr int kHbThreads = 512;
 constexpr int kHbPiece = 1024;         // columns of v staged at a time (two per thread)
 constexpr int kHbAhead = 8;            // entries of A per thread loaded before v is known
@@ -350,6 +350,8 @@ struct HbPanel {
     int k0, ib, R, own;                // CTAs 0 .. own-1 have rows, R each
     int rpc, tiles, shares;            // A v: row tiles of rpc rows, CTAs (column shares) per tile
     unsigned *bar;                     // arrivals since the reduction began: of all CTAs, of those with rows
+    const int2 *F;                     // A's columns k0+1 .. in fixed point, n entries each (kFix)
+    const unsigned *top;               // their rows' largest high words, sign off (kFix)
 };
 __host__ __device__ constexpr int hb_pitch(int R) { return R | 1; }     // odd: columns fall on different banks
 __host__ __device__ constexpr size_t hb_panel_smem(int R) {
@@ -362,6 +364,84 @@ __device__ __forceinline__ double group_sum(double x, int g) {
     return x;
 }
 
+// A v on the integer pipe.  The FP64 pipe gives two products a clock and SM,
+// 16 bytes of A, where the memory gives 24; so for large n the panel first
+// puts A's remaining columns into fixed point, 58 bits below the largest
+// entry of the row (v, at most 1, likewise: 58 bits below 1), as a high part
+// of 29 bits and a signed low part of 30 in eight bytes, what the double took.
+// A product is then four 32 x 32 -> 64 bit ones, exact, in three sums:
+// high x high (2^56 at most, turned to FP64 every 64), high x low and low x
+// high, low x low (2^58 at most, carried up every 16).  So the entries are
+// rounded once, to 2^-59 of their row's largest, and the sum over 64 columns
+// once, where the FMAs round at every column.
+//
+// Then the memory bounds A v (6.3 TB/s of A).  The two passes that make the
+// copy cost 24 bytes of traffic an entry once in 64 products.  n = 6000: a
+// panel's column 70 us at the start and 24 at the end, the reduction 380 ->
+// 316 ms; n = 3000 94 -> 87.  At n = 2000 both take 52.5 ms (the matrix lies
+// in L2, and the steps around A v are most of a column); below, the copy costs
+// more than it gives (n = 1000 19.9 -> 21.0).
+constexpr int kHbFixN = 2048;
+constexpr int kFixLow = 30, kFixBits = 58;
+// x 2^58 / 2^e to the nearest, for |x| < 2^e or a little above; parts as above.
+__device__ __forceinline__ int2 fix_parts(double x, int e) {
+    const unsigned long long u = ubits(x);
+    const int f = (int)(u >> 52) & 0x7ff;
+    const unsigned long long m = ((u & 0xfffffffffffffULL) | (f ? 0x10000000000000ULL : 0ULL)) << 10;
+    const int sh = min(62 - kFixBits - (max(f, 1) - 1023 - e), 63);          // m = |x| 2^(62 - exponent)
+    long long q = (long long)((m + (1ULL << (sh - 1))) >> sh);
+    q = u >> 63 ? -q : q;
+    const long long hi = (q + (1LL << (kFixLow - 1))) >> kFixLow;
+    return make_int2((int)hi, (int)(q - (hi << kFixLow)));
+}
+// The exponent e of fix_parts for a row whose largest high word is `top`.
+__device__ __forceinline__ int fix_exp(unsigned top) { return max((int)(top >> 20), 1) - 1022; }
+struct FixSum {
+    double s = 0.0;
+    long long hh = 0, hl = 0, ll = 0;
+    __device__ __forceinline__ void add(int2 a, int2 v) {
+        hh += (long long)a.x * v.x;
+        hl += (long long)a.x * v.y;
+        hl += (long long)a.y * v.x;
+        ll += (long long)a.y * v.y;
+    }
+    __device__ __forceinline__ void carry() {                    // after at most 16 products
+        constexpr long long mask = (1LL << kFixLow) - 1;
+        hl += ll >> kFixLow;
+        ll &= mask;
+        hh += hl >> kFixLow;
+        hl &= mask;
+    }
+    __device__ __forceinline__ void flush() {                    // after at most 64
+        s += (double)hh;
+        hh = 0;
+    }
+    // The sum, over 2^(e - 56).
+    __device__ __forceinline__ double value() {
+        carry();
+        flush();
+        return fma((double)(int)hl, 0x1p-30, s);
+    }
+};
+// Largest high word of each row over the columns k0+1 .. n-1.
+constexpr int kFixCols = 64;
+__global__ void __launch_bounds__(256) k_hb_fix_top(int n, const double *A, long long lda, int c0, unsigned *top) {
+    const int r = blockIdx.x * 256 + threadIdx.x, ca = c0 + blockIdx.y * kFixCols, ce = min(ca + kFixCols, n);
+    if (r >= n) return;
+    unsigned m = 0;
+#pragma unroll 16
+    for (int c = ca; c < ce; ++c) m = max(m, (unsigned)(ubits(A[r + (size_t)c * lda]) >> 32) & 0x7fffffffu);
+    atomicMax(top + r, m);
+}
+__global__ void __launch_bounds__(256) k_hb_fix(int n, const double *A, long long lda, int c0, const unsigned *top, int2 *F) {
+    const int r = blockIdx.x * 256 + threadIdx.x, ca = c0 + blockIdx.y * kFixCols, ce = min(ca + kFixCols, n);
+    if (r >= n) return;
+    const int e = fix_exp(top[r]);
+#pragma unroll 8
+    for (int c = ca; c < ce; ++c) F[r + (size_t)(c - c0) * n] = fix_parts(A[r + (size_t)c * lda], e);
+}
+
+template <bool kFix>
 __global__ void __launch_bounds__(kHbThreads, 1) k_hb_panel(HbPanel P) {
     extern __shared__ double hsm[];
     __shared__ int dead;
@@ -635,10 +715,15 @@ __global__ void __launch_bounds__(kHbThreads, 1) k_hb_panel(HbPanel P) {
         const int rl = tid & (P.rpc - 1), sub = tid / P.rpc, nsub = kHbThreads / P.rpc, r = rt * P.rpc + rl;
         const bool work = rt < P.tiles && r < n;
         const int pl0 = min(ce - ca, kHbPiece), sl0 = (pl0 + nsub - 1) / nsub, qa = min(sub * sl0, pl0), qb = min(qa + sl0, pl0);
-        double y0[kHbAhead], cpre[2];
+        using Entry = std::conditional_t<kFix, int2, double>;
+        const Entry *const Ap = kFix ? reinterpret_cast<const Entry *>(P.F) - (size_t)(k0 + 1) * n
+                                     : reinterpret_cast<const Entry *>(S.A);
+        const size_t ld = kFix ? (size_t)n : (size_t)S.lda;
+        Entry y0[kHbAhead];
+        double cpre[2];
 #pragma unroll
         for (int e = 0; e < kHbAhead; ++e)
-            y0[e] = work && qa + e < qb ? S.A[r + (size_t)(j + 1 + ca + qa + e) * S.lda] : 0.0;
+            y0[e] = work && qa + e < qb ? Ap[r + (size_t)(j + 1 + ca + qa + e) * ld] : Entry{};
         ok = wait(0);
         if (!ok) break;
 #pragma unroll
@@ -694,40 +779,67 @@ __global__ void __launch_bounds__(kHbThreads, 1) k_hb_panel(HbPanel P) {
         // A v
         if (rt < P.tiles) {
             double x = 0.0;                                      // one chain: four warps share a sub-partition
+            FixSum fx;
+            bool bad = false;                                    // v not finite (kFix)
+            Entry *const ve = reinterpret_cast<Entry *>(vst);
             for (int p0 = ca; p0 < ce; p0 += kHbPiece) {
                 const int pl = min(ce - p0, kHbPiece), c0 = j + 1 + p0;
                 if (p0 > ca) __syncthreads();
                 for (int c = tid, e = 0; c < pl; c += kHbThreads, ++e) {
                     const int g = c0 + c;
-                    vst[c] = g == j + 1 ? 1.0 : (p0 == ca ? cpre[e & 1] : __ldcg(S.c + g)) * rsc;
+                    const double v = g == j + 1 ? 1.0 : (p0 == ca ? cpre[e & 1] : __ldcg(S.c + g)) * rsc;
+                    if constexpr (kFix) {
+                        ve[c] = fix_parts(v, 0);
+                        bad = bad || mag(v) >= pow2_bits(1);
+                    } else {
+                        ve[c] = v;
+                    }
                 }
-                __syncthreads();
+                if (kFix) bad = __syncthreads_or(bad);
+                else __syncthreads();
                 const int sl = (pl + nsub - 1) / nsub, q0 = min(sub * sl, pl), q1 = min(q0 + sl, pl);
                 if (r < n) {
                     int q = q0;
+                    const auto add = [&](Entry a, Entry v) {
+                        if constexpr (kFix) fx.add(a, v);
+                        else x = fma(a, v, x);
+                    };
                     if (p0 == ca) {
 #pragma unroll
                         for (int e = 0; e < kHbAhead; ++e)
-                            if (q + e < q1) x = fma(y0[e], vst[q + e], x);
+                            if (q + e < q1) add(y0[e], ve[q + e]);
                         q = min(q + kHbAhead, q1);
+                        if constexpr (kFix) fx.carry();
                     }
-                    const double *a = S.A + r + (size_t)(c0 + q) * S.lda;
-                    for (; q + 15 < q1; q += 16, a += 16 * S.lda) {
-                        double y[16];
+                    const Entry *a = Ap + r + (size_t)(c0 + q) * ld;
+                    for (int z = 0; q + 15 < q1; q += 16, a += 16 * ld) {
+                        Entry y[16];
 #pragma unroll
-                        for (int e = 0; e < 16; ++e) y[e] = a[(size_t)e * S.lda];
+                        for (int e = 0; e < 16; ++e) y[e] = a[(size_t)e * ld];
 #pragma unroll
-                        for (int e = 0; e < 16; ++e) x = fma(y[e], vst[q + e], x);
+                        for (int e = 0; e < 16; ++e) add(y[e], ve[q + e]);
+                        if constexpr (kFix) {
+                            fx.carry();
+                            if ((++z & 1) == 0) fx.flush();      // with the 8 ahead and the 15 left, never 64
+                        }
                     }
                     if (q < q1) {                                // the rest, its loads in flight together too
-                        double y[15];
+                        Entry y[15];
 #pragma unroll
-                        for (int e = 0; e < 15; ++e) y[e] = q + e < q1 ? a[(size_t)e * S.lda] : 0.0;
+                        for (int e = 0; e < 15; ++e) y[e] = q + e < q1 ? a[(size_t)e * ld] : Entry{};
 #pragma unroll
                         for (int e = 0; e < 15; ++e)
-                            if (q + e < q1) x = fma(y[e], vst[q + e], x);
+                            if (q + e < q1) add(y[e], ve[q + e]);
+                    }
+                    if constexpr (kFix) {
+                        fx.carry();
+                        fx.flush();
                     }
                 }
+            }
+            if constexpr (kFix) {
+                const unsigned top = r < n ? P.top[r] : 0u;
+                x = top >= 0x7ff00000u || bad ? dg_nan() : scalbn(fx.value(), fix_exp(top) - 2 * (kFixBits - kFixLow));
             }
             if (nsub > 1) {
                 gred[tid] = x;
@@ -1289,6 +1401,7 @@ __global__ void __launch_bounds__(8 * kHbNb) k_hb_m1(const double *T, const doub
 struct HbDigits {
     unsigned char *AD, *VN, *M1, *B1, *A2, *B2;
     double *Wp, *M, *Z;
+    unsigned *top;                                               // rows' largest high words
     int *cex, *exM1, *exB, *exA2, *dk1;                          // cex: n columns of A, then [Y V]
     int cch;
 };
@@ -1304,7 +1417,8 @@ size_t hb_digits_layout(int n, unsigned char *base, HbDigits &D) {
         off += (bytes + 255) / 256 * 256;
         return base + o;
     };
-    D.AD = take((size_t)D.cch * rows16);
+    // The same place serves A's columns in fixed point while a panel runs.
+    D.AD = take(std::max((size_t)D.cch * rows16, n >= kHbFixN ? (size_t)n * n * sizeof(int2) : 0));
     D.VN = take((size_t)kDgBN * rows16);
     D.M1 = take((size_t)kDgBM * small);
     D.B1 = take(all * small);
@@ -1318,6 +1432,7 @@ size_t hb_digits_layout(int n, unsigned char *base, HbDigits &D) {
     D.exB = reinterpret_cast<int *>(take(all * sizeof(int)));
     D.exA2 = reinterpret_cast<int *>(take(all * sizeof(int)));
     D.dk1 = reinterpret_cast<int *>(take((size_t)2 * kHbNb * sizeof(int)));
+    D.top = reinterpret_cast<unsigned *>(take((size_t)n * sizeof(unsigned)));
     return off;
 }
 // The trailing columns c1 .. n-1 of panel k0.
@@ -1414,7 +1529,8 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
     while (rpc < kHbThreads && 10 * busy(rpc) < 9 * best) rpc *= 2;
     const int rtiles = (n + rpc - 1) / rpc, shares = std::max(1, ctas / rtiles);
     const bool one = rtiles <= ctas && hb_panel_smem(R) <= kHbPanelSmem &&
-                     cudaFuncSetAttribute(k_hb_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, kHbPanelSmem) == cudaSuccess;
+                     cudaFuncSetAttribute(k_hb_panel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHbPanelSmem) == cudaSuccess &&
+                     cudaFuncSetAttribute(k_hb_panel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHbPanelSmem) == cudaSuccess;
     const size_t need = 2 * (size_t)n * nb           // Y, V
                         + nb * nb                     // T
                         + (size_t)n                   // c
@@ -1462,9 +1578,17 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
             cudaMemsetAsync(S.Y + (size_t)ib * n, 0, (size_t)(kHbNb - ib) * n * sizeof(double), st) != cudaSuccess)
             return HSR_ERR_CUDA;
         if (one) {
-            HbPanel pp{S, k0, ib, R, own, rpc, rtiles, shares, S.cnt + 2};
+            const bool fix = digits && n >= kHbFixN;
+            HbPanel pp{S, k0, ib, R, own, rpc, rtiles, shares, S.cnt + 2, reinterpret_cast<const int2 *>(D.AD), D.top};
             void *args[] = {&pp};
-            if (cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_hb_panel), dim3(ctas), dim3(kHbThreads), args,
+            if (fix) {
+                const dim3 g((unsigned)(n + 255) / 256, (unsigned)((n - k0 - 1 + kFixCols - 1) / kFixCols));
+                if (cudaMemsetAsync(D.top, 0, (size_t)n * sizeof(unsigned), st) != cudaSuccess) return HSR_ERR_CUDA;
+                k_hb_fix_top<<<g, 256, 0, st>>>(n, dA, lda, k0 + 1, D.top);
+                k_hb_fix<<<g, 256, 0, st>>>(n, dA, lda, k0 + 1, D.top, reinterpret_cast<int2 *>(D.AD));
+            }
+            const void *fn = fix ? reinterpret_cast<const void *>(k_hb_panel<true>) : reinterpret_cast<const void *>(k_hb_panel<false>);
+            if (cudaLaunchCooperativeKernel(fn, dim3(ctas), dim3(kHbThreads), args,
                                             hb_panel_smem(R), st) != cudaSuccess)
                 return HSR_ERR_CUDA;
         } else {

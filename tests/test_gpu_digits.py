@@ -153,3 +153,44 @@ def test_reduction_nan_in_first_row(gpu_lib):
     tau2 = hsr.hessenberg_device(got)
     assert torch.equal(tau, tau2) and torch.equal(got[:, 1:], clean[:, 1:])
     assert torch.isnan(got[1:, 0]).all()
+
+
+@pytest.mark.parametrize("n,pad,scale,graded", [(2048, 0, 1.0, False), (2051, 1, 1e-290, False), (2112, 0, 1e280, True),
+                                                (2400, 0, 1.0, True)])
+def test_reduction_fixed_point_panel(gpu_lib, n, pad, scale, graded):
+    """Orders whose panels multiply by the matrix in fixed point: A Q = Q H to
+    within n eps |A| (as above, Q from the back-transform of the identity),
+    also with rows and columns of very different size."""
+    import torch
+    import hsrq3in_gb300 as hsr
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((n, n))
+    if graded:
+        A *= 10.0 ** rng.uniform(-6, 0, n)[:, None] * 10.0 ** rng.uniform(-6, 0, n)
+    dA = _cols(torch, A * scale, pad)
+    tau = hsr.hessenberg_device(dA)
+    Q = torch.eye(n, dtype=torch.float64, device="cuda")
+    hsr.hessenberg_apply_q_device(dA, tau, Q)                    # rows = columns of Q
+    Q = Q.T
+    H = torch.triu(dA[:, :n].T, -1) / scale
+    R = torch.from_numpy(A).cuda() @ Q - Q @ H
+    assert float(R.norm()) <= n * EPS * np.linalg.norm(A)
+
+
+def test_reduction_fixed_point_non_finite(gpu_lib):
+    """A NaN in row 0 stays there; an Inf elsewhere reaches what it reaches
+    with products in floating point."""
+    import torch
+    import hsrq3in_gb300 as hsr
+    n = 2050
+    A = np.random.default_rng(2).standard_normal((n, n))
+    ref = _cols(torch, A, 0)
+    tref = hsr.hessenberg_device(ref)
+    A[0, 1000] = np.nan
+    dA = _cols(torch, A, 0)
+    tau = hsr.hessenberg_device(dA)
+    assert torch.equal(dA[:, 1:], ref[:, 1:]) and torch.equal(tau, tref)
+    A[0, 1000], A[700, 1200] = 0.0, np.inf
+    dA = _cols(torch, A, 0)
+    hsr.hessenberg_device(dA)
+    assert not torch.isfinite(dA[2:, 1:2]).any()
