@@ -162,8 +162,8 @@ bool make_maps(CUtensorMap *m, const Layout &L, const double *H, long long ldh, 
 }
 
 // ----------------------------------------------------------- work lists
-// Phases of a tick in launch order.  phGemmTop and then phDiagNext run on the
-// side stream, concurrently with phGemmRest.
+// Phases of a tick.  phGemmTop, phDiagNext, phFinal and phNormalize run on the
+// side stream in this order, concurrently with phGemmRest.
 enum Phase {
     phNorms = 0, phInit, phDiagFirst, phPart1, phGemmTop, phDiagNext, phGemmRest, phFinal, phNormalize, phCount
 };
@@ -291,15 +291,16 @@ cudaError_t launch_tick(const PhaseSpan *sp, const DevProblem *probs, const Batc
     const bool side = sp[phGemmTop].cnt > 0 || sp[phDiagNext].cnt > 0;
     if (side) {
         if ((e = cudaEventRecord(fork, M)) != cudaSuccess || (e = cudaStreamWaitEvent(D, fork, 0)) != cudaSuccess ||
-            (e = run(phGemmTop, D)) != cudaSuccess || (e = run(phDiagNext, D)) != cudaSuccess ||
-            (e = cudaEventRecord(join, D)) != cudaSuccess)
+            (e = run(phGemmTop, D)) != cudaSuccess || (e = run(phDiagNext, D)) != cudaSuccess)
             return e;
     }
-    if ((e = run(phGemmRest, M)) != cudaSuccess) return e;
-    if (side && (e = cudaStreamWaitEvent(M, join, 0)) != cudaSuccess) return e;
+    // A problem finishes with the diagonal solve of its tile 0, above which
+    // there are no rows: its end need not wait for the others' GEMM.
     for (int ph : {phFinal, phNormalize})
-        if ((e = run(ph, M)) != cudaSuccess) return e;
-    return cudaSuccess;
+        if ((e = run(ph, side ? D : M)) != cudaSuccess) return e;
+    if (side && (e = cudaEventRecord(join, D)) != cudaSuccess) return e;
+    if ((e = run(phGemmRest, M)) != cudaSuccess) return e;
+    return side ? cudaStreamWaitEvent(M, join, 0) : cudaSuccess;
 }
 
 int validate(const hsr_batch_problem &p, int b) {
@@ -522,6 +523,7 @@ extern "C" int hsr_batch_plan_create(hsr_batch_plan **out, int nprob, const hsr_
               cudaEventCreateWithFlags(&join, cudaEventDisableTiming) == cudaSuccess;
     // First use sets the kernels' shared-memory attributes outside capture.
     if (ok) ok = launch_diag_b(pl->d_probs, pl->d_items, 0, b, cap) == cudaSuccess &&
+                 launch_finalize_b(pl->d_probs, pl->d_items, 0, cap) == cudaSuccess &&
                  launch_gemm_b(pl->d_probs, pl->d_items, 0, pl->d_maps, cap) == cudaSuccess;
     if (ok) ok = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
     bool capturing = ok;

@@ -188,18 +188,16 @@ cudaError_t launch_init(const DevProblem &P, int mode, const double *eps3_dev, i
 // evaluates the short scalar chain of each step (Givens, 1x1 solve, overflow
 // decisions) and warps 1 .. NW-1 split the vector part (the updates of
 // y(0:j-2) and of the running column) by row, one step behind the chain
-// (diag_body_pipe).  Where many CTAs share the GPU (the batched engine) one
-// warp per CTA does the same work with the fewest FP64 instructions
-// (diag_body_1w).  v (running column) and y (solution tile) live in shared
+// (diag_body_pipe).  In the persistent queue, whose warps take work of any
+// problem, one warp does the same work by itself (diag_body_1w).  v (running column) and y (solution tile) live in shared
 // memory as [row][lane]; columns of H are staged ahead with cp.async and
 // read as broadcasts.  Per-warp maxima of |y| and |v| meet in shared memory
 // once per step.  When 2*32*b doubles do not fit, v/y live in a global
 // scratch region instead (same code, generic pointers).
 constexpr int kDiagWarps = 4;     // single-problem path, v/y in global scratch
 constexpr int kDiagWarpsSmem = 8; // single-problem path, v/y in shared memory
-constexpr int kDiagWarpsB = 1;    // batched path
-// Single-problem path, 8 or 16 shifts per CTA: the rotation's chain, the
-// solve's chain and six row warps (diag_body_narrow).
+// 4, 8 or 16 shifts per CTA (few shifts, and batches): the rotation's chain,
+// the 1x1 systems, the solve's chain and five row warps (diag_body_narrow).
 constexpr int kDiagWarpsNarrow = 8;
 
 constexpr int kDiagBcast = 8;      // per-lane step results broadcast by warp 0
@@ -2390,12 +2388,6 @@ __device__ __forceinline__ void finalize_body_buf(const DevProblem &P, int bx, d
     }
 }
 
-__device__ __forceinline__ void finalize_body(const DevProblem &P, int bx, double *colnorm, int *status,
-                                              double *scale_out) {
-    __shared__ FinalizeBuf fb;
-    finalize_body_buf(P, bx, colnorm, status, scale_out, fb);
-}
-
 // The plain path's form of finalize_body_buf, on five warps for the same 32
 // columns.  Warp 0 runs the recurrence alone (the next row's carried value;
 // two FP64 instructions a row, three with a complex sine) and leaves the
@@ -2456,8 +2448,8 @@ __device__ __forceinline__ void finalize_body_ws(const DevProblem &P, int bx, do
     // commits a group: the waits count groups.
     auto stage_rot = [&](int blk) {
         const int r0 = blk * kFinRows, rows = min(kFinRows, n - r0), q = blk & 3;
-        const int c = 2 * (lane & 15);                         // Spad is a multiple of 64: columns past S exist
-        for (int t = lane >> 4; t < rows; t += 2) {
+        const int c = 2 * (lane & 15);
+        for (int t = k0 + c < P.Spad ? lane >> 4 : rows; t < rows; t += 2) {     // (Spad is even)
             const size_t at = (size_t)(r0 + t) * Spad + k0 + c;
             cp_async16(&fw.c[q][t][c], P.Cr + at);
             cp_async16(&fw.s[q][t][c], P.Sr + at);
@@ -2771,10 +2763,23 @@ __global__ void k_init_b(const DevProblem *probs, const BatchItem *items) {
     init_column(probs[it.x], it.z, threadIdx.x, blockDim.x);
 }
 
-__global__ void __launch_bounds__(32 * kDiagWarpsB) k_diag_b(const DevProblem *probs, const BatchItem *items) {
-    extern __shared__ double sm[];
-    const BatchItem it = items[blockIdx.x];
-    diag_body_1w(probs[it.x], it.y, it.z, sm, nullptr);
+// 32 / SC CTAs per item, SC shifts each, on the narrow solve's warp roles.
+// Against one warp per 32 shifts, which issues the fewest FP64 instructions but
+// one after another, a tick of tiles of 64 with 16 shifts per CTA takes: 1,131
+// items 1,747 -> 1,056 us, 463 860 -> 416, 191 832 -> 155 (8 per CTA 213, 4
+// 323), 49 720 -> 96 (97, 146).  So 16, and fewer only where those CTAs still
+// find an SM each.  A batch of 192 problems (orders 32 to 1024) 38.9 -> 33.3 ms.
+template <int SC>
+__global__ void __launch_bounds__(32 * kDiagWarpsNarrow) k_diag_b(const DevProblem *probs, const BatchItem *items) {
+    __shared__ DevProblem Ps;
+    constexpr int parts = 32 / SC;
+    const BatchItem it = items[blockIdx.x / parts];
+    if (threadIdx.x < sizeof(DevProblem) / 8)
+        reinterpret_cast<long long *>(&Ps)[threadIdx.x] =
+            reinterpret_cast<const long long *>(probs + it.x)[threadIdx.x];
+    __syncthreads();
+    const int bx = it.z * parts + blockIdx.x % parts;
+    if (bx * SC < Ps.S) diag_body_narrow<SC>(Ps, it.y, bx);
 }
 
 // One block per (problem, stage, 8 shifts); the tiles above the diagonal
@@ -2804,10 +2809,18 @@ __global__ void __launch_bounds__(256, 2) k_gemm_b(const DevProblem *__restrict_
     gemm_body<false>(P, J, lo, hi, it.z & ~kGemmTopFlag, it.w, m, m + 1, m + 2);
 }
 
-__global__ void __launch_bounds__(32) k_finalize_b(const DevProblem *probs, const BatchItem *items) {
+// The plain path's form, per item: for 192 problems of orders 32 to 1024 the
+// last tick's took 1,738 us with one warp per 32 columns, 200 us this way; the
+// batch 51.1 -> 38.9 ms.
+__global__ void __launch_bounds__(160) k_finalize_b(const DevProblem *probs, const BatchItem *items) {
+    extern __shared__ double fsm[];
+    __shared__ DevProblem Ps;
     const BatchItem it = items[blockIdx.x];
-    const DevProblem &P = probs[it.x];
-    finalize_body(P, it.z, P.colnorm, P.status, P.scale);
+    if (threadIdx.x < sizeof(DevProblem) / 8)
+        reinterpret_cast<long long *>(&Ps)[threadIdx.x] =
+            reinterpret_cast<const long long *>(probs + it.x)[threadIdx.x];
+    __syncthreads();
+    finalize_body_ws<false>(Ps, it.z, Ps.colnorm, Ps.status, Ps.scale, *reinterpret_cast<FinalizeWs *>(fsm));
 }
 
 __global__ void k_normalize_b(const DevProblem *probs, const BatchItem *items) {
@@ -2830,18 +2843,28 @@ cudaError_t launch_init_b(const DevProblem *probs, const BatchItem *items, int n
     k_init_b<<<n_items, 128, 0, st>>>(probs, items);
     return cudaGetLastError();
 }
+template <int SC>
+cudaError_t launch_diag_b_form(const DevProblem *probs, const BatchItem *items, int n_items, int bmax, cudaStream_t st) {
+    static size_t configured = 0;
+    const size_t smem = diag_narrow_smem_bytes<SC>(bmax);
+    const cudaError_t e = raise_smem_limit((const void *)k_diag_b<SC>, &configured, smem);
+    if (e != cudaSuccess || n_items <= 0) return e;
+    k_diag_b<SC><<<n_items * (32 / SC), 32 * kDiagWarpsNarrow, smem, st>>>(probs, items);
+    return cudaGetLastError();
+}
+// No items: sets the kernels' shared-memory limits only.
 cudaError_t launch_diag_b(const DevProblem *probs, const BatchItem *items, int n_items, int bmax,
                           cudaStream_t st) {
-    const size_t smem = diag_smem_bytes_nw(bmax, kDiagWarpsB);
-    if (smem < (size_t)64 * bmax * sizeof(double)) return cudaErrorInvalidValue;   // must fit shared memory
-    static size_t configured = 0;
-    {
-        const cudaError_t e = raise_smem_limit((const void *)k_diag_b, &configured, smem);
-        if (e != cudaSuccess) return e;
+    const int sms = device_sms();
+    if (n_items <= 0) {
+        const cudaError_t e4 = launch_diag_b_form<4>(probs, items, 0, bmax, st), e8 = launch_diag_b_form<8>(probs, items, 0, bmax, st);
+        if (e4 != cudaSuccess || e8 != cudaSuccess) return e4 != cudaSuccess ? e4 : e8;
+    } else if (8 * n_items <= sms) {
+        return launch_diag_b_form<4>(probs, items, n_items, bmax, st);
+    } else if (4 * n_items <= sms) {
+        return launch_diag_b_form<8>(probs, items, n_items, bmax, st);
     }
-    if (n_items <= 0) return cudaSuccess;
-    k_diag_b<<<n_items, 32 * kDiagWarpsB, smem, st>>>(probs, items);
-    return cudaGetLastError();
+    return launch_diag_b_form<16>(probs, items, n_items, bmax, st);
 }
 cudaError_t launch_part1_b(const DevProblem *probs, const BatchItem *items, int n_items, cudaStream_t st) {
     if (n_items <= 0) return cudaSuccess;
@@ -2861,8 +2884,11 @@ cudaError_t launch_gemm_b(const DevProblem *probs, const BatchItem *items, int n
     return cudaGetLastError();
 }
 cudaError_t launch_finalize_b(const DevProblem *probs, const BatchItem *items, int n_items, cudaStream_t st) {
+    static size_t configured = 0;
+    const cudaError_t e = raise_smem_limit((const void *)k_finalize_b, &configured, sizeof(FinalizeWs));
+    if (e != cudaSuccess) return e;
     if (n_items <= 0) return cudaSuccess;
-    k_finalize_b<<<n_items, 32, 0, st>>>(probs, items);
+    k_finalize_b<<<n_items, 160, sizeof(FinalizeWs), st>>>(probs, items);
     return cudaGetLastError();
 }
 cudaError_t launch_normalize_b(const DevProblem *probs, const BatchItem *items, int n_items, cudaStream_t st) {

@@ -66,3 +66,27 @@ def test_upscaled_tiles(gpu_lib, scaling, intscale):
         assert np.array_equal(dev["vr"], orc["vr"], equal_nan=True)
         assert np.array_equal(dev["scale"], orc["colscale"], equal_nan=True)
         assert np.array_equal(dev["status"], orc["status"])
+
+
+@pytest.mark.parametrize("count,tlsz", [(1, 64), (9, 16), (19, 32), (20, 64), (30, 16), (60, 32), (60, 100)])
+def test_batch_forms(gpu_lib, count, tlsz):
+    """Batches whose ticks take 4, 8 and 16 shifts per CTA, down to the last
+    problem's: each problem as the oracle solves it."""
+    import torch
+    import hsrq3in_gb300 as hsr
+    probs, ref = [], []
+    for i in range(count):
+        n = 1 + (37 * i + 100) % 150
+        H, lam = G.real_spectrum(n, i + 1)
+        wr = np.resize(G.perturbed_shifts(lam, i), (11 * i) % 70 + 1)
+        ld = n + (n & 1)
+        Hd = torch.zeros((n, ld), dtype=torch.float64)
+        Hd[:, :n] = torch.from_numpy(H.T.copy())
+        probs.append((Hd.cuda()[:, :n], torch.from_numpy(wr.copy()).cuda(),
+                      torch.zeros((wr.size, ld), dtype=torch.float64, device="cuda")))
+        ref.append(O.oracle_inverse_iteration(H, wr, tlsz, 16, intscale=1, variant="fma"))
+    plan = hsr.BatchPlan(probs, tlsz=tlsz)
+    plan.execute()
+    for (H, _, X), o in zip(probs, ref):
+        assert np.array_equal(X.cpu().numpy()[:, :H.shape[0]].T, o["vr"])
+    plan.close()
