@@ -734,6 +734,8 @@ int run_pass_c(Solver &s, int mode, int its, int off, int cnt) {
         const int cc = std::min(s.Scap, cnt - c0);
         const bool gvy = diag_vy_global((cc / 2 + 31) / 32, diag_c_ctas_per_sm(s.tlsz));
         double *gs = gvy ? w.gscratch.as<double>() : nullptr;
+        const int sc = diag_c_narrow(cc / 2);
+        const bool lone = sc == 4 || sc == 8;                   // the diagonal solves gate the stages
         DevProblem P0 = problem_for(s, off + c0, cc, 0);
         HSR_LAUNCH_C(kcSetup, M, launch_init_c(P0, mode, s.eps3_dev, its, M));
         {
@@ -753,12 +755,12 @@ int run_pass_c(Solver &s, int mode, int its, int off, int cnt) {
                              launch_gemm_c_narrow(P, J, s.fr[J - 1], s.fr[J], s.tmH, s.tmWn[J & 1], s.tmZn[J & 1], D));
             else
                 HSR_LAUNCH_C(kcGemmTop, D,
-                             launch_gemm_c(P, J, s.fr[J - 1], s.fr[J], s.tmH, s.tmW[J & 1], s.tmZ[J & 1], D));
+                             launch_gemm_c(P, J, s.fr[J - 1], s.fr[J], s.tmH, s.tmW[J & 1], s.tmZ[J & 1], false, D));
             HSR_LAUNCH_C(kcDiag, D, launch_diag_c(Pn, J - 1, s.fr[J] - s.fr[J - 1], gs, D));
             HSR_CK(cudaEventRecord(w.ev_diag, D));
             if (s.fr[J - 1] > 0)
                 HSR_LAUNCH_C(kcGemm, M,
-                             launch_gemm_c(P, J, 0, s.fr[J - 1], s.tmH, s.tmW[J & 1], s.tmZ[J & 1], M));
+                             launch_gemm_c(P, J, 0, s.fr[J - 1], s.tmH, s.tmW[J & 1], s.tmZ[J & 1], lone, M));
             HSR_CK(cudaStreamWaitEvent(M, w.ev_diag, 0));
             if (g_timing.enabled) g_timing.gemm_fma[0] += (double)s.fr[J - 1] * (2.0 * bj - 1.0) * cc;
         }

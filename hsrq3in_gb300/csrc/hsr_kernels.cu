@@ -2286,10 +2286,15 @@ cudaError_t launch_gemm_c_narrow(const DevProblem &P, int J, int row_lo, int row
     return cudaGetLastError();
 }
 
+// `lone`: shared memory for one CTA per SM only.  Beside a diagonal solve that
+// gates the stage, a chain's FP64 instruction waits for one of each GEMM warp
+// of its sub-partition; one CTA still fills the FP64 pipe.  n = 2000 with 500
+// pairs (4 per diagonal CTA): 15.4 -> 14.7 ms; 900 pairs (8) 21.8 -> 21.7;
+// n = 4000 with 1900 (16), where the GEMM gates: 122.3 -> 123.9, so not there.
 cudaError_t launch_gemm_c(const DevProblem &P, int J, int row_lo, int row_hi, const CUtensorMap &tmH,
-                          const CUtensorMap &tmW, const CUtensorMap &tmZ, cudaStream_t st) {
+                          const CUtensorMap &tmW, const CUtensorMap &tmZ, bool lone, cudaStream_t st) {
     static size_t configured = 0;
-    const size_t smem = gemm_smem_bytes();
+    const size_t smem = lone ? std::max(gemm_smem_bytes(), (size_t)120 * 1024) : gemm_smem_bytes();
     {
         const cudaError_t e = raise_smem_limit((const void *)k_gemm_c, &configured, smem);
         if (e != cudaSuccess) return e;

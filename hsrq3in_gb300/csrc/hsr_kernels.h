@@ -175,13 +175,14 @@ cudaError_t launch_queue(const DevProblem *probs, const QueueItem *items, int n_
 cudaError_t launch_init_c(const DevProblem &P, int mode, const double *eps3_dev, int its, cudaStream_t st);
 // Shared memory of k_diag_c for tile height b; *global_vy tells whether v/y
 // need the global scratch region of 4*32*b doubles per 32 pairs instead.
+int diag_c_narrow(int np);                                      // pairs per CTA, 0: the wide form
 size_t diag_c_smem_bytes(int b, bool *global_vy);
 cudaError_t launch_diag_c(const DevProblem &P, int J, int b, double *gscratch, cudaStream_t st);
 cudaError_t launch_part1_c(const DevProblem &P, int J, cudaStream_t st);
 cudaError_t launch_gemm_c_narrow(const DevProblem &P, int J, int row_lo, int row_hi, const CUtensorMap &tmH,
                                  const CUtensorMap &tmW, const CUtensorMap &tmZ, cudaStream_t st);
 cudaError_t launch_gemm_c(const DevProblem &P, int J, int row_lo, int row_hi, const CUtensorMap &tmH,
-                          const CUtensorMap &tmW, const CUtensorMap &tmZ, cudaStream_t st);
+                          const CUtensorMap &tmW, const CUtensorMap &tmZ, bool lone, cudaStream_t st);
 // colnorm/status per column (both columns of a pair), scale_out per pair.
 cudaError_t launch_finalize_c(const DevProblem &P, double *colnorm, int *status, double *scale_out,
                               cudaStream_t st);
