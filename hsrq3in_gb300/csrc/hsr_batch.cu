@@ -149,21 +149,24 @@ DevProblem make_problem(const Layout &L, char *base, const double *H, long long 
     return P;
 }
 
+// The maps of a descriptor: H, then W and Zs in 64 columns (the queue) and in 16 (the ticks).
 bool make_maps(CUtensorMap *m, const Layout &L, const double *H, long long ldh, char *base, int parity) {
     const size_t stage = (size_t)L.b * L.Spad;
+    const double *W = reinterpret_cast<const double *>(base + L.W) + parity * stage;
+    const double *Z = reinterpret_cast<const double *>(base + L.Zs) + parity * stage;
+    const unsigned long long S = (unsigned long long)L.Spad, b = (unsigned long long)L.b;
+    static_assert(kBatchMaps == 5, "H, W, Zs, W, Zs");
     return encode_tensor_map(&m[0], H, (unsigned long long)L.n, (unsigned long long)L.n,
                              (unsigned long long)ldh, kGemmBM, kGemmKC) &&
-           encode_tensor_map(&m[1], reinterpret_cast<const double *>(base + L.W) + parity * stage,
-                             (unsigned long long)L.Spad, (unsigned long long)L.b, (unsigned long long)L.Spad,
-                             kGemmBN, kGemmKC) &&
-           encode_tensor_map(&m[2], reinterpret_cast<const double *>(base + L.Zs) + parity * stage,
-                             (unsigned long long)L.Spad,
-                             (unsigned long long)L.b, (unsigned long long)L.Spad, kGemmBN, kGemmKC);
+           encode_tensor_map(&m[1], W, S, b, S, kGemmBN, kGemmKC) && encode_tensor_map(&m[2], Z, S, b, S, kGemmBN, kGemmKC) &&
+           encode_tensor_map(&m[3], W, S, b, S, kGemmBNNarrow, kGemmKC) &&
+           encode_tensor_map(&m[4], Z, S, b, S, kGemmBNNarrow, kGemmKC);
 }
 
 // ----------------------------------------------------------- work lists
-// Phases of a tick.  phGemmTop, phDiagNext, phFinal and phNormalize run on the
-// side stream in this order, concurrently with phGemmRest.
+// Phases of a tick.  phGemmTop and then phDiagNext run on a side stream,
+// concurrently with phGemmRest, and after them phFinal and phNormalize on
+// another one, concurrently with the next tick too.
 enum Phase {
     phNorms = 0, phInit, phDiagFirst, phPart1, phGemmTop, phDiagNext, phGemmRest, phFinal, phNormalize, phCount
 };
@@ -273,10 +276,34 @@ struct PhaseTimer {
     }
 };
 
-// Launches one tick: main stream M, side stream D joined back into M.
+// Streams of the ticks: the main one, D (diagonal solves), E (ends of
+// problems), and the events between them.
+struct TickStreams {
+    cudaStream_t M = nullptr, D = nullptr, E = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+    bool open(int prio) {
+        return cudaStreamCreateWithFlags(&M, cudaStreamNonBlocking) == cudaSuccess &&
+               cudaStreamCreateWithPriority(&D, cudaStreamNonBlocking, prio) == cudaSuccess &&
+               cudaStreamCreateWithPriority(&E, cudaStreamNonBlocking, prio) == cudaSuccess &&
+               cudaEventCreateWithFlags(&fork, cudaEventDisableTiming) == cudaSuccess &&
+               cudaEventCreateWithFlags(&join, cudaEventDisableTiming) == cudaSuccess;
+    }
+    void close() {
+        for (cudaStream_t x : {M, D, E})
+            if (x) cudaStreamDestroy(x);
+        for (cudaEvent_t x : {fork, join})
+            if (x) cudaEventDestroy(x);
+        *this = TickStreams();
+    }
+};
+
+// Launches one tick; D is joined back into M.  A problem ends with the
+// diagonal solve of its tile 0, above which there are no rows: its
+// finalisation waits for nothing else, nothing on M waits for it, and it runs
+// on E (`ended`: the stream that it ran on), which the caller joins.
 cudaError_t launch_tick(const PhaseSpan *sp, const DevProblem *probs, const BatchItem *items, int bmax,
-                        const CUtensorMap *maps, cudaStream_t M, cudaStream_t D, cudaEvent_t fork,
-                        cudaEvent_t join, long &launches, PhaseTimer *tm) {
+                        const CUtensorMap *maps, const TickStreams &s, cudaStream_t &ended, long &launches,
+                        PhaseTimer *tm) {
     auto run = [&](int ph, cudaStream_t st) -> cudaError_t {
         if (sp[ph].cnt == 0) return cudaSuccess;
         if (tm) tm->starts.push_back({ph, tm->record(st)});
@@ -287,20 +314,20 @@ cudaError_t launch_tick(const PhaseSpan *sp, const DevProblem *probs, const Batc
     };
     cudaError_t e = cudaSuccess;
     for (int ph : {phNorms, phInit, phDiagFirst, phPart1})
-        if ((e = run(ph, M)) != cudaSuccess) return e;
+        if ((e = run(ph, s.M)) != cudaSuccess) return e;
     const bool side = sp[phGemmTop].cnt > 0 || sp[phDiagNext].cnt > 0;
     if (side) {
-        if ((e = cudaEventRecord(fork, M)) != cudaSuccess || (e = cudaStreamWaitEvent(D, fork, 0)) != cudaSuccess ||
-            (e = run(phGemmTop, D)) != cudaSuccess || (e = run(phDiagNext, D)) != cudaSuccess)
+        if ((e = cudaEventRecord(s.fork, s.M)) != cudaSuccess || (e = cudaStreamWaitEvent(s.D, s.fork, 0)) != cudaSuccess ||
+            (e = run(phGemmTop, s.D)) != cudaSuccess || (e = run(phDiagNext, s.D)) != cudaSuccess ||
+            (e = cudaEventRecord(s.join, s.D)) != cudaSuccess)
             return e;
     }
-    // A problem finishes with the diagonal solve of its tile 0, above which
-    // there are no rows: its end need not wait for the others' GEMM.
+    ended = side && sp[phFinal].cnt > 0 ? s.E : s.M;
+    if (ended == s.E && (e = cudaStreamWaitEvent(s.E, s.join, 0)) != cudaSuccess) return e;
     for (int ph : {phFinal, phNormalize})
-        if ((e = run(ph, side ? D : M)) != cudaSuccess) return e;
-    if (side && (e = cudaEventRecord(join, D)) != cudaSuccess) return e;
-    if ((e = run(phGemmRest, M)) != cudaSuccess) return e;
-    return side ? cudaStreamWaitEvent(M, join, 0) : cudaSuccess;
+        if ((e = run(ph, ended)) != cudaSuccess) return e;
+    if ((e = run(phGemmRest, s.M)) != cudaSuccess) return e;
+    return side ? cudaStreamWaitEvent(s.M, s.join, 0) : cudaSuccess;
 }
 
 int validate(const hsr_batch_problem &p, int b) {
@@ -440,7 +467,7 @@ extern "C" int hsr_batch_plan_create(hsr_batch_plan **out, int nprob, const hsr_
     // own full Layout in the workspace area and point nbits/nan at the zero
     // area explicitly.
     std::vector<DevProblem> hp(2 * (size_t)nprob);   // two descriptors per problem (tile parity)
-    std::vector<CUtensorMap> hm(6 * (size_t)nprob);
+    std::vector<CUtensorMap> hm(2 * kBatchMaps * (size_t)nprob);
     size_t ws = zero_total;
     std::vector<std::vector<int>> frs(nprob);
     for (int i = 0; i < nprob; ++i) {
@@ -458,7 +485,7 @@ extern "C" int hsr_batch_plan_create(hsr_batch_plan **out, int nprob, const hsr_
             P.nanflag = reinterpret_cast<int *>(zbase + L.nan);
             P.status = pl->d_status + ncols;
             hp[desc(i, par)] = P;
-            if (!make_maps(&hm[3 * (size_t)desc(i, par)], L, probs[i].dH, probs[i].lddH, base, par)) {
+            if (!make_maps(&hm[kBatchMaps * (size_t)desc(i, par)], L, probs[i].dH, probs[i].lddH, base, par)) {
                 delete pl;
                 return HSR_ERR_CUDA;
             }
@@ -513,14 +540,11 @@ extern "C" int hsr_batch_plan_create(hsr_batch_plan **out, int nprob, const hsr_
 
     // Capture: zero the accumulators, then every tick, the diagonal solves of
     // the next tiles on a forked high-priority stream.
-    cudaStream_t cap = nullptr, side = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
+    TickStreams ts;
     int lo_prio = 0, hi_prio = 0;
     cudaDeviceGetStreamPriorityRange(&lo_prio, &hi_prio);
-    bool ok = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking) == cudaSuccess &&
-              cudaStreamCreateWithPriority(&side, cudaStreamNonBlocking, hi_prio) == cudaSuccess &&
-              cudaEventCreateWithFlags(&fork, cudaEventDisableTiming) == cudaSuccess &&
-              cudaEventCreateWithFlags(&join, cudaEventDisableTiming) == cudaSuccess;
+    bool ok = ts.open(hi_prio), apart = false;
+    const cudaStream_t cap = ts.M;
     // First use sets the kernels' shared-memory attributes outside capture.
     if (ok) ok = launch_diag_b(pl->d_probs, pl->d_items, 0, b, cap) == cudaSuccess &&
                  launch_finalize_b(pl->d_probs, pl->d_items, 0, cap) == cudaSuccess &&
@@ -531,15 +555,14 @@ extern "C" int hsr_batch_plan_create(hsr_batch_plan **out, int nprob, const hsr_
     if (ok) ok = cudaMemsetAsync(pl->d_err, 0, 16, cap) == cudaSuccess;
     for (auto &t : ticks) {
         if (!ok) break;
-        ok = launch_tick(t.data(), pl->d_probs, pl->d_items, b, pl->d_maps, cap, side, fork, join, pl->launches,
-                         nullptr) == cudaSuccess;
+        cudaStream_t ended = nullptr;
+        ok = launch_tick(t.data(), pl->d_probs, pl->d_items, b, pl->d_maps, ts, ended, pl->launches, nullptr) == cudaSuccess;
+        apart = apart || ended == ts.E;
     }
+    if (ok && apart) ok = cudaEventRecord(ts.join, ts.E) == cudaSuccess && cudaStreamWaitEvent(cap, ts.join, 0) == cudaSuccess;
     cudaGraph_t g = nullptr;
     const cudaError_t ce = capturing ? cudaStreamEndCapture(cap, &g) : cudaErrorInvalidValue;
-    if (cap) cudaStreamDestroy(cap);
-    if (side) cudaStreamDestroy(side);
-    if (fork) cudaEventDestroy(fork);
-    if (join) cudaEventDestroy(join);
+    ts.close();
     if (!ok || ce != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
         delete pl;
@@ -921,8 +944,7 @@ struct ActiveReq {
 struct hsr_server {
     hsr_server_config cfg{};
     int b = 64, is = 1, max_slots = 4096;
-    cudaStream_t st = nullptr, side = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
+    TickStreams ts;
     char *pool = nullptr;
     size_t pool_bytes = 0;
     PoolAlloc alloc;
@@ -937,10 +959,8 @@ struct hsr_server {
     cudaEvent_t tick_ev[2] = {nullptr, nullptr};
     std::vector<int> free_slots;
     ~hsr_server() {
-        if (st) cudaStreamSynchronize(st);
-        if (side) cudaStreamDestroy(side);
-        if (fork) cudaEventDestroy(fork);
-        if (join) cudaEventDestroy(join);
+        for (cudaStream_t x : {ts.M, ts.E})
+            if (x) cudaStreamSynchronize(x);
         for (int i = 0; i < 2; ++i) {
             if (d_items[i]) cudaFree(d_items[i]);
             if (h_items[i]) cudaFreeHost(h_items[i]);
@@ -952,7 +972,7 @@ struct hsr_server {
         if (d_maps) cudaFree(d_maps);
         if (d_err) cudaFree(d_err);
         if (pool) cudaFree(pool);
-        if (st) cudaStreamDestroy(st);
+        ts.close();
     }
 };
 
@@ -981,16 +1001,13 @@ extern "C" int hsr_server_create(hsr_server **out, const hsr_server_config *cfg)
     int lo_prio = 0, hi_prio = 0;
     cudaDeviceGetStreamPriorityRange(&lo_prio, &hi_prio);
     const size_t ndesc = 2 * (size_t)s->max_slots;   // two descriptors per slot (tile parity)
-    bool ok = cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking) == cudaSuccess &&
-              cudaStreamCreateWithPriority(&s->side, cudaStreamNonBlocking, hi_prio) == cudaSuccess &&
-              cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming) == cudaSuccess &&
-              cudaEventCreateWithFlags(&s->join, cudaEventDisableTiming) == cudaSuccess &&
+    bool ok = s->ts.open(hi_prio) &&
               cudaMalloc(&s->pool, s->pool_bytes) == cudaSuccess &&
               cudaMalloc(&s->d_probs, sizeof(DevProblem) * ndesc) == cudaSuccess &&
-              cudaMalloc(&s->d_maps, sizeof(CUtensorMap) * 3 * ndesc) == cudaSuccess &&
+              cudaMalloc(&s->d_maps, sizeof(CUtensorMap) * kBatchMaps * ndesc) == cudaSuccess &&
               cudaMalloc(&s->d_err, 16) == cudaSuccess &&
               cudaMallocHost(&s->h_prob_stage, sizeof(DevProblem) * ndesc) == cudaSuccess &&
-              cudaMallocHost(&s->h_map_stage, sizeof(CUtensorMap) * 3 * ndesc) == cudaSuccess &&
+              cudaMallocHost(&s->h_map_stage, sizeof(CUtensorMap) * kBatchMaps * ndesc) == cudaSuccess &&
               cudaEventCreateWithFlags(&s->tick_ev[0], cudaEventDisableTiming) == cudaSuccess &&
               cudaEventCreateWithFlags(&s->tick_ev[1], cudaEventDisableTiming) == cudaSuccess;
     if (!ok) {
@@ -1011,7 +1028,7 @@ extern "C" int hsr_server_replay(hsr_server *s, int nreq, hsr_request *reqs, dou
     using clock = std::chrono::steady_clock;
     const auto t0 = clock::now();
     auto elapsed = [&]() { return std::chrono::duration<double>(clock::now() - t0).count(); };
-    cudaStream_t st = s->st;
+    cudaStream_t st = s->ts.M;
     const int b = s->b;
 
     std::vector<int> order(nreq);
@@ -1061,7 +1078,8 @@ extern "C" int hsr_server_replay(hsr_server *s, int nreq, hsr_request *reqs, dou
     std::vector<char> finished(nreq, 0);
     auto fail = [&](cudaError_t e) -> int {
         (void)cudaStreamSynchronize(st);
-        (void)cudaStreamSynchronize(s->side);
+        (void)cudaStreamSynchronize(s->ts.D);
+        (void)cudaStreamSynchronize(s->ts.E);
         for (auto &a : active)
             if (a.done) cudaEventDestroy(a.done);
         for (int i = 0; i < nreq; ++i)
@@ -1164,12 +1182,12 @@ extern "C" int hsr_server_replay(hsr_server *s, int nreq, hsr_request *reqs, dou
             const int d0 = desc(a.slot, 0);
             for (int par = 0; par < 2; ++par) {
                 s->h_prob_stage[d0 + par] = make_problem(a.L, base, dH, a.ldh, dwr, dX, a.ldx, s->is, s->d_err, par);
-                make_maps(&s->h_map_stage[3 * (size_t)(d0 + par)], a.L, dH, a.ldh, base, par);
+                make_maps(&s->h_map_stage[kBatchMaps * (size_t)(d0 + par)], a.L, dH, a.ldh, base, par);
             }
             SRV_CK(cudaMemcpyAsync(s->d_probs + d0, s->h_prob_stage + d0, 2 * sizeof(DevProblem),
                                    cudaMemcpyHostToDevice, st));
-            SRV_CK(cudaMemcpyAsync(s->d_maps + 3 * (size_t)d0, s->h_map_stage + 3 * (size_t)d0,
-                                   6 * sizeof(CUtensorMap), cudaMemcpyHostToDevice, st));
+            SRV_CK(cudaMemcpyAsync(s->d_maps + kBatchMaps * (size_t)d0, s->h_map_stage + kBatchMaps * (size_t)d0,
+                                   2 * kBatchMaps * sizeof(CUtensorMap), cudaMemcpyHostToDevice, st));
             add_setup(tl, a.slot, a.L);
             flops += 2.0 * (double)r.n * r.n * r.nrhs;
             a.stage = a.L.T - 1;
@@ -1221,8 +1239,8 @@ extern "C" int hsr_server_replay(hsr_server *s, int nreq, hsr_request *reqs, dou
         pack_tick(tl, s->h_items[parity], 0, spans);
         SRV_CK(cudaMemcpyAsync(s->d_items[parity], s->h_items[parity], sizeof(BatchItem) * count,
                                cudaMemcpyHostToDevice, st));
-        SRV_CK(launch_tick(spans, s->d_probs, s->d_items[parity], b, s->d_maps, st, s->side, s->fork, s->join,
-                           launches, tm));
+        cudaStream_t ended = nullptr;
+        SRV_CK(launch_tick(spans, s->d_probs, s->d_items[parity], b, s->d_maps, s->ts, ended, launches, tm));
         // Requests that finished this tick: copy results to the host.
         for (auto &a : active) {
             if (a.retiring) continue;
@@ -1233,26 +1251,32 @@ extern "C" int hsr_server_replay(hsr_server *s, int nreq, hsr_request *reqs, dou
                 double *dX = reinterpret_cast<double *>(reinterpret_cast<char *>(dwr) + up((size_t)r.nrhs * 8, 256));
                 if (void *Xm = mapped_view(r.vr)) {   // the caller's padding rows stay untouched
                     ++launches;
-                    SRV_CK(copy_cols(static_cast<double *>(Xm), r.ldvr, dX, a.ldx, r.n, r.nrhs, st));
+                    SRV_CK(copy_cols(static_cast<double *>(Xm), r.ldvr, dX, a.ldx, r.n, r.nrhs, ended));
                 } else {
                     SRV_CK(cudaMemcpy2DAsync(r.vr, (size_t)r.ldvr * 8, dX, a.ldx * 8, (size_t)r.n * 8, r.nrhs,
-                                             cudaMemcpyDeviceToHost, st));
+                                             cudaMemcpyDeviceToHost, ended));
                 }
                 SRV_CK(cudaMemcpyAsync(a.h_status, base + a.L.status, r.nrhs * sizeof(int), cudaMemcpyDeviceToHost,
-                                       st));
+                                       ended));
                 SRV_CK(cudaEventCreateWithFlags(&a.done, cudaEventDisableTiming));
-                SRV_CK(cudaEventRecord(a.done, st));
+                SRV_CK(cudaEventRecord(a.done, ended));
                 a.retiring = true;
             } else {
                 --a.stage;
             }
         }
-        SRV_CK(cudaEventRecord(s->tick_ev[parity], st));
+        // This tick's item lists are read on both streams.
+        if (ended == s->ts.E) {
+            SRV_CK(cudaEventRecord(s->ts.join, st));
+            SRV_CK(cudaStreamWaitEvent(ended, s->ts.join, 0));
+        }
+        SRV_CK(cudaEventRecord(s->tick_ev[parity], ended));
         tick_used[parity] = true;
         parity ^= 1;
         ++ticks;
     }
     SRV_CK(cudaStreamSynchronize(st));
+    SRV_CK(cudaStreamSynchronize(s->ts.E));
     int errw = 0;
     SRV_CK(cudaMemcpy(&errw, s->d_err, sizeof(int), cudaMemcpyDeviceToHost));
 #undef SRV_CK

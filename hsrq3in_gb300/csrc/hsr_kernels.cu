@@ -2794,24 +2794,33 @@ __global__ void __launch_bounds__(256) k_part1_b(const DevProblem *probs, const 
     part1_block(probs[it.x], it.y, it.z * kPart1Shifts);
 }
 
+// 16-column tiles, four CTAs per item's 64 columns: no work for the columns
+// between the problem's last and a multiple of 64, shorter last waves, and
+// about the wide tiles' rate when all is full.  192 problems of orders 32 to
+// 1024 31.55 -> 30.05 ms, 40 served requests 26.6 -> 25.5; 1500 of 32 to 256
+// (tiles of 32) 21.3 -> 20.5; 500 of 200 to 230 with 0.3 n shifts 7.86 -> 7.03;
+// 100 of 512 with 512 shifts 32.75 -> 33.03.
 __global__ void __launch_bounds__(256, 2) k_gemm_b(const DevProblem *__restrict__ probs,
                                                   const BatchItem *__restrict__ items,
                                                   const CUtensorMap *maps) {
+    constexpr int BN = kGemmBNNarrow, parts = kGemmBN / BN;
     // The descriptor is staged in shared memory: its fields are reloaded
     // where used instead of occupying registers next to the accumulators.
     __shared__ DevProblem Ps;
     static_assert(sizeof(DevProblem) % 8 == 0 && sizeof(DevProblem) / 8 <= 256, "descriptor copy");
-    const BatchItem it = items[blockIdx.x];
+    const BatchItem it = items[blockIdx.x / parts];
     if (threadIdx.x < sizeof(DevProblem) / 8)
         reinterpret_cast<long long *>(&Ps)[threadIdx.x] =
             reinterpret_cast<const long long *>(probs + it.x)[threadIdx.x];
     __syncthreads();
     const DevProblem &P = Ps;
-    const CUtensorMap *m = maps + 3 * (size_t)it.x;
+    const CUtensorMap *m = maps + kBatchMaps * (size_t)it.x;
     const int J = it.y;
     const bool top = (it.z & kGemmTopFlag) != 0;
     const int lo = top ? P.fr[J - 1] : 0, hi = top ? P.fr[J] : P.fr[J - 1];
-    gemm_body<false>(P, J, lo, hi, it.z & ~kGemmTopFlag, it.w, m, m + 1, m + 2);
+    const int by = it.w * parts + blockIdx.x % parts;
+    if (by * BN >= P.S) return;
+    gemm_body<false, BN>(P, J, lo, hi, it.z & ~kGemmTopFlag, by, m, m + 3, m + 4);
 }
 
 // The plain path's form, per item: for 192 problems of orders 32 to 1024 the
@@ -2879,13 +2888,13 @@ cudaError_t launch_part1_b(const DevProblem *probs, const BatchItem *items, int 
 cudaError_t launch_gemm_b(const DevProblem *probs, const BatchItem *items, int n_items, const CUtensorMap *maps,
                           cudaStream_t st) {
     static size_t configured = 0;
-    const size_t smem = gemm_smem_bytes();
+    const size_t smem = gemm_narrow_smem_bytes();
     {
         const cudaError_t e = raise_smem_limit((const void *)k_gemm_b, &configured, smem);
         if (e != cudaSuccess) return e;
     }
     if (n_items <= 0) return cudaSuccess;
-    k_gemm_b<<<n_items, 256, smem, st>>>(probs, items, maps);
+    k_gemm_b<<<n_items * (kGemmBN / kGemmBNNarrow), 256, smem, st>>>(probs, items, maps);
     return cudaGetLastError();
 }
 cudaError_t launch_finalize_b(const DevProblem *probs, const BatchItem *items, int n_items, cudaStream_t st) {
@@ -3003,7 +3012,7 @@ __global__ void __launch_bounds__(kQueueThreads, 2) k_queue(const DevProblem *__
                     fence_proxy_async_global();    // operands other CTAs wrote, read by TMA below
                     fence_proxy_async_smem();      // this CTA's earlier generic use of the ring
                 }
-                const CUtensorMap *m = maps + 3 * (size_t)it.x;
+                const CUtensorMap *m = maps + kBatchMaps * (size_t)it.x;
                 const int J = it.y;
                 const bool top = (it.z & kGemmTopFlag) != 0;
                 const int lo = top ? P.fr[J - 1] : 0, hi = top ? P.fr[J] : P.fr[J - 1];

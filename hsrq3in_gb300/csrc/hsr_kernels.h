@@ -131,6 +131,7 @@ cudaError_t launch_init_b(const DevProblem *probs, const BatchItem *items, int n
 cudaError_t launch_diag_b(const DevProblem *probs, const BatchItem *items, int n_items, int bmax,
                           cudaStream_t st);
 cudaError_t launch_part1_b(const DevProblem *probs, const BatchItem *items, int n_items, cudaStream_t st);
+constexpr int kBatchMaps = 5;   // tensor maps of a descriptor: H; W, Zs in 64 and in 16 columns
 cudaError_t launch_gemm_b(const DevProblem *probs, const BatchItem *items, int n_items, const CUtensorMap *maps,
                           cudaStream_t st);
 cudaError_t launch_finalize_b(const DevProblem *probs, const BatchItem *items, int n_items, cudaStream_t st);
