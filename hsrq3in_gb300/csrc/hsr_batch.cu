@@ -158,9 +158,9 @@ bool make_maps(CUtensorMap *m, const Layout &L, const double *H, long long ldh, 
     static_assert(kBatchMaps == 5, "H, W, Zs, W, Zs");
     return encode_tensor_map(&m[0], H, (unsigned long long)L.n, (unsigned long long)L.n,
                              (unsigned long long)ldh, kGemmBM, kGemmKC) &&
-           encode_tensor_map(&m[1], W, S, b, S, kGemmBN, kGemmKC) && encode_tensor_map(&m[2], Z, S, b, S, kGemmBN, kGemmKC) &&
-           encode_tensor_map(&m[3], W, S, b, S, kGemmBNNarrow, kGemmKC) &&
-           encode_tensor_map(&m[4], Z, S, b, S, kGemmBNNarrow, kGemmKC);
+           encode_tensor_map(&m[1], W, S, b, S, kGemmBNWide, kGemmKC) && encode_tensor_map(&m[2], Z, S, b, S, kGemmBNWide, kGemmKC) &&
+           encode_tensor_map(&m[3], W, S, b, S, kGemmBN, kGemmKC) &&
+           encode_tensor_map(&m[4], Z, S, b, S, kGemmBN, kGemmKC);
 }
 
 // ----------------------------------------------------------- work lists
@@ -204,7 +204,7 @@ bool add_stage(TickLists &tl, int slot, const Layout &L, const std::vector<int> 
         const int p = desc(slot, J), pn = desc(slot, J - 1);
         const int sbp = (L.S + kPart1Shifts - 1) / kPart1Shifts;
         for (int x = 0; x < sbp; ++x) tl.v[phPart1].push_back(make_int4(p, J, x, 0));
-        const int cbs = (L.S + kGemmBN - 1) / kGemmBN;
+        const int cbs = (L.S + kGemmBNWide - 1) / kGemmBNWide;
         const int top = (fr[J] - (fr[J - 1] & ~7) + kGemmBM - 1) / kGemmBM;
         for (int r = 0; r < top; ++r)
             for (int c = 0; c < cbs; ++c) tl.v[phGemmTop].push_back(make_int4(p, J, r | kGemmTopFlag, c));
@@ -666,7 +666,7 @@ void build_queue(const hsr_batch_plan *pl, int dw, std::vector<QueueItem> &out, 
         const int sb32 = (L.S + 31) / 32;
         cnt[i] = Counts{(L.n + kNormRows - 1) / kNormRows, (L.S + kQueueInitCols - 1) / kQueueInitCols,
                         (sb32 + dw - 1) / dw, (L.S + kPart1Shifts - 1) / kPart1Shifts,
-                        (sb32 + kQueueFinalBlocks - 1) / kQueueFinalBlocks, (L.S + kGemmBN - 1) / kGemmBN};
+                        (sb32 + kQueueFinalBlocks - 1) / kQueueFinalBlocks, (L.S + kGemmBNWide - 1) / kGemmBNWide};
     }
     std::vector<QueueItem> ph[phCount];
     auto flush = [&]() {

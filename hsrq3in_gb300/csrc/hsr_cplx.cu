@@ -13,8 +13,8 @@
 //               the 1x1 systems on warps of their own
 //   k_part1_c   the exact no-rescale test per (tile, pair), the full complex
 //               Part 1 of update-task.c:68-226 where a decision can fire
-//   k_gemm_c, k_gemm_cn  the real GEMM over H (hsr_kernels.cu) with a complex
-//               epilogue: the imaginary parts are just more columns of W and Zs
+//   k_gemm_c    the real GEMM over H (hsr_kernels.cu) with a complex epilogue:
+//               the imaginary parts are just more columns of W and Zs
 //   k_finalize<true>  (hsr_kernels.cu) reconciliation, complex back-transform,
 //               2-norm, convergence
 // Layout: pair p holds its real part in column 2p and its imaginary part in

@@ -248,7 +248,6 @@ struct Solver {
     cudaStream_t st;
     Workspace *w;
     CUtensorMap tmH, tmW[2], tmZ[2];
-    CUtensorMap tmWn[2], tmZn[2];   // 16-column boxes for launch_gemm_narrow
     double *eps3_dev;
     int *d_status;     // [S] per final column
     double *d_colnorm; // [S]
@@ -341,15 +340,11 @@ int run_pass(Solver &s, int mode, int its, int off, int cnt) {
                 g_timing.drop_last();
             }
             HSR_CK(fe);
-            if (fused) {
-                // Few shifts: the top GEMM ran inside the diagonal CTAs.
-            } else if (gemm_prefers_narrow(s.fr[J] - s.fr[J - 1], cc))
-                HSR_LAUNCH_C(kcGemmTop, D, launch_gemm_narrow(P, J, s.fr[J - 1], s.fr[J], s.tmH, s.tmWn[J & 1],
-                                                              s.tmZn[J & 1], D));
-            else
+            if (!fused) {                                        // (few shifts: the top GEMM ran inside the diagonal CTAs)
                 HSR_LAUNCH_C(kcGemmTop, D,
                              launch_gemm(P, J, s.fr[J - 1], s.fr[J], s.tmH, s.tmW[J & 1], s.tmZ[J & 1], D));
-            if (!fused) HSR_LAUNCH_C(kcDiag, D, launch_diag(Pn, J - 1, s.fr[J] - s.fr[J - 1], gs, D));
+                HSR_LAUNCH_C(kcDiag, D, launch_diag(Pn, J - 1, s.fr[J] - s.fr[J - 1], gs, D));
+            }
             HSR_CK(cudaEventRecord(w.ev_diag, D));
             if (s.fr[J - 1] > 0)
                 HSR_LAUNCH_C(kcGemm, M, launch_gemm(P, J, 0, s.fr[J - 1], s.tmH, s.tmW[J & 1], s.tmZ[J & 1], M));
@@ -454,12 +449,6 @@ int solve_device(int n, const double *dH, long long ldh, int S, double *dwr, int
         !make_map(&s.tmZ[1], w.Zs.as<double>() + (size_t)tlsz * Sp, Sp, (unsigned long long)tlsz, Sp, kGemmBN,
                   kGemmKC))
         return HSR_ERR_CUDA;
-    for (int par = 0; par < 2; ++par)
-        if (!make_map(&s.tmWn[par], w.W.as<double>() + (size_t)par * tlsz * Sp, Sp, (unsigned long long)tlsz, Sp,
-                      kGemmBNNarrow, kGemmKC) ||
-            !make_map(&s.tmZn[par], w.Zs.as<double>() + (size_t)par * tlsz * Sp, Sp, (unsigned long long)tlsz, Sp,
-                      kGemmBNNarrow, kGemmKC))
-            return HSR_ERR_CUDA;
 
     // Norms and eps3.
     unsigned long long *bits = w.bits.as<unsigned long long>();
@@ -735,7 +724,9 @@ int run_pass_c(Solver &s, int mode, int its, int off, int cnt) {
         const bool gvy = diag_vy_global((cc / 2 + 31) / 32, diag_c_ctas_per_sm(s.tlsz));
         double *gs = gvy ? w.gscratch.as<double>() : nullptr;
         const int sc = diag_c_narrow(cc / 2);
-        const bool lone = sc == 4 || sc == 8;                   // the diagonal solves gate the stages
+        // Diagonal CTAs on most SMs, and stages that they gate rather than the
+        // GEMM: one GEMM CTA per SM beside them (launch_gemm_c).
+        const bool most = sc > 0 && 2 * ((cc / 2 + sc - 1) / sc) > device_sms();
         DevProblem P0 = problem_for(s, off + c0, cc, 0);
         HSR_LAUNCH_C(kcSetup, M, launch_init_c(P0, mode, s.eps3_dev, its, M));
         {
@@ -750,17 +741,14 @@ int run_pass_c(Solver &s, int mode, int its, int off, int cnt) {
             HSR_LAUNCH_C(kcPart1, M, launch_part1_c(P, J, M));
             HSR_CK(cudaEventRecord(w.ev_top, M));
             HSR_CK(cudaStreamWaitEvent(D, w.ev_top, 0));
-            if (gemm_prefers_narrow(s.fr[J] - s.fr[J - 1], cc))
-                HSR_LAUNCH_C(kcGemmTop, D,
-                             launch_gemm_c_narrow(P, J, s.fr[J - 1], s.fr[J], s.tmH, s.tmWn[J & 1], s.tmZn[J & 1], D));
-            else
-                HSR_LAUNCH_C(kcGemmTop, D,
-                             launch_gemm_c(P, J, s.fr[J - 1], s.fr[J], s.tmH, s.tmW[J & 1], s.tmZ[J & 1], false, D));
+            HSR_LAUNCH_C(kcGemmTop, D,
+                         launch_gemm_c(P, J, s.fr[J - 1], s.fr[J], s.tmH, s.tmW[J & 1], s.tmZ[J & 1], false, D));
             HSR_LAUNCH_C(kcDiag, D, launch_diag_c(Pn, J - 1, s.fr[J] - s.fr[J - 1], gs, D));
             HSR_CK(cudaEventRecord(w.ev_diag, D));
             if (s.fr[J - 1] > 0)
                 HSR_LAUNCH_C(kcGemm, M,
-                             launch_gemm_c(P, J, 0, s.fr[J - 1], s.tmH, s.tmW[J & 1], s.tmZ[J & 1], lone, M));
+                             launch_gemm_c(P, J, 0, s.fr[J - 1], s.tmH, s.tmW[J & 1], s.tmZ[J & 1],
+                                           most && (long long)s.fr[J - 1] * cc <= kLoneElements, M));
             HSR_CK(cudaStreamWaitEvent(M, w.ev_diag, 0));
             if (g_timing.enabled) g_timing.gemm_fma[0] += (double)s.fr[J - 1] * (2.0 * bj - 1.0) * cc;
         }
@@ -855,12 +843,6 @@ int solve_device_cplx(int n, const double *dH, long long ldh, int np, double *dw
         !make_map(&s.tmZ[1], w.Zs.as<double>() + (size_t)tlsz * Sp, Sp, (unsigned long long)tlsz, Sp, kGemmBN,
                   kGemmKC))
         return HSR_ERR_CUDA;
-    for (int par = 0; par < 2; ++par)
-        if (!make_map(&s.tmWn[par], w.W.as<double>() + (size_t)par * tlsz * Sp, Sp, (unsigned long long)tlsz, Sp,
-                      kGemmBNNarrow, kGemmKC) ||
-            !make_map(&s.tmZn[par], w.Zs.as<double>() + (size_t)par * tlsz * Sp, Sp, (unsigned long long)tlsz, Sp,
-                      kGemmBNNarrow, kGemmKC))
-            return HSR_ERR_CUDA;
 
     unsigned long long *bits = w.bits.as<unsigned long long>();
     HSR_CK(cudaMemsetAsync(bits, 0, (2 * (size_t)T * T + 2) * 8, st));

@@ -1938,19 +1938,25 @@ cudaError_t launch_part1(const DevProblem &P, int J, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------------ GEMM
-// CTA tile: 64 rows x 64 shifts, both operand halves; 256 threads, each with
-// a 4x4 block of both accumulators.  A = H(rows, l-1 .. l+b-2) and the two
-// B tiles arrive by TMA in 16-column chunks through a 3-stage mbarrier ring.
-// Each accumulator sums k = 0 .. b-1 in order with fma, the same order as
-// the oracle's dot products.  Warp w owns rows 8w .. 8w+7 of the tile, so a
-// warp whose rows all lie outside [row_lo, row_hi) -- the partial blocks at
-// the ragged first tile and at unaligned tile starts -- skips the FMA loop:
-// masked lanes would cost the FP64 pipe as much as live ones.
-// BN = 64 is the main tile.  BN = 16 serves the short GEMM over the rows of
-// the next diagonal tile when the 64-column tiles would leave most SMs idle:
-// that GEMM gates the next diagonal solve, and 16-column tiles spread its
-// sequential K loop over four times as many CTAs.  Every accumulator sums
-// the same products in the same order in both shapes.
+// CTA tile: 64 rows x 16 shifts, both operand halves; 256 threads, each with
+// one row and four columns of both accumulators.  A = H(rows, l-1 .. l+b-2)
+// and the two B tiles arrive by TMA in 16-column chunks through a 3-stage
+// mbarrier ring.  Each accumulator sums k = 0 .. b-1 in order with fma, the
+// same order as the oracle's dot products.  Warp w owns rows 8w .. 8w+7 of the
+// tile, so a warp whose rows all lie outside [row_lo, row_hi) -- the partial
+// blocks at the ragged first tile and at unaligned tile starts -- skips the FMA
+// loop: masked lanes would cost the FP64 pipe as much as live ones.
+//
+// Bound by the FP64 pipe (64 cycles of a sub-partition per warp's FMA, against
+// which the operands' shared-memory reads, five per eight FMAs, are nothing),
+// so the tile is narrow: less padding past the last shift, and a last wave of
+// 35 us tiles where 64 columns, 4x4 a thread, make it 138.  The 64-column tile
+// takes, 16 columns take: n = 1000 with 1000 shifts 4.26 -> 3.96 ms,
+// n = 2000 with 1000 shifts through host buffers 12.6 -> 11.1, n = 3001 with
+// 301 12.2 -> 11.6, n = 4000 with 4000 126.5 -> 122.5, n = 6000 with 1280
+// 91.4 -> 86.9, n = 10^4 with 10^4 1748 -> 1743; complex, n = 3000 with 1200
+// pairs 50.4 -> 46.8.  BN = 64 is left for the persistent queue, whose items
+// are 64 columns.
 template <int BN>
 struct GemmSmemT {
     double A[kGemmStages][kGemmKC][kGemmBM];
@@ -1958,17 +1964,14 @@ struct GemmSmemT {
     double Z[kGemmStages][kGemmKC][BN];
     uint64_t full[kGemmStages];
 };
-using GemmSmem = GemmSmemT<kGemmBN>;
-
-size_t gemm_smem_bytes() { return sizeof(GemmSmem) + 128; }
-size_t gemm_narrow_smem_bytes() { return sizeof(GemmSmemT<kGemmBNNarrow>) + 128; }
+size_t gemm_smem_bytes() { return sizeof(GemmSmemT<kGemmBN>) + 128; }
+static size_t gemm_wide_smem_bytes() { return sizeof(GemmSmemT<kGemmBNWide>) + 128; }
 
 // Complex-shift epilogue: columns (2p, 2p+1) hold the real and imaginary
 // parts of pair p, the same thread owns both, and every scalar of the real
 // epilogue becomes its complex counterpart (crossover coefficient pi, Part-1
 // ytilde, shift mu, zlast, the old crossover column); the bound folded into
 // ynorm is the largest cabs1 of the pair's rows, kept at column 2p.
-template <int BN>
 __device__ __forceinline__ void gemm_epilogue_cplx(const DevProblem &P, int J, int row_lo, int row_hi, int row0,
                                                    int col0, const double *eaw, const double *eaz, int kEpiLd) {
     const int tid = threadIdx.x;
@@ -1983,8 +1986,8 @@ __device__ __forceinline__ void gemm_epilogue_cplx(const DevProblem &P, int J, i
     if (I < 0) I = 0;
     const int key = rowok ? I : -1;
     const double hl1 = rowok ? P.H[row + (size_t)(l - 1) * P.ldh] : 0.0;
-    for (int j = 0; j < BN / 4; j += 2) {
-        const int cc = cg * (BN / 4) + j;
+    for (int j = 0; j < kGemmBN / 4; j += 2) {
+        const int cc = cg * (kGemmBN / 4) + j;
         const int col = col0 + cc;
         if (col >= P.S) break;
         const dcplx pik = cmk(P.pi[col], P.pi[col + 1]);
@@ -2037,11 +2040,11 @@ __device__ __forceinline__ void gemm_epilogue_cplx(const DevProblem &P, int J, i
     }
 }
 
-template <bool kCplx, int BN = kGemmBN>
+template <bool kCplx, int BN>
 __device__ __forceinline__ void gemm_body(const DevProblem &P, int J, int row_lo, int row_hi, int bx, int by,
                                           const CUtensorMap *tmH, const CUtensorMap *tmW,
                                           const CUtensorMap *tmZ) {
-    static_assert(BN == kGemmBN || BN == kGemmBNNarrow, "tile widths");
+    static_assert(BN == kGemmBN || (BN == kGemmBNWide && !kCplx), "tile widths");
     // Threads per row of the tile (4 columns each) and rows per thread.
     constexpr int TC = BN / 4, RPT = kGemmBM * TC / 256;
     static_assert(RPT == 4 || RPT == 1, "thread tile");
@@ -2164,7 +2167,7 @@ __device__ __forceinline__ void gemm_body(const DevProblem &P, int J, int row_lo
     }
     __syncthreads();
     if constexpr (kCplx) {
-        gemm_epilogue_cplx<BN>(P, J, row_lo, row_hi, row0, col0, eaw, eaz, kEpiLd);
+        gemm_epilogue_cplx(P, J, row_lo, row_hi, row0, col0, eaw, eaz, kEpiLd);
         return;
     }
 
@@ -2200,50 +2203,13 @@ __device__ __forceinline__ void gemm_body(const DevProblem &P, int J, int row_lo
 __global__ void __launch_bounds__(256, 2)
 k_gemm(DevProblem P, int J, int row_lo, int row_hi, const __grid_constant__ CUtensorMap tmH,
        const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmZ) {
-    gemm_body<false>(P, J, row_lo, row_hi, blockIdx.x, blockIdx.y, &tmH, &tmW, &tmZ);
-}
-
-__global__ void __launch_bounds__(256, 2)
-k_gemm_n(DevProblem P, int J, int row_lo, int row_hi, const __grid_constant__ CUtensorMap tmH,
-         const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmZ) {
-    gemm_body<false, kGemmBNNarrow>(P, J, row_lo, row_hi, blockIdx.x, blockIdx.y, &tmH, &tmW, &tmZ);
-}
-
-// The GEMM over [row_lo, row_hi) with 16-column tiles; tmW/tmZ must have a
-// 16 x 16 box.
-cudaError_t launch_gemm_narrow(const DevProblem &P, int J, int row_lo, int row_hi, const CUtensorMap &tmH,
-                               const CUtensorMap &tmW, const CUtensorMap &tmZ, cudaStream_t st) {
-    if (row_hi <= row_lo || P.S <= 0) return cudaSuccess;
-    static size_t configured = 0;
-    static bool carve = false;
-    const size_t smem = gemm_narrow_smem_bytes();
-    cudaError_t e = prefer_max_shared((const void *)k_gemm_n, &carve);
-    if (e == cudaSuccess) e = raise_smem_limit((const void *)k_gemm_n, &configured, smem);
-    if (e != cudaSuccess) return e;
-    const int span = row_hi - (row_lo & ~7);
-    dim3 g((span + kGemmBM - 1) / kGemmBM, (P.S + kGemmBNNarrow - 1) / kGemmBNNarrow);
-    k_gemm_n<<<g, 256, smem, st>>>(P, J, row_lo, row_hi, tmH, tmW, tmZ);
-    return cudaGetLastError();
-}
-
-// Whether the 16-column tiles should serve a GEMM over `rows` rows: when the
-// 64-column tiles would fill fewer than half of the SMs.
-bool gemm_prefers_narrow(int rows, int S) {
-    static const int sms = []() {
-        int dev = 0, n = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-            return 0;
-        return n;
-    }();
-    const long ctas = (long)((rows + kGemmBM - 1) / kGemmBM) * ((S + kGemmBN - 1) / kGemmBN);
-    return sms > 0 && 2 * ctas < sms;
+    gemm_body<false, kGemmBN>(P, J, row_lo, row_hi, blockIdx.x, blockIdx.y, &tmH, &tmW, &tmZ);
 }
 
 __global__ void __launch_bounds__(256, 2)
 k_gemm_c(DevProblem P, int J, int row_lo, int row_hi, const __grid_constant__ CUtensorMap tmH,
          const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmZ) {
-    gemm_body<true>(P, J, row_lo, row_hi, blockIdx.x, blockIdx.y, &tmH, &tmW, &tmZ);
+    gemm_body<true, kGemmBN>(P, J, row_lo, row_hi, blockIdx.x, blockIdx.y, &tmH, &tmW, &tmZ);
 }
 
 cudaError_t launch_gemm(const DevProblem &P, int J, int row_lo, int row_hi, const CUtensorMap &tmH,
@@ -2263,34 +2229,13 @@ cudaError_t launch_gemm(const DevProblem &P, int J, int row_lo, int row_hi, cons
     return cudaGetLastError();
 }
 
-__global__ void __launch_bounds__(256, 2)
-k_gemm_cn(DevProblem P, int J, int row_lo, int row_hi, const __grid_constant__ CUtensorMap tmH,
-          const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmZ) {
-    gemm_body<true, kGemmBNNarrow>(P, J, row_lo, row_hi, blockIdx.x, blockIdx.y, &tmH, &tmW, &tmZ);
-}
-
-// launch_gemm_narrow with the complex epilogue, for the rows of the next tile
-// that gate its diagonal solve: at n = 2000 with 500 pairs (160 rows, 1000
-// columns) 169 us a tile on 189 CTAs, against 340 us on 48 CTAs with the
-// 64-column tiles; the solve 18.28 -> 17.73 ms.
-cudaError_t launch_gemm_c_narrow(const DevProblem &P, int J, int row_lo, int row_hi, const CUtensorMap &tmH,
-                                 const CUtensorMap &tmW, const CUtensorMap &tmZ, cudaStream_t st) {
-    static size_t configured = 0;
-    const size_t smem = gemm_narrow_smem_bytes();
-    const cudaError_t e = raise_smem_limit((const void *)k_gemm_cn, &configured, smem);
-    if (e != cudaSuccess) return e;
-    if (row_hi <= row_lo) return cudaSuccess;
-    const int span = row_hi - (row_lo & ~7);
-    dim3 g((span + kGemmBM - 1) / kGemmBM, (P.S + kGemmBNNarrow - 1) / kGemmBNNarrow);
-    k_gemm_cn<<<g, 256, smem, st>>>(P, J, row_lo, row_hi, tmH, tmW, tmZ);
-    return cudaGetLastError();
-}
-
 // `lone`: shared memory for one CTA per SM only.  Beside a diagonal solve that
 // gates the stage, a chain's FP64 instruction waits for one of each GEMM warp
-// of its sub-partition; one CTA still fills the FP64 pipe.  n = 2000 with 500
-// pairs (4 per diagonal CTA): 15.4 -> 14.7 ms; 900 pairs (8) 21.8 -> 21.7;
-// n = 4000 with 1900 (16), where the GEMM gates: 122.3 -> 123.9, so not there.
+// of its sub-partition; one CTA still fills the FP64 pipe.  With it for GEMMs
+// of at most 2^20 elements: n = 2000 with 500 pairs 13.65 -> 13.28 ms, n = 3000
+// with 400 20.5 -> 20.1; for all: 13.21 and 20.4, but n = 3000 with 1200 pairs,
+// where the GEMM gates the first stages, 46.7 -> 48.8 (46.6 with the limit).
+// The real solves did not gain.
 cudaError_t launch_gemm_c(const DevProblem &P, int J, int row_lo, int row_hi, const CUtensorMap &tmH,
                           const CUtensorMap &tmW, const CUtensorMap &tmZ, bool lone, cudaStream_t st) {
     static size_t configured = 0;
@@ -2803,7 +2748,7 @@ __global__ void __launch_bounds__(256) k_part1_b(const DevProblem *probs, const 
 __global__ void __launch_bounds__(256, 2) k_gemm_b(const DevProblem *__restrict__ probs,
                                                   const BatchItem *__restrict__ items,
                                                   const CUtensorMap *maps) {
-    constexpr int BN = kGemmBNNarrow, parts = kGemmBN / BN;
+    constexpr int BN = kGemmBN, parts = kGemmBNWide / BN;
     // The descriptor is staged in shared memory: its fields are reloaded
     // where used instead of occupying registers next to the accumulators.
     __shared__ DevProblem Ps;
@@ -2888,13 +2833,13 @@ cudaError_t launch_part1_b(const DevProblem *probs, const BatchItem *items, int 
 cudaError_t launch_gemm_b(const DevProblem *probs, const BatchItem *items, int n_items, const CUtensorMap *maps,
                           cudaStream_t st) {
     static size_t configured = 0;
-    const size_t smem = gemm_narrow_smem_bytes();
+    const size_t smem = gemm_smem_bytes();
     {
         const cudaError_t e = raise_smem_limit((const void *)k_gemm_b, &configured, smem);
         if (e != cudaSuccess) return e;
     }
     if (n_items <= 0) return cudaSuccess;
-    k_gemm_b<<<n_items * (kGemmBN / kGemmBNNarrow), 256, smem, st>>>(probs, items, maps);
+    k_gemm_b<<<n_items * (kGemmBNWide / kGemmBN), 256, smem, st>>>(probs, items, maps);
     return cudaGetLastError();
 }
 cudaError_t launch_finalize_b(const DevProblem *probs, const BatchItem *items, int n_items, cudaStream_t st) {
@@ -2927,12 +2872,12 @@ __host__ __device__ inline size_t queue_diag_warp_bytes(int b) {
     return diag_small_bytes(b, 1) + (size_t)64 * b * sizeof(double);
 }
 int queue_diag_warps(int bmax) {
-    const size_t budget = gemm_smem_bytes();
+    const size_t budget = gemm_wide_smem_bytes();
     int w = (int)(budget / queue_diag_warp_bytes(bmax));
     return w < 1 ? 1 : (w > 8 ? 8 : w);
 }
 size_t queue_smem_bytes(int bmax) {
-    size_t need = gemm_smem_bytes();
+    size_t need = gemm_wide_smem_bytes();
     const size_t diag = queue_diag_warps(bmax) * queue_diag_warp_bytes(bmax);
     const size_t fin = (size_t)kQueueFinalBlocks * sizeof(FinalizeBuf);
     if (diag + 128 > need) need = diag + 128;     // + room to align the base to 128 bytes
@@ -3016,10 +2961,10 @@ __global__ void __launch_bounds__(kQueueThreads, 2) k_queue(const DevProblem *__
                 const int J = it.y;
                 const bool top = (it.z & kGemmTopFlag) != 0;
                 const int lo = top ? P.fr[J - 1] : 0, hi = top ? P.fr[J] : P.fr[J - 1];
-                gemm_body<false>(P, J, lo, hi, it.z & ~kGemmTopFlag, it.w, m, m + 1, m + 2);
+                gemm_body<false, kGemmBNWide>(P, J, lo, hi, it.z & ~kGemmTopFlag, it.w, m, m + 1, m + 2);
                 __syncthreads();
                 if (tid == 0) {
-                    GemmSmem &gs = *reinterpret_cast<GemmSmem *>(smd);
+                    GemmSmemT<kGemmBNWide> &gs = *reinterpret_cast<GemmSmemT<kGemmBNWide> *>(smd);
                     for (int st = 0; st < kGemmStages; ++st) mbar_inval(&gs.full[st]);
                 }
                 break;

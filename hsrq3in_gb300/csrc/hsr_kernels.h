@@ -100,12 +100,6 @@ cudaError_t launch_part1(const DevProblem &P, int J, cudaStream_t st);
 cudaError_t launch_gemm(const DevProblem &P, int J, int row_lo, int row_hi, const CUtensorMap &tmH,
                         const CUtensorMap &tmW, const CUtensorMap &tmZ, cudaStream_t st);
 size_t gemm_smem_bytes();
-// The same GEMM with 16-column tiles (tmW/tmZ with a 16 x 16 box), for the
-// short GEMM that gates the next diagonal solve when 64-column tiles would
-// leave most SMs idle (gemm_prefers_narrow).
-cudaError_t launch_gemm_narrow(const DevProblem &P, int J, int row_lo, int row_hi, const CUtensorMap &tmH,
-                               const CUtensorMap &tmW, const CUtensorMap &tmZ, cudaStream_t st);
-bool gemm_prefers_narrow(int rows, int S);
 cudaError_t launch_finalize(const DevProblem &P, double *colnorm, int *status,
                             double *scale_out, cudaStream_t st);
 cudaError_t launch_normalize(const DevProblem &P, const double *colnorm,
@@ -176,12 +170,11 @@ cudaError_t launch_queue(const DevProblem *probs, const QueueItem *items, int n_
 cudaError_t launch_init_c(const DevProblem &P, int mode, const double *eps3_dev, int its, cudaStream_t st);
 // Shared memory of k_diag_c for tile height b; *global_vy tells whether v/y
 // need the global scratch region of 4*32*b doubles per 32 pairs instead.
+constexpr long long kLoneElements = 1 << 20;                     // rows x columns of such a GEMM at most
 int diag_c_narrow(int np);                                      // pairs per CTA, 0: the wide form
 size_t diag_c_smem_bytes(int b, bool *global_vy);
 cudaError_t launch_diag_c(const DevProblem &P, int J, int b, double *gscratch, cudaStream_t st);
 cudaError_t launch_part1_c(const DevProblem &P, int J, cudaStream_t st);
-cudaError_t launch_gemm_c_narrow(const DevProblem &P, int J, int row_lo, int row_hi, const CUtensorMap &tmH,
-                                 const CUtensorMap &tmW, const CUtensorMap &tmZ, cudaStream_t st);
 cudaError_t launch_gemm_c(const DevProblem &P, int J, int row_lo, int row_hi, const CUtensorMap &tmH,
                           const CUtensorMap &tmW, const CUtensorMap &tmZ, bool lone, cudaStream_t st);
 // colnorm/status per column (both columns of a pair), scale_out per pair.
@@ -201,8 +194,8 @@ cudaError_t launch_probe_dmma(double *out, int blocks, int iters, cudaStream_t s
 cudaError_t launch_selftest_arith(unsigned long long per_thread, unsigned long long seed, unsigned long long *cnt,
                                   int blocks, cudaStream_t st);
 
-constexpr int kGemmBM = 64, kGemmBN = 64, kGemmKC = 16, kGemmStages = 3;
-constexpr int kGemmBNNarrow = 16;       // column tile of the narrow GEMM (launch_gemm_narrow)
+constexpr int kGemmBM = 64, kGemmBN = 16, kGemmKC = 16, kGemmStages = 3;
+constexpr int kGemmBNWide = 64;         // columns of a batched GEMM item, and the queue's tile
 constexpr int kGemmTopFlag = 1 << 30;   // batched GEMM item: rows of tile J-1
 
 }  // namespace hsr
