@@ -171,7 +171,7 @@ def oracle_csolve_1x1(smin, tr, ti, lr, li, xr, xi, intscale=0):
 # ---------------------------------------------------------------- reference
 def reference_available() -> bool:
     return os.path.exists(os.path.join(_build.REF_DIR, "libhsrq3in_ref.so")) or \
-        os.path.isdir(_build.REFERENCE_SRC)
+        os.path.isfile(os.path.join(_build.REFERENCE_SRC, "inverse_iteration.c"))
 
 
 def _ref_lib(intscale: int) -> C.CDLL:
