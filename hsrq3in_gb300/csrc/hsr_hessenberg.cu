@@ -16,7 +16,9 @@
 // panel's earlier reflectors, a_j - Y V(j,:)^T from the right and
 // (I - V T^T V^T) from the left; then its reflector is generated, and
 // Y(:, i) = tau (A v - Y (V^T v)), T(:, i) = -tau T (V^T v), T(i,i) = tau.
-// Three launches per column:
+// All columns of a panel run in one cooperative launch (k_hb_panel); only
+// where the rows do not fit its shared memory (n above about 25,000) three
+// launches per column do the same:
 //   k_hb_step    rows in parallel: finishes the previous column (Y, V and T
 //                columns, its reflector into A) and starts this one,
 //                c = a_j - Y V(j,:)^T, with partial V^T c; the last block to

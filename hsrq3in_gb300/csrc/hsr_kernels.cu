@@ -45,7 +45,7 @@ cudaError_t raise_smem_limit(const void *func, size_t *configured, size_t smem) 
 }
 
 // Ask for the largest shared-memory carveout for a kernel of the plain
-// path's look-ahead.  The GEMM of the rows above (two 74 KB CTAs per SM) and
+// path's look-ahead.  The GEMM of the rows above (two CTAs per SM) and
 // the diagonal kernel of the next tile run at the same time; an SM set up
 // with a small carveout for whichever CTA arrived first could not take the
 // other kernel's CTAs beside it.  HSR_CARVEOUT=0 leaves the default.
