@@ -1475,24 +1475,47 @@ cudaError_t hb_trailing(const HbState &S, const HbDigits &D, int k0, int c1, int
     return err != cudaSuccess ? err : cudaGetLastError();
 }
 
+// A thread's scratch for sums and counters.  Its users on different streams are
+// ordered by an event (not inside a stream capture, whose replays the caller orders).
 struct HhScratch {
     int device = -1;
     double *p = nullptr;
     size_t bytes = 0;
-    ~HhScratch() {
+    cudaEvent_t ev = nullptr;
+    cudaStream_t last = nullptr;
+    bool used = false;
+    ~HhScratch() { release(); }
+    void release() {
         if (p) cudaFree(p);
-    }
-    cudaError_t ensure(size_t b, int dev) {
-        if (device == dev && b <= bytes) return cudaSuccess;
-        if (p) cudaFree(p);
+        if (ev) cudaEventDestroy(ev);
         p = nullptr;
+        ev = nullptr;
         bytes = 0;
-        cudaError_t e = cudaMalloc(&p, b);
-        if (e == cudaSuccess) {
+        used = false;
+    }
+    static bool capturing(cudaStream_t st) {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
+            cudaGetLastError();
+            return true;
+        }
+        return cs != cudaStreamCaptureStatusNone;
+    }
+    cudaError_t ensure(size_t b, int dev, cudaStream_t st) {
+        if (device != dev || b > bytes) {
+            release();
+            const cudaError_t e = cudaMalloc(&p, b);
+            if (e != cudaSuccess) return e;
             bytes = b;
             device = dev;
         }
-        return e;
+        return used && last != st && !capturing(st) ? cudaStreamWaitEvent(st, ev, 0) : cudaSuccess;
+    }
+    void done(cudaStream_t st) {
+        if (capturing(st) || (!ev && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess)) return;
+        cudaEventRecord(ev, st);
+        last = st;
+        used = true;
     }
 };
 
@@ -1542,7 +1565,7 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
                         + nb + 8                      // sc
                         + (size_t)(kHbMaxSplit + 2) * nb * n   // W partials, W, W2
                         + 4;                          // counters
-    if (sc.ensure(need * sizeof(double), dev) != cudaSuccess) return HSR_ERR_NOMEM;
+    if (sc.ensure(need * sizeof(double), dev, st) != cudaSuccess) return HSR_ERR_NOMEM;
     HbState S{};
     S.A = dA;
     S.lda = lda;
@@ -1635,6 +1658,7 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
             return HSR_ERR_CUDA;
     }
     if (digits) dg.done(st);
+    sc.done(st);
     return cudaGetLastError() == cudaSuccess ? HSR_OK : HSR_ERR_CUDA;
 }
 
@@ -1652,7 +1676,7 @@ extern "C" int hsr_hessenberg_apply_q_device(int n, const double *dA, int lda, c
     const size_t nb = kHbNb;
     const size_t need = (size_t)n * nb + 2 * nb * nb + (size_t)kHbMaxSplit * nb * nb +
                         (size_t)(kHbMaxSplit + 2) * nb * ncols;
-    if (sc.ensure(need * sizeof(double), dev) != cudaSuccess) return HSR_ERR_NOMEM;
+    if (sc.ensure(need * sizeof(double), dev, st) != cudaSuccess) return HSR_ERR_NOMEM;
     double *V = sc.p, *G = V + (size_t)n * nb, *T = G + nb * nb, *Gp = T + nb * nb;
     double *Wp = Gp + (size_t)kHbMaxSplit * nb * nb, *W = Wp + (size_t)kHbMaxSplit * nb * ncols,
            *W2 = W + nb * (size_t)ncols;
@@ -1689,5 +1713,6 @@ extern "C" int hsr_hessenberg_apply_q_device(int n, const double *dA, int lda, c
                 cudaSuccess)
             return HSR_ERR_CUDA;
     }
+    sc.done(st);
     return cudaGetLastError() == cudaSuccess ? HSR_OK : HSR_ERR_CUDA;
 }

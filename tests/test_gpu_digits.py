@@ -194,3 +194,32 @@ def test_reduction_fixed_point_non_finite(gpu_lib):
     dA = _cols(torch, A, 0)
     hsr.hessenberg_device(dA)
     assert not torch.isfinite(dA[2:, 1:2]).any()
+
+
+def test_reductions_on_two_streams(gpu_lib):
+    """One thread, two streams, no wait between the calls: each reduction and
+    back-transform (with digits, and small enough to go without) gives what it
+    gives alone."""
+    import torch
+    import hsrq3in_gb300 as hsr
+    rng = np.random.default_rng(8)
+    for n in (20, 300):
+        A = [rng.standard_normal((n, n)) for _ in range(6)]
+        X = rng.standard_normal((n, 7))
+        ref = []
+        for a in A:
+            d, x = _cols(torch, a, 0), _cols(torch, X, 0)
+            t = hsr.hessenberg_device(d)
+            hsr.hessenberg_apply_q_device(d, t, x)
+            ref.append((d, t, x))
+        st = [torch.cuda.Stream(), torch.cuda.Stream()]
+        got = [(_cols(torch, a, 0), _cols(torch, X, 0)) for a in A]
+        torch.cuda.synchronize()
+        tau = []
+        for i, (d, x) in enumerate(got):
+            with torch.cuda.stream(st[i & 1]):
+                tau.append(hsr.hessenberg_device(d, stream=st[i & 1]))
+                hsr.hessenberg_apply_q_device(d, tau[-1], x, stream=st[i & 1])
+        torch.cuda.synchronize()
+        for (d, x), t, (rd, rt, rx) in zip(got, tau, ref):
+            assert torch.equal(d, rd) and torch.equal(t, rt) and torch.equal(x, rx)
