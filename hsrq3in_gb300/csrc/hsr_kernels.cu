@@ -1678,13 +1678,23 @@ void record_fused_top(int S, bool on) {
 // Whether the narrow diagonal kernel also computes the top GEMM of its own
 // rows: HSR_FUSED_TOP (0 or 1) first, then the autotuner's trial value, then
 // its recorded choice for the nearest shift count within a factor of two,
-// else yes.  Either form gives the same result bit for bit.
+// else where the diagonal CTAs are on more than three quarters of the SMs: on
+// fewer, those SMs alone would do the rows that a GEMM of 64x16 tiles spreads
+// over all.  Inside / separate: n = 3001 with 301 shifts (76 CTAs) 11.6 / 10.7
+// ms, n = 1000 with 300 2.94 / 2.62, n = 4096 with 640 24.4 / 23.8, n = 48
+// 298 / 283 us; n = 1000 with 1000 (125 CTAs, tiles of 160) 3.92 / 4.12 ms.
+// Either form gives the same result bit for bit.
 bool fused_top_for(int S) {
     const char *env = getenv("HSR_FUSED_TOP");
     if (env && (env[0] == '0' || env[0] == '1')) return env[0] == '1';
     if (t_fused_trial >= 0) return t_fused_trial != 0;
-    std::lock_guard<std::mutex> g(g_spc_mu);
-    return nearest_tuned(g_fused_tuned, S) != 2;
+    {
+        std::lock_guard<std::mutex> g(g_spc_mu);
+        const int tuned = nearest_tuned(g_fused_tuned, S);
+        if (tuned) return tuned == 1;
+    }
+    const int sc = narrow_shifts(S);
+    return 4 * ((S + sc - 1) / sc) > 3 * device_sms();
 }
 
 // Shifts per diagonal CTA.  HSR_DIAG_SHIFTS_PER_CTA (8, 16 or 32) first,
