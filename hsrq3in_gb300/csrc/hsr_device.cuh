@@ -40,8 +40,14 @@ __device__ __forceinline__ unsigned long long abs_bits(double x) {
     unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffULL;
     return b > 0x7ff0000000000000ULL ? 0ULL : b;
 }
-__device__ __forceinline__ double from_bits(unsigned long long b) {
+__host__ __device__ __forceinline__ double from_bits(unsigned long long b) {
+#ifdef __CUDA_ARCH__
     return __longlong_as_double((long long)b);
+#else
+    double x;
+    memcpy(&x, &b, 8);
+    return x;
+#endif
 }
 __device__ __forceinline__ unsigned long long umax64(unsigned long long a, unsigned long long b) {
     return a > b ? a : b;

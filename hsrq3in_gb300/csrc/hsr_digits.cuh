@@ -296,7 +296,7 @@ __device__ __forceinline__ bool dg_wait(uint64_t *bar, uint32_t parity) {
 }
 
 // x 2^e for any e, results outside the normal range included.
-static __device__ __noinline__ double dg_ldexp_rare(double x, int e) { return ldexp(x, e); }
+static __host__ __device__ __noinline__ double dg_ldexp_rare(double x, int e) { return ldexp(x, e); }
 __device__ __forceinline__ double dg_ldexp(double x, int e) {
     const int f = (int)((ubits(x) >> 52) & 0x7ff);
     if (is_zero(x)) return x;
@@ -307,7 +307,15 @@ __device__ __forceinline__ double dg_ldexp(double x, int e) {
 // FP64 instructions less, 64 clocks of a sub-partition each): the sum's sign
 // and magnitude, its leading 64 bits, rounded to 53 (ties up; what lies below
 // the 64 bits does not enter).  Results outside the normal range: ldexp.
-__device__ __forceinline__ double dg_value(long long hi, long long lo, int e) {
+// Both forms compile for the host too, where a test checks them.
+__host__ __device__ __forceinline__ int dg_clz(unsigned long long x) {   // x != 0
+#ifdef __CUDA_ARCH__
+    return __clzll((long long)x);
+#else
+    return __builtin_clzll(x);
+#endif
+}
+__host__ __device__ __forceinline__ double dg_value(long long hi, long long lo, int e) {
     long long H = hi + (lo >> 36);
     unsigned long long L = (unsigned long long)lo & ((1ULL << 36) - 1);
     const unsigned long long sign = (unsigned long long)H & 0x8000000000000000ULL;
@@ -322,7 +330,7 @@ __device__ __forceinline__ double dg_value(long long hi, long long lo, int e) {
         L = 0;
         e -= 36;
     }
-    const int z = __clzll(H);                                    // 1 .. 63
+    const int z = dg_clz((unsigned long long)H);                 // 1 .. 63
     unsigned long long m = ((unsigned long long)H << z) | ((L << 28) >> (64 - z));
     int f = 1023 + 63 + 36 - z + e;
     m = (m >> 11) + ((m >> 10) & 1ULL);                          // 2^52 .. 2^53
@@ -330,13 +338,15 @@ __device__ __forceinline__ double dg_value(long long hi, long long lo, int e) {
     return from_bits(sign | (((unsigned long long)(f - 1) << 52) + m));
 }
 
-// The same for one word, T 2^(e - 55), |T| <= 2^62.
-__device__ __forceinline__ double dg_value(long long T, int e) {
+// The same for one word, T 2^(e - 55), |T| <= 2^62.  The rounding bit is added
+// after the shift: bit 63 of a << z is set, so adding it before could carry out.
+__host__ __device__ __forceinline__ double dg_value(long long T, int e) {
     if (T == 0) return 0.0;
     const unsigned long long sign = (unsigned long long)T & 0x8000000000000000ULL;
     const unsigned long long a = (unsigned long long)(T < 0 ? -T : T);
-    const int z = __clzll((long long)a);
-    const unsigned long long m = ((a << z) + (1ULL << 10)) >> 11;    // a <= 2^62: no carry out of 64 bits
+    const int z = dg_clz(a);
+    unsigned long long m = a << z;
+    m = (m >> 11) + ((m >> 10) & 1ULL);                          // 2^52 .. 2^53
     const int f = 1023 + 63 - z - 55 + e;
     if (f <= 0 || f >= 0x7fe) return dg_ldexp_rare(from_bits(sign | (0x3ffULL << 52)) * (double)m, f - 1075);
     return from_bits(sign | (((unsigned long long)(f - 1) << 52) + m));
