@@ -223,3 +223,31 @@ def test_reductions_on_two_streams(gpu_lib):
         torch.cuda.synchronize()
         for (d, x), t, (rd, rt, rx) in zip(got, tau, ref):
             assert torch.equal(d, rd) and torch.equal(t, rt) and torch.equal(x, rx)
+
+
+def test_back_transform_sum_below_power_of_two(gpu_lib):
+    """An update whose exact sum lies 2^-53 below 4: five reflectors meet in
+    row 150 with (2^-27, 1, 1, 1, 1) (-2^-26, 1, 1, 1, 1)^T, the rest of the
+    block is the identity and the first block random.  Tolerance as above."""
+    import torch
+    import hsrq3in_gb300 as hsr
+    n, r = 160, 150
+    A, tau = _reflectors(np.random.default_rng(4), n)
+    A[:, 128:] = np.triu(A, -1)[:, 128:]
+    tau[128:] = 0.0
+    tau[128:133] = 1.0
+    A[r, 128:133] = [2.0 ** -27, 1, 1, 1, 1]
+    X = np.zeros((n, 2))
+    X[129:134, 0] = [2.0 ** -26, 4, 3, 2, 1]
+    X[129:134, 1] = [-2.0 ** -26, -4, -3, -2, -1]
+    dX = _cols(torch, X, 0)
+    hsr.hessenberg_apply_q_device(_cols(torch, A, 0), torch.from_numpy(tau).cuda(), dX)
+    R = X.astype(np.longdouble)
+    for k in range(n - 3, -1, -1):
+        v = A[k + 1:, k].astype(np.longdouble)
+        v[0] = 1.0
+        R[k + 1:] -= np.outer(v, tau[k] * (v[:, None] * R[k + 1:]).sum(0))
+        if k == 128:
+            assert np.array_equal(R[r], np.longdouble([-1, 1]) * (4 - np.longdouble(2) ** -53))
+    err = np.sqrt(((dX.cpu().numpy().T - R) ** 2).sum(0)) / np.sqrt((R * R).sum(0))
+    assert err.max() <= n * EPS, err.max()
