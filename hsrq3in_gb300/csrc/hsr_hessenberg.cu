@@ -562,8 +562,9 @@ __global__ void __launch_bounds__(kHbThreads, 1) k_hb_panel(HbPanel P) {
     };
     // xnorm (or, as good a test for 0, its square) to sc[0], alpha to sc[1],
     // beta to sc[2], 1 / (alpha - beta) to sc[4].  With all of c(j+1 :) in the middle range beta is one
-    // square root of the sum of squares.
-    auto norms_in = [&](int j, const double *in) {
+    // square root of the sum of squares.  `again`: after the rescaling, whose
+    // caller needs xnorm itself and has an alpha that is not the stored one.
+    auto norms_in = [&](int j, const double *in, bool again) {
         if (tid < 32) {
             double x[3][5];
             Nrm3 tot;
@@ -592,7 +593,7 @@ __global__ void __launch_bounds__(kHbThreads, 1) k_hb_panel(HbPanel P) {
             if (tid == 0) {
                 const unsigned long long ma = mag(alpha);
                 double xn = tot.amed, beta = alpha;
-                if (!ends && (ma == 0 || (ma > pow2_bits(-500) && ma < pow2_bits(486))) && mag(xn) > pow2_bits(-900)) {
+                if (!again && !ends && (ma == 0 || (ma > pow2_bits(-500) && ma < pow2_bits(486))) && mag(xn) > pow2_bits(-900)) {
                     beta = sqrt(fma(alpha, alpha, xn));
                     beta = ubits(alpha) >> 63 ? beta : neg(beta);
                 } else {
@@ -734,7 +735,7 @@ __global__ void __launch_bounds__(kHbThreads, 1) k_hb_panel(HbPanel P) {
             cpre[e] = rt < P.tiles && c < pl0 ? __ldcg(S.c + j + 1 + ca + c) : 0.0;
         }
         // dlarfg, the same in every CTA.
-        norms_in(j, S.partn);
+        norms_in(j, S.partn, false);
         double xnorm = sc[0], alpha = sc[1], beta = sc[2];
         const double safmin = 0x1p-969, rsafmn = 0x1p+969;       // dlamch('S') / dlamch('E')
         int knt = 0;
@@ -753,7 +754,7 @@ __global__ void __launch_bounds__(kHbThreads, 1) k_hb_panel(HbPanel P) {
             arrive(0);
             ok = wait(0);
             if (!ok) break;
-            norms_in(j, again);                                  // (alpha as stored is the unscaled one)
+            norms_in(j, again, true);
             xnorm = sc[0];
             beta = -copysign(lapy2(alpha, xnorm), alpha);
             __syncthreads();

@@ -90,3 +90,29 @@ def test_dense_pipeline(gpu_lib):
     R = A @ X - X * sol["wr"][None, :]
     res = np.linalg.norm(R, axis=0) / (np.linalg.norm(A) * np.linalg.norm(X, axis=0))
     assert np.all(res <= 100 * n * EPS), res.max()
+
+
+@pytest.mark.parametrize("n,scale,leading", [(5, 1e-300, 0), (60, 1e-300, 0), (60, 1e-305, 1), (300, 1e-300, 2),
+                                             (60, 1.0, 1)])
+def test_zero_subdiagonal_at_the_safe_minimum(gpu_lib, n, scale, leading):
+    """Columns whose reflector starts from an exact 0 above entries that need
+    the safe-minimum rescaling: `leading` columns that are zero below the
+    diagonal, then one with a zero on the subdiagonal.  A Q = Q H and Q^T Q = I
+    with Q formed in extended precision, to within n eps as 2n Householder
+    transformations leave it."""
+    L = np.longdouble
+    A = np.random.default_rng(n + leading).standard_normal((n, n))
+    for k in range(leading):
+        A[k + 1:, k] = 0.0
+    A[leading + 1, leading] = 0.0
+    _, _, F, tau = _reduce(A * scale)
+    Q = np.eye(n, dtype=L)
+    for k in range(n - 3, -1, -1):
+        v = F[k + 1:, k].astype(L)
+        v[0] = 1.0
+        Q[k + 1:] -= np.outer(v, tau[k] * (v[:, None] * Q[k + 1:]).sum(0))
+    G = np.array([(Q * Q[:, c:c + 1]).sum(0) for c in range(n)]) - np.eye(n)
+    assert float(np.sqrt((G * G).sum())) <= n * EPS * np.sqrt(n)
+    H = np.triu(F, -1).astype(L) / scale
+    R = np.array([(A * Q[:, c]).sum(1) - (Q[:, :c + 2] * H[:c + 2, c]).sum(1) for c in range(n)])
+    assert float(np.sqrt((R * R).sum())) <= n * EPS * np.linalg.norm(A)
