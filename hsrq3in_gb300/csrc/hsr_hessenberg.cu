@@ -1243,7 +1243,8 @@ bool hq_digits(int n, const double *dA, int lda, const double *dtau, int ncols, 
     int *exX = reinterpret_cast<int *>(b + oEx), *exW = exX + ncols, *exVA = exW + cch, *exV = exVA + vrb * kHqNb,
         *exT = exV + gmax * kHqNb;
     *rc = HSR_ERR_CUDA;
-    k_dg_exp_k<<<ncols, 256, 0, st>>>(HqCols{dX, ldx, ncols, n}, n, nullptr, 0, exX);
+    // Over the rows that reflectors touch: row 0 stays what it is.
+    k_dg_exp_k<<<ncols, 256, 0, st>>>(HqCols{dX + 1, ldx, ncols, n - 1}, n - 1, nullptr, 0, exX);
     for (int last = nblk - 1; last >= 0; last -= gmax) {
         const int ng = std::min(gmax, last + 1);
         const HqGroup h{dA, lda, n, last * kHqNb, (n - 1 - last * kHqNb + kHqNb - 1) / kHqNb};

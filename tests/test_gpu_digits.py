@@ -251,3 +251,22 @@ def test_back_transform_sum_below_power_of_two(gpu_lib):
             assert np.array_equal(R[r], np.longdouble([-1, 1]) * (4 - np.longdouble(2) ** -53))
     err = np.sqrt(((dX.cpu().numpy().T - R) ** 2).sum(0)) / np.sqrt((R * R).sum(0))
     assert err.max() <= n * EPS, err.max()
+
+
+@pytest.mark.parametrize("n", [40, 200, 389])
+def test_back_transform_first_row(gpu_lib, n):
+    """Row 0 takes part in no reflector: whatever is there, the other rows are
+    what they are without it, bit for bit, and it stays."""
+    import torch
+    import hsrq3in_gb300 as hsr
+    rng = np.random.default_rng(n)
+    A, tau = _reflectors(rng, n)
+    dA, dtau = _cols(torch, A, 0), torch.from_numpy(tau).cuda()
+    X = np.repeat(rng.standard_normal((n, 1)), 5, axis=1)
+    X[0] = [0.5, 1e20, -1e300, np.inf, np.nan]
+    dX = _cols(torch, X, 1)
+    hsr.hessenberg_apply_q_device(dA, dtau, dX)
+    got = dX.cpu().numpy()
+    assert np.isfinite(got[0]).all() and np.array_equal(got[:, 0], X[0], equal_nan=True)
+    for c in range(1, 5):
+        assert np.array_equal(got[c, 1:n], got[0, 1:n]), c
