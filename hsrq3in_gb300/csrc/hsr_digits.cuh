@@ -138,6 +138,11 @@ __device__ __forceinline__ int dg_dk(const int *dk, int k) {     // no scaling b
     return d <= -kDgBad / 2 || d >= kDgBad / 2 ? 0 : d;
 }
 
+// Digit products are for operands whose entries are of like size; a call that
+// leaves the choice to the device passes a word `off` to every launch, which
+// does nothing where the word is not 0 (the caller's other form then runs).
+__device__ __forceinline__ bool dg_off(const int *off) { return off && *off != 0; }
+
 // ---------------------------------------------------------- preparation
 // Exponents and digits of an operand of R rows and K columns, read through a
 // loader ld(r, k) (0 outside the operand).  dk (optional): exponents taken
@@ -146,8 +151,10 @@ __device__ __forceinline__ int dg_dk(const int *dk, int k) {     // no scaling b
 
 // Rows contiguous along k: a block per row.
 template <class Ld>
-__global__ void __launch_bounds__(256) k_dg_exp_k(Ld ld, int K, const int *dk, int sign, int *ex) {
+__global__ void __launch_bounds__(256) k_dg_exp_k(Ld ld, int K, const int *dk, int sign, int *ex,
+                                                  const int *off) {
     __shared__ int red[8];
+    if (dg_off(off)) return;
     const int r = blockIdx.x;
     int m = kDgZero;
     for (int k = threadIdx.x; k < K; k += blockDim.x) {
@@ -182,7 +189,9 @@ __global__ void __launch_bounds__(256) k_dg_exp_r(Ld ld, int R, int K, int span,
 // both the loads and the 16-byte stores of a warp cover whole sectors.
 template <class Ld, bool RC>
 __global__ void __launch_bounds__(256) k_dg_split(Ld ld, int RB, int Rpad, long long steps, const int *ex,
-                                                  const int *dk, int sign, int R, int K, unsigned char *out) {
+                                                  const int *dk, int sign, int R, int K, unsigned char *out,
+                                                  const int *off) {
+    if (dg_off(off)) return;
     const int t = threadIdx.x;
     const int r = RC ? blockIdx.x * 32 + (t & 31) : blockIdx.x * 8 + (t & 7);
     const int c8 = RC ? blockIdx.y * 8 + (t >> 5) : blockIdx.y * 32 + (t >> 3);
@@ -205,9 +214,10 @@ __global__ void __launch_bounds__(256) k_dg_split(Ld ld, int RB, int Rpad, long 
 // groups one group of eight columns each.
 template <class Ld, bool RC>
 __global__ void __launch_bounds__(RC ? 512 : 128) k_dg_small(Ld ld, int RB, int R, int Rpad, int K, const int *dk,
-                                                             int sign, int *ex, unsigned char *out) {
+                                                             int sign, int *ex, unsigned char *out, const int *off) {
     constexpr int ROWS = RC ? 32 : 8;
     __shared__ int red[ROWS][17];
+    if (dg_off(off)) return;
     const int t = threadIdx.x, rr = RC ? t & 31 : t & 7, c8 = RC ? t >> 5 : t >> 3;
     const int r = blockIdx.x * ROWS + rr;
     const int steps = (K + kDgBK - 1) / kDgBK;
@@ -443,11 +453,12 @@ __device__ __forceinline__ bool dg_group(uint32_t tmem, uint64_t da, uint64_t db
 // this form 3.7 ms; the fma chain on the FP64 pipe 114 ms.
 template <class Epi>
 __global__ void __launch_bounds__(64 + 32 * Epi::kWarps, 1)
-k_dg_gemm(const unsigned char *__restrict__ A, const unsigned char *__restrict__ B, int tiles, Epi epi) {
+k_dg_gemm(const unsigned char *__restrict__ A, const unsigned char *__restrict__ B, int tiles, Epi epi, const int *off) {
     extern __shared__ __align__(1024) unsigned char dg_sm[];
     __shared__ __align__(8) uint64_t full[kDgStages], empty[kDgStages], acc_full[kDgGroups], acc_empty[kDgGroups];
     __shared__ uint32_t tmem_base;
     __shared__ int failed;
+    if (dg_off(off)) return;
     const int tid = threadIdx.x, wid = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     if (tid == 0) {
         for (int i = 0; i < kDgStages; ++i) {
@@ -745,11 +756,11 @@ inline int dg_parts(int tiles, int sms, int most, int steps, int &per) {
 }
 template <class Epi>
 inline cudaError_t dg_gemm(int tiles, int sms, const unsigned char *A, const unsigned char *B, const Epi &epi,
-                           cudaStream_t st) {
+                           const int *off, cudaStream_t st) {
     const cudaError_t e =
         cudaFuncSetAttribute(k_dg_gemm<Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDgSmem);
     if (e != cudaSuccess) return e;
-    k_dg_gemm<Epi><<<std::min(tiles, sms), 64 + 32 * Epi::kWarps, kDgSmem, st>>>(A, B, tiles, epi);
+    k_dg_gemm<Epi><<<std::min(tiles, sms), 64 + 32 * Epi::kWarps, kDgSmem, st>>>(A, B, tiles, epi, off);
     return cudaGetLastError();
 }
 

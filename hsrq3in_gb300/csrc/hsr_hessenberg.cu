@@ -29,8 +29,13 @@
 //   k_hb_gemv    A(:, j+1 : n-1) v in column chunks, and partial V^T v
 // After the panel the trailing columns c1 = k0 + nb ... get both sides of
 // the block reflector: in one rank-128 product by digits on the tensor cores
-// (hb_trailing), or with FP64 GEMMs (k_hb_gemm, DFMA, 64x64 tiles):
+// (hb_trailing), or with FP64 GEMMs (k_hb_plain, DFMA, 64x64 tiles):
 //   A(:, c1:) -= Y V(c1:, :)^T;  W = T^T V^T A(k0+1:, c1:);  A(k0+1:, c1:) -= V W
+// Digits and fixed point hold an entry by a window below the largest one of its
+// row or column, FP64 by 53 bits of its own.  They are for matrices whose
+// entries are of like size (k_hb_even decides, on the device); where rows or
+// columns differ, the reduction in FP64 keeps the small ones accurate, and it
+// runs in FP64 throughout.
 // The "last block" reductions use a completion counter and a fixed summation
 // order: no block waits for another, and results are reproducible run to run.
 #include "../../include/hsrq3in_gb300.h"
@@ -354,6 +359,7 @@ struct HbPanel {
     unsigned *bar;                     // arrivals since the reduction began: of all CTAs, of those with rows
     const int2 *F;                     // A's columns k0+1 .. in fixed point, n entries each (kFix)
     const unsigned *top;               // their rows' largest high words, sign off (kFix)
+    const int *uneven;                 // k_hb_panel<true> runs where it is 0, <false> where it is not (null: runs)
 };
 __host__ __device__ constexpr int hb_pitch(int R) { return R | 1; }     // odd: columns fall on different banks
 __host__ __device__ constexpr size_t hb_panel_smem(int R) {
@@ -427,7 +433,9 @@ struct FixSum {
 };
 // Largest high word of each row over the columns k0+1 .. n-1.
 constexpr int kFixCols = 64;
-__global__ void __launch_bounds__(256) k_hb_fix_top(int n, const double *A, long long lda, int c0, unsigned *top) {
+__global__ void __launch_bounds__(256) k_hb_fix_top(int n, const double *A, long long lda, int c0, unsigned *top,
+                                                    const int *uneven) {
+    if (dg_off(uneven)) return;
     const int r = blockIdx.x * 256 + threadIdx.x, ca = c0 + blockIdx.y * kFixCols, ce = min(ca + kFixCols, n);
     if (r >= n) return;
     unsigned m = 0;
@@ -435,7 +443,9 @@ __global__ void __launch_bounds__(256) k_hb_fix_top(int n, const double *A, long
     for (int c = ca; c < ce; ++c) m = max(m, (unsigned)(ubits(A[r + (size_t)c * lda]) >> 32) & 0x7fffffffu);
     atomicMax(top + r, m);
 }
-__global__ void __launch_bounds__(256) k_hb_fix(int n, const double *A, long long lda, int c0, const unsigned *top, int2 *F) {
+__global__ void __launch_bounds__(256) k_hb_fix(int n, const double *A, long long lda, int c0, const unsigned *top, int2 *F,
+                                                const int *uneven) {
+    if (dg_off(uneven)) return;
     const int r = blockIdx.x * 256 + threadIdx.x, ca = c0 + blockIdx.y * kFixCols, ce = min(ca + kFixCols, n);
     if (r >= n) return;
     const int e = fix_exp(top[r]);
@@ -447,6 +457,7 @@ template <bool kFix>
 __global__ void __launch_bounds__(kHbThreads, 1) k_hb_panel(HbPanel P) {
     extern __shared__ double hsm[];
     __shared__ int dead;
+    if (P.uneven && (*P.uneven != 0) == kFix) return;            // uniform over the grid, ahead of every barrier
     const HbState &S = P.S;
     const int tid = threadIdx.x, n = S.n, k0 = P.k0, R = P.R, Rp = hb_pitch(R), G = gridDim.x, b = blockIdx.x;
     double *const Ys = hsm, *const Vs = Ys + kHbNb * Rp, *const Ts = Vs + kHbNb * Rp;      // T(p, q) at p + 65 q
@@ -884,29 +895,49 @@ __global__ void __launch_bounds__(kHbThreads, 1) k_hb_panel(HbPanel P) {
     }
 }
 
-// C(i, j) = beta C(i, j) + alpha sum_k A(i, k) B(k, j) over k in this block's
-// split-K range, with A(i, k) = A[i*sai + k*sak], B(k, j) = B[k*sbk + j*sbj]
-// (one of each pair of strides is 1: loads coalesce along it) and
-// C(i, j) = C[i + j*ldc + blockIdx.z*cz].  64x64 tiles, 256 threads with a
-// 4x4 block each, K in chunks of 16 through shared memory; the sum over k is
-// one fma chain in k order.
+// C(i, j) = beta C(i, j) + alpha sum_k A(i, k) B(k, j), with A(i, k) =
+// A[i*sai + k*sak], B(k, j) = B[k*sbk + j*sbj] (one of each pair of strides is
+// 1: loads coalesce along it) and C(i, j) = C[i + j*ldc + z*cz], where part z
+// of nz takes k = z kc .. .  64x64 tiles, 256 threads with a 4x4 block each, K
+// in chunks of 16 through shared memory; the sum over k is one fma chain in k
+// order.  CTA c takes tiles c, c + gridDim.x, ...
 constexpr int kHbTm = 64, kHbTk = 16;
-__global__ void __launch_bounds__(256, 2)
-k_hb_gemm(int M, int N, int K, int kc, double alpha, const double *A, long long sai, long long sak,
-          const double *B, long long sbk, long long sbj, double beta, double *C, long long ldc, long long cz) {
-    __shared__ __align__(16) double As[kHbTk][kHbTm + 2];
-    __shared__ __align__(16) double Bs[kHbTk][kHbTm + 2];
+struct HbGemm {
+    int M, N, K, nz, kc;
+    double alpha;
+    const double *A;
+    long long sai, sak;
+    const double *B;
+    long long sbk, sbj;
+    double beta;
+    double *C;
+    long long ldc, cz;
+};
+// Parts of K for `split` of them at most, in whole chunks.
+__host__ __device__ __forceinline__ int hb_kc(int K, int split) {
+    return ((K + split - 1) / split + kHbTk - 1) / kHbTk * kHbTk;
+}
+__host__ __device__ __forceinline__ int hb_parts(int K, int split) {
+    const int kc = hb_kc(K, split);
+    return (K + kc - 1) / kc;
+}
+struct HbTiles {
+    __align__(16) double A[kHbTk][kHbTm + 2];
+    __align__(16) double B[kHbTk][kHbTm + 2];
+};
+__device__ __forceinline__ void hb_gemm_tile(const HbGemm &g, int bx, int by, int bz, HbTiles &sm) {
+    double (&As)[kHbTk][kHbTm + 2] = sm.A, (&Bs)[kHbTk][kHbTm + 2] = sm.B;
     const int tid = threadIdx.x;
-    const int i0 = blockIdx.x * kHbTm, j0 = blockIdx.y * kHbTm;
-    const int kb = blockIdx.z * kc, ke = min(K, kb + kc);
+    const int i0 = bx * kHbTm, j0 = by * kHbTm;
+    const int kb = bz * g.kc, ke = min(g.K, kb + g.kc);
     const int tr = tid >> 4, tc = tid & 15;
     double acc[4][4];
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
         for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
-    const bool a_i = sai == 1;                 // A contiguous along i (else along k)
-    const bool b_k = sbk == 1;                 // B contiguous along k (else along j)
+    const bool a_i = g.sai == 1;                 // A contiguous along i (else along k)
+    const bool b_k = g.sbk == 1;                 // B contiguous along k (else along j)
     for (int k = kb; k < ke; k += kHbTk) {
         double ra[4], rb[4];
 #pragma unroll
@@ -915,12 +946,12 @@ k_hb_gemm(int M, int N, int K, int kc, double alpha, const double *A, long long 
             if (a_i) { ii = tid & 63; kk = (tid >> 6) + 4 * e; }
             else { kk = tid & 15; ii = (tid >> 4) + 16 * e; }
             const int gi = i0 + ii, gk = k + kk;
-            ra[e] = (gi < M && gk < ke) ? A[(size_t)gi * sai + (size_t)gk * sak] : 0.0;
+            ra[e] = (gi < g.M && gk < ke) ? g.A[(size_t)gi * g.sai + (size_t)gk * g.sak] : 0.0;
             int jj, kq;
             if (b_k) { kq = tid & 15; jj = (tid >> 4) + 16 * e; }
             else { jj = tid & 63; kq = (tid >> 6) + 4 * e; }
             const int gj = j0 + jj, gq = k + kq;
-            rb[e] = (gj < N && gq < ke) ? B[(size_t)gq * sbk + (size_t)gj * sbj] : 0.0;
+            rb[e] = (gj < g.N && gq < ke) ? g.B[(size_t)gq * g.sbk + (size_t)gj * g.sbj] : 0.0;
         }
         __syncthreads();
 #pragma unroll
@@ -945,41 +976,192 @@ k_hb_gemm(int M, int N, int K, int kc, double alpha, const double *A, long long 
                 for (int b = 0; b < 4; ++b) acc[a][b] = fma(av[a], bv[b], acc[a][b]);
         }
     }
-    double *Cz = C + (size_t)blockIdx.z * cz;
+    double *Cz = g.C + (size_t)bz * g.cz;
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
         const int gj = j0 + 4 * tc + b;
-        if (gj >= N) continue;
+        if (gj >= g.N) continue;
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
             const int gi = i0 + 4 * tr + a;
-            if (gi >= M) continue;
-            double *cp = Cz + gi + (size_t)gj * ldc;
-            const double v = alpha * acc[a][b];
-            *cp = beta == 0.0 ? v : fma(beta, *cp, v);
+            if (gi >= g.M) continue;
+            double *cp = Cz + gi + (size_t)gj * g.ldc;
+            const double v = g.alpha * acc[a][b];
+            *cp = g.beta == 0.0 ? v : fma(g.beta, *cp, v);
         }
     }
 }
-
-// W(q, j) = sum over s of Wp[s](q, j), in order.
-__global__ void k_hb_sumk(int M, int N, int nsplit, const double *Wp, long long ldw, long long cz, double *W) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= M * N) return;
-    const int q = e % M, j = e / M;
-    double s = 0.0;
-    for (int z = 0; z < nsplit; ++z) s += Wp[(size_t)z * cz + q + (size_t)j * ldw];
-    W[q + (size_t)j * ldw] = s;
+__host__ __device__ __forceinline__ int hb_gemm_tiles(const HbGemm &g) {
+    return g.M <= 0 || g.N <= 0 ? 0 : ((g.M + kHbTm - 1) / kHbTm) * ((g.N + kHbTm - 1) / kHbTm) * g.nz;
+}
+__device__ __forceinline__ void hb_gemm_run(const HbGemm &g, HbTiles &sm) {
+    const int mt = (g.M + kHbTm - 1) / kHbTm, nt = (g.N + kHbTm - 1) / kHbTm, total = hb_gemm_tiles(g);
+    for (int t = blockIdx.x; t < total; t += gridDim.x) {
+        const int z = t / (mt * nt), r = t - z * mt * nt, by = r / mt;
+        hb_gemm_tile(g, r - by * mt, by, z, sm);
+        __syncthreads();                                         // before the next tile's first chunk
+    }
+}
+// W(q, j) = sum over z of Wp[z](q, j), in order.
+__device__ __forceinline__ void hb_sum_parts(int M, int N, int nz, const double *Wp, long long ldw, long long cz, double *W) {
+    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < (long long)M * N; e += (long long)gridDim.x * blockDim.x) {
+        const long long q = e % M, j = e / M;
+        double s = 0.0;
+        for (int z = 0; z < nz; ++z) s += Wp[(size_t)z * cz + q + (size_t)j * ldw];
+        W[q + (size_t)j * ldw] = s;
+    }
 }
 
+// A grid barrier for kernels launched cooperatively, as in k_hb_panel: `word`
+// counts arrivals since it was zeroed, in whole rounds: every launch that uses
+// the word has the same grid.
+// False once one gave up after kHbSpin polls.
+struct GridBar {
+    unsigned *word, target, G;
+    __device__ __forceinline__ GridBar(unsigned *w) : word(w), target(0), G(gridDim.x) {
+        // Arrivals of this launch cannot complete a round before this CTA's own.
+        if (threadIdx.x == 0) target = (*reinterpret_cast<volatile unsigned *>(w) & ~kHbDead) / G * G;
+    }
+    __device__ __forceinline__ bool meet() {
+        bool dead = false;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(word) : "memory");
+            target += G;
+            unsigned it = 0, v;
+            do {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
+            } while (!(v & kHbDead) && (int)(v - target) < 0 && ++it < kHbSpin);
+            if (it >= kHbSpin) atomicOr(word, kHbDead);
+            dead = it >= kHbSpin || (v & kHbDead);
+        }
+        return __syncthreads_or(dead) == 0;
+    }
+};
+
+// The trailing columns c1 .. n-1 of panel k0 in FP64, five phases: A(:, c1:)
+// -= Y V(c1:, :)^T; the parts of V^T A(k0+1:, c1:); their sums W; T^T W; and
+// A(k0+1:, c1:) -= V (T^T W).  One cooperative launch for all (first = 0, last
+// = 5), so that a panel whose product runs by digits passes over it in one
+// launch and not in five, or one launch a phase.
+struct HbPlain {
+    HbState S;
+    int k0, ib, c1, split;
+    double *Wp, *W, *W2;
+    unsigned *bar;
+    const int *uneven;                 // runs where it is not 0 (null: runs)
+};
+constexpr int kHbPlainPhases = 5;
+__global__ void __launch_bounds__(256, 2) k_hb_plain(HbPlain P, int first, int last) {
+    __shared__ HbTiles sm;
+    if (P.uneven && *P.uneven == 0) return;
+    const HbState &S = P.S;
+    const long long n = S.n, nb = kHbNb, m = n - P.c1, kr = n - P.k0 - 1;
+    double *const A1 = S.A + (size_t)P.c1 * S.lda, *const A2 = A1 + (P.k0 + 1);
+    const double *const V = S.V + (P.k0 + 1);
+    GridBar bar(P.bar);
+    for (int ph = first; ph < last; ++ph) {
+        if (ph == 2) {
+            hb_sum_parts(P.ib, (int)m, hb_parts((int)kr, P.split), P.Wp, nb, nb * m, P.W);
+        } else {
+            HbGemm g;
+            if (ph == 0) g = HbGemm{(int)n, (int)m, P.ib, 1, P.ib, -1.0, S.Y, 1, n, S.V + P.c1, n, 1, 1.0, A1, S.lda, 0};
+            if (ph == 1)
+                g = HbGemm{P.ib, (int)m, (int)kr, hb_parts((int)kr, P.split), hb_kc((int)kr, P.split), 1.0, V, n, 1, A2, 1,
+                           S.lda, 0.0, P.Wp, nb, nb * m};
+            if (ph == 3) g = HbGemm{P.ib, (int)m, P.ib, 1, P.ib, 1.0, S.T, nb, 1, P.W, 1, nb, 0.0, P.W2, nb, 0};
+            if (ph == 4) g = HbGemm{(int)kr, (int)m, P.ib, 1, P.ib, -1.0, V, 1, n, P.W2, 1, nb, 1.0, A2, S.lda, 0};
+            hb_gemm_run(g, sm);
+        }
+        if (ph + 1 < last && !bar.meet()) {
+            if (blockIdx.x == 0)
+                for (int q = threadIdx.x; q < n; q += blockDim.x) S.tau[q] = dg_nan();
+            return;
+        }
+    }
+}
+// All phases of a kernel k(P, first, last) in one cooperative launch, or, where
+// the device refuses that, one by one.
+template <class Params>
+cudaError_t launch_phases(void (*kernel)(Params, int, int), Params P, int phases, int grid, cudaStream_t st) {
+    int first = 0;
+    void *args[] = {&P, &first, &phases};
+    const cudaError_t e =
+        cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel), dim3(grid), dim3(256), args, 0, st);
+    if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported) return e;
+    cudaGetLastError();
+    for (; first < phases; ++first) kernel<<<grid, 256, 0, st>>>(P, first, first + 1);
+    return cudaGetLastError();
+}
+
+// Whether the sizes of A's entries allow digits and fixed point: in every row
+// but the first (no reflector touches it) and in every column, three fifths of
+// the entries lie within 2^8 of the largest of all.  Then every reflector mixes
+// entries of like size, and FP64 itself leaves errors of the size of the
+// largest entry's rounding everywhere.  |Q^T A Q - H| scaled by 1 / (d_i d_j)
+// for A = D G D, G of N(0,1) entries, relative to |G|, in FP64 / by digits, n =
+// 160 (2100): d from 1 to 2^-3 1.9e-15 / 1.6e-15 (5.3e-15 / 5.0e-15), to 2^-10
+// 1.1e-14 / 1.1e-14 (2.4e-14 / 2.1e-14), to 1e-16 4.6e-13 / 3e-4 (5.5e-13 /
+// 2e-3); those with d down to 2^-4 (n = 2100) and beyond are refused.  The
+// check reads A once: n = 700 13.36 -> 13.45 ms with the launches that do
+// nothing, n = 6000 316.0 -> 317.5.  Refused, d to 1e-12: n = 700 15.9 ms, n =
+// 4000 326.
+constexpr int kHbEvenBits = 8;
+constexpr int kHbEvenCols = 64;        // columns per CTA
+__device__ __forceinline__ bool hb_few(int low, int of) { return 5 * low <= 2 * of; }
+// cex: exponents of A's columns over rows 1 ..; low: 2 n counts, zeroed, of the
+// rows' and the columns' smaller (or non-finite) entries; cnt: a counter, zeroed.
+__global__ void __launch_bounds__(256) k_hb_even(int n, const double *A, long long lda, const int *cex, int *low, unsigned *cnt,
+                                                 int *uneven) {
+    __shared__ int red[8], col[kHbEvenCols];
+    const int tid = threadIdx.x, r = 1 + blockIdx.x * 256 + tid, c0 = blockIdx.y * kHbEvenCols, cols = min(kHbEvenCols, n - c0);
+    int top = kDgZero;
+    for (int c = tid; c < n; c += 256) top = dg_bad(cex[c]) ? top : max(top, cex[c]);
+    top = __reduce_max_sync(0xffffffffu, top);
+    if ((tid & 31) == 0) red[tid >> 5] = top;
+    if (tid < kHbEvenCols) col[tid] = 0;
+    __syncthreads();
+    for (int w = 0; w < 8; ++w) top = max(top, red[w]);
+    int mine = 0;
+#pragma unroll 4
+    for (int c = 0; c < cols; ++c) {
+        const int e = r < n ? dg_exp(A[r + (size_t)(c0 + c) * lda]) : top;
+        const bool small = e < top - kHbEvenBits || dg_bad(e);
+        const unsigned b = __ballot_sync(0xffffffffu, small);
+        if ((tid & 31) == 0 && b) atomicAdd(&col[c], __popc(b));
+        mine += small;
+    }
+    if (mine) atomicAdd(&low[r], mine);
+    __syncthreads();
+    if (tid < cols && col[tid]) atomicAdd(&low[n + c0 + tid], col[tid]);
+    // The last CTA decides.
+    __shared__ bool am_last;
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) am_last = atomicAdd(cnt, 1u) == gridDim.x * gridDim.y - 1;
+    __syncthreads();
+    if (!am_last) return;
+    __threadfence();
+    bool bad = false;
+    for (int q = tid; q < n; q += 256) bad = bad || !hb_few(__ldcg(&low[n + q]), n - 1) || (q > 0 && !hb_few(__ldcg(&low[q]), n));
+    bad = __syncthreads_or(bad);
+    if (tid == 0) *uneven = bad;
+}
+
+// The same as launches of their own.
+__global__ void __launch_bounds__(256, 2) k_hb_gemm(HbGemm g) {
+    __shared__ HbTiles sm;
+    hb_gemm_run(g, sm);
+}
+__global__ void k_hb_sumk(int M, int N, int nz, const double *Wp, long long ldw, long long cz, double *W) {
+    hb_sum_parts(M, N, nz, Wp, ldw, cz, W);
+}
 cudaError_t hb_gemm(int M, int N, int K, double alpha, const double *A, long long sai, long long sak,
                     const double *B, long long sbk, long long sbj, double beta, double *C, long long ldc,
                     int nsplit, long long cz, cudaStream_t st) {
     if (M <= 0 || N <= 0) return cudaSuccess;
-    int kc = K;
-    if (nsplit > 1) kc = (((K + nsplit - 1) / nsplit) + kHbTk - 1) / kHbTk * kHbTk;
-    const int nz = kc > 0 ? (K + kc - 1) / kc : 1;
-    dim3 g((M + kHbTm - 1) / kHbTm, (N + kHbTm - 1) / kHbTm, nz < 1 ? 1 : nz);
-    k_hb_gemm<<<g, 256, 0, st>>>(M, N, K, kc > 0 ? kc : 1, alpha, A, sai, sak, B, sbk, sbj, beta, C, ldc, cz);
+    const HbGemm g{M, N, K, hb_parts(K, nsplit), hb_kc(K, nsplit), alpha, A, sai, sak, B, sbk, sbj, beta, C, ldc, cz};
+    k_hb_gemm<<<hb_gemm_tiles(g), 256, 0, st>>>(g);
     return cudaGetLastError();
 }
 
@@ -1244,21 +1426,21 @@ bool hq_digits(int n, const double *dA, int lda, const double *dtau, int ncols, 
         *exT = exV + gmax * kHqNb;
     *rc = HSR_ERR_CUDA;
     // Over the rows that reflectors touch: row 0 stays what it is.
-    k_dg_exp_k<<<ncols, 256, 0, st>>>(HqCols{dX + 1, ldx, ncols, n - 1}, n - 1, nullptr, 0, exX);
+    k_dg_exp_k<<<ncols, 256, 0, st>>>(HqCols{dX + 1, ldx, ncols, n - 1}, n - 1, nullptr, 0, exX, nullptr);
     for (int last = nblk - 1; last >= 0; last -= gmax) {
         const int ng = std::min(gmax, last + 1);
         const HqGroup h{dA, lda, n, last * kHqNb, (n - 1 - last * kHqNb + kHqNb - 1) / kHqNb};
         const int rmax = h.rblocks(ng - 1), gz = std::min(kHqMaxSplit, std::max(1, 2 * sms / (2 * ng)));
-        k_dg_exp_k<<<ng * kHqNb, 256, 0, st>>>(HqVCols{h}, n - h.k0(ng - 1) - 1, nullptr, 0, exV);
+        k_dg_exp_k<<<ng * kHqNb, 256, 0, st>>>(HqVCols{h}, n - h.k0(ng - 1) - 1, nullptr, 0, exV, nullptr);
         const dim3 gv(kHqNb / 8, (unsigned)((2 * rmax * ksteps + 31) / 32), ng);
         k_hq_vcols<kDgBM><<<gv, 256, 0, st>>>(h, exV, VM);
         k_hq_vcols<kDgBN><<<gv, 256, 0, st>>>(h, exV, VN);
         k_hq_vrows<<<dim3(rmax * (kHqNb / 32), ng), 512, 0, st>>>(h, exVA, VA);
-        if (dg_gemm(2 * gz * ng, sms, VM, VN, HqGram{h, gz, exV, S}, st) != cudaSuccess) return true;
+        if (dg_gemm(2 * gz * ng, sms, VM, VN, HqGram{h, gz, exV, S}, nullptr, st) != cudaSuccess) return true;
         k_hq_thalf<<<dim3(ng, 2), 4 * kHqHalf, 0, st>>>(h, dtau, S, gz, T);
         k_hq_tcross<<<dim3(ng, kHqHalf / 8), 8 * kHqHalf, 0, st>>>(h, S, gz, T);
         k_dg_small<HqT, true><<<ng * (kHqNb / 32), 512, 0, st>>>(HqT{T}, kDgBM, ng * kHqNb, ng * kHqNb, kHqNb, nullptr, 0,
-                                                                exT, TM);
+                                                                exT, TM, nullptr);
         for (int c0 = 0; c0 < ncols; c0 += cch) {
             const int cols = std::min(cch, ncols - c0), cb = (cols + kDgBN - 1) / kDgBN;
             for (int g = 0; g < ng; ++g) {
@@ -1266,20 +1448,20 @@ bool hq_digits(int n, const double *dA, int lda, const double *dtau, int ncols, 
                 const long long at = h.before(g);
                 double *X = dX + (size_t)c0 * ldx + k0 + 1;
                 k_dg_split<HqCols, false><<<dim3(cb * (kDgBN / 8), (unsigned)((2 * steps + 31) / 32)), 256, 0, st>>>(
-                    HqCols{X, ldx, cols, kr}, kDgBN, cb * kDgBN, steps, exX + c0, nullptr, 0, cols, kr, XN);
+                    HqCols{X, ldx, cols, kr}, kDgBN, cb * kDgBN, steps, exX + c0, nullptr, 0, cols, kr, XN, nullptr);
                 int per = 0;
                 const int nz = dg_parts(cb, sms, kHqMaxSplit, steps, per);
                 const DgStoreLong e1{1, cb, steps, per, kHqNb, cols, exV + g * kHqNb, exX + c0, Wp, 1, kHqNb,
                                      (long long)kHqNb * cols};
-                if (dg_gemm(cb * nz, sms, VM + (size_t)at * vblock, XN, e1, st) != cudaSuccess) return true;
+                if (dg_gemm(cb * nz, sms, VM + (size_t)at * vblock, XN, e1, nullptr, st) != cudaSuccess) return true;
                 k_dg_small<HqSum, false><<<cb * (kDgBN / 8), 128, 0, st>>>(HqSum{Wp, nz, (long long)kHqNb * cols}, kDgBN,
-                                                                         cols, cb * kDgBN, kHqNb, nullptr, 0, exW, WN);
+                                                                         cols, cb * kDgBN, kHqNb, nullptr, 0, exW, WN, nullptr);
                 const DgStoreShort e2{1, cb, ksteps, ksteps, kHqNb, cols, exT + g * kHqNb, exW, W2, 1, kHqNb, 0};
-                if (dg_gemm(cb, sms, TM + (size_t)g * kHqNb * small, WN, e2, st) != cudaSuccess) return true;
+                if (dg_gemm(cb, sms, TM + (size_t)g * kHqNb * small, WN, e2, nullptr, st) != cudaSuccess) return true;
                 k_dg_small<HqSum, false><<<cb * (kDgBN / 8), 128, 0, st>>>(HqSum{W2, 1, 0}, kDgBN, cols, cb * kDgBN, kHqNb,
-                                                                         nullptr, 0, exW, WN);
+                                                                         nullptr, 0, exW, WN, nullptr);
                 const DgUpdate e3{rb, ksteps, kr, cols, exVA + at * kHqNb, exW, X, ldx, exX + c0, 0};
-                if (dg_gemm(rb * cb, sms, VA + (size_t)at * vblock, WN, e3, st) != cudaSuccess) return true;
+                if (dg_gemm(rb * cb, sms, VA + (size_t)at * vblock, WN, e3, nullptr, st) != cudaSuccess) return true;
             }
         }
     }
@@ -1372,9 +1554,10 @@ struct HbB2 {
 // M1 = [T^T, -T^T VY] (VY: the last 64 columns of W0), eight columns per CTA,
 // and their exponents.
 __global__ void __launch_bounds__(8 * kHbNb) k_hb_m1(const double *T, const double *VYp, int nz, long long cz, double *M,
-                                                     int *dk) {
+                                                     int *dk, const int *off) {
     __shared__ double vy[8][kHbNb];
     __shared__ int red[8][2];
+    if (dg_off(off)) return;
     const int q = threadIdx.x % kHbNb, c = threadIdx.x / kHbNb, k = blockIdx.x * 8 + c;
     double v;
     if (k < kHbNb) {
@@ -1406,6 +1589,7 @@ struct HbDigits {
     unsigned char *AD, *VN, *M1, *B1, *A2, *B2;
     double *Wp, *M, *Z;
     unsigned *top;                                               // rows' largest high words
+    int *low, *uneven;                                           // k_hb_even's counts and result
     int *cex, *exM1, *exB, *exA2, *dk1;                          // cex: n columns of A, then [Y V]
     int cch;
 };
@@ -1437,17 +1621,19 @@ size_t hb_digits_layout(int n, unsigned char *base, HbDigits &D) {
     D.exA2 = reinterpret_cast<int *>(take(all * sizeof(int)));
     D.dk1 = reinterpret_cast<int *>(take((size_t)2 * kHbNb * sizeof(int)));
     D.top = reinterpret_cast<unsigned *>(take((size_t)n * sizeof(unsigned)));
+    D.low = reinterpret_cast<int *>(take((size_t)(2 * n + 2) * sizeof(int)));   // the last two: counter, result
+    D.uneven = D.low + 2 * n + 1;
     return off;
 }
-// The trailing columns c1 .. n-1 of panel k0.
+// The trailing columns c1 .. n-1 of panel k0, where the matrix is even.
 cudaError_t hb_trailing(const HbState &S, const HbDigits &D, int k0, int c1, int sms, cudaStream_t st) {
     const int n = S.n, m = n - c1, kr = n - k0 - 1, total = m + kHbNb;
     const int steps = (kr + kDgBK - 1) / kDgBK;
     constexpr int ksteps = 2 * kHbNb / kDgBK;
     const int *exY = D.cex + n, *exV = exY + kHbNb;
-    k_dg_exp_k<<<2 * kHbNb, 256, 0, st>>>(HbPanelCols{S.Y, S.V, n, k0}, kr, nullptr, 0, D.cex + n);
+    k_dg_exp_k<<<2 * kHbNb, 256, 0, st>>>(HbPanelCols{S.Y, S.V, n, k0}, kr, nullptr, 0, D.cex + n, D.uneven);
     k_dg_split<HbVCols, false><<<dim3(kDgBN / 8, (unsigned)((2 * steps + 31) / 32)), 256, 0, st>>>(
-        HbVCols{S.V, n, k0}, kDgBN, kDgBN, steps, exV, nullptr, 0, kHbNb, kr, D.VN);
+        HbVCols{S.V, n, k0}, kDgBN, kDgBN, steps, exV, nullptr, 0, kHbNb, kr, D.VN, D.uneven);
     int per = 0;
     const int tiles = (std::min(total, D.cch) + kDgBM - 1) / kDgBM;
     const int nz = dg_parts(tiles, sms, kHbParts, steps, per);
@@ -1455,25 +1641,25 @@ cudaError_t hb_trailing(const HbState &S, const HbDigits &D, int k0, int c1, int
     for (int c = 0; c < total; c += D.cch) {
         const int cols = std::min(D.cch, total - c), mb = (cols + kDgBM - 1) / kDgBM;
         k_dg_split<HbTrail, false><<<dim3(mb * (kDgBM / 8), (unsigned)((2 * steps + 31) / 32)), 256, 0, st>>>(
-            HbTrail{S.A, S.Y, S.lda, n, k0, c1 + c}, kDgBM, mb * kDgBM, steps, D.cex + c1 + c, nullptr, 0, cols, kr, D.AD);
+            HbTrail{S.A, S.Y, S.lda, n, k0, c1 + c}, kDgBM, mb * kDgBM, steps, D.cex + c1 + c, nullptr, 0, cols, kr, D.AD, D.uneven);
         const DgStoreLong e{mb, 1, steps, per, cols, kHbNb, D.cex + c1 + c, exV, D.Wp + (size_t)kHbNb * c, kHbNb, 1, cz};
-        const cudaError_t err = dg_gemm(mb * nz, sms, D.AD, D.VN, e, st);
+        const cudaError_t err = dg_gemm(mb * nz, sms, D.AD, D.VN, e, D.uneven, st);
         if (err != cudaSuccess) return err;
     }
-    k_hb_m1<<<2 * kHbNb / 8, 8 * kHbNb, 0, st>>>(S.T, D.Wp + (size_t)kHbNb * m, nz, cz, D.M, D.dk1);
-    k_dg_small<HbM1, true><<<kDgBM / 32, 512, 0, st>>>(HbM1{D.M}, kDgBM, kHbNb, kDgBM, 2 * kHbNb, D.dk1, -1, D.exM1, D.M1);
+    k_hb_m1<<<2 * kHbNb / 8, 8 * kHbNb, 0, st>>>(S.T, D.Wp + (size_t)kHbNb * m, nz, cz, D.M, D.dk1, D.uneven);
+    k_dg_small<HbM1, true><<<kDgBM / 32, 512, 0, st>>>(HbM1{D.M}, kDgBM, kHbNb, kDgBM, 2 * kHbNb, D.dk1, -1, D.exM1, D.M1, D.uneven);
     const int nb = (m + kDgBN - 1) / kDgBN, rb = (n + kDgBM - 1) / kDgBM;
     k_dg_small<HbB1, false><<<nb * (kDgBN / 8), 128, 0, st>>>(HbB1{D.Wp, S.V, nz, n, c1, cz}, kDgBN, m, nb * kDgBN,
-                                                              2 * kHbNb, D.dk1, 1, D.exB, D.B1);
+                                                              2 * kHbNb, D.dk1, 1, D.exB, D.B1, D.uneven);
     const DgStoreShort ez{1, nb, ksteps, ksteps, kHbNb, m, D.exM1, D.exB, D.Z, 1, kHbNb, 0};
-    cudaError_t err = dg_gemm(nb, sms, D.M1, D.B1, ez, st);
+    cudaError_t err = dg_gemm(nb, sms, D.M1, D.B1, ez, D.uneven, st);
     if (err != cudaSuccess) return err;
     k_dg_small<HbA2, true><<<rb * (kDgBM / 32), 512, 0, st>>>(HbA2{S.Y, S.V, n}, kDgBM, n, rb * kDgBM, 2 * kHbNb, D.cex + n,
-                                                              -1, D.exA2, D.A2);
+                                                              -1, D.exA2, D.A2, D.uneven);
     k_dg_small<HbB2, false><<<nb * (kDgBN / 8), 128, 0, st>>>(HbB2{S.V, D.Z, n, c1}, kDgBN, m, nb * kDgBN, 2 * kHbNb,
-                                                              D.cex + n, 1, D.exB, D.B2);
+                                                              D.cex + n, 1, D.exB, D.B2, D.uneven);
     const DgUpdate eu{rb, ksteps, n, m, D.exA2, D.exB, S.A + (size_t)c1 * S.lda, S.lda, D.cex + c1, k0 + 1};
-    err = dg_gemm(rb * nb, sms, D.A2, D.B2, eu, st);
+    err = dg_gemm(rb * nb, sms, D.A2, D.B2, eu, D.uneven, st);
     return err != cudaSuccess ? err : cudaGetLastError();
 }
 
@@ -1594,7 +1780,10 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
     if (digits) {
         hb_digits_layout(n, dg.p, D);
         // Exponents of A's columns over the rows that reflectors touch.
-        k_dg_exp_k<<<n, 256, 0, st>>>(HqCols{dA + 1, lda, n, n - 1}, n - 1, nullptr, 0, D.cex);
+        k_dg_exp_k<<<n, 256, 0, st>>>(HqCols{dA + 1, lda, n, n - 1}, n - 1, nullptr, 0, D.cex, nullptr);
+        if (cudaMemsetAsync(D.low, 0, (size_t)(2 * n + 2) * sizeof(int), st) != cudaSuccess) return HSR_ERR_CUDA;
+        k_hb_even<<<dim3((n + 254) / 256, (n + kHbEvenCols - 1) / kHbEvenCols), 256, 0, st>>>(
+            n, dA, lda, D.cex, D.low, reinterpret_cast<unsigned *>(D.low + 2 * n), D.uneven);
     }
     for (int k0 = 0; k0 < n - 2; k0 += kHbNb) {
         const int ib = std::min(kHbNb, n - 2 - k0);
@@ -1606,17 +1795,20 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
             return HSR_ERR_CUDA;
         if (one) {
             const bool fix = digits && n >= kHbFixN;
-            HbPanel pp{S, k0, ib, R, own, rpc, rtiles, shares, S.cnt + 2, reinterpret_cast<const int2 *>(D.AD), D.top};
+            HbPanel pp{S, k0, ib, R, own, rpc, rtiles, shares, S.cnt + 2, reinterpret_cast<const int2 *>(D.AD), D.top,
+                       fix ? D.uneven : nullptr};
             void *args[] = {&pp};
             if (fix) {
                 const dim3 g((unsigned)(n + 255) / 256, (unsigned)((n - k0 - 1 + kFixCols - 1) / kFixCols));
                 if (cudaMemsetAsync(D.top, 0, (size_t)n * sizeof(unsigned), st) != cudaSuccess) return HSR_ERR_CUDA;
-                k_hb_fix_top<<<g, 256, 0, st>>>(n, dA, lda, k0 + 1, D.top);
-                k_hb_fix<<<g, 256, 0, st>>>(n, dA, lda, k0 + 1, D.top, reinterpret_cast<int2 *>(D.AD));
+                k_hb_fix_top<<<g, 256, 0, st>>>(n, dA, lda, k0 + 1, D.top, D.uneven);
+                k_hb_fix<<<g, 256, 0, st>>>(n, dA, lda, k0 + 1, D.top, reinterpret_cast<int2 *>(D.AD), D.uneven);
+                if (cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_hb_panel<true>), dim3(ctas), dim3(kHbThreads),
+                                                args, hb_panel_smem(R), st) != cudaSuccess)
+                    return HSR_ERR_CUDA;
             }
-            const void *fn = fix ? reinterpret_cast<const void *>(k_hb_panel<true>) : reinterpret_cast<const void *>(k_hb_panel<false>);
-            if (cudaLaunchCooperativeKernel(fn, dim3(ctas), dim3(kHbThreads), args,
-                                            hb_panel_smem(R), st) != cudaSuccess)
+            if (cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_hb_panel<false>), dim3(ctas), dim3(kHbThreads),
+                                            args, hb_panel_smem(R), st) != cudaSuccess)
                 return HSR_ERR_CUDA;
         } else {
             int nchp = 0;
@@ -1632,32 +1824,13 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
         }
         const int c1 = k0 + ib, m = n - c1;
         if (m <= 0) continue;
-        if (digits) {
-            if (hb_trailing(S, D, k0, c1, sms, st) != cudaSuccess) return HSR_ERR_CUDA;
-            continue;
-        }
-        // Right: A(:, c1:) -= Y V(c1:, :)^T
-        if (hb_gemm(n, m, ib, -1.0, S.Y, 1, n, S.V + c1, n, 1, 1.0, dA + (size_t)c1 * lda, lda, 1, 0, st) !=
-            cudaSuccess)
-            return HSR_ERR_CUDA;
-        // Left: W = T^T (V(k0+1:, :)^T A(k0+1:, c1:)); A(k0+1:, c1:) -= V(k0+1:, :) W
-        const int kr = n - k0 - 1;
-        const int tiles = ((m + kHbTm - 1) / kHbTm) * ((ib + kHbTm - 1) / kHbTm);
-        int split = (2 * sms + tiles - 1) / tiles;
-        split = std::max(1, std::min(split, std::min(kHbMaxSplit, (kr + kHbTk - 1) / kHbTk)));
-        if (hb_gemm(ib, m, kr, 1.0, S.V + (k0 + 1), n, 1, dA + (k0 + 1) + (size_t)c1 * lda, 1, lda, 0.0, Wp, nb,
-                    split, nb * (long long)m, st) != cudaSuccess)
-            return HSR_ERR_CUDA;
-        {
-            int kc = (((kr + split - 1) / split) + kHbTk - 1) / kHbTk * kHbTk;
-            const int nz = (kr + kc - 1) / kc;
-            const int tot = ib * m;
-            k_hb_sumk<<<(tot + 255) / 256, 256, 0, st>>>(ib, m, nz, Wp, nb, nb * (long long)m, W);
-        }
-        if (hb_gemm(ib, m, ib, 1.0, S.T, nb, 1, W, 1, nb, 0.0, W2, nb, 1, 0, st) != cudaSuccess ||
-            hb_gemm(kr, m, ib, -1.0, S.V + (k0 + 1), 1, n, W2, 1, nb, 1.0, dA + (k0 + 1) + (size_t)c1 * lda, lda, 1,
-                    0, st) != cudaSuccess)
-            return HSR_ERR_CUDA;
+        if (digits && hb_trailing(S, D, k0, c1, sms, st) != cudaSuccess) return HSR_ERR_CUDA;
+        // In FP64, where the matrix is not even or there are no digits.
+        const int kr = n - k0 - 1, mt = (m + kHbTm - 1) / kHbTm;
+        const int split = std::max(1, std::min((2 * sms + mt - 1) / mt, std::min(kHbMaxSplit, (kr + kHbTk - 1) / kHbTk)));
+        const HbPlain hp{S, k0, ib, c1, split, Wp, W, W2, S.cnt + 4, digits ? D.uneven : nullptr};
+        const int nt = (n + kHbTm - 1) / kHbTm, grid = std::min(2 * sms, nt * nt);   // the same for all panels (GridBar)
+        if (launch_phases(k_hb_plain, hp, kHbPlainPhases, grid, st) != cudaSuccess) return HSR_ERR_CUDA;
     }
     if (digits) dg.done(st);
     sc.done(st);

@@ -173,7 +173,10 @@ void hsr_release_workspace(void);
  * dlarfg): on exit the upper-Hessenberg part of dA holds H, column k below
  * the subdiagonal holds v_k(k+2 .. n-1) (v_k(k+1) = 1 implied), dtau[n] the
  * factors, and A = Q H Q^T with Q = H_0 ... H_{n-3}, H_k = I - tau_k v_k v_k^T.
- * Enqueued on `stream`; all pointers are device pointers.  No reference
+ * Where the entries of dA are of like size (decided on the device), products
+ * run on the tensor cores and in fixed point with errors no larger than FP64's;
+ * otherwise in FP64, so that the small rows and columns of a graded matrix stay
+ * accurate.  Enqueued on `stream`; all pointers are device pointers.  No reference
  * counterpart in the solver itself. */
 int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, void *stream);
 /* X <- Q X for the Q of hsr_hessenberg_device (LAPACK dormhr 'L','N'):

@@ -270,3 +270,87 @@ def test_back_transform_first_row(gpu_lib, n):
     assert np.isfinite(got[0]).all() and np.array_equal(got[:, 0], X[0], equal_nan=True)
     for c in range(1, 5):
         assert np.array_equal(got[c, 1:n], got[0, 1:n]), c
+
+
+def _form_q(torch, F, tau):
+    """Q of the reflectors in F (columns as usual) and tau, one by one in FP64."""
+    n = F.shape[0]
+    Q = torch.eye(n, dtype=torch.float64, device="cuda")
+    for k in range(n - 3, -1, -1):
+        v = F[k + 1:, k].clone()
+        v[0] = 1.0
+        Q[k + 1:] -= tau[k] * torch.outer(v, v @ Q[k + 1:])
+    return Q
+
+
+def _reduce_one_by_one(torch, A):
+    """dgehd2 in FP64: the reflectors one by one."""
+    F, n = A.clone(), A.shape[0]
+    tau = torch.zeros(n, dtype=torch.float64, device="cuda")
+    for k in range(n - 2):
+        x = F[k + 1:, k].clone()
+        beta = -torch.copysign(torch.linalg.norm(x), x[0])
+        tau[k] = (beta - x[0]) / beta
+        v = x / (x[0] - beta)
+        v[0] = 1.0
+        F[:, k + 1:] -= tau[k] * torch.outer(F[:, k + 1:] @ v, v)
+        F[k + 1:, k + 1:] -= tau[k] * torch.outer(v, v @ F[k + 1:, k + 1:])
+        F[k + 1, k] = beta
+        F[k + 2:, k] = v[1:]
+    return F, tau
+
+
+@pytest.mark.parametrize("n,pad,decades", [(33, 0, 10), (130, 1, 16), (160, 0, 30), (300, 0, 12), (2100, 0, 16)])
+def test_reduction_keeps_graded_rows(gpu_lib, n, pad, decades):
+    """A = D G D with D falling over many decades: the Householder reduction in
+    FP64 keeps the small rows and columns, (Q^T A Q - H)_ij of the size of d_i
+    d_j eps.  Within ten times of the reflectors one by one in FP64, whose sums
+    run in another order; a window below the largest entry would lose
+    everything (1e9 times and more)."""
+    import torch
+    import hsrq3in_gb300 as hsr
+    d = 10.0 ** (-decades * np.arange(n) / (n - 1))
+    A = np.random.default_rng(n).standard_normal((n, n)) * d[:, None] * d
+    dA = _cols(torch, A, pad)
+    tau = hsr.hessenberg_device(dA)
+    assert torch.all(dA[:, n:] == 5.0)
+    At, D = torch.from_numpy(A).cuda(), torch.from_numpy(d).cuda()
+    err = []
+    for F, t in ((dA[:, :n].T.contiguous(), tau), _reduce_one_by_one(torch, At)):
+        Q = _form_q(torch, F, t)
+        err.append(float(((Q.T @ At @ Q - torch.triu(F, -1)) / D[:, None] / D).abs().max()))
+    assert err[0] <= 10 * err[1], err
+
+
+@pytest.mark.parametrize("n,pad", [(32, 0), (65, 1), (130, 0), (321, 3), (2049, 0)])
+@pytest.mark.parametrize("form", ["zero", "eye", "band", "permutation", "sparse", "hessenberg", "blocks", "even"])
+def test_reduction_of_any_form(gpu_lib, n, pad, form):
+    """Matrices that the digit products take and that they leave to FP64: A Q =
+    Q H and Q^T Q = I to within n eps as in test_reduction_backward_error."""
+    import torch
+    import hsrq3in_gb300 as hsr
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((n, n))
+    if form == "zero":
+        A[:] = 0.0
+    elif form == "eye":
+        A = np.eye(n) + 1e-9 * A
+    elif form == "band":
+        A = np.tril(np.triu(A, -3), 2)
+    elif form == "permutation":
+        A = np.eye(n)[rng.permutation(n)]
+    elif form == "sparse":
+        A *= rng.random((n, n)) < 0.1
+    elif form == "hessenberg":
+        A = np.triu(A, -1)
+    elif form == "blocks":
+        A[: n // 2, n // 2:] *= 1e9
+        A[n // 2:, : n // 2] *= 1e-9
+    else:
+        A = rng.uniform(0.0, 1.0, (n, n))
+    dA = _cols(torch, A, pad)
+    tau = hsr.hessenberg_device(dA)
+    F = dA[:, :n].T.contiguous()
+    At, Q = torch.from_numpy(A).cuda(), _form_q(torch, F, tau)
+    assert float((Q.T @ Q - torch.eye(n, dtype=torch.float64, device="cuda")).norm()) <= n * EPS * np.sqrt(n)
+    assert float((At @ Q - Q @ torch.triu(F, -1)).norm()) <= n * EPS * np.linalg.norm(A)
