@@ -139,8 +139,10 @@ __device__ __forceinline__ int dg_dk(const int *dk, int k) {     // no scaling b
 }
 
 // Digit products are for operands whose entries are of like size; a call that
-// leaves the choice to the device passes a word `off` to every launch, which
-// does nothing where the word is not 0 (the caller's other form then runs).
+// leaves the choice to the device passes a word `off` to the splits and the
+// products, which store nothing where the word is not 0 (the caller's other
+// form then runs).  They read it beside their first loads or set-up: ahead of
+// them it cost 0.7 us a launch.
 __device__ __forceinline__ bool dg_off(const int *off) { return off && *off != 0; }
 
 // ---------------------------------------------------------- preparation
@@ -151,10 +153,8 @@ __device__ __forceinline__ bool dg_off(const int *off) { return off && *off != 0
 
 // Rows contiguous along k: a block per row.
 template <class Ld>
-__global__ void __launch_bounds__(256) k_dg_exp_k(Ld ld, int K, const int *dk, int sign, int *ex,
-                                                  const int *off) {
+__global__ void __launch_bounds__(256) k_dg_exp_k(Ld ld, int K, const int *dk, int sign, int *ex) {
     __shared__ int red[8];
-    if (dg_off(off)) return;
     const int r = blockIdx.x;
     int m = kDgZero;
     for (int k = threadIdx.x; k < K; k += blockDim.x) {
@@ -191,7 +191,7 @@ template <class Ld, bool RC>
 __global__ void __launch_bounds__(256) k_dg_split(Ld ld, int RB, int Rpad, long long steps, const int *ex,
                                                   const int *dk, int sign, int R, int K, unsigned char *out,
                                                   const int *off) {
-    if (dg_off(off)) return;
+    const bool skip = dg_off(off);
     const int t = threadIdx.x;
     const int r = RC ? blockIdx.x * 32 + (t & 31) : blockIdx.x * 8 + (t & 7);
     const int c8 = RC ? blockIdx.y * 8 + (t >> 5) : blockIdx.y * 32 + (t >> 3);
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(256) k_dg_split(Ld ld, int RB, int Rpad, long 
         const int k = c8 * 8 + e;
         u[e] = dg_digits(x[e], dk && k < K ? base - sign * dk[k] : base);
     }
-    dg_store8(u, out + dg_place(r, c8, RB, steps), RB * kDgBK * 2);
+    if (!skip) dg_store8(u, out + dg_place(r, c8, RB, steps), RB * kDgBK * 2);
 }
 
 // Exponents and digits in one pass for K <= 128: a thread keeps its eight
@@ -214,10 +214,9 @@ __global__ void __launch_bounds__(256) k_dg_split(Ld ld, int RB, int Rpad, long 
 // groups one group of eight columns each.
 template <class Ld, bool RC>
 __global__ void __launch_bounds__(RC ? 512 : 128) k_dg_small(Ld ld, int RB, int R, int Rpad, int K, const int *dk,
-                                                             int sign, int *ex, unsigned char *out, const int *off) {
+                                                             int sign, int *ex, unsigned char *out) {
     constexpr int ROWS = RC ? 32 : 8;
     __shared__ int red[ROWS][17];
-    if (dg_off(off)) return;
     const int t = threadIdx.x, rr = RC ? t & 31 : t & 7, c8 = RC ? t >> 5 : t >> 3;
     const int r = blockIdx.x * ROWS + rr;
     const int steps = (K + kDgBK - 1) / kDgBK;
@@ -458,7 +457,7 @@ k_dg_gemm(const unsigned char *__restrict__ A, const unsigned char *__restrict__
     __shared__ __align__(8) uint64_t full[kDgStages], empty[kDgStages], acc_full[kDgGroups], acc_empty[kDgGroups];
     __shared__ uint32_t tmem_base;
     __shared__ int failed;
-    if (dg_off(off)) return;
+    const bool skip = dg_off(off);
     const int tid = threadIdx.x, wid = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     if (tid == 0) {
         for (int i = 0; i < kDgStages; ++i) {
@@ -483,6 +482,7 @@ k_dg_gemm(const unsigned char *__restrict__ A, const unsigned char *__restrict__
     const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
     unsigned char *const sa = reinterpret_cast<unsigned char *>(((uintptr_t)dg_sm + 1023) & ~(uintptr_t)1023);
     unsigned char *const sb = sa + kDgStages * kDgABytes;
+    if (skip) tiles = 0;
     const uint32_t sa0 = __shfl_sync(0xffffffffu, smem_u32(sa), 0), sb0 = sa0 + kDgStages * kDgABytes;
 
     if (wid == 0) {

@@ -994,9 +994,10 @@ __device__ __forceinline__ void hb_gemm_tile(const HbGemm &g, int bx, int by, in
 __host__ __device__ __forceinline__ int hb_gemm_tiles(const HbGemm &g) {
     return g.M <= 0 || g.N <= 0 ? 0 : ((g.M + kHbTm - 1) / kHbTm) * ((g.N + kHbTm - 1) / kHbTm) * g.nz;
 }
-__device__ __forceinline__ void hb_gemm_run(const HbGemm &g, HbTiles &sm) {
+// `skip`: tiles of another product handed out just before.
+__device__ __forceinline__ void hb_gemm_run(const HbGemm &g, HbTiles &sm, int skip = 0) {
     const int mt = (g.M + kHbTm - 1) / kHbTm, nt = (g.N + kHbTm - 1) / kHbTm, total = hb_gemm_tiles(g);
-    for (int t = blockIdx.x; t < total; t += gridDim.x) {
+    for (int t = (blockIdx.x + gridDim.x - skip % gridDim.x) % gridDim.x; t < total; t += gridDim.x) {
         const int z = t / (mt * nt), r = t - z * mt * nt, by = r / mt;
         hb_gemm_tile(g, r - by * mt, by, z, sm);
         __syncthreads();                                         // before the next tile's first chunk
@@ -1103,91 +1104,146 @@ cudaError_t launch_phases(void (*kernel)(Params, int, int), Params P, int phases
 // 160 (2100): d from 1 to 2^-3 1.9e-15 / 1.6e-15 (5.3e-15 / 5.0e-15), to 2^-10
 // 1.1e-14 / 1.1e-14 (2.4e-14 / 2.1e-14), to 1e-16 4.6e-13 / 3e-4 (5.5e-13 /
 // 2e-3); those with d down to 2^-4 (n = 2100) and beyond are refused.  The
-// check reads A once: n = 700 13.36 -> 13.45 ms with the launches that do
-// nothing, n = 6000 316.0 -> 317.5.  Refused, d to 1e-12: n = 700 15.9 ms, n =
-// 4000 326.
+// check reads A once: n = 700 13.15 -> 13.19 ms with the launches that do
+// nothing, n = 6000 316.4 -> 317.7.  Refused, d to 1e-12: n = 700 16.1 ms, n =
+// 4000 317.
 constexpr int kHbEvenBits = 8;
-constexpr int kHbEvenCols = 64;        // columns per CTA
 __device__ __forceinline__ bool hb_few(int low, int of) { return 5 * low <= 2 * of; }
+// Counts of the entries that small(x, c) holds of rows r = r0 + tid (in or not)
+// and columns c0 .. c0 + 31, into low[r] and low[n + c]; get(c): an entry.
+constexpr int kEvenCols = 32;
+template <class Get, class Small>
+__device__ __forceinline__ void even_count(int n, int r, int c0, int cols, const Get &get, const Small &small, int *low) {
+    __shared__ int col[kEvenCols];
+    const int tid = threadIdx.x, lane = tid & 31;
+    if (tid < kEvenCols) col[tid] = 0;
+    __syncthreads();
+    int mine = 0, ours = 0;                                      // of this row; lane c: of column c, these 32 rows
+#pragma unroll
+    for (int c = 0; c < kEvenCols; c += 16) {
+        double x[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) x[q] = get(c0 + min(c + q, cols - 1));
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            const bool s = c + q < cols && small(x[q], c + q);
+            const unsigned b = __ballot_sync(0xffffffffu, s);
+            if (lane == c + q) ours = __popc(b);
+            mine += s;
+        }
+    }
+    if (mine) atomicAdd(&low[r], mine);
+    if (ours) atomicAdd(&col[lane], ours);
+    __syncthreads();
+    if (tid < cols && col[tid]) atomicAdd(&low[n + c0 + tid], col[tid]);
+}
+// The CTA that counted last (of a 2-d grid) sees all counts.
+__device__ __forceinline__ bool even_last(unsigned *cnt) {
+    __shared__ bool am_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) am_last = atomicAdd(cnt, 1u) == gridDim.x * gridDim.y - 1;
+    __syncthreads();
+    if (am_last) __threadfence();
+    return am_last;
+}
 // cex: exponents of A's columns over rows 1 ..; low: 2 n counts, zeroed, of the
 // rows' and the columns' smaller (or non-finite) entries; cnt: a counter, zeroed.
 __global__ void __launch_bounds__(256) k_hb_even(int n, const double *A, long long lda, const int *cex, int *low, unsigned *cnt,
                                                  int *uneven) {
-    __shared__ int red[8], col[kHbEvenCols];
-    const int tid = threadIdx.x, r = 1 + blockIdx.x * 256 + tid, c0 = blockIdx.y * kHbEvenCols, cols = min(kHbEvenCols, n - c0);
+    __shared__ int red[8];
+    const int tid = threadIdx.x, r = 1 + blockIdx.x * 256 + tid, c0 = blockIdx.y * kEvenCols, cols = min(kEvenCols, n - c0);
     int top = kDgZero;
     for (int c = tid; c < n; c += 256) top = dg_bad(cex[c]) ? top : max(top, cex[c]);
     top = __reduce_max_sync(0xffffffffu, top);
     if ((tid & 31) == 0) red[tid >> 5] = top;
-    if (tid < kHbEvenCols) col[tid] = 0;
     __syncthreads();
     for (int w = 0; w < 8; ++w) top = max(top, red[w]);
-    int mine = 0;
-#pragma unroll 4
-    for (int c = 0; c < cols; ++c) {
-        const int e = r < n ? dg_exp(A[r + (size_t)(c0 + c) * lda]) : top;
-        const bool small = e < top - kHbEvenBits || dg_bad(e);
-        const unsigned b = __ballot_sync(0xffffffffu, small);
-        if ((tid & 31) == 0 && b) atomicAdd(&col[c], __popc(b));
-        mine += small;
-    }
-    if (mine) atomicAdd(&low[r], mine);
-    __syncthreads();
-    if (tid < cols && col[tid]) atomicAdd(&low[n + c0 + tid], col[tid]);
-    // The last CTA decides.
-    __shared__ bool am_last;
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) am_last = atomicAdd(cnt, 1u) == gridDim.x * gridDim.y - 1;
-    __syncthreads();
-    if (!am_last) return;
-    __threadfence();
+    even_count(n, r, c0, cols, [&](int c) { return r < n ? A[r + (size_t)c * lda] : 0.0; },
+               [&](double x, int) {
+                   const int e = dg_exp(x);
+                   return r < n && (e < top - kHbEvenBits || dg_bad(e));
+               }, low);
+    if (!even_last(cnt)) return;
     bool bad = false;
     for (int q = tid; q < n; q += 256) bad = bad || !hb_few(__ldcg(&low[n + q]), n - 1) || (q > 0 && !hb_few(__ldcg(&low[q]), n));
     bad = __syncthreads_or(bad);
     if (tid == 0) *uneven = bad;
 }
 
-// The same as launches of their own.
-__global__ void __launch_bounds__(256, 2) k_hb_gemm(HbGemm g) {
+// Back-transform Q X in FP64, blocked like LAPACK dormhr ('L', 'N'): the panels
+// of the reduction in reverse order, X(k0+1:, :) -= V (T (V^T X(k0+1:, :))),
+// with V rebuilt from the reflectors stored in A and T from V and tau (dlarft:
+// T(0:i, i) = -tau_i T(0:i, 0:i) (V^T V)(0:i, i), T(i, i) = tau_i).  Six phases a
+// panel: V; the parts of V^T V and V^T X; their sums G and W; T; T W; X.  One
+// cooperative launch for all panels, so that a call which the digits take
+// passes over it in one launch.
+struct HqPlain {
+    int n, ncols;
+    const double *A;
+    long long lda;
+    const double *tau;
+    double *X;
+    long long ldx;
+    double *V, *T, *G, *Gp, *W, *Wp, *W2;
+    int splitg, splitw;                // parts of the sums over rows, at most
+    unsigned *bar;
+    const int *uneven;                 // runs where it is not 0 (null: runs)
+};
+constexpr int kHqPlainPhases = 6;
+__global__ void __launch_bounds__(256, 2) k_hq_plain(HqPlain P, int first, int last) {
     __shared__ HbTiles sm;
-    hb_gemm_run(g, sm);
-}
-__global__ void k_hb_sumk(int M, int N, int nz, const double *Wp, long long ldw, long long cz, double *W) {
-    hb_sum_parts(M, N, nz, Wp, ldw, cz, W);
-}
-cudaError_t hb_gemm(int M, int N, int K, double alpha, const double *A, long long sai, long long sak,
-                    const double *B, long long sbk, long long sbj, double beta, double *C, long long ldc,
-                    int nsplit, long long cz, cudaStream_t st) {
-    if (M <= 0 || N <= 0) return cudaSuccess;
-    const HbGemm g{M, N, K, hb_parts(K, nsplit), hb_kc(K, nsplit), alpha, A, sai, sak, B, sbk, sbj, beta, C, ldc, cz};
-    k_hb_gemm<<<hb_gemm_tiles(g), 256, 0, st>>>(g);
-    return cudaGetLastError();
-}
-
-// Back-transform Q X, blocked like LAPACK dormhr ('L', 'N'): the panels of
-// the reduction in reverse order, X(k0+1:, :) -= V (T (V^T X(k0+1:, :))), with
-// V rebuilt from the reflectors stored in A and T from V and tau (dlarft:
-// T(0:i, i) = -tau_i T(0:i, 0:i) (V^T V)(0:i, i), T(i, i) = tau_i).
-__global__ void k_hq_vpanel(int n, const double *A, long long lda, int k0, double *V) {
-    const int i = blockIdx.y, j = k0 + i;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x)
-        V[r + (size_t)i * n] = r == j + 1 ? 1.0 : (r >= j + 2 ? A[r + (size_t)j * lda] : 0.0);
-}
-
-__global__ void k_hq_tfactor(int ib, const double *tau, const double *G, double *T) {
-    for (int i = 0; i < ib; ++i) {
-        const double t = tau[i];
-        for (int p = threadIdx.x; p < i; p += blockDim.x) {
-            double s = 0.0;
-            for (int q = p; q < i; ++q) s = fma(T[p + (size_t)q * kHbNb], G[q + (size_t)i * kHbNb], s);
-            T[p + (size_t)i * kHbNb] = -t * s;
+    if (P.uneven && *P.uneven == 0) return;
+    const long long n = P.n, nb = kHbNb, nc = P.ncols;
+    const int panels = (P.n - 3) / kHbNb + 1;
+    GridBar bar(P.bar);
+    for (int ph = first; ph < last; ++ph) {
+        const int k0 = (panels - 1 - ph / kHqPlainPhases) * kHbNb, ib = min(kHbNb, P.n - 2 - k0), kr = P.n - k0 - 1;
+        const double *const V = P.V + (k0 + 1);
+        double *const X = P.X + (k0 + 1);
+        const int zg = hb_parts(kr, P.splitg), zw = hb_parts(kr, P.splitw);
+        switch (ph % kHqPlainPhases) {
+        case 0:
+            for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n * ib; e += (long long)gridDim.x * blockDim.x) {
+                const int i = (int)(e / n), r = (int)(e - i * n), j = k0 + i;
+                P.V[e] = r == j + 1 ? 1.0 : (r >= j + 2 ? P.A[r + (size_t)j * P.lda] : 0.0);
+            }
+            break;
+        case 1:
+            {
+                const HbGemm w{ib, P.ncols, kr, zw, hb_kc(kr, P.splitw), 1.0, V, n, 1, X, 1, P.ldx, 0.0, P.Wp, nb, nb * nc};
+                hb_gemm_run(w, sm);
+                hb_gemm_run(HbGemm{ib, ib, kr, zg, hb_kc(kr, P.splitg), 1.0, V, n, 1, V, 1, n, 0.0, P.Gp, nb, nb * ib}, sm,
+                            hb_gemm_tiles(w));
+            }
+            break;
+        case 2:
+            hb_sum_parts(ib, ib, zg, P.Gp, nb, nb * ib, P.G);
+            hb_sum_parts(ib, P.ncols, zw, P.Wp, nb, nb * nc, P.W);
+            break;
+        case 3:
+            for (int i = 0; blockIdx.x == 0 && i < ib; ++i) {
+                const double t = P.tau[k0 + i];
+                for (int p = threadIdx.x; p < i; p += blockDim.x) {
+                    double s = 0.0;
+                    for (int q = p; q < i; ++q) s = fma(P.T[p + (size_t)q * kHbNb], P.G[q + (size_t)i * kHbNb], s);
+                    P.T[p + (size_t)i * kHbNb] = -t * s;
+                }
+                for (int p = i + threadIdx.x; p < kHbNb; p += blockDim.x) P.T[p + (size_t)i * kHbNb] = p == i ? t : 0.0;
+                __syncthreads();
+            }
+            break;
+        case 4:
+            hb_gemm_run(HbGemm{ib, P.ncols, ib, 1, ib, 1.0, P.T, 1, nb, P.W, 1, nb, 0.0, P.W2, nb, 0}, sm);
+            break;
+        default:
+            hb_gemm_run(HbGemm{kr, P.ncols, ib, 1, ib, -1.0, V, 1, n, P.W2, 1, nb, 1.0, X, P.ldx, 0}, sm);
         }
-        if (threadIdx.x == 0) {
-            T[i + (size_t)i * kHbNb] = t;
-            for (int p = i + 1; p < kHbNb; ++p) T[p + (size_t)i * kHbNb] = 0.0;
+        if (ph + 1 < last && !bar.meet()) {
+            if (blockIdx.x == 0)
+                for (long long e = threadIdx.x; e < (n - 1) * nc; e += blockDim.x) P.X[1 + e % (n - 1) + (e / (n - 1)) * P.ldx] = dg_nan();
+            return;
         }
-        __syncthreads();
     }
 }
 
@@ -1200,14 +1256,56 @@ __global__ void k_hq_tfactor(int ib, const double *tau, const double *G, double 
 // X -= V (T W).
 constexpr int kHqNb = 128;
 // Smallest order: a reflector of the DFMA form costs about 5.5 us (three thin
-// products and a serial factor per 64), this form 215 us and 0.5 us each
-// (n = 20: 155 us as DFMA; 64: 337 against 225; 300: 1,780 against 390;
-// 5000 with 2500 columns: 175.4 ms against 8.5).  The DFMA form also stays for
-// a scratch buffer that cannot be had.
+// products and a serial factor per 64), this form 240 us and 0.5 us each
+// (n = 32: 139 us as DFMA; 64: 360 against 248; 300: 1,665 against 411; 4000
+// with 2000 columns: 85.7 ms against 5.3).  The DFMA form also stays for
+// reflectors that are not even and for a scratch buffer that cannot be had.
 constexpr int kHqDigitsN = 40;
 // Most scratch for digits of X's columns and of V (three layouts) at a time.
 constexpr size_t kHqXBytes = (size_t)1 << 30, kHqVBytes = (size_t)4 << 30;
 constexpr int kHqMaxSplit = 16;
+
+// Whether the reflectors allow digits.  A column of X is held by a window below
+// its largest entry in rows 1 ..; that loses nothing where the reflectors carry
+// an entry of that size into every row, whose rounding in FP64 is then as large.
+// So in every column of V with kHqEvenMin entries below its 1, and in every row
+// with as many, three fifths of the entries have to be at least 2^-5 / sqrt(m),
+// m the length of the column (a reflector's norm is at most sqrt(2) and that of
+// a random one's entries about 1 / sqrt(m)), and tau not near 0.  Reflectors of
+// D G D on columns D G', G and G' of N(0,1) entries, error row by row relative
+// to the row's largest, in FP64 / by digits: d down to 1e-8 (n = 45) 2.5e-15 /
+// 2.6e-9, to 1e-12 (n = 300) 3.3e-15 / 2.3e-7.  The check reads V once: n = 64
+// 232 -> 248 us, n = 700 622 -> 650, n = 5000 with 2500 columns 8.56 -> 8.70 ms.
+// Refused, n = 700 with 350 columns 3.86 ms, n = 4000 with 2000 86.
+constexpr int kHqEvenBits = 5, kHqEvenMin = 32;
+// low: 2 n counts, zeroed, of the rows' and the columns' smaller entries; cnt: a
+// counter, zeroed.
+__global__ void __launch_bounds__(256) k_hq_even(int n, const double *A, long long lda, const double *tau, int *low, unsigned *cnt,
+                                                 int *uneven) {
+    __shared__ int least[kEvenCols];                             // smallest exponent of a column that counts
+    const int tid = threadIdx.x, r = blockIdx.x * 256 + tid, c0 = blockIdx.y * kEvenCols, cols = min(kEvenCols, n - 2 - c0);
+    if ((int)(blockIdx.x + 1) * 256 > c0 + 2) {                  // some row is below some column's 1
+        if (tid < kEvenCols) {
+            const int m = max(n - 1 - (c0 + tid), 1);
+            const unsigned long long t = tid < cols ? ubits(tau[c0 + tid]) : 0;      // mixing: 0.5 <= tau, no NaN
+            least[tid] = t < pow2_bits(-1) || t >= kInfBits ? INT_MAX : 1022 - kHqEvenBits - ((32 - __clz(m)) >> 1);
+        }
+        even_count(n, r, c0, cols, [&](int c) { return r < n && r >= c + 2 ? A[r + (size_t)c * lda] : 0.0; },
+                   [&](double x, int c) {
+                       const int e = dg_exp(x);
+                       return r < n && r >= c0 + c + 2 && (e < least[c] || dg_bad(e));
+                   }, low);
+    }
+    if (!even_last(cnt)) return;
+    bool bad = false;
+    for (int q = tid; q < n; q += 256) {
+        const int below = n - 2 - q, left = q - 1;               // entries of column q and of row q
+        bad = bad || (below >= kHqEvenMin && !hb_few(__ldcg(&low[n + q]), below)) ||
+              (left >= kHqEvenMin && !hb_few(__ldcg(&low[q]), left));
+    }
+    bad = __syncthreads_or(bad);
+    if (tid == 0) *uneven = bad;
+}
 
 // The blocks of a group, last first: block g of the group begins at reflector
 // k0(g) and has rows k0 + 1 .. n - 1.  Its row blocks of 128 count from the
@@ -1217,6 +1315,7 @@ struct HqGroup {
     const double *A;
     long long lda;
     int n, klast, rb0;                                           // klast: k0 of block 0
+    const int *off;
     __host__ __device__ __forceinline__ int k0(int g) const { return klast - g * kHqNb; }
     __host__ __device__ __forceinline__ int rblocks(int g) const { return rb0 + g; }
     __host__ __device__ __forceinline__ long long before(int g) const {      // row blocks of blocks 0 .. g-1
@@ -1243,6 +1342,7 @@ template <int RB>
 __global__ void __launch_bounds__(256) k_hq_vcols(HqGroup h, const int *ex, unsigned char *out) {
     const int t = threadIdx.x, g = blockIdx.z, r = blockIdx.x * 8 + (t & 7), c8 = blockIdx.y * 32 + (t >> 3);
     const int steps = h.rblocks(g) * (kHqNb / kDgBK);
+    if (dg_off(h.off)) return;
     if (c8 >= 2 * steps) return;
     const int base = max(ex[g * kHqNb + r], kDgZero) - 9, i0 = h.k0(g) + 1 + c8 * 8;
     unsigned long long u[8];
@@ -1254,7 +1354,7 @@ __global__ void __launch_bounds__(256) k_hq_vcols(HqGroup h, const int *ex, unsi
 __global__ void __launch_bounds__(512) k_hq_vrows(HqGroup h, int *ex, unsigned char *out) {
     __shared__ int red[32][17];
     const int t = threadIdx.x, g = blockIdx.y, rr = t & 31, c8 = t >> 5, r = blockIdx.x * 32 + rr;
-    if (r - rr >= h.rblocks(g) * kHqNb) return;                  // uniform over the block
+    if (dg_off(h.off) || r - rr >= h.rblocks(g) * kHqNb) return; // uniform over the block
     double x[8];
     int m = kDgZero;
 #pragma unroll
@@ -1348,6 +1448,7 @@ __device__ __forceinline__ double hq_gram(const double *S, int nz, int p, int i)
 }
 __global__ void __launch_bounds__(4 * kHqHalf) k_hq_thalf(HqGroup h, const double *tau, const double *Sp, int nz, double *T) {
     __shared__ double ts[kHqHalf * (kHqHalf + 1) / 2], ss[kHqHalf * (kHqHalf + 1) / 2], part[4][kHqHalf];
+    if (dg_off(h.off)) return;
     const int p = threadIdx.x % kHqHalf, w = threadIdx.x / kHqHalf, o = blockIdx.y * kHqHalf;
     const int k0 = h.k0(blockIdx.x) + o, ib = max(0, min(kHqHalf, h.n - 2 - k0));
     const double *S = Sp + (size_t)blockIdx.x * nz * kHqNb * kHqNb + o + (size_t)o * kHqNb;
@@ -1370,8 +1471,9 @@ __global__ void __launch_bounds__(4 * kHqHalf) k_hq_thalf(HqGroup h, const doubl
         }
     }
 }
-__global__ void __launch_bounds__(8 * kHqHalf) k_hq_tcross(HqGroup, const double *Sp, int nz, double *T) {
+__global__ void __launch_bounds__(8 * kHqHalf) k_hq_tcross(HqGroup h, const double *Sp, int nz, double *T) {
     __shared__ double s12[kHqHalf][kHqHalf + 1], t22[kHqHalf][8], u[kHqHalf][8];
+    if (dg_off(h.off)) return;
     const int p = threadIdx.x % kHqHalf, c = threadIdx.x / kHqHalf, col = blockIdx.y * 8 + c;
     const double *S = Sp + (size_t)blockIdx.x * nz * kHqNb * kHqNb + (size_t)kHqHalf * kHqNb;   // S(0.., 64..)
     double *To = T + (size_t)blockIdx.x * kHqNb * kHqNb;
@@ -1394,9 +1496,10 @@ __global__ void __launch_bounds__(8 * kHqHalf) k_hq_tcross(HqGroup, const double
     To[kHqHalf + p + (size_t)col * kHqNb] = 0.0;                 // T21
 }
 
+// Enqueues the digit form, which does nothing where *uneven (set here) is not 0.
 // False when the scratch cannot be had: nothing has been enqueued then.
 bool hq_digits(int n, const double *dA, int lda, const double *dtau, int ncols, double *dX, int ldx, int dev, int sms,
-               cudaStream_t st, int *rc) {
+               cudaStream_t st, const int **uneven, int *rc) {
     static thread_local DgScratch dg;
     constexpr int ksteps = kHqNb / kDgBK;
     constexpr size_t vblock = (size_t)kHqNb * kHqNb * kDgDigits * 2, small = (size_t)kHqNb * kDgDigits * 2;
@@ -1417,30 +1520,34 @@ bool hq_digits(int n, const double *dA, int lda, const double *dtau, int ncols, 
                  oVA = take(vrb * vblock), oTM = take((size_t)gmax * kHqNb * small), oWN = take((size_t)cch * small),
                  oS = take((size_t)gmax * kHqMaxSplit * kHqNb * kHqNb * 8), oT = take((size_t)gmax * kHqNb * kHqNb * 8),
                  oWp = take((size_t)kHqMaxSplit * kHqNb * cch * 8), oW2 = take((size_t)kHqNb * cch * 8),
-                 oEx = take(((size_t)ncols + cch + vrb * kHqNb + (size_t)2 * gmax * kHqNb) * sizeof(int));
+                 oEx = take(((size_t)ncols + cch + vrb * kHqNb + (size_t)2 * gmax * kHqNb + 2 * n + 2) * sizeof(int));
     if (!dg.ensure(off, dev, st)) return false;
     unsigned char *const b = dg.p, *XN = b + oXN, *VM = b + oVM, *VN = b + oVN, *VA = b + oVA, *TM = b + oTM, *WN = b + oWN;
     double *S = reinterpret_cast<double *>(b + oS), *T = reinterpret_cast<double *>(b + oT),
            *Wp = reinterpret_cast<double *>(b + oWp), *W2 = reinterpret_cast<double *>(b + oW2);
     int *exX = reinterpret_cast<int *>(b + oEx), *exW = exX + ncols, *exVA = exW + cch, *exV = exVA + vrb * kHqNb,
-        *exT = exV + gmax * kHqNb;
+        *exT = exV + gmax * kHqNb, *low = exT + gmax * kHqNb, *gate = low + 2 * n + 1;
+    *uneven = gate;
     *rc = HSR_ERR_CUDA;
+    if (cudaMemsetAsync(low, 0, (size_t)(2 * n + 2) * sizeof(int), st) != cudaSuccess) return true;
+    k_hq_even<<<dim3((n + 255) / 256, (n - 2 + kEvenCols - 1) / kEvenCols), 256, 0, st>>>(
+        n, dA, lda, dtau, low, reinterpret_cast<unsigned *>(low + 2 * n), gate);
     // Over the rows that reflectors touch: row 0 stays what it is.
-    k_dg_exp_k<<<ncols, 256, 0, st>>>(HqCols{dX + 1, ldx, ncols, n - 1}, n - 1, nullptr, 0, exX, nullptr);
+    k_dg_exp_k<<<ncols, 256, 0, st>>>(HqCols{dX + 1, ldx, ncols, n - 1}, n - 1, nullptr, 0, exX);
     for (int last = nblk - 1; last >= 0; last -= gmax) {
         const int ng = std::min(gmax, last + 1);
-        const HqGroup h{dA, lda, n, last * kHqNb, (n - 1 - last * kHqNb + kHqNb - 1) / kHqNb};
+        const HqGroup h{dA, lda, n, last * kHqNb, (n - 1 - last * kHqNb + kHqNb - 1) / kHqNb, gate};
         const int rmax = h.rblocks(ng - 1), gz = std::min(kHqMaxSplit, std::max(1, 2 * sms / (2 * ng)));
-        k_dg_exp_k<<<ng * kHqNb, 256, 0, st>>>(HqVCols{h}, n - h.k0(ng - 1) - 1, nullptr, 0, exV, nullptr);
+        k_dg_exp_k<<<ng * kHqNb, 256, 0, st>>>(HqVCols{h}, n - h.k0(ng - 1) - 1, nullptr, 0, exV);
         const dim3 gv(kHqNb / 8, (unsigned)((2 * rmax * ksteps + 31) / 32), ng);
         k_hq_vcols<kDgBM><<<gv, 256, 0, st>>>(h, exV, VM);
         k_hq_vcols<kDgBN><<<gv, 256, 0, st>>>(h, exV, VN);
         k_hq_vrows<<<dim3(rmax * (kHqNb / 32), ng), 512, 0, st>>>(h, exVA, VA);
-        if (dg_gemm(2 * gz * ng, sms, VM, VN, HqGram{h, gz, exV, S}, nullptr, st) != cudaSuccess) return true;
+        if (dg_gemm(2 * gz * ng, sms, VM, VN, HqGram{h, gz, exV, S}, gate, st) != cudaSuccess) return true;
         k_hq_thalf<<<dim3(ng, 2), 4 * kHqHalf, 0, st>>>(h, dtau, S, gz, T);
         k_hq_tcross<<<dim3(ng, kHqHalf / 8), 8 * kHqHalf, 0, st>>>(h, S, gz, T);
         k_dg_small<HqT, true><<<ng * (kHqNb / 32), 512, 0, st>>>(HqT{T}, kDgBM, ng * kHqNb, ng * kHqNb, kHqNb, nullptr, 0,
-                                                                exT, TM, nullptr);
+                                                                exT, TM);
         for (int c0 = 0; c0 < ncols; c0 += cch) {
             const int cols = std::min(cch, ncols - c0), cb = (cols + kDgBN - 1) / kDgBN;
             for (int g = 0; g < ng; ++g) {
@@ -1448,20 +1555,20 @@ bool hq_digits(int n, const double *dA, int lda, const double *dtau, int ncols, 
                 const long long at = h.before(g);
                 double *X = dX + (size_t)c0 * ldx + k0 + 1;
                 k_dg_split<HqCols, false><<<dim3(cb * (kDgBN / 8), (unsigned)((2 * steps + 31) / 32)), 256, 0, st>>>(
-                    HqCols{X, ldx, cols, kr}, kDgBN, cb * kDgBN, steps, exX + c0, nullptr, 0, cols, kr, XN, nullptr);
+                    HqCols{X, ldx, cols, kr}, kDgBN, cb * kDgBN, steps, exX + c0, nullptr, 0, cols, kr, XN, gate);
                 int per = 0;
                 const int nz = dg_parts(cb, sms, kHqMaxSplit, steps, per);
                 const DgStoreLong e1{1, cb, steps, per, kHqNb, cols, exV + g * kHqNb, exX + c0, Wp, 1, kHqNb,
                                      (long long)kHqNb * cols};
-                if (dg_gemm(cb * nz, sms, VM + (size_t)at * vblock, XN, e1, nullptr, st) != cudaSuccess) return true;
+                if (dg_gemm(cb * nz, sms, VM + (size_t)at * vblock, XN, e1, gate, st) != cudaSuccess) return true;
                 k_dg_small<HqSum, false><<<cb * (kDgBN / 8), 128, 0, st>>>(HqSum{Wp, nz, (long long)kHqNb * cols}, kDgBN,
-                                                                         cols, cb * kDgBN, kHqNb, nullptr, 0, exW, WN, nullptr);
+                                                                         cols, cb * kDgBN, kHqNb, nullptr, 0, exW, WN);
                 const DgStoreShort e2{1, cb, ksteps, ksteps, kHqNb, cols, exT + g * kHqNb, exW, W2, 1, kHqNb, 0};
-                if (dg_gemm(cb, sms, TM + (size_t)g * kHqNb * small, WN, e2, nullptr, st) != cudaSuccess) return true;
+                if (dg_gemm(cb, sms, TM + (size_t)g * kHqNb * small, WN, e2, gate, st) != cudaSuccess) return true;
                 k_dg_small<HqSum, false><<<cb * (kDgBN / 8), 128, 0, st>>>(HqSum{W2, 1, 0}, kDgBN, cols, cb * kDgBN, kHqNb,
-                                                                         nullptr, 0, exW, WN, nullptr);
+                                                                         nullptr, 0, exW, WN);
                 const DgUpdate e3{rb, ksteps, kr, cols, exVA + at * kHqNb, exW, X, ldx, exX + c0, 0};
-                if (dg_gemm(rb * cb, sms, VA + (size_t)at * vblock, WN, e3, nullptr, st) != cudaSuccess) return true;
+                if (dg_gemm(rb * cb, sms, VA + (size_t)at * vblock, WN, e3, gate, st) != cudaSuccess) return true;
             }
         }
     }
@@ -1554,10 +1661,9 @@ struct HbB2 {
 // M1 = [T^T, -T^T VY] (VY: the last 64 columns of W0), eight columns per CTA,
 // and their exponents.
 __global__ void __launch_bounds__(8 * kHbNb) k_hb_m1(const double *T, const double *VYp, int nz, long long cz, double *M,
-                                                     int *dk, const int *off) {
+                                                     int *dk) {
     __shared__ double vy[8][kHbNb];
     __shared__ int red[8][2];
-    if (dg_off(off)) return;
     const int q = threadIdx.x % kHbNb, c = threadIdx.x / kHbNb, k = blockIdx.x * 8 + c;
     double v;
     if (k < kHbNb) {
@@ -1631,7 +1737,7 @@ cudaError_t hb_trailing(const HbState &S, const HbDigits &D, int k0, int c1, int
     const int steps = (kr + kDgBK - 1) / kDgBK;
     constexpr int ksteps = 2 * kHbNb / kDgBK;
     const int *exY = D.cex + n, *exV = exY + kHbNb;
-    k_dg_exp_k<<<2 * kHbNb, 256, 0, st>>>(HbPanelCols{S.Y, S.V, n, k0}, kr, nullptr, 0, D.cex + n, D.uneven);
+    k_dg_exp_k<<<2 * kHbNb, 256, 0, st>>>(HbPanelCols{S.Y, S.V, n, k0}, kr, nullptr, 0, D.cex + n);
     k_dg_split<HbVCols, false><<<dim3(kDgBN / 8, (unsigned)((2 * steps + 31) / 32)), 256, 0, st>>>(
         HbVCols{S.V, n, k0}, kDgBN, kDgBN, steps, exV, nullptr, 0, kHbNb, kr, D.VN, D.uneven);
     int per = 0;
@@ -1646,18 +1752,18 @@ cudaError_t hb_trailing(const HbState &S, const HbDigits &D, int k0, int c1, int
         const cudaError_t err = dg_gemm(mb * nz, sms, D.AD, D.VN, e, D.uneven, st);
         if (err != cudaSuccess) return err;
     }
-    k_hb_m1<<<2 * kHbNb / 8, 8 * kHbNb, 0, st>>>(S.T, D.Wp + (size_t)kHbNb * m, nz, cz, D.M, D.dk1, D.uneven);
-    k_dg_small<HbM1, true><<<kDgBM / 32, 512, 0, st>>>(HbM1{D.M}, kDgBM, kHbNb, kDgBM, 2 * kHbNb, D.dk1, -1, D.exM1, D.M1, D.uneven);
+    k_hb_m1<<<2 * kHbNb / 8, 8 * kHbNb, 0, st>>>(S.T, D.Wp + (size_t)kHbNb * m, nz, cz, D.M, D.dk1);
+    k_dg_small<HbM1, true><<<kDgBM / 32, 512, 0, st>>>(HbM1{D.M}, kDgBM, kHbNb, kDgBM, 2 * kHbNb, D.dk1, -1, D.exM1, D.M1);
     const int nb = (m + kDgBN - 1) / kDgBN, rb = (n + kDgBM - 1) / kDgBM;
     k_dg_small<HbB1, false><<<nb * (kDgBN / 8), 128, 0, st>>>(HbB1{D.Wp, S.V, nz, n, c1, cz}, kDgBN, m, nb * kDgBN,
-                                                              2 * kHbNb, D.dk1, 1, D.exB, D.B1, D.uneven);
+                                                              2 * kHbNb, D.dk1, 1, D.exB, D.B1);
     const DgStoreShort ez{1, nb, ksteps, ksteps, kHbNb, m, D.exM1, D.exB, D.Z, 1, kHbNb, 0};
     cudaError_t err = dg_gemm(nb, sms, D.M1, D.B1, ez, D.uneven, st);
     if (err != cudaSuccess) return err;
     k_dg_small<HbA2, true><<<rb * (kDgBM / 32), 512, 0, st>>>(HbA2{S.Y, S.V, n}, kDgBM, n, rb * kDgBM, 2 * kHbNb, D.cex + n,
-                                                              -1, D.exA2, D.A2, D.uneven);
+                                                              -1, D.exA2, D.A2);
     k_dg_small<HbB2, false><<<nb * (kDgBN / 8), 128, 0, st>>>(HbB2{S.V, D.Z, n, c1}, kDgBN, m, nb * kDgBN, 2 * kHbNb,
-                                                              D.cex + n, 1, D.exB, D.B2, D.uneven);
+                                                              D.cex + n, 1, D.exB, D.B2);
     const DgUpdate eu{rb, ksteps, n, m, D.exA2, D.exB, S.A + (size_t)c1 * S.lda, S.lda, D.cex + c1, k0 + 1};
     err = dg_gemm(rb * nb, sms, D.A2, D.B2, eu, D.uneven, st);
     return err != cudaSuccess ? err : cudaGetLastError();
@@ -1780,9 +1886,9 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
     if (digits) {
         hb_digits_layout(n, dg.p, D);
         // Exponents of A's columns over the rows that reflectors touch.
-        k_dg_exp_k<<<n, 256, 0, st>>>(HqCols{dA + 1, lda, n, n - 1}, n - 1, nullptr, 0, D.cex, nullptr);
+        k_dg_exp_k<<<n, 256, 0, st>>>(HqCols{dA + 1, lda, n, n - 1}, n - 1, nullptr, 0, D.cex);
         if (cudaMemsetAsync(D.low, 0, (size_t)(2 * n + 2) * sizeof(int), st) != cudaSuccess) return HSR_ERR_CUDA;
-        k_hb_even<<<dim3((n + 254) / 256, (n + kHbEvenCols - 1) / kHbEvenCols), 256, 0, st>>>(
+        k_hb_even<<<dim3((n + 254) / 256, (n + kEvenCols - 1) / kEvenCols), 256, 0, st>>>(
             n, dA, lda, D.cex, D.low, reinterpret_cast<unsigned *>(D.low + 2 * n), D.uneven);
     }
     for (int k0 = 0; k0 < n - 2; k0 += kHbNb) {
@@ -1829,7 +1935,8 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
         const int kr = n - k0 - 1, mt = (m + kHbTm - 1) / kHbTm;
         const int split = std::max(1, std::min((2 * sms + mt - 1) / mt, std::min(kHbMaxSplit, (kr + kHbTk - 1) / kHbTk)));
         const HbPlain hp{S, k0, ib, c1, split, Wp, W, W2, S.cnt + 4, digits ? D.uneven : nullptr};
-        const int nt = (n + kHbTm - 1) / kHbTm, grid = std::min(2 * sms, nt * nt);   // the same for all panels (GridBar)
+        const int nt = (n + kHbTm - 1) / kHbTm;
+        const int grid = std::min(sms, nt * std::max(nt, kHbMaxSplit));   // the same for all panels (GridBar)
         if (launch_phases(k_hb_plain, hp, kHbPlainPhases, grid, st) != cudaSuccess) return HSR_ERR_CUDA;
     }
     if (digits) dg.done(st);
@@ -1846,48 +1953,26 @@ extern "C" int hsr_hessenberg_apply_q_device(int n, const double *dA, int lda, c
     int dev = 0, sms = 0, rc = HSR_OK;
     if (cudaGetDevice(&dev) != cudaSuccess) return HSR_ERR_CUDA;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (n >= kHqDigitsN && hq_digits(n, dA, lda, dtau, ncols, dX, ldx, dev, sms, st, &rc))
-        return rc;
     const size_t nb = kHbNb;
     const size_t need = (size_t)n * nb + 2 * nb * nb + (size_t)kHbMaxSplit * nb * nb +
-                        (size_t)(kHbMaxSplit + 2) * nb * ncols;
+                        (size_t)(kHbMaxSplit + 2) * nb * ncols + 1;
     if (sc.ensure(need * sizeof(double), dev, st) != cudaSuccess) return HSR_ERR_NOMEM;
-    double *V = sc.p, *G = V + (size_t)n * nb, *T = G + nb * nb, *Gp = T + nb * nb;
-    double *Wp = Gp + (size_t)kHbMaxSplit * nb * nb, *W = Wp + (size_t)kHbMaxSplit * nb * ncols,
-           *W2 = W + nb * (size_t)ncols;
-    auto split_for = [&](int tiles, int kr) {
-        int sp = (2 * sms + tiles - 1) / tiles;
-        return std::max(1, std::min(sp, std::min(kHbMaxSplit, (kr + kHbTk - 1) / kHbTk)));
-    };
-    auto sum_parts = [&](int M, int N, int kr, int sp, const double *parts, double *out) {
-        const int kc = (((kr + sp - 1) / sp) + kHbTk - 1) / kHbTk * kHbTk;
-        const int nz = (kr + kc - 1) / kc;
-        k_hb_sumk<<<(M * N + 255) / 256, 256, 0, st>>>(M, N, nz, parts, nb, nb * (long long)N, out);
-    };
-    const int last = ((n - 3) / kHbNb) * kHbNb;
-    for (int k0 = last; k0 >= 0; k0 -= kHbNb) {
-        const int ib = std::min(kHbNb, n - 2 - k0);
-        const int kr = n - k0 - 1;
-        k_hq_vpanel<<<dim3((n + 255) / 256 < 64 ? (n + 255) / 256 : 64, ib), 256, 0, st>>>(n, dA, lda, k0, V);
-        // G = V^T V over rows k0+1 .., then T (dlarft, forward, columnwise).
-        const int sg = split_for(1, kr);
-        if (hb_gemm(ib, ib, kr, 1.0, V + (k0 + 1), n, 1, V + (k0 + 1), 1, n, 0.0, Gp, nb, sg, nb * (long long)ib,
-                    st) != cudaSuccess)
-            return HSR_ERR_CUDA;
-        sum_parts(ib, ib, kr, sg, Gp, G);
-        k_hq_tfactor<<<1, 64, 0, st>>>(ib, dtau + k0, G, T);
-        // X(k0+1:, :) -= V (T (V^T X(k0+1:, :)))
-        const int tiles = (ncols + kHbTm - 1) / kHbTm;
-        const int sp = split_for(tiles, kr);
-        if (hb_gemm(ib, ncols, kr, 1.0, V + (k0 + 1), n, 1, dX + (k0 + 1), 1, ldx, 0.0, Wp, nb, sp,
-                    nb * (long long)ncols, st) != cudaSuccess)
-            return HSR_ERR_CUDA;
-        sum_parts(ib, ncols, kr, sp, Wp, W);
-        if (hb_gemm(ib, ncols, ib, 1.0, T, 1, nb, W, 1, nb, 0.0, W2, nb, 1, 0, st) != cudaSuccess ||
-            hb_gemm(kr, ncols, ib, -1.0, V + (k0 + 1), 1, n, W2, 1, nb, 1.0, dX + (k0 + 1), ldx, 1, 0, st) !=
-                cudaSuccess)
-            return HSR_ERR_CUDA;
-    }
+    const int *uneven = nullptr;
+    if (n >= kHqDigitsN && hq_digits(n, dA, lda, dtau, ncols, dX, ldx, dev, sms, st, &uneven, &rc) && rc != HSR_OK) return rc;
+    // In FP64, where the reflectors are not even or there are no digits.
+    HqPlain P{};
+    P.n = n, P.ncols = ncols, P.A = dA, P.lda = lda, P.tau = dtau, P.X = dX, P.ldx = ldx, P.uneven = uneven;
+    P.V = sc.p, P.G = P.V + (size_t)n * nb, P.T = P.G + nb * nb, P.Gp = P.T + nb * nb;
+    P.Wp = P.Gp + (size_t)kHbMaxSplit * nb * nb, P.W = P.Wp + (size_t)kHbMaxSplit * nb * ncols;
+    P.W2 = P.W + nb * (size_t)ncols;
+    P.bar = reinterpret_cast<unsigned *>(P.W2 + nb * (size_t)ncols);
+    const int ct = (ncols + kHbTm - 1) / kHbTm, rt = (n + kHbTm - 1) / kHbTm;
+    P.splitg = std::min(2 * sms, kHbMaxSplit);
+    P.splitw = std::max(1, std::min((2 * sms + ct - 1) / ct, kHbMaxSplit));
+    if (cudaMemsetAsync(P.bar, 0, sizeof(double), st) != cudaSuccess ||
+        launch_phases(k_hq_plain, P, kHqPlainPhases * ((n - 3) / kHbNb + 1), std::min(sms, ct * std::max(rt, kHbMaxSplit)), st) !=
+            cudaSuccess)
+        return HSR_ERR_CUDA;
     sc.done(st);
     return cudaGetLastError() == cudaSuccess ? HSR_OK : HSR_ERR_CUDA;
 }

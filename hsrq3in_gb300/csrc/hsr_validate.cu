@@ -371,7 +371,7 @@ extern "C" int hsr_residuals_device(int n, const double *dH, int lddH, int ncols
                 const int cols = std::min(cch, ncols - c0), cb = (cols + kDgBN - 1) / kDgBN;
                 const double *Xc = dX + (size_t)c0 * lddX;
                 const ValX lx{Xc, lddX, n, cols};
-                k_dg_exp_k<<<cols, 256, 0, st>>>(lx, n, hcol, 1, xex, nullptr);
+                k_dg_exp_k<<<cols, 256, 0, st>>>(lx, n, hcol, 1, xex);
                 k_dg_split<ValX, false><<<dim3(cb * (kDgBN / 8), (unsigned)((2 * steps + 31) / 32)), 256, 0, st>>>(
                     lx, kDgBN, cb * kDgBN, steps, xex, hcol, 1, cols, n, xdig, nullptr);
                 k_val_cols<<<(cols + 127) / 128, 128, 0, st>>>(cols, dwr + c0, hmax, xmax + c0, xex, vcol);

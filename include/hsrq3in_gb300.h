@@ -181,7 +181,9 @@ void hsr_release_workspace(void);
 int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, void *stream);
 /* X <- Q X for the Q of hsr_hessenberg_device (LAPACK dormhr 'L','N'):
  * back-transforms eigenvectors of H to eigenvectors of A, or forms Q from
- * X = I.  dX is n x ncols, leading dimension ldx. */
+ * X = I.  dX is n x ncols, leading dimension ldx.  Products run on the tensor
+ * cores where the reflectors' entries are of like size (decided on the device),
+ * else in FP64, as in the reduction. */
 int hsr_hessenberg_apply_q_device(int n, const double *dA, int lda, const double *dtau,
                                   int ncols, double *dX, int ldx, void *stream);
 

@@ -289,6 +289,8 @@ def _reduce_one_by_one(torch, A):
     tau = torch.zeros(n, dtype=torch.float64, device="cuda")
     for k in range(n - 2):
         x = F[k + 1:, k].clone()
+        if not torch.any(x[1:]):
+            continue                             # tau = 0
         beta = -torch.copysign(torch.linalg.norm(x), x[0])
         tau[k] = (beta - x[0]) / beta
         v = x / (x[0] - beta)
@@ -354,3 +356,68 @@ def test_reduction_of_any_form(gpu_lib, n, pad, form):
     At, Q = torch.from_numpy(A).cuda(), _form_q(torch, F, tau)
     assert float((Q.T @ Q - torch.eye(n, dtype=torch.float64, device="cuda")).norm()) <= n * EPS * np.sqrt(n)
     assert float((At @ Q - Q @ torch.triu(F, -1)).norm()) <= n * EPS * np.linalg.norm(A)
+
+
+@pytest.mark.parametrize("n,ncols,pad,decades", [(45, 3, 0, 8), (130, 65, 1, 10), (200, 5, 0, 25), (300, 30, 0, 12)])
+def test_back_transform_keeps_graded_rows(gpu_lib, n, ncols, pad, decades):
+    """Reflectors of a graded matrix on columns graded alike: FP64 keeps the
+    small rows.  Row by row, relative to the row's largest entry, within ten
+    times of the reflectors one by one in FP64, whose sums run in another
+    order; both against extended precision."""
+    import torch
+    import hsrq3in_gb300 as hsr
+    rng = np.random.default_rng(n)
+    d = 10.0 ** (-decades * np.arange(n) / (n - 1))
+    F, tau = _reduce_one_by_one(torch, torch.from_numpy(rng.standard_normal((n, n)) * d[:, None] * d).cuda())
+    A, tau = F.cpu().numpy(), tau.cpu().numpy()
+    X = rng.standard_normal((n, ncols)) * d[:, None]
+    dX = _cols(torch, X, pad)
+    hsr.hessenberg_apply_q_device(_cols(torch, A, pad), torch.from_numpy(tau).cuda(), dX)
+    got = dX.cpu().numpy()
+    assert np.all(got[:, n:] == 5.0)
+    R, S = X.astype(np.longdouble), X.copy()
+    for k in range(n - 3, -1, -1):
+        v = A[k + 1:, k].copy()
+        v[0] = 1.0
+        S[k + 1:] -= np.outer(v, tau[k] * (v[:, None] * S[k + 1:]).sum(0))
+        v = v.astype(np.longdouble)
+        R[k + 1:] -= np.outer(v, tau[k] * (v[:, None] * R[k + 1:]).sum(0))
+    scale = np.abs(R).max(1)[:, None]
+    err = [float((np.abs(Z - R) / scale).max()) for Z in (got[:, :n].T, S)]
+    assert err[0] <= 10 * err[1], err
+
+
+@pytest.mark.parametrize("n,ncols", [(40, 1), (65, 64), (130, 65), (321, 7)])
+@pytest.mark.parametrize("form", ["identity", "hessenberg", "band", "sparse", "first", "late"])
+def test_back_transform_of_any_form(gpu_lib, n, ncols, form):
+    """Reflectors that the digit products take and that they leave to FP64, and
+    columns of one large entry: within n eps of extended precision, column by
+    column, as in test_back_transform_against_extended."""
+    import torch
+    import hsrq3in_gb300 as hsr
+    rng = np.random.default_rng(n)
+    M = rng.standard_normal((n, n))
+    X = rng.standard_normal((n, ncols))
+    if form == "identity":
+        M[np.tril_indices(n, -2)] = 0.0
+    elif form == "hessenberg":
+        M[np.tril_indices(n, -2)] *= 1e-14
+    elif form == "band":
+        M = np.tril(M, 3)
+    elif form == "sparse":
+        M *= rng.random((n, n)) < 0.2
+    elif form == "first":
+        X[2:] *= 1e-25
+    else:
+        X[: n // 2] = 0.0
+    F, tau = _reduce_one_by_one(torch, torch.from_numpy(M).cuda())
+    A, tau = F.cpu().numpy(), tau.cpu().numpy()
+    dX = _cols(torch, X, 0)
+    hsr.hessenberg_apply_q_device(_cols(torch, A, 0), torch.from_numpy(tau).cuda(), dX)
+    R = X.astype(np.longdouble)
+    for k in range(n - 3, -1, -1):
+        v = A[k + 1:, k].astype(np.longdouble)
+        v[0] = 1.0
+        R[k + 1:] -= np.outer(v, tau[k] * (v[:, None] * R[k + 1:]).sum(0))
+    err = np.sqrt(((dX.cpu().numpy().T - R) ** 2).sum(0)) / np.sqrt((R * R).sum(0))
+    assert err.max() <= n * EPS, err.max()
