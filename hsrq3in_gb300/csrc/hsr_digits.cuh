@@ -687,57 +687,6 @@ struct DgUpdate {
     }
 };
 
-// Host side: one growing device buffer per thread.  A call on another stream
-// than the last one first waits for that one's work.
-struct DgScratch {
-    int device = -1;
-    unsigned char *p = nullptr;
-    size_t bytes = 0;
-    cudaEvent_t ev = nullptr;
-    cudaStream_t last = nullptr;
-    bool used = false;
-    ~DgScratch() {
-        if (p) cudaFree(p);
-        if (ev) cudaEventDestroy(ev);
-    }
-    // False when the buffer cannot be had (too little memory, or it would have
-    // to grow inside a stream capture): the caller has a path without it.
-    bool ensure(size_t b, int dev, cudaStream_t st) {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        if (device != dev || b > bytes) {
-            if (cs != cudaStreamCaptureStatusNone) return false;
-            if (p) cudaFree(p);
-            if (ev) cudaEventDestroy(ev);
-            p = nullptr;
-            ev = nullptr;
-            bytes = 0;
-            used = false;
-            device = dev;
-            if (cudaMalloc(&p, b) != cudaSuccess || cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
-                cudaGetLastError();
-                if (p) cudaFree(p);
-                p = nullptr;
-                return false;
-            }
-            bytes = b;
-        }
-        if (cs == cudaStreamCaptureStatusNone && used && last != st && cudaStreamWaitEvent(st, ev, 0) != cudaSuccess)
-            return false;
-        capturing = cs != cudaStreamCaptureStatusNone;
-        return true;
-    }
-    void done(cudaStream_t st) {
-        if (capturing) return;
-        cudaEventRecord(ev, st);
-        last = st;
-        used = true;
-    }
-    bool capturing = false;
-};
 // Parts of a sum over `steps` stages for `tiles` tiles (per: stages of a
 // part): as many as give the fewest stages on the busiest SM, five stages'
 // time counted for the end of each part.

@@ -41,6 +41,7 @@
 #include "../../include/hsrq3in_gb300.h"
 #include "hsr_device.cuh"
 #include "hsr_digits.cuh"
+#include "hsr_scratch.h"
 
 #include <algorithm>
 #include <cfloat>
@@ -1496,40 +1497,58 @@ __global__ void __launch_bounds__(8 * kHqHalf) k_hq_tcross(HqGroup h, const doub
     To[kHqHalf + p + (size_t)col * kHqNb] = 0.0;                 // T21
 }
 
-// Enqueues the digit form, which does nothing where *uneven (set here) is not 0.
-// False when the scratch cannot be had: nothing has been enqueued then.
-bool hq_digits(int n, const double *dA, int lda, const double *dtau, int ncols, double *dX, int ldx, int dev, int sms,
-               cudaStream_t st, const int **uneven, int *rc) {
-    static thread_local DgScratch dg;
-    constexpr int ksteps = kHqNb / kDgBK;
-    constexpr size_t vblock = (size_t)kHqNb * kHqNb * kDgDigits * 2, small = (size_t)kHqNb * kDgDigits * 2;
-    const int nblk = (n - 3) / kHqNb + 1;                        // blocks of reflectors
+// Scratch of the digit form, laid out once.
+struct HqDigits {
+    unsigned char *XN, *VM, *VN, *VA, *TM, *WN;
+    double *S, *T, *Wp, *W2;
+    int *exX, *exW, *exVA, *exV, *exT, *low;                     // low: k_hq_even's counts, a counter and the result
+    int nblk, cch, gmax;                                         // blocks of reflectors, columns at a time, blocks of a group
+};
+constexpr size_t kHqVBlock = (size_t)kHqNb * kHqNb * kDgDigits * 2, kHqSmall = (size_t)kHqNb * kDgDigits * 2;
+size_t hq_digits_layout(int n, int ncols, unsigned char *base, HqDigits &D) {
+    D.nblk = (n - 3) / kHqNb + 1;
     const int rbmax = (n - 1 + kHqNb - 1) / kHqNb;               // row blocks of the first one
     const size_t per_row = (size_t)rbmax * kHqNb * kDgDigits * 2;
     const size_t fit = std::max<size_t>(1, kHqXBytes / (per_row * kDgBN)) * kDgBN;
-    const int cch = (int)std::min<size_t>(fit, (size_t)((ncols + kDgBN - 1) / kDgBN) * kDgBN);
-    const int gmax = (int)std::max<size_t>(1, std::min<size_t>(nblk, kHqVBytes / (3 * vblock * rbmax)));
-    const size_t vrb = (size_t)gmax * rbmax;                     // row blocks of a group, at most
+    D.cch = (int)std::min<size_t>(fit, (size_t)((ncols + kDgBN - 1) / kDgBN) * kDgBN);
+    D.gmax = (int)std::max<size_t>(1, std::min<size_t>(D.nblk, kHqVBytes / (3 * kHqVBlock * rbmax)));
+    const size_t vrb = (size_t)D.gmax * rbmax;                   // row blocks of a group, at most
     size_t off = 0;
     const auto take = [&](size_t bytes) {
         const size_t o = off;
         off += (bytes + 255) / 256 * 256;
-        return o;
+        return base + o;
     };
-    const size_t oXN = take((size_t)cch * per_row), oVM = take(vrb * vblock), oVN = take(vrb * vblock),
-                 oVA = take(vrb * vblock), oTM = take((size_t)gmax * kHqNb * small), oWN = take((size_t)cch * small),
-                 oS = take((size_t)gmax * kHqMaxSplit * kHqNb * kHqNb * 8), oT = take((size_t)gmax * kHqNb * kHqNb * 8),
-                 oWp = take((size_t)kHqMaxSplit * kHqNb * cch * 8), oW2 = take((size_t)kHqNb * cch * 8),
-                 oEx = take(((size_t)ncols + cch + vrb * kHqNb + (size_t)2 * gmax * kHqNb + 2 * n + 2) * sizeof(int));
-    if (!dg.ensure(off, dev, st)) return false;
-    unsigned char *const b = dg.p, *XN = b + oXN, *VM = b + oVM, *VN = b + oVN, *VA = b + oVA, *TM = b + oTM, *WN = b + oWN;
-    double *S = reinterpret_cast<double *>(b + oS), *T = reinterpret_cast<double *>(b + oT),
-           *Wp = reinterpret_cast<double *>(b + oWp), *W2 = reinterpret_cast<double *>(b + oW2);
-    int *exX = reinterpret_cast<int *>(b + oEx), *exW = exX + ncols, *exVA = exW + cch, *exV = exVA + vrb * kHqNb,
-        *exT = exV + gmax * kHqNb, *low = exT + gmax * kHqNb, *gate = low + 2 * n + 1;
+    D.XN = take((size_t)D.cch * per_row);
+    D.VM = take(vrb * kHqVBlock);
+    D.VN = take(vrb * kHqVBlock);
+    D.VA = take(vrb * kHqVBlock);
+    D.TM = take((size_t)D.gmax * kHqNb * kHqSmall);
+    D.WN = take((size_t)D.cch * kHqSmall);
+    D.S = reinterpret_cast<double *>(take((size_t)D.gmax * kHqMaxSplit * kHqNb * kHqNb * 8));
+    D.T = reinterpret_cast<double *>(take((size_t)D.gmax * kHqNb * kHqNb * 8));
+    D.Wp = reinterpret_cast<double *>(take((size_t)kHqMaxSplit * kHqNb * D.cch * 8));
+    D.W2 = reinterpret_cast<double *>(take((size_t)kHqNb * D.cch * 8));
+    D.exX = reinterpret_cast<int *>(take(((size_t)ncols + D.cch + vrb * kHqNb + (size_t)2 * D.gmax * kHqNb + 2 * n + 2) * sizeof(int)));
+    D.exW = D.exX + ncols;
+    D.exVA = D.exW + D.cch;
+    D.exV = D.exVA + vrb * kHqNb;
+    D.exT = D.exV + D.gmax * kHqNb;
+    D.low = D.exT + D.gmax * kHqNb;
+    return off;
+}
+// Enqueues the digit form, which does nothing where *uneven (set here) is not 0.
+cudaError_t hq_digits(const HqDigits &D, int n, const double *dA, int lda, const double *dtau, int ncols, double *dX, int ldx,
+                      int sms, cudaStream_t st, const int **uneven) {
+    constexpr int ksteps = kHqNb / kDgBK;
+    constexpr size_t vblock = kHqVBlock, small = kHqSmall;
+    const int nblk = D.nblk, cch = D.cch, gmax = D.gmax;
+    unsigned char *const XN = D.XN, *VM = D.VM, *VN = D.VN, *VA = D.VA, *TM = D.TM, *WN = D.WN;
+    double *S = D.S, *T = D.T, *Wp = D.Wp, *W2 = D.W2;
+    int *exX = D.exX, *exW = D.exW, *exVA = D.exVA, *exV = D.exV, *exT = D.exT, *low = D.low, *gate = low + 2 * n + 1;
+    cudaError_t e = cudaMemsetAsync(low, 0, (size_t)(2 * n + 2) * sizeof(int), st);
+    if (e != cudaSuccess) return e;
     *uneven = gate;
-    *rc = HSR_ERR_CUDA;
-    if (cudaMemsetAsync(low, 0, (size_t)(2 * n + 2) * sizeof(int), st) != cudaSuccess) return true;
     k_hq_even<<<dim3((n + 255) / 256, (n - 2 + kEvenCols - 1) / kEvenCols), 256, 0, st>>>(
         n, dA, lda, dtau, low, reinterpret_cast<unsigned *>(low + 2 * n), gate);
     // Over the rows that reflectors touch: row 0 stays what it is.
@@ -1543,7 +1562,7 @@ bool hq_digits(int n, const double *dA, int lda, const double *dtau, int ncols, 
         k_hq_vcols<kDgBM><<<gv, 256, 0, st>>>(h, exV, VM);
         k_hq_vcols<kDgBN><<<gv, 256, 0, st>>>(h, exV, VN);
         k_hq_vrows<<<dim3(rmax * (kHqNb / 32), ng), 512, 0, st>>>(h, exVA, VA);
-        if (dg_gemm(2 * gz * ng, sms, VM, VN, HqGram{h, gz, exV, S}, gate, st) != cudaSuccess) return true;
+        if ((e = dg_gemm(2 * gz * ng, sms, VM, VN, HqGram{h, gz, exV, S}, gate, st)) != cudaSuccess) return e;
         k_hq_thalf<<<dim3(ng, 2), 4 * kHqHalf, 0, st>>>(h, dtau, S, gz, T);
         k_hq_tcross<<<dim3(ng, kHqHalf / 8), 8 * kHqHalf, 0, st>>>(h, S, gz, T);
         k_dg_small<HqT, true><<<ng * (kHqNb / 32), 512, 0, st>>>(HqT{T}, kDgBM, ng * kHqNb, ng * kHqNb, kHqNb, nullptr, 0,
@@ -1560,21 +1579,19 @@ bool hq_digits(int n, const double *dA, int lda, const double *dtau, int ncols, 
                 const int nz = dg_parts(cb, sms, kHqMaxSplit, steps, per);
                 const DgStoreLong e1{1, cb, steps, per, kHqNb, cols, exV + g * kHqNb, exX + c0, Wp, 1, kHqNb,
                                      (long long)kHqNb * cols};
-                if (dg_gemm(cb * nz, sms, VM + (size_t)at * vblock, XN, e1, gate, st) != cudaSuccess) return true;
+                if ((e = dg_gemm(cb * nz, sms, VM + (size_t)at * vblock, XN, e1, gate, st)) != cudaSuccess) return e;
                 k_dg_small<HqSum, false><<<cb * (kDgBN / 8), 128, 0, st>>>(HqSum{Wp, nz, (long long)kHqNb * cols}, kDgBN,
                                                                          cols, cb * kDgBN, kHqNb, nullptr, 0, exW, WN);
                 const DgStoreShort e2{1, cb, ksteps, ksteps, kHqNb, cols, exT + g * kHqNb, exW, W2, 1, kHqNb, 0};
-                if (dg_gemm(cb, sms, TM + (size_t)g * kHqNb * small, WN, e2, gate, st) != cudaSuccess) return true;
+                if ((e = dg_gemm(cb, sms, TM + (size_t)g * kHqNb * small, WN, e2, gate, st)) != cudaSuccess) return e;
                 k_dg_small<HqSum, false><<<cb * (kDgBN / 8), 128, 0, st>>>(HqSum{W2, 1, 0}, kDgBN, cols, cb * kDgBN, kHqNb,
                                                                          nullptr, 0, exW, WN);
                 const DgUpdate e3{rb, ksteps, kr, cols, exVA + at * kHqNb, exW, X, ldx, exX + c0, 0};
-                if (dg_gemm(rb * cb, sms, VA + (size_t)at * vblock, WN, e3, gate, st) != cudaSuccess) return true;
+                if ((e = dg_gemm(rb * cb, sms, VA + (size_t)at * vblock, WN, e3, gate, st)) != cudaSuccess) return e;
             }
         }
     }
-    dg.done(st);
-    *rc = cudaGetLastError() == cudaSuccess ? HSR_OK : HSR_ERR_CUDA;
-    return true;
+    return cudaGetLastError();
 }
 
 // ------------------------------------------------ trailing update by digits
@@ -1769,50 +1786,6 @@ cudaError_t hb_trailing(const HbState &S, const HbDigits &D, int k0, int c1, int
     return err != cudaSuccess ? err : cudaGetLastError();
 }
 
-// A thread's scratch for sums and counters.  Its users on different streams are
-// ordered by an event (not inside a stream capture, whose replays the caller orders).
-struct HhScratch {
-    int device = -1;
-    double *p = nullptr;
-    size_t bytes = 0;
-    cudaEvent_t ev = nullptr;
-    cudaStream_t last = nullptr;
-    bool used = false;
-    ~HhScratch() { release(); }
-    void release() {
-        if (p) cudaFree(p);
-        if (ev) cudaEventDestroy(ev);
-        p = nullptr;
-        ev = nullptr;
-        bytes = 0;
-        used = false;
-    }
-    static bool capturing(cudaStream_t st) {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
-            cudaGetLastError();
-            return true;
-        }
-        return cs != cudaStreamCaptureStatusNone;
-    }
-    cudaError_t ensure(size_t b, int dev, cudaStream_t st) {
-        if (device != dev || b > bytes) {
-            release();
-            const cudaError_t e = cudaMalloc(&p, b);
-            if (e != cudaSuccess) return e;
-            bytes = b;
-            device = dev;
-        }
-        return used && last != st && !capturing(st) ? cudaStreamWaitEvent(st, ev, 0) : cudaSuccess;
-    }
-    void done(cudaStream_t st) {
-        if (capturing(st) || (!ev && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess)) return;
-        cudaEventRecord(ev, st);
-        last = st;
-        used = true;
-    }
-};
-
 }  // namespace
 }  // namespace hsr
 
@@ -1823,7 +1796,7 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (cudaMemsetAsync(dtau, 0, (size_t)n * sizeof(double), st) != cudaSuccess) return HSR_ERR_CUDA;
     if (n <= 2) return HSR_OK;
-    static thread_local HhScratch sc;
+    static thread_local Scratch sc;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return HSR_ERR_CUDA;
     const int nblk = (n + kHbRows - 1) / kHbRows;
@@ -1859,12 +1832,17 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
                         + nb + 8                      // sc
                         + (size_t)(kHbMaxSplit + 2) * nb * n   // W partials, W, W2
                         + 4;                          // counters
-    if (sc.ensure(need * sizeof(double), dev, st) != cudaSuccess) return HSR_ERR_NOMEM;
+    // The digits' part behind it, where there is memory for it.
+    const size_t plain = (need * sizeof(double) + 255) / 256 * 256;
+    HbDigits D{};
+    const ScratchUse use(sc, n >= kHbDigitsN ? plain + hb_digits_layout(n, nullptr, D) : plain, plain, dev, st);
+    if (!use) return HSR_ERR_NOMEM;
+    const bool digits = use.bytes() > plain;
     HbState S{};
     S.A = dA;
     S.lda = lda;
     S.n = n;
-    double *p = sc.p;
+    double *p = reinterpret_cast<double *>(use.get());
     S.Y = p; p += (size_t)n * nb;
     S.V = p; p += (size_t)n * nb;
     S.T = p; p += nb * nb;
@@ -1880,11 +1858,8 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
     S.cnt = reinterpret_cast<unsigned int *>(p);
     S.tau = dtau;
     if (cudaMemsetAsync(S.cnt, 0, 4 * sizeof(double), st) != cudaSuccess) return HSR_ERR_CUDA;
-    static thread_local DgScratch dg;
-    HbDigits D{};
-    const bool digits = n >= kHbDigitsN && dg.ensure(hb_digits_layout(n, nullptr, D), dev, st);
     if (digits) {
-        hb_digits_layout(n, dg.p, D);
+        hb_digits_layout(n, use.get() + plain, D);
         // Exponents of A's columns over the rows that reflectors touch.
         k_dg_exp_k<<<n, 256, 0, st>>>(HqCols{dA + 1, lda, n, n - 1}, n - 1, nullptr, 0, D.cex);
         if (cudaMemsetAsync(D.low, 0, (size_t)(2 * n + 2) * sizeof(int), st) != cudaSuccess) return HSR_ERR_CUDA;
@@ -1939,8 +1914,6 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
         const int grid = std::min(sms, nt * std::max(nt, kHbMaxSplit));   // the same for all panels (GridBar)
         if (launch_phases(k_hb_plain, hp, kHbPlainPhases, grid, st) != cudaSuccess) return HSR_ERR_CUDA;
     }
-    if (digits) dg.done(st);
-    sc.done(st);
     return cudaGetLastError() == cudaSuccess ? HSR_OK : HSR_ERR_CUDA;
 }
 
@@ -1949,20 +1922,26 @@ extern "C" int hsr_hessenberg_apply_q_device(int n, const double *dA, int lda, c
     if (n <= 0 || lda < n || ncols < 0 || ldx < n || !dA || !dtau || (ncols > 0 && !dX)) return HSR_ERR_ARG;
     if (ncols == 0 || n <= 2) return HSR_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    static thread_local HhScratch sc;
-    int dev = 0, sms = 0, rc = HSR_OK;
+    static thread_local Scratch sc;
+    int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return HSR_ERR_CUDA;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const size_t nb = kHbNb;
     const size_t need = (size_t)n * nb + 2 * nb * nb + (size_t)kHbMaxSplit * nb * nb +
                         (size_t)(kHbMaxSplit + 2) * nb * ncols + 1;
-    if (sc.ensure(need * sizeof(double), dev, st) != cudaSuccess) return HSR_ERR_NOMEM;
+    const size_t plain = (need * sizeof(double) + 255) / 256 * 256;
+    HqDigits D{};
+    const ScratchUse use(sc, n >= kHqDigitsN ? plain + hq_digits_layout(n, ncols, nullptr, D) : plain, plain, dev, st);
+    if (!use) return HSR_ERR_NOMEM;
     const int *uneven = nullptr;
-    if (n >= kHqDigitsN && hq_digits(n, dA, lda, dtau, ncols, dX, ldx, dev, sms, st, &uneven, &rc) && rc != HSR_OK) return rc;
+    if (use.bytes() > plain) {
+        hq_digits_layout(n, ncols, use.get() + plain, D);
+        if (hq_digits(D, n, dA, lda, dtau, ncols, dX, ldx, sms, st, &uneven) != cudaSuccess) return HSR_ERR_CUDA;
+    }
     // In FP64, where the reflectors are not even or there are no digits.
     HqPlain P{};
     P.n = n, P.ncols = ncols, P.A = dA, P.lda = lda, P.tau = dtau, P.X = dX, P.ldx = ldx, P.uneven = uneven;
-    P.V = sc.p, P.G = P.V + (size_t)n * nb, P.T = P.G + nb * nb, P.Gp = P.T + nb * nb;
+    P.V = reinterpret_cast<double *>(use.get()), P.G = P.V + (size_t)n * nb, P.T = P.G + nb * nb, P.Gp = P.T + nb * nb;
     P.Wp = P.Gp + (size_t)kHbMaxSplit * nb * nb, P.W = P.Wp + (size_t)kHbMaxSplit * nb * ncols;
     P.W2 = P.W + nb * (size_t)ncols;
     P.bar = reinterpret_cast<unsigned *>(P.W2 + nb * (size_t)ncols);
@@ -1973,6 +1952,5 @@ extern "C" int hsr_hessenberg_apply_q_device(int n, const double *dA, int lda, c
         launch_phases(k_hq_plain, P, kHqPlainPhases * ((n - 3) / kHbNb + 1), std::min(sms, ct * std::max(rt, kHbMaxSplit)), st) !=
             cudaSuccess)
         return HSR_ERR_CUDA;
-    sc.done(st);
     return cudaGetLastError() == cudaSuccess ? HSR_OK : HSR_ERR_CUDA;
 }

@@ -30,6 +30,7 @@
 #include "../../include/hsrq3in_gb300.h"
 #include "hsr_device.cuh"
 #include "hsr_digits.cuh"
+#include "hsr_scratch.h"
 
 #include <algorithm>
 #include <cmath>
@@ -299,15 +300,6 @@ struct ValEpi {
     }
 };
 
-struct ValScratch {
-    int device = -1;
-    void *p = nullptr;
-    size_t bytes = 0;
-    ~ValScratch() {
-        if (p) cudaFree(p);
-    }
-};
-
 }  // namespace
 }  // namespace hsr
 
@@ -319,29 +311,12 @@ extern "C" int hsr_residuals_device(int n, const double *dH, int lddH, int ncols
         return HSR_ERR_ARG;
     if (ncols == 0) return HSR_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    static thread_local ValScratch sc;
+    static thread_local Scratch sc;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return HSR_ERR_CUDA;
-    const size_t need = (size_t)(2 + 3 * (size_t)ncols) * 8;
-    if (sc.device != dev || sc.bytes < need) {
-        if (sc.p) cudaFree(sc.p);
-        sc.p = nullptr;
-        sc.bytes = 0;
-        if (cudaMalloc(&sc.p, need) != cudaSuccess) return HSR_ERR_NOMEM;
-        sc.bytes = need;
-        sc.device = dev;
-    }
-    unsigned long long *hmax = static_cast<unsigned long long *>(sc.p);
-    double *hsum = reinterpret_cast<double *>(hmax + 1);
-    unsigned long long *xmax = hmax + 2;
-    double *xsum = reinterpret_cast<double *>(xmax + ncols);
-    double *rsum = xsum + ncols;
-    if (cudaMemsetAsync(hmax, 0, 16, st) != cudaSuccess ||
-        cudaMemsetAsync(rsum, 0, (size_t)ncols * 8, st) != cudaSuccess)
-        return HSR_ERR_CUDA;
     // Digits: rows of H and columns of x in chunks of at most kValHBytes and
-    // kValXBytes, exponents (hcol, hex, xex) beside them.
-    static thread_local DgScratch dg;
+    // kValXBytes, exponents (hcol, hex, xex) beside them; behind the sums, where
+    // there is memory for it.
     const long long steps = (n + kDgBK - 1) / kDgBK;
     const size_t per_row = (size_t)steps * kDgBK * kDgDigits * 2;
     const auto chunk = [&](size_t cap, int count, int block) {
@@ -350,9 +325,20 @@ extern "C" int hsr_residuals_device(int n, const double *dH, int lddH, int ncols
     };
     const int rch = chunk(kValHBytes, n, kDgBM), cch = chunk(kValXBytes, ncols, kDgBN);
     const size_t hbytes = (size_t)rch * per_row, xbytes = (size_t)cch * per_row;
-    const bool digits = n >= kValDigitsN &&
-                        dg.ensure(hbytes + xbytes + (size_t)cch * sizeof(ValCol) + (size_t)(n + rch + cch) * sizeof(int), dev, st);
-    unsigned char *hdig = dg.p, *xdig = hdig + hbytes;
+    const size_t sums = ((size_t)(2 + 3 * (size_t)ncols) * 8 + 255) / 256 * 256;
+    const size_t dbytes = hbytes + xbytes + (size_t)cch * sizeof(ValCol) + (size_t)(n + rch + cch) * sizeof(int);
+    const ScratchUse use(sc, n < kValDigitsN ? sums : sums + dbytes, sums, dev, st);
+    if (!use) return HSR_ERR_NOMEM;
+    const bool digits = use.bytes() > sums;
+    unsigned long long *hmax = reinterpret_cast<unsigned long long *>(use.get());
+    double *hsum = reinterpret_cast<double *>(hmax + 1);
+    unsigned long long *xmax = hmax + 2;
+    double *xsum = reinterpret_cast<double *>(xmax + ncols);
+    double *rsum = xsum + ncols;
+    if (cudaMemsetAsync(hmax, 0, 16, st) != cudaSuccess ||
+        cudaMemsetAsync(rsum, 0, (size_t)ncols * 8, st) != cudaSuccess)
+        return HSR_ERR_CUDA;
+    unsigned char *hdig = use.get() + sums, *xdig = hdig + hbytes;
     ValCol *vcol = reinterpret_cast<ValCol *>(xdig + xbytes);
     int *hcol = digits ? reinterpret_cast<int *>(vcol + cch) : nullptr, *hex = hcol + n, *xex = hex + rch;
     int sms = 1;
@@ -379,7 +365,6 @@ extern "C" int hsr_residuals_device(int n, const double *dH, int lddH, int ncols
                 if (dg_gemm(rb * cb, sms, hdig, xdig, epi, nullptr, st) != cudaSuccess) return HSR_ERR_CUDA;
             }
         }
-        dg.done(st);
         k_val_final<<<(ncols + 127) / 128, 128, 0, st>>>(ncols, hmax, xmax, hsum, xsum, rsum, d_res);
         return cudaGetLastError() == cudaSuccess ? HSR_OK : HSR_ERR_CUDA;
     }
