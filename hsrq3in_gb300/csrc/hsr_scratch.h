@@ -9,8 +9,10 @@ namespace hsr {
 // One growing device buffer of a host thread for one entry point.  A call holds
 // it by a ScratchUse from before its first launch until after its last one.
 //
-// Outside a stream capture the calls on different streams are ordered by an
-// event.  Inside one, a call gets memory that belongs to the graph (an
+// Outside a stream capture every call waits for the last one by an event, also
+// on what looks like the same stream: a new stream can have the handle of one
+// that was destroyed with its work still running (on the same stream the wait
+// costs nothing on the device).  Inside one, a call gets memory that belongs to the graph (an
 // allocation and a free node): the thread's buffer, which a later call may
 // replace and the thread's end frees, never enters a graph, and replays need no
 // order against direct calls.
@@ -19,7 +21,6 @@ struct Scratch {
     void *p = nullptr;
     size_t bytes = 0;
     cudaEvent_t ev = nullptr;
-    cudaStream_t last = nullptr;
     bool used = false;
     ~Scratch() { release(); }
     void release() {
@@ -51,14 +52,13 @@ class ScratchUse {
             p_ = nullptr;
             if (want == least) break;
         }
-        if (p_ && !captured_ && s.used && s.last != st && cudaStreamWaitEvent(st, s.ev, 0) != cudaSuccess) p_ = nullptr;
+        if (p_ && !captured_ && s.used && cudaStreamWaitEvent(st, s.ev, 0) != cudaSuccess) p_ = nullptr;
     }
     ~ScratchUse() {
         if (!p_) return;
         if (captured_) {
             cudaFreeAsync(p_, st_);
         } else if (cudaEventRecord(s_.ev, st_) == cudaSuccess) {
-            s_.last = st_;
             s_.used = true;
         }
     }

@@ -97,3 +97,33 @@ def test_replay_beside_direct_calls(gpu_lib):
     torch.cuda.synchronize()
     _same(torch, out, ref)
     _same(torch, direct, qref)
+
+
+def test_streams_that_come_and_go(gpu_lib):
+    """One thread, each call on a stream of its own that is destroyed behind
+    it with the work still enqueued, residuals included: a new stream may get a
+    destroyed one's handle."""
+    import ctypes
+    import torch
+    import hsrq3in_gb300 as hsr
+    rt = ctypes.CDLL("libcudart.so." + torch.version.cuda.split(".")[0])
+    probs = [_problem(torch, n, 90, False, n) for n in (600, 300, 500, 200, 60)]
+    ref = [_all(hsr, torch, *p) for p in probs]
+    torch.cuda.synchronize()
+
+    class Stream:
+        cuda_stream = None
+    for _ in range(3):
+        outs, copies = [], [(A0.clone(), X0.clone()) for A0, X0, _ in probs]
+        torch.cuda.synchronize()
+        for (A0, X0, wr), (A, X) in zip(probs, copies):
+            s, h = Stream(), ctypes.c_void_p()
+            assert rt.cudaStreamCreateWithFlags(ctypes.byref(h), 1) == 0
+            s.cuda_stream = h.value
+            tau = hsr.hessenberg_device(A, stream=s)
+            hsr.hessenberg_apply_q_device(A, tau, X, stream=s)
+            outs.append((A, tau, X, hsr.residuals_device(A0, wr, X0, stream=s)))
+            assert rt.cudaStreamDestroy(h) == 0
+        torch.cuda.synchronize()
+        for got, r in zip(outs, ref):
+            _same(torch, got, r)
