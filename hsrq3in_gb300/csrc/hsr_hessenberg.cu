@@ -1263,7 +1263,7 @@ constexpr int kHqNb = 128;
 // reflectors that are not even and for a scratch buffer that cannot be had.
 constexpr int kHqDigitsN = 40;
 // Most scratch for digits of X's columns and of V (three layouts) at a time.
-constexpr size_t kHqXBytes = (size_t)1 << 30, kHqVBytes = (size_t)4 << 30;
+constexpr size_t kHqXBytes = (size_t)1 << 30, kHqVBytes = (size_t)4 << 30;   // (V of n = 10,000: 2.5 GB)
 constexpr int kHqMaxSplit = 16;
 
 // Whether the reflectors allow digits.  A column of X is held by a window below
@@ -1511,8 +1511,11 @@ size_t hq_digits_layout(int n, int ncols, unsigned char *base, HqDigits &D) {
     const size_t per_row = (size_t)rbmax * kHqNb * kDgDigits * 2;
     const size_t fit = std::max<size_t>(1, kHqXBytes / (per_row * kDgBN)) * kDgBN;
     D.cch = (int)std::min<size_t>(fit, (size_t)((ncols + kDgBN - 1) / kDgBN) * kDgBN);
-    D.gmax = (int)std::max<size_t>(1, std::min<size_t>(D.nblk, kHqVBytes / (3 * kHqVBlock * rbmax)));
-    const size_t vrb = (size_t)D.gmax * rbmax;                   // row blocks of a group, at most
+    // Row blocks of a group, at most: the g first blocks have rbmax, rbmax - 1, ... of them.
+    const auto rows_of = [&](size_t g) { return g * rbmax - g * (g - 1) / 2; };
+    D.gmax = 1;
+    while (D.gmax < D.nblk && 3 * kHqVBlock * rows_of(D.gmax + 1) <= kHqVBytes) ++D.gmax;
+    const size_t vrb = rows_of(D.gmax);
     size_t off = 0;
     const auto take = [&](size_t bytes) {
         const size_t o = off;
@@ -1602,7 +1605,7 @@ cudaError_t hq_digits(const HqDigits &D, int n, const double *dA, int lda, const
 // so the trailing columns are read once for W0 and read and written once for
 // A -= [Y V] [V(c1:, :)^T; Z], where the two sides one after the other pass
 // over them five times.  V^T Y comes with W0 (Y's columns follow A's).
-constexpr size_t kHbDigitBytes = (size_t)2 << 30;   // most scratch for digits of A's columns at a time
+constexpr size_t kHbDigitBytes = (size_t)2 << 30;   // most scratch for digits of A's columns at a time (or 8 n^2 bytes, below)
 constexpr int kHbParts = 16;
 // Smallest order: the DFMA form's thin products take about 65 us each on the
 // few SMs they fill (n = 10, no trailing product worth the name: 331 us
@@ -1716,7 +1719,7 @@ struct HbDigits {
     int *cex, *exM1, *exB, *exA2, *dk1;                          // cex: n columns of A, then [Y V]
     int cch;
 };
-size_t hb_digits_layout(int n, unsigned char *base, HbDigits &D) {
+size_t hb_digits_layout(int n, bool fix, unsigned char *base, HbDigits &D) {
     const size_t rows16 = (size_t)((n + kDgBK - 1) / kDgBK) * kDgBK * kDgDigits * 2;   // bytes of one column's digits
     const size_t all = (size_t)(n + kHbNb + kDgBM - 1) / kDgBM * kDgBM;
     const size_t fit = std::max<size_t>(1, kHbDigitBytes / (rows16 * kDgBM)) * kDgBM;
@@ -1728,8 +1731,9 @@ size_t hb_digits_layout(int n, unsigned char *base, HbDigits &D) {
         off += (bytes + 255) / 256 * 256;
         return base + o;
     };
-    // The same place serves A's columns in fixed point while a panel runs.
-    D.AD = take(std::max((size_t)D.cch * rows16, n >= kHbFixN ? (size_t)n * n * sizeof(int2) : 0));
+    // The same place serves A's columns in fixed point while a panel runs (fix:
+    // 8 n^2 bytes, 5 GB at the largest order whose panel is one launch).
+    D.AD = take(std::max((size_t)D.cch * rows16, fix ? (size_t)n * n * sizeof(int2) : 0));
     D.VN = take((size_t)kDgBN * rows16);
     D.M1 = take((size_t)kDgBM * small);
     D.B1 = take(all * small);
@@ -1835,7 +1839,8 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
     // The digits' part behind it, where there is memory for it.
     const size_t plain = (need * sizeof(double) + 255) / 256 * 256;
     HbDigits D{};
-    const ScratchUse use(sc, n >= kHbDigitsN ? plain + hb_digits_layout(n, nullptr, D) : plain, plain, dev, st);
+    const bool fixes = one && n >= kHbFixN;
+    const ScratchUse use(sc, n >= kHbDigitsN ? plain + hb_digits_layout(n, fixes, nullptr, D) : plain, plain, dev, st);
     if (!use) return HSR_ERR_NOMEM;
     const bool digits = use.bytes() > plain;
     HbState S{};
@@ -1859,7 +1864,7 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
     S.tau = dtau;
     if (cudaMemsetAsync(S.cnt, 0, 4 * sizeof(double), st) != cudaSuccess) return HSR_ERR_CUDA;
     if (digits) {
-        hb_digits_layout(n, use.get() + plain, D);
+        hb_digits_layout(n, fixes, use.get() + plain, D);
         // Exponents of A's columns over the rows that reflectors touch.
         k_dg_exp_k<<<n, 256, 0, st>>>(HqCols{dA + 1, lda, n, n - 1}, n - 1, nullptr, 0, D.cex);
         if (cudaMemsetAsync(D.low, 0, (size_t)(2 * n + 2) * sizeof(int), st) != cudaSuccess) return HSR_ERR_CUDA;
@@ -1875,7 +1880,7 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
             cudaMemsetAsync(S.Y + (size_t)ib * n, 0, (size_t)(kHbNb - ib) * n * sizeof(double), st) != cudaSuccess)
             return HSR_ERR_CUDA;
         if (one) {
-            const bool fix = digits && n >= kHbFixN;
+            const bool fix = digits && fixes;
             HbPanel pp{S, k0, ib, R, own, rpc, rtiles, shares, S.cnt + 2, reinterpret_cast<const int2 *>(D.AD), D.top,
                        fix ? D.uneven : nullptr};
             void *args[] = {&pp};

@@ -8,6 +8,7 @@
 #include "hsr_common.h"
 #include "hsr_device.cuh"
 #include "hsr_kernels.h"
+#include "hsr_scratch.h"
 #include "../../include/hsrq3in_gb300.h"
 
 #include <algorithm>
@@ -1221,7 +1222,10 @@ int hsr_last_kernel_times(double *ms, long *launches, double *gemm_fma) {
     return kcCount;
 }
 
-void hsr_release_workspace(void) { ws().release(); }
+void hsr_release_workspace(void) {
+    ws().release();
+    Scratch::release_all();
+}
 
 int hsr_selftest_arith(long long per_thread, unsigned long long seed, long long counts[4]) {
     if (per_thread < 0 || !counts) return record_status(HSR_ERR_ARG, cudaSuccess);

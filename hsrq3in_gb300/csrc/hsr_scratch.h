@@ -16,13 +16,34 @@ namespace hsr {
 // allocation and a free node): the thread's buffer, which a later call may
 // replace and the thread's end frees, never enters a graph, and replays need no
 // order against direct calls.
+//
+// A thread's buffers keep their largest size until release_all
+// (hsr_release_workspace) or its end.
 struct Scratch {
     int device = -1;
     void *p = nullptr;
     size_t bytes = 0;
     cudaEvent_t ev = nullptr;
     bool used = false;
-    ~Scratch() { release(); }
+    Scratch *next;                                               // the thread's others
+    static Scratch *&first() {
+        static thread_local Scratch *f = nullptr;
+        return f;
+    }
+    Scratch() : next(first()) { first() = this; }
+    ~Scratch() {
+        for (Scratch **s = &first(); *s; s = &(*s)->next)
+            if (*s == this) {
+                *s = next;
+                break;
+            }
+        release();
+    }
+    Scratch(const Scratch &) = delete;
+    Scratch &operator=(const Scratch &) = delete;
+    static void release_all() {
+        for (Scratch *s = first(); s; s = s->next) s->release();
+    }
     void release() {
         if (p) cudaFree(p);
         if (ev) cudaEventDestroy(ev);

@@ -163,7 +163,11 @@ long hsr_last_launch_count(void);
 void hsr_set_kernel_timing(int enable);
 int hsr_last_kernel_times(double *ms, long *launches, double *gemm_fma);
 
-/* Release cached device workspaces of this thread. */
+/* Release the cached device workspaces of this thread: the solvers' and the
+ * scratch of the reduction (at most 2 GB of digits, or 8 n^2 bytes up to n of
+ * about 25,000), the back-transform (at most 1 GB for X and 4 GB for the
+ * reflectors) and the residuals (at most 3 GB), which keep their largest size
+ * until then or the thread's end.  Waits for the work that uses them. */
 void hsr_release_workspace(void);
 
 /* ------------------------------------------ Hessenberg reduction (device) */

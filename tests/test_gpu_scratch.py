@@ -127,3 +127,38 @@ def test_streams_that_come_and_go(gpu_lib):
         torch.cuda.synchronize()
         for got, r in zip(outs, ref):
             _same(torch, got, r)
+
+
+def test_release_gives_everything_back(gpu_lib):
+    """hsr_release_workspace frees the scratch of all three, which is no more
+    than what their digits take (a triangle of V three times, n = 3000: 24
+    blocks of 128 reflectors, 300 of their 128 x 128 blocks at 256 KB, 2 MB of
+    Gram parts a block, and X;
+    8 n^2 bytes for the reduction; H and X for the residuals), and later calls
+    get it anew."""
+    import torch
+    import hsrq3in_gb300 as hsr
+    n, ncols, mb = 3000, 64, 2.0 ** 20
+    A0, X0, wr = _problem(torch, n, ncols, False, 6)
+    A, X = A0.clone(), X0.clone()
+    lib = hsr.load()
+    _all(hsr, torch, A0, X0, wr)                                # library and allocator pools loaded
+    lib.hsr_release_workspace()
+    torch.cuda.synchronize()
+
+    def used(f):
+        before = torch.cuda.mem_get_info()[0]
+        f()
+        torch.cuda.synchronize()
+        return (before - torch.cuda.mem_get_info()[0]) / mb
+    tau = torch.zeros(n, dtype=torch.float64, device="cuda")
+    res = torch.zeros(ncols, dtype=torch.float64, device="cuda")
+    base = torch.cuda.mem_get_info()[0]
+    red = used(lambda: lib.hsr_hessenberg_device(n, A.data_ptr(), n, tau.data_ptr(), None))
+    back = used(lambda: lib.hsr_hessenberg_apply_q_device(n, A.data_ptr(), n, tau.data_ptr(), ncols, X.data_ptr(), n, None))
+    val = used(lambda: lib.hsr_residuals_device(n, A0.data_ptr(), n, ncols, wr.data_ptr(), X0.data_ptr(), n, res.data_ptr(),
+                                                None))
+    assert 50 < red < 300 and 3 * 300 / 4 <= back < 3 * 300 / 4 + 80 and 100 < val < 200, (red, back, val)
+    lib.hsr_release_workspace()
+    assert torch.cuda.mem_get_info()[0] == base
+    _same(torch, _all(hsr, torch, A0, X0, wr), (A, tau, X, res))
