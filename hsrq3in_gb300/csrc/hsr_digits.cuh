@@ -592,12 +592,12 @@ k_dg_gemm(const unsigned char *__restrict__ A, const unsigned char *__restrict__
     dg_fence_after();
     if (wid == 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
-    if (failed) epi.poison();
+    if (failed) epi.poison(threadIdx.x, blockDim.x);
 }
 
 // ------------------------------------------------------------- epilogues
 __device__ __forceinline__ bool dg_bad(int ex) { return ex >= kDgBad / 2; }
-__device__ __forceinline__ double dg_nan() { return __longlong_as_double(0x7ff8000000000000LL); }
+__host__ __device__ __forceinline__ double dg_nan() { return from_bits(0x7ff8000000000000ULL); }
 
 // Stages [0, steps) of every tile cut into nz parts of `per` stages; part z
 // of C(i, j) goes to out[z * cz + i * si + j * sj].
@@ -625,9 +625,12 @@ struct DgStore {
             if (i < M && j0 + c < N) o[(size_t)c * sj] = dg_bad(er) || dg_bad(ec) ? dg_nan() : v;
         }
     }
-    __device__ void poison() const {
-        for (long long e = threadIdx.x; e < (long long)M * N; e += blockDim.x)
-            out[(e % M) * si + (e / M) * sj] = dg_nan();
+    // Every part: the tile that failed may be of any, and the others' owners
+    // may still store theirs.
+    __host__ __device__ void poison(int thread, int threads) const {
+        for (int z = 0; z * per < steps; ++z)
+            for (long long e = thread; e < (long long)M * N; e += threads)
+                out[z * cz + (e % M) * si + (e / M) * sj] = dg_nan();
     }
 };
 using DgStoreLong = DgStore<DgTwo<16>, 16>;
@@ -682,8 +685,8 @@ struct DgUpdate {
             if (m > cl) atomicMax(&cex[jl], m);
         }
     }
-    __device__ void poison() const {
-        for (long long e = threadIdx.x; e < (long long)M * N; e += blockDim.x) C[(e % M) + (e / M) * ldc] = dg_nan();
+    __device__ void poison(int thread, int threads) const {
+        for (long long e = thread; e < (long long)M * N; e += threads) C[(e % M) + (e / M) * ldc] = dg_nan();
     }
 };
 

@@ -1400,8 +1400,10 @@ struct HqGram {
             o[(size_t)c * kHqNb] = dg_bad(er) || dg_bad(ec) ? dg_nan() : v;
         }
     }
-    __device__ void poison() const {
-        for (int e = threadIdx.x; e < nz * kHqNb * kHqNb; e += blockDim.x) S[e] = dg_nan();
+    // The group's block 0, which the back-transform takes first and whose rows
+    // every later block mixes into all of X.
+    __device__ void poison(int thread, int threads) const {
+        for (int e = thread; e < nz * kHqNb * kHqNb; e += threads) S[e] = dg_nan();
     }
 };
 // Rows of the operand are columns of a column-major matrix.

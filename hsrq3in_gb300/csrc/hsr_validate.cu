@@ -295,8 +295,8 @@ struct ValEpi {
         r2[0] += __shfl_xor_sync(0xffffffffu, r2[0], 16);
         if (lane < NC && col0 + lane < cols) atomicAdd(&rsum[col0 + lane], r2[0]);
     }
-    __device__ void poison() const {
-        for (int c = threadIdx.x; c < cols; c += blockDim.x) rsum[c] = __longlong_as_double(0x7ff8000000000000LL);
+    __device__ void poison(int thread, int threads) const {
+        for (int c = thread; c < cols; c += threads) rsum[c] = __longlong_as_double(0x7ff8000000000000LL);
     }
 };
 
