@@ -17,8 +17,8 @@
 // (I - V T^T V^T) from the left; then its reflector is generated, and
 // Y(:, i) = tau (A v - Y (V^T v)), T(:, i) = -tau T (V^T v), T(i,i) = tau.
 // All columns of a panel run in one cooperative launch (k_hb_panel); only
-// where the rows do not fit its shared memory (n above about 25,000) three
-// launches per column do the same:
+// where the rows do not fit its shared memory (n above about 25,000), or the
+// device refuses such a launch, three launches per column do the same:
 //   k_hb_step    rows in parallel: finishes the previous column (Y, V and T
 //                columns, its reflector into A) and starts this one,
 //                c = a_j - Y V(j,:)^T, with partial V^T c; the last block to
@@ -46,6 +46,8 @@
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
+#include <cstdlib>
+#include <cstring>
 #include <cuda_runtime.h>
 #include <type_traits>
 
@@ -1082,6 +1084,8 @@ __global__ void __launch_bounds__(256, 2) k_hb_plain(HbPlain P, int first, int l
         }
     }
 }
+// A cooperative launch that this device, or what is left of it, cannot take.
+bool refused(cudaError_t e) { return e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported; }
 // All phases of a kernel k(P, first, last) in one cooperative launch, or, where
 // the device refuses that, one by one.
 template <class Params>
@@ -1090,7 +1094,7 @@ cudaError_t launch_phases(void (*kernel)(Params, int, int), Params P, int phases
     void *args[] = {&P, &first, &phases};
     const cudaError_t e =
         cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel), dim3(grid), dim3(256), args, 0, st);
-    if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported) return e;
+    if (!refused(e)) return e;
     cudaGetLastError();
     for (; first < phases; ++first) kernel<<<grid, 256, 0, st>>>(P, first, first + 1);
     return cudaGetLastError();
@@ -1826,7 +1830,8 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
     for (int h = 32; h <= kHbThreads; h *= 2) best = std::max(best, busy(h));
     while (rpc < kHbThreads && 10 * busy(rpc) < 9 * best) rpc *= 2;
     const int rtiles = (n + rpc - 1) / rpc, shares = std::max(1, ctas / rtiles);
-    const bool one = rtiles <= ctas && hb_panel_smem(R) <= kHbPanelSmem &&
+    const char *env = getenv("HSR_HESS_PANEL");                  // "steps": three launches a column at any order
+    bool one = !(env && !strcmp(env, "steps")) && rtiles <= ctas && hb_panel_smem(R) <= kHbPanelSmem &&
                      cudaFuncSetAttribute(k_hb_panel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHbPanelSmem) == cudaSuccess &&
                      cudaFuncSetAttribute(k_hb_panel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHbPanelSmem) == cudaSuccess;
     const size_t need = 2 * (size_t)n * nb           // Y, V
@@ -1886,19 +1891,25 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
             HbPanel pp{S, k0, ib, R, own, rpc, rtiles, shares, S.cnt + 2, reinterpret_cast<const int2 *>(D.AD), D.top,
                        fix ? D.uneven : nullptr};
             void *args[] = {&pp};
-            if (fix) {
+            const auto panel = [&](const void *fn) {
+                return cudaLaunchCooperativeKernel(fn, dim3(ctas), dim3(kHbThreads), args, hb_panel_smem(R), st);
+            };
+            // (First: where it is refused, neither form runs.)
+            const cudaError_t e = panel(reinterpret_cast<const void *>(k_hb_panel<false>));
+            if (refused(e)) {
+                cudaGetLastError();
+                one = false;
+            } else if (e != cudaSuccess) {
+                return HSR_ERR_CUDA;
+            } else if (fix) {
                 const dim3 g((unsigned)(n + 255) / 256, (unsigned)((n - k0 - 1 + kFixCols - 1) / kFixCols));
                 if (cudaMemsetAsync(D.top, 0, (size_t)n * sizeof(unsigned), st) != cudaSuccess) return HSR_ERR_CUDA;
                 k_hb_fix_top<<<g, 256, 0, st>>>(n, dA, lda, k0 + 1, D.top, D.uneven);
                 k_hb_fix<<<g, 256, 0, st>>>(n, dA, lda, k0 + 1, D.top, reinterpret_cast<int2 *>(D.AD), D.uneven);
-                if (cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_hb_panel<true>), dim3(ctas), dim3(kHbThreads),
-                                                args, hb_panel_smem(R), st) != cudaSuccess)
-                    return HSR_ERR_CUDA;
+                if (panel(reinterpret_cast<const void *>(k_hb_panel<true>)) != cudaSuccess) return HSR_ERR_CUDA;
             }
-            if (cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_hb_panel<false>), dim3(ctas), dim3(kHbThreads),
-                                            args, hb_panel_smem(R), st) != cudaSuccess)
-                return HSR_ERR_CUDA;
-        } else {
+        }
+        if (!one) {
             int nchp = 0;
             for (int i = 0; i < ib; ++i) {
                 const int j = k0 + i;

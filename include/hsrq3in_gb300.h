@@ -180,7 +180,11 @@ void hsr_release_workspace(void);
  * Where the entries of dA are of like size (decided on the device), products
  * run on the tensor cores and in fixed point with errors no larger than FP64's;
  * otherwise in FP64, so that the small rows and columns of a graded matrix stay
- * accurate.  Enqueued on `stream`; all pointers are device pointers.  No reference
+ * accurate.  Enqueued on `stream`; all pointers are device pointers.  The call
+ * returns before the device has run it: a wait between the thread blocks of a
+ * panel, or for a copy, that runs out (none does unless the device stalls for
+ * seconds) is not in the status but leaves NaN in dtau and dA; likewise in dX
+ * below and in the residuals.  No reference
  * counterpart in the solver itself. */
 int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, void *stream);
 /* X <- Q X for the Q of hsr_hessenberg_device (LAPACK dormhr 'L','N'):

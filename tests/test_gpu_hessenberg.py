@@ -116,3 +116,22 @@ def test_zero_subdiagonal_at_the_safe_minimum(gpu_lib, n, scale, leading):
     H = np.triu(F, -1).astype(L) / scale
     R = np.array([(A * Q[:, c]).sum(1) - (Q[:, :c + 2] * H[:c + 2, c]).sum(1) for c in range(n)])
     assert float(np.sqrt((R * R).sum())) <= n * EPS * np.linalg.norm(A)
+
+
+@pytest.mark.parametrize("n,scale", [(3, 1.0), (64, 1.0), (67, 1e-300), (130, 1.0), (300, 1e150), (2100, 1.0)])
+def test_three_launches_a_column(gpu_lib, monkeypatch, n, scale):
+    """The form for orders whose panel does not fit one launch (and for devices
+    that refuse a cooperative one), forced: A Q = Q H and Q^T Q = I, with a zero
+    on the subdiagonal of A's first column."""
+    import torch
+    import hsrq3in_gb300 as hsr
+    monkeypatch.setenv("HSR_HESS_PANEL", "steps")
+    A = np.random.default_rng(n).standard_normal((n, n))
+    A[1, 0] = 0.0
+    dA, tau, out, _ = _reduce(A * scale)
+    one = hsr.hessenberg_device(torch.zeros_like(dA))           # and of a zero matrix
+    assert not torch.any(one)
+    Q = torch.from_numpy(_form_q(dA, tau, n)).cuda()
+    H, At = torch.from_numpy(np.triu(out, -1) / scale).cuda(), torch.from_numpy(A).cuda()
+    assert float((Q.T @ Q - torch.eye(n, dtype=torch.float64, device="cuda")).norm()) <= 50 * n * EPS
+    assert float((At @ Q - Q @ H).norm()) / np.linalg.norm(A) <= 50 * n * EPS
