@@ -1617,22 +1617,13 @@ int device_sms() {
     return sms;
 }
 
-// Shifts per CTA of a launch: diag_shifts_per_cta, and where that is 8 and
-// CTAs of 4 still find an SM each, 4: the rows and the fused top GEMM are
-// bound by the FP64 pipes of the SMs that take part (n = 3001, 301 shifts,
-// tile 200: 14.6 ms with 8, 12.4 with 4).
-int narrow_shifts(int S) {
-    const int sc = diag_shifts_per_cta(S);
-    return sc == 8 && (S + 3) / 4 <= device_sms() ? 4 : sc;
-}
-
 // Tile J's diagonal solve preceded by stage J+1's GEMM over tile J's rows,
 // in one launch, when the narrow forms apply; false (nothing launched) when
 // the wide form is used and the caller runs the two launches.
 bool launch_diag_fused(const DevProblem &P, const DevProblem &Pg, int J, int b, cudaStream_t st,
                        cudaError_t *err) {
     if (!fused_top_for(P.S)) return false;
-    switch (narrow_shifts(P.S)) {
+    switch (diag_shifts_per_cta(P.S)) {
     case 4: *err = launch_diag_narrow_fused<4, kDiagWarpsNarrow>(P, Pg, J, b, st); return true;
     case 8: *err = launch_diag_narrow_fused<8, kDiagWarpsNarrow>(P, Pg, J, b, st); return true;
     case 16: *err = launch_diag_narrow_fused<16, kDiagWarpsNarrow>(P, Pg, J, b, st); return true;
@@ -1693,37 +1684,39 @@ bool fused_top_for(int S) {
         const int tuned = nearest_tuned(g_fused_tuned, S);
         if (tuned) return tuned == 1;
     }
-    const int sc = narrow_shifts(S);
+    const int sc = diag_shifts_per_cta(S);
     return 4 * ((S + sc - 1) / sc) > 3 * device_sms();
 }
 
-// Shifts per diagonal CTA.  HSR_DIAG_SHIFTS_PER_CTA (8, 16 or 32) first,
-// then the autotuner's trial value, then its recorded choice for the nearest
-// shift count within a factor of two; otherwise 32 (a lane per shift) while
-// the 32-shift CTAs cover the GPU, fewer when they would leave most SMs idle
-// -- 16 below half the SMs, 8 below a quarter.  Every choice gives the same
-// result bit for bit.
+// Shifts per diagonal CTA.  HSR_DIAG_SHIFTS_PER_CTA (4, 8, 16 or 32) first and
+// as it is; then the autotuner's trial value, then its recorded choice for the
+// nearest shift count within a factor of two; otherwise 32 (a lane per shift)
+// while the 32-shift CTAs cover the GPU, fewer when they would leave most SMs
+// idle -- 16 below half the SMs, 8 below a quarter.  Where one of these gives 8
+// and CTAs of 4 still find an SM each, 4: the rows and the fused top GEMM are
+// bound by the FP64 pipes of the SMs that take part (n = 3001, 301 shifts, tile
+// 200: 14.6 ms with 8, 12.4 with 4).  So a trial of 8 times what a recorded 8
+// runs.  Every choice gives the same result bit for bit.
 int diag_shifts_per_cta(int S) {
     const char *env = getenv("HSR_DIAG_SHIFTS_PER_CTA");   // read per launch: tests switch it
     const int forced = env ? atoi(env) : 0;
-    if (forced == 8 || forced == 16 || forced == 32) return forced;
-    if (t_spc_trial) return t_spc_trial;
-    {
-        std::lock_guard<std::mutex> g(g_spc_mu);
-        const int best = nearest_tuned(g_spc_tuned, S);
-        if (best) return best;
-    }
+    if (forced == 4 || forced == 8 || forced == 16 || forced == 32) return forced;
     const int sms = device_sms();
-    const int wide = (S + 31) / 32;
-    if (sms <= 0) return 32;
-    if (4 * wide <= sms) return 8;
-    if (2 * wide <= sms) return 16;
-    return 32;
+    int sc = t_spc_trial;
+    if (!sc) {
+        std::lock_guard<std::mutex> g(g_spc_mu);
+        sc = nearest_tuned(g_spc_tuned, S);
+    }
+    if (!sc) {
+        const int wide = (S + 31) / 32;
+        sc = sms <= 0 ? 32 : 4 * wide <= sms ? 8 : 2 * wide <= sms ? 16 : 32;
+    }
+    return sc == 8 && (S + 3) / 4 <= sms ? 4 : sc;
 }
 
 cudaError_t launch_diag(const DevProblem &P, int J, int b, double *gscratch, cudaStream_t st) {
     const int grid = (P.S + 31) / 32;
-    switch (narrow_shifts(P.S)) {
+    switch (diag_shifts_per_cta(P.S)) {
     case 4: return launch_diag_narrow<4, kDiagWarpsNarrow>(P, J, b, st);
     case 8: return launch_diag_narrow<8, kDiagWarpsNarrow>(P, J, b, st);
     case 16: return launch_diag_narrow<16, kDiagWarpsNarrow>(P, J, b, st);

@@ -79,14 +79,16 @@ bool launch_diag_fused(const DevProblem &P, const DevProblem &Pg, int J, int b, 
                        cudaError_t *err);
 // Top-GEMM form of the narrow diagonal kernel: fused (true) or a separate
 // launch -- the HSR_FUSED_TOP override, else this thread's autotuning trial
-// (-1: none), else the tuned entry of the nearest shift count, else fused.
+// (-1: none), else the tuned entry of the nearest shift count, else by how many
+// SMs the diagonal CTAs are on.
 bool fused_top_for(int S);
 void set_fused_top_trial(int on);
 void record_fused_top(int S, bool on);
-// Shifts per CTA the diagonal kernel uses for S shifts: 8, 16 or 32 -- the
+// Shifts per CTA the diagonal kernel uses for S shifts: 4, 8, 16 or 32 -- the
 // HSR_DIAG_SHIFTS_PER_CTA override, else this thread's autotuning trial, else
 // the tuned entry of the nearest shift count (record_diag_shifts), else a rule
-// by how many SMs the 32-shift CTAs would fill.
+// by how many SMs the 32-shift CTAs would fill; 4 for an 8 of the last three
+// where those CTAs find an SM each.
 int diag_shifts_per_cta(int S);
 void set_diag_shifts_trial(int sc);      // 0 ends the trial
 void record_diag_shifts(int S, int sc);

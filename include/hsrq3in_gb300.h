@@ -265,8 +265,8 @@ int hsr_batch_plan_queue_info(const hsr_batch_plan *plan, int *engine, long *ite
 /* Plain-path autotuner: times hsr_inverse_iteration_device on the caller's
  * problem (device pointers; dwr is restored, dvr overwritten) for each
  * candidate tlsz in `cand` (ms_out[i], optional, gets candidate i's time),
- * then, at the fastest tlsz, for 8, 16 and 32 shifts per diagonal CTA
- * (spc_ms[0..2], optional), and, where the fastest of those is 8 or 16,
+ * then, at the fastest tlsz, for 8 (4 where those CTAs still find an SM each),
+ * 16 and 32 shifts per diagonal CTA (spc_ms[0..2], optional), and, where the fastest of those is 8 or 16,
  * with the GEMM of each tile's own rows run inside the diagonal CTAs or as
  * its own launch (fused_ms[1] and fused_ms[0], optional; -1 where it does
  * not apply).  It records the fastest tlsz for order n, the fastest shifts

@@ -90,3 +90,26 @@ def test_batch_forms(gpu_lib, count, tlsz):
     for (H, _, X), o in zip(probs, ref):
         assert np.array_equal(X.cpu().numpy()[:, :H.shape[0]].T, o["vr"])
     plan.close()
+
+
+@pytest.mark.parametrize("n,tlsz,nrhs", [(203, 40, 77), (260, 160, 609), (300, 64, 1217)])
+def test_forced_shifts_per_cta(gpu_lib, monkeypatch, n, tlsz, nrhs):
+    """A forced number of shifts per diagonal CTA is the one that runs: the
+    kernels' instantiation shows in a trace, the result is the oracle's."""
+    import torch
+    import hsrq3in_gb300 as hsr
+    from torch.profiler import ProfilerActivity, profile
+    H, lam = G.real_spectrum(n, n)
+    wr = np.resize(G.perturbed_shifts(lam, 3), nrhs)
+    orc = O.oracle_inverse_iteration(H, wr, tlsz, 16, intscale=1, variant="fma")
+    for sc in (4, 8, 16, 32):
+        monkeypatch.setenv("HSR_DIAG_SHIFTS_PER_CTA", str(sc))
+        for _ in range(2):                       # a process's first trace can come back empty
+            with profile(activities=[ProfilerActivity.CUDA]) as prof:
+                dev = hsr.inverse_iteration(H, wr, tlsz, 16)
+                torch.cuda.synchronize()
+            diag = [e.key for e in prof.key_averages() if "k_diag" in e.key]
+            if diag:
+                break
+        assert diag and all(("k_diag_n" in k and "<%d, " % sc in k) if sc < 32 else "k_diag_n" not in k for k in diag), (sc, diag)
+        assert np.array_equal(dev["vr"], orc["vr"])
