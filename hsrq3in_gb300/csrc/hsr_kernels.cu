@@ -1622,7 +1622,7 @@ int device_sms() {
 // the wide form is used and the caller runs the two launches.
 bool launch_diag_fused(const DevProblem &P, const DevProblem &Pg, int J, int b, cudaStream_t st,
                        cudaError_t *err) {
-    if (!fused_top_for(P.S)) return false;
+    if (!fused_top_for(P.S, b)) return false;
     switch (diag_shifts_per_cta(P.S)) {
     case 4: *err = launch_diag_narrow_fused<4, kDiagWarpsNarrow>(P, Pg, J, b, st); return true;
     case 8: *err = launch_diag_narrow_fused<8, kDiagWarpsNarrow>(P, Pg, J, b, st); return true;
@@ -1669,13 +1669,18 @@ void record_fused_top(int S, bool on) {
 // Whether the narrow diagonal kernel also computes the top GEMM of its own
 // rows: HSR_FUSED_TOP (0 or 1) first, then the autotuner's trial value, then
 // its recorded choice for the nearest shift count within a factor of two,
-// else where the diagonal CTAs are on more than three quarters of the SMs: on
-// fewer, those SMs alone would do the rows that a GEMM of 64x16 tiles spreads
-// over all.  Inside / separate: n = 3001 with 301 shifts (76 CTAs) 11.6 / 10.7
-// ms, n = 1000 with 300 2.94 / 2.62, n = 4096 with 640 24.4 / 23.8, n = 48
-// 298 / 283 us; n = 1000 with 1000 (125 CTAs, tiles of 160) 3.92 / 4.12 ms.
-// Either form gives the same result bit for bit.
-bool fused_top_for(int S) {
+// else with 8 shifts per CTA, more than three quarters of the SMs taken and 144
+// to 192 rows in the tile.  Fewer CTAs leave those SMs alone with rows that a
+// GEMM of 64x16 tiles spreads over all; lower tiles do not pay for the wait of
+// the CTA's own columns; more than 192 rows are a second pass
+// (top_rows_staged).  Separate / inside, ms: n = 2000 with 1000 shifts, tiles of
+// 96 10.55 / 11.08, 128 10.56 / 10.94, 144 10.56 / 10.54, 160 11.02 / 10.71, 192
+// 11.27 / 10.56, 200 11.00 / 11.99; with 700 shifts (88 CTAs), 160, 8.82 / 8.95;
+// n = 3001 with 1200, 160, 23.55 / 23.42, 200 23.85 / 25.62.  4 shifts per CTA, n
+// = 1300 with 600 (150 CTAs), tiles of 160 4.42 / 5.02; 16 shifts, n = 3001 with
+// 2400 (150), 160 42.33 / 42.72, 64 43.87 / 44.08.  Either form gives the same
+// result bit for bit.
+bool fused_top_for(int S, int b) {
     const char *env = getenv("HSR_FUSED_TOP");
     if (env && (env[0] == '0' || env[0] == '1')) return env[0] == '1';
     if (t_fused_trial >= 0) return t_fused_trial != 0;
@@ -1684,8 +1689,7 @@ bool fused_top_for(int S) {
         const int tuned = nearest_tuned(g_fused_tuned, S);
         if (tuned) return tuned == 1;
     }
-    const int sc = diag_shifts_per_cta(S);
-    return 4 * ((S + sc - 1) / sc) > 3 * device_sms();
+    return diag_shifts_per_cta(S) == 8 && 4 * ((S + 7) / 8) > 3 * device_sms() && b >= 144 && b <= 192;
 }
 
 // Shifts per diagonal CTA.  HSR_DIAG_SHIFTS_PER_CTA (4, 8, 16 or 32) first and

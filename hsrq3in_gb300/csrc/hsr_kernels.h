@@ -80,8 +80,8 @@ bool launch_diag_fused(const DevProblem &P, const DevProblem &Pg, int J, int b, 
 // Top-GEMM form of the narrow diagonal kernel: fused (true) or a separate
 // launch -- the HSR_FUSED_TOP override, else this thread's autotuning trial
 // (-1: none), else the tuned entry of the nearest shift count, else by how many
-// SMs the diagonal CTAs are on.
-bool fused_top_for(int S);
+// SMs the diagonal CTAs are on and the tile's rows b.
+bool fused_top_for(int S, int b);
 void set_fused_top_trial(int on);
 void record_fused_top(int S, bool on);
 // Shifts per CTA the diagonal kernel uses for S shifts: 4, 8, 16 or 32 -- the
