@@ -139,10 +139,10 @@ __device__ __forceinline__ int dg_dk(const int *dk, int k) {     // no scaling b
 }
 
 // Digit products are for operands whose entries are of like size; a call that
-// leaves the choice to the device passes a word `off` to the splits and the
-// products, which store nothing where the word is not 0 (the caller's other
-// form then runs).  They read it beside their first loads or set-up: ahead of
-// them it cost 0.7 us a launch.
+// leaves the choice to the device passes a word `off` to the products, which
+// store nothing where it is not 0 (the caller's other form then runs).  Only
+// the warps that store read it, beside the first products: read at the start of
+// every product and split it cost the back-transform of n = 5000 1.5%.
 __device__ __forceinline__ bool dg_off(const int *off) { return off && *off != 0; }
 
 // ---------------------------------------------------------- preparation
@@ -189,9 +189,7 @@ __global__ void __launch_bounds__(256) k_dg_exp_r(Ld ld, int R, int K, int span,
 // both the loads and the 16-byte stores of a warp cover whole sectors.
 template <class Ld, bool RC>
 __global__ void __launch_bounds__(256) k_dg_split(Ld ld, int RB, int Rpad, long long steps, const int *ex,
-                                                  const int *dk, int sign, int R, int K, unsigned char *out,
-                                                  const int *off) {
-    const bool skip = dg_off(off);
+                                                  const int *dk, int sign, int R, int K, unsigned char *out) {
     const int t = threadIdx.x;
     const int r = RC ? blockIdx.x * 32 + (t & 31) : blockIdx.x * 8 + (t & 7);
     const int c8 = RC ? blockIdx.y * 8 + (t >> 5) : blockIdx.y * 32 + (t >> 3);
@@ -206,7 +204,7 @@ __global__ void __launch_bounds__(256) k_dg_split(Ld ld, int RB, int Rpad, long 
         const int k = c8 * 8 + e;
         u[e] = dg_digits(x[e], dk && k < K ? base - sign * dk[k] : base);
     }
-    if (!skip) dg_store8(u, out + dg_place(r, c8, RB, steps), RB * kDgBK * 2);
+    dg_store8(u, out + dg_place(r, c8, RB, steps), RB * kDgBK * 2);
 }
 
 // Exponents and digits in one pass for K <= 128: a thread keeps its eight
@@ -457,7 +455,6 @@ k_dg_gemm(const unsigned char *__restrict__ A, const unsigned char *__restrict__
     __shared__ __align__(8) uint64_t full[kDgStages], empty[kDgStages], acc_full[kDgGroups], acc_empty[kDgGroups];
     __shared__ uint32_t tmem_base;
     __shared__ int failed;
-    const bool skip = dg_off(off);
     const int tid = threadIdx.x, wid = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     if (tid == 0) {
         for (int i = 0; i < kDgStages; ++i) {
@@ -482,7 +479,6 @@ k_dg_gemm(const unsigned char *__restrict__ A, const unsigned char *__restrict__
     const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
     unsigned char *const sa = reinterpret_cast<unsigned char *>(((uintptr_t)dg_sm + 1023) & ~(uintptr_t)1023);
     unsigned char *const sb = sa + kDgStages * kDgABytes;
-    if (skip) tiles = 0;
     const uint32_t sa0 = __shfl_sync(0xffffffffu, smem_u32(sa), 0), sb0 = sa0 + kDgStages * kDgABytes;
 
     if (wid == 0) {
@@ -559,6 +555,7 @@ k_dg_gemm(const unsigned char *__restrict__ A, const unsigned char *__restrict__
         const int quad = wid & 3, part = (wid - 2) >> 2;
         const int row = quad * 32 + lane;
         const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(part * kCols);
+        const bool skip = dg_off(off);
         unsigned chunk = 0;
         bool ok = true;
         for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
@@ -583,7 +580,7 @@ k_dg_gemm(const unsigned char *__restrict__ A, const unsigned char *__restrict__
                     for (int c = 0; c < kCols; ++c) sum.add(g, c, v[c]);
                 }
             }
-            if (ok) epi.finish(q, q.bx * kDgBM + row, q.by * kDgBN + part * kCols, sum);
+            if (ok && !skip) epi.finish(q, q.bx * kDgBM + row, q.by * kDgBN + part * kCols, sum);
         }
         if (!ok) failed = 1;
     }
@@ -592,7 +589,7 @@ k_dg_gemm(const unsigned char *__restrict__ A, const unsigned char *__restrict__
     dg_fence_after();
     if (wid == 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
-    if (failed) epi.poison(threadIdx.x, blockDim.x);
+    if (failed && !dg_off(off)) epi.poison(threadIdx.x, blockDim.x);
 }
 
 // ------------------------------------------------------------- epilogues

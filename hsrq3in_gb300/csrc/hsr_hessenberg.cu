@@ -1109,9 +1109,9 @@ cudaError_t launch_phases(void (*kernel)(Params, int, int), Params P, int phases
 // 160 (2100): d from 1 to 2^-3 1.9e-15 / 1.6e-15 (5.3e-15 / 5.0e-15), to 2^-10
 // 1.1e-14 / 1.1e-14 (2.4e-14 / 2.1e-14), to 1e-16 4.6e-13 / 3e-4 (5.5e-13 /
 // 2e-3); those with d down to 2^-4 (n = 2100) and beyond are refused.  The
-// check reads A once: n = 700 13.15 -> 13.19 ms with the launches that do
-// nothing, n = 6000 316.4 -> 317.7.  Refused, d to 1e-12: n = 700 16.1 ms, n =
-// 4000 317.
+// check reads A once: n = 700 13.35 -> 13.38 ms with the launches that do
+// nothing, n = 4000 138.1 -> 139.2, n = 6000 316.4 -> 317.7.  Refused, d to
+// 1e-12: n = 700 16.4 ms, n = 4000 324.
 constexpr int kHbEvenBits = 8;
 __device__ __forceinline__ bool hb_few(int low, int of) { return 5 * low <= 2 * of; }
 // Counts of the entries that small(x, c) holds of rows r = r0 + tid (in or not)
@@ -1262,8 +1262,8 @@ __global__ void __launch_bounds__(256, 2) k_hq_plain(HqPlain P, int first, int l
 constexpr int kHqNb = 128;
 // Smallest order: a reflector of the DFMA form costs about 5.5 us (three thin
 // products and a serial factor per 64), this form 240 us and 0.5 us each
-// (n = 32: 139 us as DFMA; 64: 360 against 248; 300: 1,665 against 411; 4000
-// with 2000 columns: 85.7 ms against 5.3).  The DFMA form also stays for
+// (n = 32: 139 us as DFMA; 64: 360 against 257; 300: 1,665 against 411; 4000
+// with 2000 columns: 85.7 ms against 5.2).  The DFMA form also stays for
 // reflectors that are not even and for a scratch buffer that cannot be had.
 constexpr int kHqDigitsN = 40;
 // Most scratch for digits of X's columns and of V (three layouts) at a time.
@@ -1280,8 +1280,8 @@ constexpr int kHqMaxSplit = 16;
 // D G D on columns D G', G and G' of N(0,1) entries, error row by row relative
 // to the row's largest, in FP64 / by digits: d down to 1e-8 (n = 45) 2.5e-15 /
 // 2.6e-9, to 1e-12 (n = 300) 3.3e-15 / 2.3e-7.  The check reads V once: n = 64
-// 232 -> 248 us, n = 700 622 -> 650, n = 5000 with 2500 columns 8.56 -> 8.70 ms.
-// Refused, n = 700 with 350 columns 3.86 ms, n = 4000 with 2000 86.
+// 238 -> 257 us, n = 700 625 -> 643, n = 5000 with 2500 columns 8.53 -> 8.60 ms.
+// Refused, n = 700 with 350 columns 4.0 ms, n = 4000 with 2000 89.
 constexpr int kHqEvenBits = 5, kHqEvenMin = 32;
 // low: 2 n counts, zeroed, of the rows' and the columns' smaller entries; cnt: a
 // counter, zeroed.
@@ -1583,7 +1583,7 @@ cudaError_t hq_digits(const HqDigits &D, int n, const double *dA, int lda, const
                 const long long at = h.before(g);
                 double *X = dX + (size_t)c0 * ldx + k0 + 1;
                 k_dg_split<HqCols, false><<<dim3(cb * (kDgBN / 8), (unsigned)((2 * steps + 31) / 32)), 256, 0, st>>>(
-                    HqCols{X, ldx, cols, kr}, kDgBN, cb * kDgBN, steps, exX + c0, nullptr, 0, cols, kr, XN, gate);
+                    HqCols{X, ldx, cols, kr}, kDgBN, cb * kDgBN, steps, exX + c0, nullptr, 0, cols, kr, XN);
                 int per = 0;
                 const int nz = dg_parts(cb, sms, kHqMaxSplit, steps, per);
                 const DgStoreLong e1{1, cb, steps, per, kHqNb, cols, exV + g * kHqNb, exX + c0, Wp, 1, kHqNb,
@@ -1766,7 +1766,7 @@ cudaError_t hb_trailing(const HbState &S, const HbDigits &D, int k0, int c1, int
     const int *exY = D.cex + n, *exV = exY + kHbNb;
     k_dg_exp_k<<<2 * kHbNb, 256, 0, st>>>(HbPanelCols{S.Y, S.V, n, k0}, kr, nullptr, 0, D.cex + n);
     k_dg_split<HbVCols, false><<<dim3(kDgBN / 8, (unsigned)((2 * steps + 31) / 32)), 256, 0, st>>>(
-        HbVCols{S.V, n, k0}, kDgBN, kDgBN, steps, exV, nullptr, 0, kHbNb, kr, D.VN, D.uneven);
+        HbVCols{S.V, n, k0}, kDgBN, kDgBN, steps, exV, nullptr, 0, kHbNb, kr, D.VN);
     int per = 0;
     const int tiles = (std::min(total, D.cch) + kDgBM - 1) / kDgBM;
     const int nz = dg_parts(tiles, sms, kHbParts, steps, per);
@@ -1774,7 +1774,7 @@ cudaError_t hb_trailing(const HbState &S, const HbDigits &D, int k0, int c1, int
     for (int c = 0; c < total; c += D.cch) {
         const int cols = std::min(D.cch, total - c), mb = (cols + kDgBM - 1) / kDgBM;
         k_dg_split<HbTrail, false><<<dim3(mb * (kDgBM / 8), (unsigned)((2 * steps + 31) / 32)), 256, 0, st>>>(
-            HbTrail{S.A, S.Y, S.lda, n, k0, c1 + c}, kDgBM, mb * kDgBM, steps, D.cex + c1 + c, nullptr, 0, cols, kr, D.AD, D.uneven);
+            HbTrail{S.A, S.Y, S.lda, n, k0, c1 + c}, kDgBM, mb * kDgBM, steps, D.cex + c1 + c, nullptr, 0, cols, kr, D.AD);
         const DgStoreLong e{mb, 1, steps, per, cols, kHbNb, D.cex + c1 + c, exV, D.Wp + (size_t)kHbNb * c, kHbNb, 1, cz};
         const cudaError_t err = dg_gemm(mb * nz, sms, D.AD, D.VN, e, D.uneven, st);
         if (err != cudaSuccess) return err;

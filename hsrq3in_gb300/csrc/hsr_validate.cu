@@ -352,14 +352,14 @@ extern "C" int hsr_residuals_device(int n, const double *dH, int lddH, int ncols
             if (cudaMemsetAsync(hex, 0x80, (size_t)rows * sizeof(int), st) != cudaSuccess) return HSR_ERR_CUDA;
             k_dg_exp_r<<<dim3((rows + 255) / 256, (n + 127) / 128), 256, 0, st>>>(lh, rows, n, 128, hcol, -1, hex);
             k_dg_split<ValH, true><<<dim3(rb * (kDgBM / 32), (unsigned)((2 * steps + 7) / 8)), 256, 0, st>>>(
-                lh, kDgBM, rb * kDgBM, steps, hex, hcol, -1, rows, n, hdig, nullptr);
+                lh, kDgBM, rb * kDgBM, steps, hex, hcol, -1, rows, n, hdig);
             for (int c0 = 0; c0 < ncols; c0 += cch) {
                 const int cols = std::min(cch, ncols - c0), cb = (cols + kDgBN - 1) / kDgBN;
                 const double *Xc = dX + (size_t)c0 * lddX;
                 const ValX lx{Xc, lddX, n, cols};
                 k_dg_exp_k<<<cols, 256, 0, st>>>(lx, n, hcol, 1, xex);
                 k_dg_split<ValX, false><<<dim3(cb * (kDgBN / 8), (unsigned)((2 * steps + 31) / 32)), 256, 0, st>>>(
-                    lx, kDgBN, cb * kDgBN, steps, xex, hcol, 1, cols, n, xdig, nullptr);
+                    lx, kDgBN, cb * kDgBN, steps, xex, hcol, 1, cols, n, xdig);
                 k_val_cols<<<(cols + 127) / 128, 128, 0, st>>>(cols, dwr + c0, hmax, xmax + c0, xex, vcol);
                 const ValEpi epi{r0, rows, cols, (int)steps, cb, Xc, lddX, hex, vcol, rsum + c0};
                 if (dg_gemm(rb * cb, sms, hdig, xdig, epi, nullptr, st) != cudaSuccess) return HSR_ERR_CUDA;
