@@ -1086,16 +1086,24 @@ __global__ void __launch_bounds__(256, 2) k_hb_plain(HbPlain P, int first, int l
 }
 // A cooperative launch that this device, or what is left of it, cannot take.
 bool refused(cudaError_t e) { return e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported; }
+// HSR_HESS_PANEL=steps: do without cooperative launches (read per call: tests
+// switch it).
+bool without_cooperative() {
+    const char *env = getenv("HSR_HESS_PANEL");
+    return env && !strcmp(env, "steps");
+}
 // All phases of a kernel k(P, first, last) in one cooperative launch, or, where
 // the device refuses that, one by one.
 template <class Params>
 cudaError_t launch_phases(void (*kernel)(Params, int, int), Params P, int phases, int grid, cudaStream_t st) {
     int first = 0;
     void *args[] = {&P, &first, &phases};
-    const cudaError_t e =
-        cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel), dim3(grid), dim3(256), args, 0, st);
-    if (!refused(e)) return e;
-    cudaGetLastError();
+    if (!without_cooperative()) {
+        const cudaError_t e =
+            cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel), dim3(grid), dim3(256), args, 0, st);
+        if (!refused(e)) return e;
+        cudaGetLastError();
+    }
     for (; first < phases; ++first) kernel<<<grid, 256, 0, st>>>(P, first, first + 1);
     return cudaGetLastError();
 }
@@ -1830,8 +1838,7 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
     for (int h = 32; h <= kHbThreads; h *= 2) best = std::max(best, busy(h));
     while (rpc < kHbThreads && 10 * busy(rpc) < 9 * best) rpc *= 2;
     const int rtiles = (n + rpc - 1) / rpc, shares = std::max(1, ctas / rtiles);
-    const char *env = getenv("HSR_HESS_PANEL");                  // "steps": three launches a column at any order
-    bool one = !(env && !strcmp(env, "steps")) && rtiles <= ctas && hb_panel_smem(R) <= kHbPanelSmem &&
+    bool one = !without_cooperative() && rtiles <= ctas && hb_panel_smem(R) <= kHbPanelSmem &&
                      cudaFuncSetAttribute(k_hb_panel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHbPanelSmem) == cudaSuccess &&
                      cudaFuncSetAttribute(k_hb_panel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHbPanelSmem) == cudaSuccess;
     const size_t need = 2 * (size_t)n * nb           // Y, V

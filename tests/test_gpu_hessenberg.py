@@ -118,16 +118,19 @@ def test_zero_subdiagonal_at_the_safe_minimum(gpu_lib, n, scale, leading):
     assert float(np.sqrt((R * R).sum())) <= n * EPS * np.linalg.norm(A)
 
 
-@pytest.mark.parametrize("n,scale", [(3, 1.0), (64, 1.0), (67, 1e-300), (130, 1.0), (300, 1e150), (2100, 1.0)])
-def test_three_launches_a_column(gpu_lib, monkeypatch, n, scale):
-    """The form for orders whose panel does not fit one launch (and for devices
-    that refuse a cooperative one), forced: A Q = Q H and Q^T Q = I, with a zero
-    on the subdiagonal of A's first column."""
+@pytest.mark.parametrize("n,scale,graded", [(3, 1.0, False), (64, 1.0, False), (67, 1e-300, False), (130, 1.0, True),
+                                            (300, 1e150, False), (300, 1.0, True), (2100, 1.0, False)])
+def test_three_launches_a_column(gpu_lib, monkeypatch, n, scale, graded):
+    """The forms for orders whose panel does not fit one launch and for devices
+    that refuse a cooperative one, forced: A Q = Q H and Q^T Q = I, with a zero
+    on the subdiagonal of A's first column; graded: the updates in FP64 too."""
     import torch
     import hsrq3in_gb300 as hsr
     monkeypatch.setenv("HSR_HESS_PANEL", "steps")
     A = np.random.default_rng(n).standard_normal((n, n))
     A[1, 0] = 0.0
+    if graded:
+        A *= 10.0 ** (-9 * np.arange(n) / n)
     dA, tau, out, _ = _reduce(A * scale)
     one = hsr.hessenberg_device(torch.zeros_like(dA))           # and of a zero matrix
     assert not torch.any(one)
