@@ -44,13 +44,13 @@ sys.path.insert(0, HERE)
 METRIC = "FP64 eigenvectors/s at n=10k"
 UNIT = "eigenvectors/s"
 # DRAM bytes per algorithmic FMA of k_gemm, from one ncu capture of this
-# workload (n=10000, S=10000, tlsz=160; the launch over the 8080 rows above
-# tile 51: 1342.60 MB of dram__bytes_read and 1237.79 MB of
+# workload (n=10000, S=10000, tlsz=160, GEMM tiles of 64x16; the launch over
+# the 8080 rows above tile 51: 1340.06 MB of dram__bytes_read and 1238.63 MB of
 # dram__bytes_write for 8080*319*10000 FMAs; the launch over 7920 rows gives
-# the same ratio within 0.1%).  The traffic is the read and write of R and
+# the same ratio within 0.2%).  The traffic is the read and write of R and
 # X over the rows above, so it grows with rows x shifts as the FMAs do, and
 # the ratio gives each launch's traffic.
-GEMM_DRAM_BYTES_PER_FMA = (1342.602752e6 + 1237.791744e6) / (8080 * 319 * 10000)
+GEMM_DRAM_BYTES_PER_FMA = (1340.062208e6 + 1238.631936e6) / (8080 * 319 * 10000)
 
 
 def parse():

@@ -26,11 +26,17 @@
 //     1/4 where every product's bound is 1.
 //
 // What is lost is the rounding of t (2^-63 of the row's largest entry) and
-// the products with p + q >= 8 (2^-60 of the largest product), below the
-// rounding of an FP64 fma chain of any length.  The method is accurate
-// relative to the largest product of a row and a column; where the columns of
-// A (index k) differ in size a power of two per k evens them out (dk, taken
-// out of A and put into B).
+// the products with p + q >= 8 (2^-60 of the largest product).  So the method is
+// accurate relative to the largest product of a row and a column, not to the
+// sum of their products' magnitudes as an FP64 fma chain is: for operands of
+// entries of like size its error is below the chain's, for others it may be far
+// above.  Where the columns of A (index k) differ in size a power of two per k
+// evens them out (dk, taken out of A and put into B); where a result's small
+// entries count the caller checks the sizes first (hsr_hessenberg.cu: k_hb_even,
+// k_hq_even).  The residuals need no check: with their columns evened out the
+// error in a row is at most 2^-60 sqrt(n) of the largest c_k |x_k|, c_k the
+// largest entry of column k, and that of FP64 in the row where c_k lies about
+// 2^-53 of it, so the norm of r is no less accurate.
 //
 // Digits are stored tile by tile in the order in which the tensor cores read
 // shared memory (8 x 16-byte core matrices, no swizzle), so that a stage of

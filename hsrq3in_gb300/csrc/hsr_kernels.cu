@@ -1957,12 +1957,11 @@ cudaError_t launch_part1(const DevProblem &P, int J, cudaStream_t st) {
 // Bound by the FP64 pipe (64 cycles of a sub-partition per warp's FMA, against
 // which the operands' shared-memory reads, five per eight FMAs, are nothing),
 // so the tile is narrow: less padding past the last shift, and a last wave of
-// 35 us tiles where 64 columns, 4x4 a thread, make it 138.  The 64-column tile
-// takes, 16 columns take: n = 1000 with 1000 shifts 4.26 -> 3.96 ms,
-// n = 2000 with 1000 shifts through host buffers 12.6 -> 11.1, n = 3001 with
-// 301 12.2 -> 11.6, n = 4000 with 4000 126.5 -> 122.5, n = 6000 with 1280
-// 91.4 -> 86.9, n = 10^4 with 10^4 1748 -> 1743; complex, n = 3000 with 1200
-// pairs 50.4 -> 46.8.  BN = 64 is left for the persistent queue, whose items
+// 35 us tiles where 64 columns, 4x4 a thread, make it 138.  Whole solves with
+// 64-column / 16-column tiles: n = 1000 with 1000 shifts 4.26 / 3.96 ms, n =
+// 2000 with 1000 shifts through host buffers 12.6 / 11.1, n = 3001 with 301 12.2
+// / 11.6, n = 4000 with 4000 126.5 / 122.5, n = 6000 with 1280 91.4 / 86.9, n =
+// 10^4 with 10^4 1748 / 1743; complex, n = 3000 with 1200 pairs 50.4 / 46.8.  BN = 64 is left for the persistent queue, whose items
 // are 64 columns.
 template <int BN>
 struct GemmSmemT {
