@@ -1118,7 +1118,7 @@ cudaError_t launch_phases(void (*kernel)(Params, int, int), Params P, int phases
 // 1.1e-14 / 1.1e-14 (2.4e-14 / 2.1e-14), to 1e-16 4.6e-13 / 3e-4 (5.5e-13 /
 // 2e-3); those with d down to 2^-4 (n = 2100) and beyond are refused.  The
 // check reads A once: n = 700 13.35 -> 13.38 ms with the launches that do
-// nothing, n = 4000 138.1 -> 139.2, n = 6000 316.4 -> 317.7.  Refused, d to
+// nothing, n = 4000 138.3 -> 138.7, n = 6000 316.8 -> 318.7.  Refused, d to
 // 1e-12: n = 700 16.4 ms, n = 4000 324.
 constexpr int kHbEvenBits = 8;
 __device__ __forceinline__ bool hb_few(int low, int of) { return 5 * low <= 2 * of; }
@@ -1132,18 +1132,15 @@ __device__ __forceinline__ void even_count(int n, int r, int c0, int cols, const
     if (tid < kEvenCols) col[tid] = 0;
     __syncthreads();
     int mine = 0, ours = 0;                                      // of this row; lane c: of column c, these 32 rows
+    double x[kEvenCols];
 #pragma unroll
-    for (int c = 0; c < kEvenCols; c += 16) {
-        double x[16];
+    for (int c = 0; c < kEvenCols; ++c) x[c] = get(c0 + min(c, cols - 1));
 #pragma unroll
-        for (int q = 0; q < 16; ++q) x[q] = get(c0 + min(c + q, cols - 1));
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            const bool s = c + q < cols && small(x[q], c + q);
-            const unsigned b = __ballot_sync(0xffffffffu, s);
-            if (lane == c + q) ours = __popc(b);
-            mine += s;
-        }
+    for (int c = 0; c < kEvenCols; ++c) {
+        const bool s = c < cols && small(x[c], c);
+        const unsigned b = __ballot_sync(0xffffffffu, s);
+        if (lane == c) ours = __popc(b);
+        mine += s;
     }
     if (mine) atomicAdd(&low[r], mine);
     if (ours) atomicAdd(&col[lane], ours);
@@ -1270,7 +1267,7 @@ __global__ void __launch_bounds__(256, 2) k_hq_plain(HqPlain P, int first, int l
 constexpr int kHqNb = 128;
 // Smallest order: a reflector of the DFMA form costs about 5.5 us (three thin
 // products and a serial factor per 64), this form 240 us and 0.5 us each
-// (n = 32: 139 us as DFMA; 64: 360 against 257; 300: 1,665 against 411; 4000
+// (n = 32: 139 us as DFMA; 64: 360 against 249; 300: 1,665 against 411; 4000
 // with 2000 columns: 85.7 ms against 5.2).  The DFMA form also stays for
 // reflectors that are not even and for a scratch buffer that cannot be had.
 constexpr int kHqDigitsN = 40;
@@ -1288,7 +1285,7 @@ constexpr int kHqMaxSplit = 16;
 // D G D on columns D G', G and G' of N(0,1) entries, error row by row relative
 // to the row's largest, in FP64 / by digits: d down to 1e-8 (n = 45) 2.5e-15 /
 // 2.6e-9, to 1e-12 (n = 300) 3.3e-15 / 2.3e-7.  The check reads V once: n = 64
-// 238 -> 257 us, n = 700 625 -> 643, n = 5000 with 2500 columns 8.53 -> 8.60 ms.
+// 231 -> 249 us, n = 700 621 -> 641, n = 5000 with 2500 columns 8.57 -> 8.65 ms.
 // Refused, n = 700 with 350 columns 4.0 ms, n = 4000 with 2000 89.
 constexpr int kHqEvenBits = 5, kHqEvenMin = 32;
 // low: 2 n counts, zeroed, of the rows' and the columns' smaller entries; cnt: a
@@ -1515,7 +1512,8 @@ __global__ void __launch_bounds__(8 * kHqHalf) k_hq_tcross(HqGroup h, const doub
 struct HqDigits {
     unsigned char *XN, *VM, *VN, *VA, *TM, *WN;
     double *S, *T, *Wp, *W2;
-    int *exX, *exW, *exVA, *exV, *exT, *low;                     // low: k_hq_even's counts, a counter and the result
+    int *exX, *exW, *exVA, *exV, *exT, *low;                     // low: k_hq_even's counts, a counter, the result and
+                                                                 // k_hq_plain's barrier
     int nblk, cch, gmax;                                         // blocks of reflectors, columns at a time, blocks of a group
 };
 constexpr size_t kHqVBlock = (size_t)kHqNb * kHqNb * kDgDigits * 2, kHqSmall = (size_t)kHqNb * kDgDigits * 2;
@@ -1546,7 +1544,7 @@ size_t hq_digits_layout(int n, int ncols, unsigned char *base, HqDigits &D) {
     D.T = reinterpret_cast<double *>(take((size_t)D.gmax * kHqNb * kHqNb * 8));
     D.Wp = reinterpret_cast<double *>(take((size_t)kHqMaxSplit * kHqNb * D.cch * 8));
     D.W2 = reinterpret_cast<double *>(take((size_t)kHqNb * D.cch * 8));
-    D.exX = reinterpret_cast<int *>(take(((size_t)ncols + D.cch + vrb * kHqNb + (size_t)2 * D.gmax * kHqNb + 2 * n + 2) * sizeof(int)));
+    D.exX = reinterpret_cast<int *>(take(((size_t)ncols + D.cch + vrb * kHqNb + (size_t)2 * D.gmax * kHqNb + 2 * n + 3) * sizeof(int)));
     D.exW = D.exX + ncols;
     D.exVA = D.exW + D.cch;
     D.exV = D.exVA + vrb * kHqNb;
@@ -1563,7 +1561,7 @@ cudaError_t hq_digits(const HqDigits &D, int n, const double *dA, int lda, const
     unsigned char *const XN = D.XN, *VM = D.VM, *VN = D.VN, *VA = D.VA, *TM = D.TM, *WN = D.WN;
     double *S = D.S, *T = D.T, *Wp = D.Wp, *W2 = D.W2;
     int *exX = D.exX, *exW = D.exW, *exVA = D.exVA, *exV = D.exV, *exT = D.exT, *low = D.low, *gate = low + 2 * n + 1;
-    cudaError_t e = cudaMemsetAsync(low, 0, (size_t)(2 * n + 2) * sizeof(int), st);
+    cudaError_t e = cudaMemsetAsync(low, 0, (size_t)(2 * n + 3) * sizeof(int), st);
     if (e != cudaSuccess) return e;
     *uneven = gate;
     k_hq_even<<<dim3((n + 255) / 256, (n - 2 + kEvenCols - 1) / kEvenCols), 256, 0, st>>>(
@@ -1973,7 +1971,8 @@ extern "C" int hsr_hessenberg_apply_q_device(int n, const double *dA, int lda, c
     const int ct = (ncols + kHbTm - 1) / kHbTm, rt = (n + kHbTm - 1) / kHbTm;
     P.splitg = std::min(2 * sms, kHbMaxSplit);
     P.splitw = std::max(1, std::min((2 * sms + ct - 1) / ct, kHbMaxSplit));
-    if (cudaMemsetAsync(P.bar, 0, sizeof(double), st) != cudaSuccess ||
+    if (uneven) P.bar = reinterpret_cast<unsigned *>(D.low + 2 * n + 2);         // zeroed with the counts
+    if ((!uneven && cudaMemsetAsync(P.bar, 0, sizeof(double), st) != cudaSuccess) ||
         launch_phases(k_hq_plain, P, kHqPlainPhases * ((n - 3) / kHbNb + 1), std::min(sms, ct * std::max(rt, kHbMaxSplit)), st) !=
             cudaSuccess)
         return HSR_ERR_CUDA;
