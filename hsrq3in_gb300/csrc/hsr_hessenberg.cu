@@ -1112,14 +1112,17 @@ cudaError_t launch_phases(void (*kernel)(Params, int, int), Params P, int phases
 // but the first (no reflector touches it) and in every column, three fifths of
 // the entries lie within 2^8 of the largest of all.  Then every reflector mixes
 // entries of like size, and FP64 itself leaves errors of the size of the
-// largest entry's rounding everywhere.  |Q^T A Q - H| scaled by 1 / (d_i d_j)
-// for A = D G D, G of N(0,1) entries, relative to |G|, in FP64 / by digits, n =
-// 160 (2100): d from 1 to 2^-3 1.9e-15 / 1.6e-15 (5.3e-15 / 5.0e-15), to 2^-10
-// 1.1e-14 / 1.1e-14 (2.4e-14 / 2.1e-14), to 1e-16 4.6e-13 / 3e-4 (5.5e-13 /
-// 2e-3); those with d down to 2^-4 (n = 2100) and beyond are refused.  The
-// check reads A once: n = 700 13.35 -> 13.38 ms with the launches that do
-// nothing, n = 4000 138.3 -> 138.7, n = 6000 316.8 -> 318.7.  Refused, d to
-// 1e-12: n = 700 16.4 ms, n = 4000 324.
+// largest entry's rounding everywhere.  Measured, n = 160, Q^T A Q - H in extended
+// precision, by digits over FP64, median and largest ratio of the root mean
+// squares of its columns, against the bits a matrix needs: N(0,1) entries (4) 0.83,
+// 1.8; Z H Z^T, Z orthogonal (3) 0.87, 1.3; G G^T (5) 0.93, 1.7; G + 100 D (9) 0.98,
+// 2.5; a Hessenberg matrix between two reflectors (10) 0.96, 3.1; Cauchy entries
+// (16) 0.86, 5.3, cubed (49) 1.4, 38.  D G D scaled by 1 / (d_i d_j), relative to
+// G, FP64 / digits, n = 160 (4000): d from 1 to 2^-8 (14) 7.2e-15 / 6.8e-15
+// (2.3e-14 / 2.1e-14), to 2^-16 (27) 2.9e-14 / 7.5e-14 (7.3e-14 / 3.1e-13), to
+// 1e-16 4.6e-13 / 3e-4.  The check reads A once: n = 700 13.35 -> 13.38 ms with
+// the launches that do nothing, n = 4000 138.3 -> 138.7, n = 6000 316.8 -> 318.7.
+// Refused, d to 1e-12: n = 700 16.4 ms, n = 4000 324.
 constexpr int kHbEvenBits = 8;
 __device__ __forceinline__ bool hb_few(int low, int of) { return 5 * low <= 2 * of; }
 // Counts of the entries that small(x, c) holds of rows r = r0 + tid (in or not)
@@ -1279,15 +1282,18 @@ constexpr int kHqMaxSplit = 16;
 // its largest entry in rows 1 ..; that loses nothing where the reflectors carry
 // an entry of that size into every row, whose rounding in FP64 is then as large.
 // So in every column of V with kHqEvenMin entries below its 1, and in every row
-// with as many, three fifths of the entries have to be at least 2^-5 / sqrt(m),
+// with as many, three fifths of the entries have to be at least 2^-3 / sqrt(m),
 // m the length of the column (a reflector's norm is at most sqrt(2) and that of
 // a random one's entries about 1 / sqrt(m)), and tau not near 0.  Reflectors of
 // D G D on columns D G', G and G' of N(0,1) entries, error row by row relative
-// to the row's largest, in FP64 / by digits: d down to 1e-8 (n = 45) 2.5e-15 /
-// 2.6e-9, to 1e-12 (n = 300) 3.3e-15 / 2.3e-7.  The check reads V once: n = 64
+// to the row's largest, root mean square, in FP64 / by digits, n = 160 (500): d
+// from 1 to 2^-6 3.7e-16 / 3.0e-16 (4.0e-16 / 2.3e-16), to 2^-8, which is
+// refused, 3.5e-16 / 5.4e-16 (3.8e-16 / 2.9e-16), to 2^-16 3.3e-16 / 2.3e-14
+// (3.9e-16 / 1.3e-14); d to 1e-12 (n = 300), the largest, 3.3e-15 / 2.3e-7.
+// Random reflectors need 2^-2 at most.  The check reads V once: n = 64
 // 231 -> 249 us, n = 700 621 -> 641, n = 5000 with 2500 columns 8.57 -> 8.65 ms.
 // Refused, n = 700 with 350 columns 4.0 ms, n = 4000 with 2000 89.
-constexpr int kHqEvenBits = 5, kHqEvenMin = 32;
+constexpr int kHqEvenBits = 3, kHqEvenMin = 32;
 // low: 2 n counts, zeroed, of the rows' and the columns' smaller entries; cnt: a
 // counter, zeroed.
 __global__ void __launch_bounds__(256) k_hq_even(int n, const double *A, long long lda, const double *tau, int *low, unsigned *cnt,

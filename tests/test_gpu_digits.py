@@ -302,7 +302,8 @@ def _reduce_one_by_one(torch, A):
     return F, tau
 
 
-@pytest.mark.parametrize("n,pad,decades", [(33, 0, 10), (130, 1, 16), (160, 0, 30), (300, 0, 12), (2100, 0, 16)])
+@pytest.mark.parametrize("n,pad,decades", [(33, 0, 10), (130, 1, 16), (160, 0, 30), (300, 0, 12), (2100, 0, 16),
+                                           (160, 0, 2.4), (300, 1, 3.6), (2100, 0, 2.4)])   # near where FP64 takes over
 def test_reduction_keeps_graded_rows(gpu_lib, n, pad, decades):
     """A = D G D with D falling over many decades: the Householder reduction in
     FP64 keeps the small rows and columns, (Q^T A Q - H)_ij of the size of d_i
@@ -358,7 +359,8 @@ def test_reduction_of_any_form(gpu_lib, n, pad, form):
     assert float((At @ Q - Q @ torch.triu(F, -1)).norm()) <= n * EPS * np.linalg.norm(A)
 
 
-@pytest.mark.parametrize("n,ncols,pad,decades", [(45, 3, 0, 8), (130, 65, 1, 10), (200, 5, 0, 25), (300, 30, 0, 12)])
+@pytest.mark.parametrize("n,ncols,pad,decades", [(45, 3, 0, 8), (130, 65, 1, 10), (200, 5, 0, 25), (300, 30, 0, 12),
+                                                 (200, 30, 0, 1.8), (300, 5, 0, 2.4)])   # near where FP64 takes over
 def test_back_transform_keeps_graded_rows(gpu_lib, n, ncols, pad, decades):
     """Reflectors of a graded matrix on columns graded alike: FP64 keeps the
     small rows.  Row by row, relative to the row's largest entry, within ten
