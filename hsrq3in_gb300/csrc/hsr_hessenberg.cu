@@ -1121,41 +1121,54 @@ cudaError_t launch_phases(void (*kernel)(Params, int, int), Params P, int phases
 // G, FP64 / digits, n = 160 (4000): d from 1 to 2^-8 (14) 7.2e-15 / 6.8e-15
 // (2.3e-14 / 2.1e-14), to 2^-16 (27) 2.9e-14 / 7.5e-14 (7.3e-14 / 3.1e-13), to
 // 1e-16 4.6e-13 / 3e-4.  The check reads A once: n = 700 13.35 -> 13.38 ms with
-// the launches that do nothing, n = 4000 138.3 -> 138.7, n = 6000 316.8 -> 318.7.
+// the launches that do nothing, n = 4000 138.2 -> 139.3, n = 6000 317.0 -> 318.0.
 // Refused, d to 1e-12: n = 700 16.4 ms, n = 4000 324.
 constexpr int kHbEvenBits = 8;
 __device__ __forceinline__ bool hb_few(int low, int of) { return 5 * low <= 2 * of; }
-// Counts of the entries that small(x, c) holds of rows r = r0 + tid (in or not)
-// and columns c0 .. c0 + 31, into low[r] and low[n + c]; get(c): an entry.
-constexpr int kEvenCols = 32;
-template <class Get, class Small>
-__device__ __forceinline__ void even_count(int n, int r, int c0, int cols, const Get &get, const Small &small, int *low) {
-    __shared__ int col[kEvenCols];
-    const int tid = threadIdx.x, lane = tid & 31;
-    if (tid < kEvenCols) col[tid] = 0;
-    __syncthreads();
-    int mine = 0, ours = 0;                                      // of this row; lane c: of column c, these 32 rows
-    double x[kEvenCols];
+// Counts of entries by row, low[r], and by column, low[n + c]: a warp takes 32 x
+// 32 of them, a lane a row, its 32 loads in flight together, and its lane c ends
+// with column c's count; warps side by side take rows below one another.
+// get(r, c): an entry; limit(c): what the lane of column c contributes to
+// small(x, r, c, limit), which tells whether it counts.  Above the diagonal of
+// c = r + below there is nothing to count.  Bound by the latency of the loads,
+// with 16 warps an SM: V of n = 5000 (100 MB) 52 us; with the loads under the
+// conditions 120, with block-wide counts in shared memory 90 to 115.
+constexpr int kEvenTile = 32;
+template <class Get, class Limit, class Small>
+__device__ __forceinline__ void even_count(int n, int r0, int rows, int cols, int below, const Get &get, const Limit &limit,
+                                           const Small &small, int *low) {
+    const int lane = threadIdx.x & 31, nr = (rows + kEvenTile - 1) / kEvenTile, nc = (cols + kEvenTile - 1) / kEvenTile;
+    const int warps = gridDim.x * (blockDim.x >> 5);
+    for (int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < nr * nc; t += warps) {
+        const int c0 = t / nr * kEvenTile, ra = r0 + t % nr * kEvenTile, r = ra + lane;
+        if (c0 > ra + kEvenTile - 1 + below) continue;
+        double x[kEvenTile];
 #pragma unroll
-    for (int c = 0; c < kEvenCols; ++c) x[c] = get(c0 + min(c, cols - 1));
+        for (int c = 0; c < kEvenTile; ++c) x[c] = get(min(r, n - 1), min(c0 + c, cols - 1));   // unconditional loads
+        const int lim = c0 + lane < cols ? limit(c0 + lane) : 0;
+        int mine = 0, ours = 0;
 #pragma unroll
-    for (int c = 0; c < kEvenCols; ++c) {
-        const bool s = c < cols && small(x[c], c);
-        const unsigned b = __ballot_sync(0xffffffffu, s);
-        if (lane == c) ours = __popc(b);
-        mine += s;
+        for (int c = 0; c < kEvenTile; ++c) {
+            const int l = __shfl_sync(0xffffffffu, lim, c);      // by all lanes, also those past the last row
+            const bool s = r < n && c0 + c < cols && small(x[c], r, c0 + c, l);
+            const unsigned b = __ballot_sync(0xffffffffu, s);
+            if (lane == c) ours = __popc(b);
+            mine += s;
+        }
+        if (mine) atomicAdd(&low[r], mine);
+        if (ours) atomicAdd(&low[n + c0 + lane], ours);
     }
-    if (mine) atomicAdd(&low[r], mine);
-    if (ours) atomicAdd(&col[lane], ours);
-    __syncthreads();
-    if (tid < cols && col[tid]) atomicAdd(&low[n + c0 + tid], col[tid]);
 }
-// The CTA that counted last (of a 2-d grid) sees all counts.
+int even_grid(int rows, int cols, int sms) {                     // CTAs of 256 threads
+    const long long tiles = (long long)((rows + kEvenTile - 1) / kEvenTile) * ((cols + kEvenTile - 1) / kEvenTile);
+    return (int)std::min<long long>(2 * sms, (tiles + 7) / 8);
+}
+// The CTA that counted last sees all counts.
 __device__ __forceinline__ bool even_last(unsigned *cnt) {
     __shared__ bool am_last;
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) am_last = atomicAdd(cnt, 1u) == gridDim.x * gridDim.y - 1;
+    if (threadIdx.x == 0) am_last = atomicAdd(cnt, 1u) == gridDim.x - 1;
     __syncthreads();
     if (am_last) __threadfence();
     return am_last;
@@ -1165,17 +1178,17 @@ __device__ __forceinline__ bool even_last(unsigned *cnt) {
 __global__ void __launch_bounds__(256) k_hb_even(int n, const double *A, long long lda, const int *cex, int *low, unsigned *cnt,
                                                  int *uneven) {
     __shared__ int red[8];
-    const int tid = threadIdx.x, r = 1 + blockIdx.x * 256 + tid, c0 = blockIdx.y * kEvenCols, cols = min(kEvenCols, n - c0);
+    const int tid = threadIdx.x;
     int top = kDgZero;
     for (int c = tid; c < n; c += 256) top = dg_bad(cex[c]) ? top : max(top, cex[c]);
     top = __reduce_max_sync(0xffffffffu, top);
     if ((tid & 31) == 0) red[tid >> 5] = top;
     __syncthreads();
     for (int w = 0; w < 8; ++w) top = max(top, red[w]);
-    even_count(n, r, c0, cols, [&](int c) { return r < n ? A[r + (size_t)c * lda] : 0.0; },
-               [&](double x, int) {
+    even_count(n, 1, n - 1, n, n, [&](int r, int c) { return A[r + (size_t)c * lda]; }, [](int) { return 0; },
+               [&](double x, int, int, int) {
                    const int e = dg_exp(x);
-                   return r < n && (e < top - kHbEvenBits || dg_bad(e));
+                   return e < top - kHbEvenBits || dg_bad(e);
                }, low);
     if (!even_last(cnt)) return;
     bool bad = false;
@@ -1291,27 +1304,23 @@ constexpr int kHqMaxSplit = 16;
 // refused, 3.5e-16 / 5.4e-16 (3.8e-16 / 2.9e-16), to 2^-16 3.3e-16 / 2.3e-14
 // (3.9e-16 / 1.3e-14); d to 1e-12 (n = 300), the largest, 3.3e-15 / 2.3e-7.
 // Random reflectors need 2^-2 at most.  The check reads V once: n = 64
-// 231 -> 249 us, n = 700 621 -> 641, n = 5000 with 2500 columns 8.57 -> 8.65 ms.
+// 236 -> 250 us, n = 700 625 -> 640, n = 5000 with 2500 columns 8.54 -> 8.63 ms.
 // Refused, n = 700 with 350 columns 4.0 ms, n = 4000 with 2000 89.
 constexpr int kHqEvenBits = 3, kHqEvenMin = 32;
 // low: 2 n counts, zeroed, of the rows' and the columns' smaller entries; cnt: a
 // counter, zeroed.
 __global__ void __launch_bounds__(256) k_hq_even(int n, const double *A, long long lda, const double *tau, int *low, unsigned *cnt,
                                                  int *uneven) {
-    __shared__ int least[kEvenCols];                             // smallest exponent of a column that counts
-    const int tid = threadIdx.x, r = blockIdx.x * 256 + tid, c0 = blockIdx.y * kEvenCols, cols = min(kEvenCols, n - 2 - c0);
-    if ((int)(blockIdx.x + 1) * 256 > c0 + 2) {                  // some row is below some column's 1
-        if (tid < kEvenCols) {
-            const int m = max(n - 1 - (c0 + tid), 1);
-            const unsigned long long t = tid < cols ? ubits(tau[c0 + tid]) : 0;      // mixing: 0.5 <= tau, no NaN
-            least[tid] = t < pow2_bits(-1) || t >= kInfBits ? INT_MAX : 1022 - kHqEvenBits - ((32 - __clz(m)) >> 1);
-        }
-        even_count(n, r, c0, cols, [&](int c) { return r < n && r >= c + 2 ? A[r + (size_t)c * lda] : 0.0; },
-                   [&](double x, int c) {
-                       const int e = dg_exp(x);
-                       return r < n && r >= c0 + c + 2 && (e < least[c] || dg_bad(e));
-                   }, low);
-    }
+    const int tid = threadIdx.x;
+    even_count(n, 2, n - 2, n - 2, -2, [&](int r, int c) { return A[r + (size_t)c * lda]; },
+               [&](int c) {                                      // smallest exponent of column c that counts
+                   const unsigned long long t = ubits(tau[c]);   // mixing: 0.5 <= tau, no NaN
+                   return t < pow2_bits(-1) || t >= kInfBits ? INT_MAX : 1022 - kHqEvenBits - ((32 - __clz(n - 1 - c)) >> 1);
+               },
+               [&](double x, int r, int c, int least) {
+                   const int e = dg_exp(x);
+                   return r >= c + 2 && (e < least || dg_bad(e));
+               }, low);
     if (!even_last(cnt)) return;
     bool bad = false;
     for (int q = tid; q < n; q += 256) {
@@ -1570,7 +1579,7 @@ cudaError_t hq_digits(const HqDigits &D, int n, const double *dA, int lda, const
     cudaError_t e = cudaMemsetAsync(low, 0, (size_t)(2 * n + 3) * sizeof(int), st);
     if (e != cudaSuccess) return e;
     *uneven = gate;
-    k_hq_even<<<dim3((n + 255) / 256, (n - 2 + kEvenCols - 1) / kEvenCols), 256, 0, st>>>(
+    k_hq_even<<<even_grid(n, n - 2, sms), 256, 0, st>>>(
         n, dA, lda, dtau, low, reinterpret_cast<unsigned *>(low + 2 * n), gate);
     // Over the rows that reflectors touch: row 0 stays what it is.
     k_dg_exp_k<<<ncols, 256, 0, st>>>(HqCols{dX + 1, ldx, ncols, n - 1}, n - 1, nullptr, 0, exX);
@@ -1886,7 +1895,7 @@ extern "C" int hsr_hessenberg_device(int n, double *dA, int lda, double *dtau, v
         // Exponents of A's columns over the rows that reflectors touch.
         k_dg_exp_k<<<n, 256, 0, st>>>(HqCols{dA + 1, lda, n, n - 1}, n - 1, nullptr, 0, D.cex);
         if (cudaMemsetAsync(D.low, 0, (size_t)(2 * n + 2) * sizeof(int), st) != cudaSuccess) return HSR_ERR_CUDA;
-        k_hb_even<<<dim3((n + 254) / 256, (n + kEvenCols - 1) / kEvenCols), 256, 0, st>>>(
+        k_hb_even<<<even_grid(n - 1, n, sms), 256, 0, st>>>(
             n, dA, lda, D.cex, D.low, reinterpret_cast<unsigned *>(D.low + 2 * n), D.uneven);
     }
     for (int k0 = 0; k0 < n - 2; k0 += kHbNb) {
