@@ -108,8 +108,11 @@ def test_forced_shifts_per_cta(gpu_lib, monkeypatch, n, tlsz, nrhs):
             with profile(activities=[ProfilerActivity.CUDA]) as prof:
                 dev = hsr.inverse_iteration(H, wr, tlsz, 16)
                 torch.cuda.synchronize()
-            diag = [e.key for e in prof.key_averages() if "k_diag" in e.key]
+            names = [e.key for e in prof.key_averages()]
+            diag = [k for k in names if "k_diag" in k]
             if diag:
                 break
+        if not any("k_" in k for k in names):
+            pytest.skip("no kernel trace on this machine")
         assert diag and all(("k_diag_n" in k and "<%d, " % sc in k) if sc < 32 else "k_diag_n" not in k for k in diag), (sc, diag)
         assert np.array_equal(dev["vr"], orc["vr"])
